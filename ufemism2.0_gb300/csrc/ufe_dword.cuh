@@ -127,6 +127,10 @@ __device__ __forceinline__ dw2 v_pupd(dw2 r, dw bw, dw2 v, dw beta, dw2 p) {
 __device__ __forceinline__ dw2 v_sub_scaled(dw2 r, dw a, dw2 v) {
   return make_dw2(dw_add(dw_u(r), dw_neg(dw_mul(a, dw_u(v)))), dw_add(dw_v(r), dw_neg(dw_mul(a, dw_v(v)))));
 }
+// x + a*p: v_xupd in two steps
+__device__ __forceinline__ dw2 v_axpy(dw2 x, dw a, dw2 p) {
+  return make_dw2(dw_add(dw_u(x), dw_mul(a, dw_u(p))), dw_add(dw_v(x), dw_mul(a, dw_v(p))));
+}
 // x + a*p + w*s
 __device__ __forceinline__ dw2 v_xupd(dw2 x, dw a, dw2 p, dw w, dw2 s) {
   return make_dw2(dw_add(dw_add(dw_u(x), dw_mul(a, dw_u(p))), dw_mul(w, dw_u(s))),

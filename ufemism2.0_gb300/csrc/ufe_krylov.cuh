@@ -14,6 +14,8 @@
 // rows with a grid stride so the grid never exceeds the partial-sum capacity.
 #pragma once
 
+#include <math_constants.h>
+
 #include <type_traits>
 
 #include "ufe_dword.cuh"
@@ -37,6 +39,7 @@ template <class V> __device__ __forceinline__ V v_zero();
 template <> __device__ __forceinline__ double2 v_zero<double2>() { return make_double2(0.0, 0.0); }
 template <> __device__ __forceinline__ float2 v_zero<float2>() { return make_float2(0.f, 0.f); }
 template <> __device__ __forceinline__ double v_zero<double>() { return 0.0; }
+template <> __device__ __forceinline__ dw2 v_zero<dw2>() { return dw2{make_float4(0.f, 0.f, 0.f, 0.f)}; }
 // p_new = r - (beta*omega)*v + beta*p   (PETSc VecAXPBYPCZ(P, 1, -beta*omega, beta, R, V))
 __device__ __forceinline__ double2 v_pupd(double2 r, double bw, double2 v, double beta, double2 p) {
   return make_double2(fma(beta, p.x, fma(-bw, v.x, r.x)), fma(beta, p.y, fma(-bw, v.y, r.y)));
@@ -55,6 +58,10 @@ __device__ __forceinline__ float2 v_sub_scaled(float2 r, float a, float2 v) {
   return make_float2(fmaf(-a, v.x, r.x), fmaf(-a, v.y, r.y));
 }
 __device__ __forceinline__ double v_sub_scaled(double r, double a, double v) { return fma(-a, v, r); }
+// x + a*p: v_xupd in two steps
+__device__ __forceinline__ double2 v_axpy(double2 x, double a, double2 p) {
+  return make_double2(fma(a, p.x, x.x), fma(a, p.y, x.y));
+}
 // x + a*p + w*s
 __device__ __forceinline__ double2 v_xupd(double2 x, double a, double2 p, double w, double2 s) {
   return make_double2(fma(w, s.x, fma(a, p.x, x.x)), fma(w, s.y, fma(a, p.y, x.y)));
@@ -521,7 +528,7 @@ constexpr int kPersistSlots = 5;     // partial sums per block per phase
 struct __align__(128) GridSync {
   unsigned int count;
   unsigned int pad0[31];
-  unsigned int gen;     // unused by the barrier; kept zero
+  unsigned int gen;     // last stamp of the stamped exchanges (below); runs on across launches
   int err;
   unsigned int pad1[30];
 };
@@ -750,6 +757,7 @@ struct HaloMat {
   const float4 *__restrict__ rowsum;    // FP32 difference form: FP64 row sums rounded to FP32
   const int32_t *__restrict__ halo_off; // gridDim.x + 1
   const int32_t *__restrict__ halo_idx; // global rows of each block's halo
+  const uint8_t *__restrict__ halo_pub; // rows that are in some block's halo
 };
 using HaloDiffMat = HaloMat<float4>;
 
@@ -870,13 +878,6 @@ struct DotAcc {
   double v = 0.0;
   __device__ __forceinline__ void add(Vec a, Vec b) { v += v_dot(a, b); }
   __device__ __forceinline__ Part part() const { return v; }
-  static __device__ __forceinline__ Part zero() { return 0.0; }
-  static __device__ __forceinline__ Part warp_sum(Part x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-  }
-  static __device__ __forceinline__ double finish(Part x) { return x; }
 };
 template <>
 struct DotAcc<dw2> {
@@ -891,102 +892,388 @@ struct DotAcc<dw2> {
     return make_float2(t.hi, t.lo);
   }
   static __device__ __forceinline__ Part zero() { return make_float2(0.f, 0.f); }
-  static __device__ __forceinline__ Part warp_sum(Part x) {
-    dw t(x.x, x.y);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      t = dw_add(t, dw(__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o)));
-    return make_float2(t.hi, t.lo);
-  }
-  static __device__ __forceinline__ double finish(Part x) { return dw(x.x, x.y).to_double(); }
 };
 
-// Scratch of the FP64 block sums (one instance per kernel that uses it).
-__device__ __forceinline__ double *fp64_reduce_scratch() {
-  __shared__ double buf[kPersistSlots * kPersistThreads];
-  return buf;
+// ---- grid-wide sums of the persistent kernels ---------------------------------------------------
+// A phase ends with the sum of one or five values over all blocks.  Every block puts its partial sums into
+// its own slots, stamped with the number of this exchange, and every block reads all blocks' slots until
+// each carries the stamp: the partials' arrival is the barrier, so no counter is incremented and nothing
+// is loaded after the wait (a counter barrier followed by loads took two more L2 round trips).  The slots
+// exist kReplicas times, each read by its share of the blocks: 152 SMs polling one copy delay its
+// writers (wait of the p-phase on 115k triangles, mean over blocks: 6,200 cycles with two copies, 4,600 with
+// eight, 4,200 with sixteen).  All cross-block data is made of 64-bit words of 32 data bits and the 32-bit
+// stamp, so a torn read is seen and needs no fence.  Stamps run on from GridSync::gen across launches;
+// words are written again only after every block has passed the next exchange, that is, after all have
+// read them.  Every wait is bounded: a thread that polls too long, or sees that another gave up, sets
+// `err` and every block leaves its loop.
+//
+// GB300 issues an FP64 instruction of a warp in 64 cycles per quarter SM whatever its active mask
+// (measured: 0.50 lanes/clk per quarter, 65-cycle latency, 565 per division, ~615 per square root), and an
+// instruction line that is not in the SM's instruction cache costs hundreds.  So the sums keep FP64
+// instructions few and spread over the quarters' warps, run one piece of code in all of them (separate
+// code per warp made the s-phase's sums 5x slower), skip the tree levels that would only add zeros, and
+// compare on bit patterns; loops off the critical path stay rolled.  Every sum keeps one fixed order:
+// threads as a binary tree (t + 512, 256, ... 32, then xor 16 ... 1), blocks b, b + 32, ... per lane,
+// then xor 16 ... 1.
+struct __align__(16) ExSlot {   // one FP64 value
+  unsigned long long lo, hi;
+};
+struct __align__(32) ExRow {    // one 16-byte vector entry
+  unsigned long long w[4];
+};
+constexpr unsigned int kExchangePolls = 1u << 22;
+constexpr int kHaloMaxBlocks = 160;
+constexpr int kReplicas = 8;
+constexpr size_t kExSlots = 2 * (size_t)kReplicas * kPersistSlots * kHaloMaxBlocks;   // p-phase, s-phase
+
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void st_words(void *p, unsigned long long a, unsigned long long b) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void ld_words(const void *p, unsigned long long &a, unsigned long long &b) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ unsigned long long word(unsigned int data, unsigned int stamp) {
+  return (unsigned long long)data | ((unsigned long long)stamp << 32);
+}
+__device__ __forceinline__ bool stamped(unsigned long long w, unsigned int stamp) { return (unsigned int)(w >> 32) == stamp; }
+
+__device__ __forceinline__ void slot_publish(ExSlot *p, double x, unsigned int stamp) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  st_words(p, word((unsigned int)u, stamp), word((unsigned int)(u >> 32), stamp));
+}
+// true when the poll loop has to give up
+__device__ __forceinline__ bool poll_expired(unsigned int &polls, GridSync *gs) {
+  if (++polls >= kExchangePolls || ((polls & 255u) == 0u && *((volatile int *)&gs->err))) {
+    atomicExch(&gs->err, 1);
+    return true;
+  }
+  return false;
+}
+// the slots of one exchange: value k of block b in replica c
+__device__ __forceinline__ int slot_index(int k, int b, int c) {
+  return (c * kPersistSlots + k) * kHaloMaxBlocks + b;
+}
+// Waits for this exchange's words, two 16-byte items per thread at a time (one after the other, the second's
+// round trip follows the first's): all blocks' np partials to sp[k * kHaloMaxBlocks + block] (shared memory),
+// and the entries of the nhalo rows hg[] of `rows` to halo[].  False after a timeout.
+__device__ __forceinline__ bool exchange_wait(int np, const ExSlot *slots, double *sp, const ExRow *rows,
+                                              const int *hg, int nhalo, double *halo, unsigned int stamp,
+                                              GridSync *gs) {
+  const int ns = np * kHaloMaxBlocks, n = ns + 2 * nhalo, G = (int)gridDim.x;
+  slots += slot_index(0, 0, (int)blockIdx.x % kReplicas);
+  bool ok = true;
+  // item t: slot t = k * kHaloMaxBlocks + block, then halo row (t - ns) / 2's halves; null: nothing to wait for
+  auto item = [&](int t) -> const void * {
+    if (t < ns) return t % kHaloMaxBlocks < G ? (const void *)(slots + t) : nullptr;
+    return t < n ? (const void *)(rows[hg[(t - ns) >> 1]].w + 2 * ((t - ns) & 1)) : nullptr;
+  };
+  auto put = [&](int t, unsigned long long a, unsigned long long b) {
+    (t < ns ? sp : halo - ns)[t] = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+  };
+#pragma unroll 1
+  for (int t = threadIdx.x; t < n; t += 2 * (int)blockDim.x) {
+    const int t2 = t + (int)blockDim.x;
+    const void *p0 = item(t), *p1 = item(t2);
+    unsigned long long a = 0, b = 0, c = 0, d = 0;
+    unsigned int polls = 0;
+    for (;;) {
+      if (p0) ld_words(p0, a, b);
+      if (p1) ld_words(p1, c, d);
+      if ((!p0 || (stamped(a, stamp) && stamped(b, stamp))) && (!p1 || (stamped(c, stamp) && stamped(d, stamp)))) break;
+      if (poll_expired(polls, gs)) {
+        ok = false;
+        break;
+      }
+    }
+    put(t, a, b);
+    if (t2 < n) put(t2, c, d);
+  }
+  return ok;
+}
+// the lane's part of the sum of value k over the blocks: blocks lane, lane + 32, ... in this order.  The trip
+// count is the same in all lanes: shuffles after a loop that lanes leave one by one took ~450 cycles each.
+__device__ __forceinline__ double lane_blocks(const double *sp, int k, int lane) {
+  const double *q = sp + k * kHaloMaxBlocks;
+  double v = q[lane];
+#pragma unroll 1
+  for (int b = 32; b < (int)gridDim.x; b += 32) v = lane + b < (int)gridDim.x ? v + q[lane + b] : v;
+  return v;
+}
+// the warp's index in a register the compiler knows to be uniform: branches on it are, too
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// A vector entry for the blocks that have its row in their halo.
+template <class Vec>
+__device__ __forceinline__ void row_publish(ExRow *p, Vec x, unsigned int stamp) {
+  static_assert(sizeof(Vec) == 16, "16-byte vector entries");
+  uint4 q;
+  memcpy(&q, &x, 16);
+  st_words(p->w, word(q.x, stamp), word(q.y, stamp));
+  st_words(p->w + 2, word(q.z, stamp), word(q.w, stamp));
+}
+// FP64 butterfly sums of a (in lanes below 16) and b (in the others); not inlined, to be fetched once
+__device__ __forceinline__ double warp_fold_sum(double a, double b) {
+  const bool up = threadIdx.x & 16;
+  double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double fp64_div(double a, double b) { return a / b; }
+// Double-word sums.  Two butterflies' step in one addition: lanes with `bit` clear go on with a, the others
+// with b (fold(a, a, bit) is a butterfly step).  Not inlined: a double-word addition is 20 instructions.
+__device__ __forceinline__ dw dw_fold(dw a, dw b, int bit) {
+  const bool up = threadIdx.x & bit;
+  const dw keep(up ? b.hi : a.hi, up ? b.lo : a.lo), send(up ? a.hi : b.hi, up ? a.lo : b.lo);
+  return dw_add(keep, dw(__shfl_xor_sync(0xffffffffu, send.hi, bit), __shfl_xor_sync(0xffffffffu, send.lo, bit)));
+}
+__device__ __forceinline__ dw dw_warp_sum(dw a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a = dw_fold(a, a, o);
+  return a;
 }
 
-// block sum of NP accumulators (fixed tree), written by thread 0 to part[blockIdx.x * NP + k].
-// FP64 sums run as a shared-memory tree down to one warp: a butterfly of shuffles would issue
-// 5 FP64 adds per warp per value, and FP64 issue is scarce on GB300.  Double-word sums stay in
-// shuffles (FP32 pipe).
-template <int NP, class Acc>
-__device__ __forceinline__ void block_partials_acc(const Acc (&acc)[NP], double *part) {
+// Sum the first np (1 or 5) accumulators over the block's first nact threads (the others hold zero) and publish
+// them.  scratch: np * min(nact, blockDim) doubles (FP64 parts) or np * 32 float2 (double-word parts).
+// kFence: the block's other writes are read after the exchange and have to be visible before the sums are.
+template <bool kFence, class Acc>
+__device__ __forceinline__ void block_publish(int np, const Acc (&acc)[kPersistSlots], int nact, void *scratch,
+                                              ExSlot *slots, unsigned int stamp) {
   using P = typename Acc::Part;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   if constexpr (std::is_same<P, double>::value) {
-    double *t = fp64_reduce_scratch();
-    const int n = blockDim.x;   // a power of two
+    double *t = static_cast<double *>(scratch);
+    if (tid < nact) {
+      t[tid] = acc[0].part();
+      if (np == 5)
 #pragma unroll
-    for (int k = 0; k < NP; ++k) t[k * n + threadIdx.x] = acc[k].part();
+        for (int k = 1; k < 5; ++k) t[k * nact + tid] = acc[k].part();
+    }
     __syncthreads();
-    for (int st = n >> 1; st >= 32; st >>= 1) {
-      if ((int)threadIdx.x < st)
-#pragma unroll
-        for (int k = 0; k < NP; ++k) t[k * n + threadIdx.x] += t[k * n + threadIdx.x + st];
+#pragma unroll 1
+    for (int st = 512; st >= 256; st >>= 1) {
+      if (st >= nact) continue;
+      if (tid < st && tid + st < nact)
+#pragma unroll 1
+        for (int k = 0; k < np; ++k) t[k * nact + tid] += t[k * nact + tid + st];
       __syncthreads();
     }
-    if (warp == 0) {
-#pragma unroll
-      for (int k = 0; k < NP; ++k) {
-        const double v = Acc::warp_sum(t[k * n + lane]);
-        if (lane == 0) part[(int64_t)blockIdx.x * NP + k] = v;
+    // value k in warp k, so that each quarter of the SM has one; a fifth value folds into warp 0's butterfly
+    if (warp < min(np, 4)) {
+      const int n = min(nact, 256), nseg = (n + 31) >> 5;
+      double v0 = 0.0, v = 0.0;
+#pragma unroll 1
+      for (int k = warp; k < np; k += 4) {
+        v0 = v;
+        const double *q = t + k * nact + lane;
+        auto seg = [&](int j) { return lane + 32 * j < n ? q[32 * j] : 0.0; };
+        double a = seg(0), b = nseg > 2 ? seg(2) : 0.0, c = nseg > 1 ? seg(1) : 0.0, d = nseg > 3 ? seg(3) : 0.0;
+        if (nseg > 4) a += seg(4);
+        if (nseg > 6) b += seg(6);
+        if (nseg > 5) c += seg(5);
+        if (nseg > 7) d += seg(7);
+        if (nseg > 2) a += b;
+        if (nseg > 3) c += d;
+        v = nseg > 1 ? a + c : a;
       }
+      const bool two = np == 5 && warp == 0;   // v0 is value 0 and v value 4
+      v = warp_fold_sum(two ? v0 : v, v);
+      // every lane holds the sum: lane c writes replica c (of value 4: lane 16 + c)
+      if (kFence) fence_acq_rel_gpu();
+      if (lane < kReplicas || (two && lane >= 16 && lane < 16 + kReplicas))
+        slot_publish(slots + slot_index(warp + ((lane >> 4) << 2), blockIdx.x, lane & 15), v, stamp);
     }
   } else {
-    __shared__ P red[NP][32];
+    float2 *red = static_cast<float2 *>(scratch);
+    const int nw = (nact + 31) >> 5;
+    if (warp < nw) {
+      dw x[5];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      const P v = Acc::warp_sum(acc[k].part());
-      if (lane == 0) red[k][warp] = v;
+      for (int k = 0; k < 5; ++k) {
+        const float2 q = acc[k].part();
+        x[k] = dw(q.x, q.y);
+      }
+      if (np == 1) {
+        const dw v = dw_warp_sum(x[0]);
+        if (lane == 0) red[warp] = make_float2(v.hi, v.lo);
+      } else {
+        // 8 double-word additions instead of 25: value 0 ends in lane 0, 1 in 16, 2 in 8, 3 in 24, 4 in 4
+        const dw ab = dw_fold(x[0], x[1], 16), cd = dw_fold(x[2], x[3], 16), e = dw_fold(x[4], x[4], 16);
+        const dw abcd = dw_fold(ab, cd, 8), e8 = dw_fold(e, e, 8);
+        dw v = dw_fold(abcd, e8, 4);
+        v = dw_fold(v, v, 2);
+        v = dw_fold(v, v, 1);
+        if ((lane & 7) == 0) red[((lane >> 4) + ((lane >> 3) & 1) * 2) * 32 + warp] = make_float2(v.hi, v.lo);
+        if (lane == 4) red[4 * 32 + warp] = make_float2(v.hi, v.lo);
+      }
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-#pragma unroll
-      for (int k = 0; k < NP; ++k) {
-        const P v = Acc::warp_sum(lane < nw ? red[k][lane] : Acc::zero());
-        if (lane == 0) part[(int64_t)blockIdx.x * NP + k] = Acc::finish(v);
-      }
+    if (warp < np) {
+      const float2 q = lane < nw ? red[warp * 32 + lane] : make_float2(0.f, 0.f);
+      const dw v = dw_warp_sum(dw(q.x, q.y));
+      if (kFence) fence_acq_rel_gpu();
+      if (lane < kReplicas) slot_publish(slots + slot_index(warp, blockIdx.x, lane), v.to_double(), stamp);
     }
   }
 }
 
-// After a phase's barrier: the block loads all blocks' partials at once (one L2 round trip,
-// one value per thread; the grid holds at most kHaloMaxBlocks blocks), warp k sums value k in
-// block order, and thread 0 runs update(tot) on the block's shared scalars.  Every thread sees
-// the result after the closing barrier.
-constexpr int kHaloMaxBlocks = kPersistThreads / kPersistSlots;
-__device__ __forceinline__ double *phase_scratch() {
-  __shared__ double buf[kPersistThreads + kPersistSlots];
-  return buf;
+// ---- the scalar recurrence, after an exchange -------------------------------------------------------
+__device__ __forceinline__ bool bits_nan(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
 }
-template <int NP, class F>
-__device__ __forceinline__ void phase_update(const double *part, F &&update) {
-  double *sp = phase_scratch();
-  double *tot = sp + kPersistThreads;
-  const int n = (int)gridDim.x * NP;
-  if ((int)threadIdx.x < n) sp[threadIdx.x] = __ldcg(part + threadIdx.x);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < NP) {
-    double v = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) v += sp[b * NP + warp];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) tot[warp] = v;
+__device__ __forceinline__ bool bits_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull; }
+// a <= b for values that are not negative and not NaN (their bit patterns order as they do)
+__device__ __forceinline__ bool bits_le(double a, double b) {
+  return (unsigned long long)__double_as_longlong(a) <= (unsigned long long)__double_as_longlong(b);
+}
+
+// coefficients in the solve's arithmetic: [0] beta, [1] beta * omega_old, [2] alpha, [3] omega
+template <class R>
+struct __align__(16) PhaseScalars {
+  KrylovScalars s;
+  int finish;         // 1 when the last iteration's x/r update is still to be applied
+  double res2;        // |r|^2 of the last iteration, >= 0
+  double lo2, hi2;    // lo2 < |r|^2 < hi2: |r| is certainly above ttol and below the divergence limit
+  double tot[kPersistSlots];
+  __align__(8) unsigned char rs_raw[4 * sizeof(R)];
+  __device__ __forceinline__ R *rs() { return reinterpret_cast<R *>(rs_raw); }
+  // thread 0, at the start
+  __device__ __forceinline__ void open(const KrylovScalars *ks) {
+    s = *ks;
+    rs()[0] = (R)s.beta;
+    rs()[1] = (R)(s.beta * s.omegaold);
+    finish = 0;
+    res2 = s.dp * s.dp;
+    // squares that a relative margin of 1e-12 keeps clear of the roundings of the square and of the root;
+    // where a square leaves the normal range every iteration takes the root (lo2 = inf or hi2 = 0)
+    const double a = s.ttol * s.ttol * (1.0 + 1e-12), d = 1e4 * s.rnorm0, b = d * d * (1.0 - 1e-12);
+    lo2 = (s.ttol == 0.0 || (a > 1e-290 && a < 1e300)) ? a : CUDART_INF;
+    hi2 = (b > 1e-290 && b < 1e300) ? b : 0.0;
+  }
+};
+
+// The stopping tests of an iteration whose squared residual norm does not decide them, or that ends the solve.
+template <class R>
+static __device__ __noinline__ void stop_tests(PhaseScalars<R> &ph, double res2, double rho_new, bool zero) {
+  KrylovScalars &s = ph.s;
+  const double dp = sqrt(res2);
+  s.dp = dp;
+  if (zero) { s.tbreak = 1; s.active = 0; s.status = UFE_OK; s.dp = 0.0; }
+  else if (bits_nan(dp)) { s.status = UFE_ERR_NAN; s.active = 0; }
+  else if (bits_le(dp, s.ttol)) { s.active = 0; }
+  else if (bits_le(1e4 * s.rnorm0, dp)) { s.status = UFE_ERR_DIVERGED; s.active = 0; }
+  else if (s.it >= s.max_it) { s.status = UFE_WARN_KRYLOV_MAXIT; s.active = 0; }
+  else if (bits_zero(rho_new)) { s.status = UFE_ERR_DIVERGED; s.active = 0; }
+}
+template <class R>
+static __device__ __noinline__ void stop_failed(PhaseScalars<R> &ph, int status) {
+  ph.s.status = status;
+  ph.s.active = 0;
+  if (ph.s.it > 0) ph.s.dp = sqrt(ph.res2);
+}
+
+// The scalars after an exchange; every thread of the block calls it, and sees the result after it.
+// P-phase: alpha from (v, r^).  S-phase: omega, rho, beta and the stopping tests from (s,t), (t,t), (s,s), (s,r^),
+// (t,r^).  Four warps, one on each quarter of the SM, sum the values, the two of rho in one butterfly.  Warps 0
+// and 1 form omega; warp 0 goes on to the next iteration's coefficients (both divisions of beta in one
+// instruction, in two lanes) while warp 1 does the stopping tests, on the squared residual norm where that
+// decides them: the root (~615 cycles) is taken only near a limit and in the iteration that stops.
+template <class R>
+__device__ __forceinline__ void after_exchange(PhaseScalars<R> &ph, const double *sp, bool s_phase) {
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  if (warp < (s_phase ? 4 : 1)) {   // one piece of code for all: instruction fetches are a cost here
+    // warp 0 (s,t) or (v,r^), 1 (t,t), 2 (s,r^) and (t,r^), 3 (s,s)
+    const int k = warp < 2 ? warp : 5 - warp;
+    double a = 0.0, b = 0.0;
+#pragma unroll 1
+    for (int q = k;; q = 4) {
+      a = b;
+      b = lane_blocks(sp, q, lane);
+      if (warp != 2 || q == 4) break;
+    }
+    const double v = warp_fold_sum(warp == 2 ? a : b, b);
+    if (lane == 0) ph.tot[k] = v;
+    if (warp == 2 && lane == 16) ph.tot[4] = v;
+    if (warp >= 2) asm volatile("bar.arrive 2, 128;" ::: "memory");
+  }
+  if (warp < (s_phase ? 2 : 1)) {
+    if (s_phase) asm volatile("bar.sync 1, 64;" ::: "memory");
+    else __syncwarp();
+    // P: alpha = rho / (v,r^);  S: omega = (s,t) / (t,t)
+    const double st = ph.tot[0], den = ph.tot[s_phase ? 1 : 0];
+    const bool zero = bits_zero(den), nan = bits_nan(den);
+    const double w = (s_phase && zero) ? 0.0 : fp64_div(s_phase ? st : ph.s.rho, den);
+    if (!s_phase) {
+      const R a = (R)w;
+      if (lane == 0) {
+        ph.finish = 0;   // the staging applied the previous iteration's x/r update
+        if (nan || zero) {
+          stop_failed(ph, nan ? UFE_ERR_NAN : UFE_ERR_DIVERGED);
+        } else {
+          ph.s.alpha = w;
+          ph.rs()[2] = a;
+        }
+      }
+    } else {
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      const double ss = ph.tot[2], rho_new = ph.tot[3] - w * ph.tot[4];
+      const bool fail = (zero && !bits_zero(ss)) || nan;
+      if (warp == 0) {
+        const double rho_old = ph.s.rho;
+        const double q = fp64_div(lane == 0 ? rho_new : ph.s.alpha, lane == 0 ? rho_old : w);
+        const double beta = __shfl_sync(0xffffffffu, q, 0) * __shfl_sync(0xffffffffu, q, 1);
+        const double bw = beta * w;
+        const R c = (R)(lane == 0 ? beta : lane == 1 ? bw : w);
+        if (!fail) {
+          if (lane < 3) ph.rs()[lane == 2 ? 3 : lane] = c;
+          if (lane == 0) {
+            ph.s.omega = w;
+            ph.s.rhoold = rho_old;
+            ph.s.omegaold = w;
+            ph.s.rho = rho_new;
+            ph.s.beta = beta;
+          }
+        }
+      } else {
+        const double res2 = fmax(ss - w * (2.0 * st - w * den), 0.0);
+        if (lane == 0) {
+          if (fail) {
+            stop_failed(ph, zero ? UFE_ERR_DIVERGED : UFE_ERR_NAN);
+          } else {
+            ph.finish = 1;   // this iteration's x/r update is due from here on
+            ph.res2 = res2;
+            const int it = ph.s.it + 1;
+            ph.s.it = it;
+            ph.s.total_its += 1;
+            if (zero || it >= ph.s.max_it || bits_zero(rho_new) || bits_le(res2, ph.lo2) || bits_le(ph.hi2, res2))
+              stop_tests(ph, res2, rho_new, zero);
+          }
+        }
+      }
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) update(tot);
-  __syncthreads();
+}
+
+// block 0, at the end: the result and the next launch's first stamp (every block read this launch's
+// before its first exchange; after a timeout another block may be one exchange further)
+__device__ __forceinline__ void persist_close(KrylovScalars &s, bool ok, KrylovScalars *ks, GridSync *gs,
+                                              unsigned int stamp) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    if (!ok) {
+      s.status = UFE_ERR_DEVICE;
+      s.active = 0;
+    }
+    *ks = s;
+    gs->gen = stamp + 4u;
+  }
 }
 
 // The whole BiCGStab solve in one launch (one 1024-thread block per SM): each block owns the
 // contiguous rows [blockIdx.x * rpb, ...) and stages its patch (own rows, then halo rows) in
-// shared memory for the two SpMVs.  The scalar recurrence (divisions, square root, stopping
-// tests) runs once per block, in thread 0, on the block's shared copy of the scalars; the other
-// threads read the coefficients of the next phase from shared memory, already in the solve's
-// arithmetic (FP64, FP32 or double-word).
+// shared memory for the two SpMVs.  The scalar recurrence runs once per block, on the block's
+// shared copy of the scalars; the other threads read the coefficients of the next phase from
+// shared memory, already in the solve's arithmetic (FP64, FP32 or double-word).
 //
 // Two grid-wide reductions per iteration instead of three.  The s-phase also forms (s, r^) and
 // (t, r^), so the scalars of r_{k+1} = s - omega t follow without reducing over r:
@@ -995,39 +1282,38 @@ __device__ __forceinline__ void phase_update(const double *part, F &&update) {
 // is formed on the fly from its s and t; each row's owner writes x and r).  The iterates are
 // those of PETSc's KSPBCGS; only the rounding of rho and of the residual norm differs.  The
 // x/r update of the last iteration runs after the loop.
+//
+// This form takes any number of rows per block and keeps every vector in global memory; meshes of at
+// most one row per thread run k_bicgstab_resident below.
 template <class Vec, class Blk>
 __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> m, KV<Vec> v, KrylovScalars *ks,
-                                                                   double *part, GridSync *gs) {
+                                                                   ExSlot *slots, GridSync *gs) {
   using R = typename ScalarOf<Vec>::T;
+  constexpr bool kDw = std::is_same<Vec, dw2>::value;
   extern __shared__ __align__(16) unsigned char tab_raw[];
   Vec *tab = reinterpret_cast<Vec *>(tab_raw);
-  __shared__ KrylovScalars s;
-  __shared__ int finish;   // 1 when the last iteration's x/r update is still to be applied
-  // coefficients in the solve's arithmetic: [0] beta, [1] beta * omega_old, [2] alpha, [3] omega
-  __shared__ __align__(16) unsigned char rs_raw[4 * sizeof(R)];
-  R *rs = reinterpret_cast<R *>(rs_raw);
-  if (threadIdx.x == 0) {
-    s = *ks;
-    rs[0] = (R)s.beta;
-    rs[1] = (R)(s.beta * s.omegaold);
-    finish = 0;
-  }
+  __shared__ PhaseScalars<R> ph;
+  __shared__ double sp[kPersistSlots * kHaloMaxBlocks];
+  __shared__ __align__(16) unsigned char scratch[kDw ? kPersistSlots * 32 * sizeof(float2)
+                                                     : kPersistSlots * kPersistThreads * sizeof(double)];
+  if (threadIdx.x == 0) ph.open(ks);
   __syncthreads();
-  if (!s.active) return;
-  double *partP = part, *partS = part + kPersistMaxBlocks * kPersistSlots;
-  unsigned int gen = 0;   // barrier arrival target (thread 0)
+  if (!ph.s.active) return;
+  ExSlot *slotP = slots, *slotS = slots + kReplicas * kPersistSlots * kHaloMaxBlocks;
+  unsigned int stamp = *((volatile unsigned int *)&gs->gen);
   const int r0 = blockIdx.x * m.rpb;
   const int r1 = min(m.items, r0 + m.rpb);
   const int own = max(r1 - r0, 0);
+  const int nact = min(own, (int)blockDim.x);
   const int h0 = __ldg(m.halo_off + blockIdx.x);
   const int nloc = own + (__ldg(m.halo_off + blockIdx.x + 1) - h0);
   bool ok = true, pending = false;   // pending: iteration k-1's x/r update not yet applied
   for (;;) {
-    const int cur = s.it & 1, nxt = cur ^ 1;
+    const int cur = ph.s.it & 1, nxt = cur ^ 1;
     // -- [x <- x + alpha p + omega s; r <- s - omega t]  p <- r - beta omega v + beta p (staged);
     //    v <- D^-1 A p;  (v, r^)
     {
-      const R beta = rs[0], bw = rs[1], ap = rs[2], wp = rs[3];
+      const R beta = ph.rs()[0], bw = ph.rs()[1], ap = ph.rs()[2], wp = ph.rs()[3];
       const Vec *__restrict__ Po = v.P[cur];
       const Vec *__restrict__ Vo = v.V[cur];
       for (int e = threadIdx.x; e < nloc; e += blockDim.x) {
@@ -1049,31 +1335,24 @@ __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> 
         if (e < own) v.P[nxt][g] = pn;
       }
       __syncthreads();
-      DotAcc<Vec> acc[1];
+      DotAcc<Vec> acc[kPersistSlots];
       for (int il = threadIdx.x; il < own; il += blockDim.x) {
         const int i = r0 + il;
         const Vec vn = v_mul(v.dinv[i], halo_row(m, i, il, tab));
         v.V[nxt][i] = vn;
         acc[0].add(vn, v.RP[i]);
       }
-      block_partials_acc<1>(acc, partP);
-      if (!(ok = grid_barrier(gs, gen))) break;
-      phase_update<1>(partP, [&](const double *tot) {
-        finish = 0;   // the staging above applied the previous iteration's x/r update
-        const double d1 = tot[0];
-        if (d1 == 0.0 || isnan(d1)) {
-          s.status = isnan(d1) ? UFE_ERR_NAN : UFE_ERR_DIVERGED;
-          s.active = 0;
-        } else {
-          s.alpha = s.rho / d1;
-          rs[2] = (R)s.alpha;
-        }
-      });
-      if (!s.active) break;
+      ++stamp;
+      block_publish<true>(1, acc, nact, scratch, slotP, stamp);
+      ok = exchange_wait(1, slotP, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
+      fence_acq_rel_gpu();
+      if (!(ok = __syncthreads_and(ok) != 0)) break;
+      after_exchange(ph, sp, false);
+      if (!ph.s.active) break;
     }
     // -- s <- r - alpha v (staged);  t <- D^-1 A s;  (s,t), (t,t), (s,s), (s,r^), (t,r^)
     {
-      const R alpha = rs[2];
+      const R alpha = ph.rs()[2];
       const Vec *__restrict__ Vn = v.V[nxt];
       for (int e = threadIdx.x; e < nloc; e += blockDim.x) {
         const int g = e < own ? r0 + e : __ldg(m.halo_idx + h0 + e - own);
@@ -1095,53 +1374,20 @@ __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> 
         acc[3].add(si, rp);
         acc[4].add(ti, rp);
       }
-      block_partials_acc<5>(acc, partS);
-      if (!(ok = grid_barrier(gs, gen))) break;
-      phase_update<5>(partS, [&](const double *tot) {
-        if (tot[1] == 0.0) {
-          if (tot[2] != 0.0) {
-            s.status = UFE_ERR_DIVERGED;
-            s.active = 0;
-            return;
-          }
-          s.omega = 0.0;
-          s.tbreak = 1;
-        } else if (isnan(tot[1])) {
-          s.status = UFE_ERR_NAN;
-          s.active = 0;
-          return;
-        } else {
-          s.omega = tot[0] / tot[1];
-        }
-        const double w = s.omega;
-        finish = 1;   // this iteration's x/r update is due from here on
-        s.it += 1;
-        s.total_its += 1;
-        const double rho_new = tot[3] - w * tot[4];
-        const double dp = sqrt(fmax(tot[2] - w * (2.0 * tot[0] - w * tot[1]), 0.0));
-        s.dp = dp;
-        s.rhoold = s.rho;
-        s.omegaold = w;
-        s.rho = rho_new;
-        if (s.tbreak) { s.active = 0; s.status = UFE_OK; s.dp = 0.0; }
-        else if (isnan(dp)) { s.status = UFE_ERR_NAN; s.active = 0; }
-        else if (dp <= s.ttol) { s.active = 0; }
-        else if (dp >= 1e4 * s.rnorm0) { s.status = UFE_ERR_DIVERGED; s.active = 0; }
-        else if (s.it >= s.max_it) { s.status = UFE_WARN_KRYLOV_MAXIT; s.active = 0; }
-        else if (rho_new == 0.0) { s.status = UFE_ERR_DIVERGED; s.active = 0; }
-        else s.beta = (s.rho / s.rhoold) * (s.alpha / s.omegaold);
-        rs[0] = (R)s.beta;
-        rs[1] = (R)(s.beta * w);
-        rs[3] = (R)w;
-      });
-      if (!s.active) break;
+      ++stamp;
+      block_publish<true>(5, acc, nact, scratch, slotS, stamp);
+      ok = exchange_wait(5, slotS, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
+      fence_acq_rel_gpu();
+      if (!(ok = __syncthreads_and(ok) != 0)) break;
+      after_exchange(ph, sp, true);
+      if (!ph.s.active) break;
       pending = true;
     }
   }
   // the x/r update of the last iteration
-  if (ok && finish) {
-    const R alpha = rs[2], omega = rs[3];
-    const int nxt = ((s.it - 1) & 1) ^ 1;   // the parity p was written with in that iteration
+  if (ok && ph.finish) {
+    const R alpha = ph.rs()[2], omega = ph.rs()[3];
+    const int nxt = ((ph.s.it - 1) & 1) ^ 1;   // the parity p was written with in that iteration
     for (int il = threadIdx.x; il < own; il += blockDim.x) {
       const int i = r0 + il;
       const Vec si = v.S[i];
@@ -1149,11 +1395,243 @@ __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> 
       v.R[i] = v_sub_scaled(si, omega, v.T[i]);
     }
   }
-  if (threadIdx.x == 0) {
-    if (!ok) {
-      s.status = UFE_ERR_DEVICE;
-      s.active = 0;
-    }
-    if (blockIdx.x == 0) *ks = s;
+  persist_close(ph.s, ok, ks, gs, stamp);
+}
+
+// ---- one row per thread: the vectors and as much of the matrix as fits stay on the SM ---------------
+// One matrix row's sum, block by block in storage order (the halves of a block as stored: 16 bytes each).
+template <class Vec>
+struct RowSum;
+template <>
+struct RowSum<double2> {
+  double2 y = make_double2(0.0, 0.0);
+  __device__ __forceinline__ void mac(uint4 h0, uint4 h1, double2 x) {
+    const double ax = __hiloint2double(h0.y, h0.x), ay = __hiloint2double(h0.w, h0.z);
+    const double az = __hiloint2double(h1.y, h1.x), aw = __hiloint2double(h1.w, h1.z);
+    y.x = fma(ay, x.y, fma(ax, x.x, y.x));
+    y.y = fma(aw, x.y, fma(az, x.x, y.y));
   }
+  __device__ __forceinline__ double2 result() const { return y; }
+};
+template <>
+struct RowSum<dw2> {
+  dw_acc yu, yv;
+  __device__ __forceinline__ void mac(uint4 h, uint4 l, dw2 xx) {
+    const float4 x = xx.q;
+    yu.mac(__uint_as_float(h.x), __uint_as_float(l.x), x.x, x.z);
+    yu.mac(__uint_as_float(h.y), __uint_as_float(l.y), x.y, x.w);
+    yv.mac(__uint_as_float(h.z), __uint_as_float(l.z), x.x, x.z);
+    yv.mac(__uint_as_float(h.w), __uint_as_float(l.w), x.y, x.w);
+  }
+  __device__ __forceinline__ dw2 result() const { return make_dw2(yu.result(), yv.result()); }
+};
+
+// Shared-memory layout of k_bicgstab_resident for a block shape; `depth` blocks per row are kept.
+struct ResidentLayout {
+  int rows, local, halo, slots, depth;   // largest numbers of a block: rows, patch entries, halo entries, slots;
+                                         // blocks kept per row
+  size_t scratch_bytes;            // block_publish's scratch
+  __host__ __device__ size_t tab() const { return 0; }
+  __host__ __device__ size_t vec() const { return tab() + 16ull * local; }              // x, r^, D^-1 of own rows
+  __host__ __device__ size_t hvec() const { return vec() + 3 * 16ull * rows; }          // r, p, v, t of halo rows
+  __host__ __device__ size_t hidx() const { return hvec() + 4 * 16ull * halo; }
+  __host__ __device__ size_t scratch() const { return hidx() + (4ull * halo + 15) / 16 * 16; }
+  __host__ __device__ size_t lcol() const { return scratch() + (scratch_bytes + 15) / 16 * 16; }
+  __host__ __device__ size_t blocks() const { return lcol() + (2ull * slots + 15) / 16 * 16; }
+  __host__ __device__ size_t bytes() const { return blocks() + 32ull * depth * rows; }
+};
+
+// k_bicgstab_halo's iteration with one thread per own row: r, p, v and t of the row stay in the thread's
+// registers, s in the staged table, x, r^, D^-1, the local column indices and the first `depth` blocks of
+// every row in shared memory for the whole solve.  Only v and t of the rows in another block's halo leave
+// the SM, as stamped entries that arrive during the exchange's wait: a halo row's r, p and s are formed again
+// from them with the owner's operations on the owner's operands (same values) instead of being loaded.
+// Same sums in the same order as k_bicgstab_halo.
+//
+// What bounds it: small meshes are a chain of latencies -- per iteration two L2 exchanges (~3,000 cycles with 152
+// blocks, 1,400 with 37), the FP64 pipe (64 cycles per instruction and warp: 4 per stored block, so ~3,300 for a
+// row of 13) and the scalar recurrence (~2,000 and ~3,300); the double-word form on 115k triangles is bound by
+// the L2 stream of the blocks that do not fit.  Per iteration, with the counter-barrier kernel it replaces
+// beside it: FP64 11.6 us (20.8) on 1,154 triangles, 14.0 (21.2) on 16,662, 35.0 (39.7) on 115,383; double-word
+// 19.3 us (25.4) on 115,383.  Fewer threads leave more registers and loads in flight to each, so the launch
+// takes 512, 768 or 1024 by the rows per block.
+template <class Vec, class Blk, int NT>
+__global__ void __launch_bounds__(NT, 1) k_bicgstab_resident(HaloMat<Blk> m, KV<Vec> v, KrylovScalars *ks,
+                                                             ExSlot *slots, ExRow *xv, ExRow *xt, GridSync *gs,
+                                                             ResidentLayout lay) {
+  using R = typename ScalarOf<Vec>::T;
+  static_assert(sizeof(Vec) == 16 && sizeof(Blk) == 32, "16-byte vector entries and 32-byte blocks");
+  extern __shared__ __align__(16) unsigned char smem[];
+  Vec *tab = reinterpret_cast<Vec *>(smem + lay.tab());
+  Vec *sx = reinterpret_cast<Vec *>(smem + lay.vec());
+  Vec *srp = sx + lay.rows, *sdinv = srp + lay.rows;
+  Vec *hr = reinterpret_cast<Vec *>(smem + lay.hvec()), *hp = hr + lay.halo, *hv = hp + lay.halo, *ht = hv + lay.halo;
+  int *hg = reinterpret_cast<int *>(smem + lay.hidx());
+  void *scratch = smem + lay.scratch();
+  uint16_t *slc = reinterpret_cast<uint16_t *>(smem + lay.lcol());
+  uint4 *sb0 = reinterpret_cast<uint4 *>(smem + lay.blocks()), *sb1 = sb0 + (size_t)lay.depth * lay.rows;
+  __shared__ PhaseScalars<R> ph;
+  __shared__ double sp[kPersistSlots * kHaloMaxBlocks];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) ph.open(ks);
+  __syncthreads();
+  if (!ph.s.active) return;
+  ExSlot *slotP = slots, *slotS = slots + kReplicas * kPersistSlots * kHaloMaxBlocks;
+  unsigned int stamp = *((volatile unsigned int *)&gs->gen);
+  const int r0 = blockIdx.x * m.rpb;
+  const int r1 = min(m.items, r0 + m.rpb);
+  const int own = max(r1 - r0, 0);
+  const int h0 = __ldg(m.halo_off + blockIdx.x);
+  const int nloc = own + (__ldg(m.halo_off + blockIdx.x + 1) - h0);
+  const bool mine = tid < own;
+  const int nhalo = nloc - own, g = r0 + tid;
+  const uint4 *__restrict__ gblk = reinterpret_cast<const uint4 *>(m.sblk);
+  // this row's slots: global slot of its first block, their number, and the slice's place in slc
+  int base = 0, width = 0, lbase = 0;
+  if (mine) {
+    const int sl = g >> 5;
+    const int s0 = __ldg(m.soff + sl);
+    base = s0 + lane;
+    width = (__ldg(m.soff + sl + 1) - s0) >> 5;
+    lbase = s0 - __ldg(m.soff + (r0 >> 5)) + lane;
+  }
+  const int kept = min(width, lay.depth);
+  Vec r = v_zero<Vec>(), p = v_zero<Vec>(), vv = v_zero<Vec>(), tt = v_zero<Vec>(), x1 = v_zero<Vec>();
+  {
+    const int cur = ph.s.it & 1;
+#pragma unroll 1
+    for (int h = tid; h < nhalo; h += NT) {
+      const int j = __ldg(m.halo_idx + h0 + h);
+      hg[h] = j;
+      hr[h] = v.R[j];
+      hp[h] = v.P[cur][j];
+      hv[h] = v.V[cur][j];
+    }
+    if (mine) {
+      r = v.R[g];
+      p = v.P[cur][g];
+      vv = v.V[cur][g];
+    }
+    if (mine) {
+      sx[tid] = v.X[g];
+      srp[tid] = v.RP[g];
+      sdinv[tid] = v.dinv[g];
+#pragma unroll 1
+      for (int k = 0; k < width; ++k) slc[lbase + 32 * k] = (uint16_t)__ldg(m.lcol + base + 32 * k);
+#pragma unroll 1
+      for (int k = 0; k < kept; ++k) {
+        const int64_t q = 2ll * (base + 32 * k);
+        sb0[k * lay.rows + tid] = gblk[q];
+        sb1[k * lay.rows + tid] = gblk[q + 1];
+      }
+    }
+  }
+  __syncthreads();
+  const bool pub = mine && __ldg(m.halo_pub + g);   // the row is in another block's halo
+  auto spmv_row = [&]() {   // row `tid` times the staged vector
+    RowSum<Vec> y;
+    // the blocks that are not kept come last: the first of them is on its way during the kept ones
+    uint4 a0, a1;
+    const uint4 *gq = gblk + 2ll * (base + 32 * kept);
+    if (kept < width) {
+      a0 = __ldg(gq);
+      a1 = __ldg(gq + 1);
+    }
+    const uint16_t *lc = slc + lbase;
+    const uint4 *q0 = sb0 + tid, *q1 = sb1 + tid;
+    constexpr int kUnroll = std::is_same<Vec, double2>::value ? 2 : 1;
+#pragma unroll kUnroll
+    for (int k = 0; k < kept; ++k, lc += 32, q0 += lay.rows, q1 += lay.rows) y.mac(*q0, *q1, tab[*lc]);
+#pragma unroll 1
+    for (int k = kept; k < width; ++k, lc += 32) {
+      const uint4 c0 = a0, c1 = a1;
+      gq += 64;
+      if (k + 1 < width) {
+        a0 = __ldg(gq);
+        a1 = __ldg(gq + 1);
+      }
+      y.mac(c0, c1, tab[*lc]);
+    }
+    return y.result();
+  };
+  bool ok = true, s_phase = false;
+  int pending = 0;   // iteration k-1's x/r update not yet applied
+  // Two passes of one loop body per iteration, so that the product, the sums and the wait are fetched as one
+  // piece of code each.
+#pragma unroll 1
+  for (;;) {
+    if (!s_phase) {
+      // [x <- x + alpha p + omega s; r <- s - omega t]  p <- r - beta omega v + beta p (staged)
+      const R beta = ph.rs()[0], bw = ph.rs()[1], wp = ph.rs()[3];
+#pragma unroll 1
+      for (int h = NT - 1 - tid; h < nhalo; h += NT) {   // the last threads first: they have no own row
+        Vec rh = hr[h];
+        if (pending) {
+          rh = v_sub_scaled(tab[own + h], wp, ht[h]);
+          hr[h] = rh;
+        }
+        const Vec pn = v_pupd(rh, bw, hv[h], beta, hp[h]);
+        hp[h] = pn;
+        tab[own + h] = pn;
+      }
+      if (mine) {
+        if (pending) {
+          const Vec sg = tab[tid];
+          r = v_sub_scaled(sg, wp, tt);
+          sx[tid] = v_axpy(x1, wp, sg);
+        }
+        p = v_pupd(r, bw, vv, beta, p);
+        tab[tid] = p;
+      }
+    } else {
+      // s <- r - alpha v (staged)
+      const R alpha = ph.rs()[2];
+#pragma unroll 1
+      for (int h = NT - 1 - tid; h < nhalo; h += NT) tab[own + h] = v_sub_scaled(hr[h], alpha, hv[h]);
+      if (mine) tab[tid] = v_sub_scaled(r, alpha, vv);
+    }
+    __syncthreads();
+    // v <- D^-1 A p;  (v, r^)      or      t <- D^-1 A s;  (s,t), (t,t), (s,s), (s,r^), (t,r^)
+    ++stamp;
+    DotAcc<Vec> acc[kPersistSlots];
+    if (mine) {
+      const Vec y = v_mul(sdinv[tid], spmv_row()), rp = srp[tid];
+      if (pub) row_publish((s_phase ? xt : xv) + g, y, stamp);
+      if (!s_phase) {
+        vv = y;
+        acc[0].add(y, rp);
+      } else {
+        tt = y;
+        const Vec si = tab[tid];
+        acc[0].add(si, y);
+        acc[1].add(y, y);
+        acc[2].add(si, si);
+        acc[3].add(si, rp);
+        acc[4].add(y, rp);
+      }
+    }
+    const int np = s_phase ? 5 : 1;
+    block_publish<false>(np, acc, own, scratch, s_phase ? slotS : slotP, stamp);
+    if (mine && s_phase) x1 = v_axpy(sx[tid], ph.rs()[2], p);   // half of the x update, while the sums travel
+    ok = exchange_wait(np, s_phase ? slotS : slotP, sp, s_phase ? xt : xv, hg, nhalo,
+                       reinterpret_cast<double *>(s_phase ? ht : hv), stamp, gs);
+    if (!(ok = __syncthreads_and(ok) != 0)) break;
+    after_exchange(ph, sp, s_phase);
+    if (!ph.s.active) break;
+    pending |= s_phase;
+    s_phase = !s_phase;
+    asm volatile("" : "+r"(pending));   // one copy of the body: the first passes are not peeled
+  }
+  if (mine) {
+    Vec x = sx[tid];
+    if (ok && ph.finish) {   // the x/r update of the last iteration
+      const R omega = ph.rs()[3];
+      const Vec si = tab[tid];
+      x = v_axpy(x1, omega, si);
+      r = v_sub_scaled(si, omega, tt);
+    }
+    v.X[g] = x;
+    v.R[g] = r;
+  }
+  persist_close(ph.s, ok, ks, gs, stamp);
 }

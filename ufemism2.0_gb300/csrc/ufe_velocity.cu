@@ -630,7 +630,10 @@ __global__ void k_inner_init(int nTri, const double2 *R, float2 *R32, float2 *RP
                              double inner_rtol, int max_it, double *partials, unsigned int *tickets,
                              CondArg cond, GridSync *gsync) {
   // reset the persistent solve's grid barrier (nothing else uses it now)
-  if (gsync && blockIdx.x == 0 && threadIdx.x == 0) *gsync = GridSync{0u, 0u, 0, 0};
+  if (gsync && blockIdx.x == 0 && threadIdx.x == 0) {
+    gsync->count = 0u;
+    gsync->err = 0;
+  }
   double acc[1] = {0.0};
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nTri; t += stride) {
@@ -1118,7 +1121,7 @@ void build_sell(ufe_ctx *ctx, Work *w) {
   const int32_t G = std::max(1, std::min<int32_t>(std::min<int32_t>(sms, nsl), kHaloMaxBlocks));
   const int32_t rpb = ((n + G - 1) / G + 31) / 32 * 32;
   std::vector<int32_t> hoff(G + 1, 0), hidx, lcol(nslots, 0);
-  int32_t maxlocal = 0;
+  int32_t maxlocal = 0, maxhalo = 0;
   std::vector<int32_t> halo;
   for (int32_t b = 0; b < G; ++b) {
     const int32_t r0 = std::min(n, b * rpb), r1 = std::min(n, r0 + rpb);
@@ -1138,12 +1141,25 @@ void build_sell(ufe_ctx *ctx, Work *w) {
     hidx.insert(hidx.end(), halo.begin(), halo.end());
     hoff[b + 1] = (int32_t)hidx.size();
     maxlocal = std::max(maxlocal, own + (int32_t)halo.size());
+    maxhalo = std::max(maxhalo, (int32_t)halo.size());
   }
   w->halo_G = G;
   w->halo_rpb = rpb;
   w->halo_maxlocal = maxlocal;
+  w->halo_maxhalo = maxhalo;
+  w->halo_maxslots = 0;
+  for (int32_t b = 0; b < G; ++b) {
+    const int32_t r0 = std::min(n, b * rpb), r1 = std::min(n, r0 + rpb);
+    if (r1 > r0) w->halo_maxslots = std::max(w->halo_maxslots, off[(r1 + 31) / 32] - off[r0 / 32]);
+  }
+  w->halo_maxwidth = 0;
+  for (int32_t sl = 0; sl < nsl; ++sl) w->halo_maxwidth = std::max(w->halo_maxwidth, (off[sl + 1] - off[sl]) / 32);
   w->halo_off = up(hoff);
   w->halo_idx = up(hidx);
+  std::vector<uint8_t> pub(n, 0);
+  for (int32_t j : hidx) pub[j] = 1;
+  w->halo_pub = alloc_n<uint8_t>(n);
+  UFE_CUDA(cudaMemcpy(w->halo_pub, pub.data(), n, cudaMemcpyHostToDevice));
   w->halo_lcol = up(lcol);
   w->sell_blk = alloc_n<double4>(nslots);
   w->sell_blk32 = alloc_n<float4>(nslots);
@@ -1208,6 +1224,8 @@ Work *ensure_work(ufe_ctx *ctx) {
   build_sell(ctx, w);
   w->ppart = alloc_n<double>((size_t)3 * kPersistMaxBlocks * kPersistSlots);
   w->gsync = alloc_n<GridSync>(1);
+  w->xslots = alloc_n<ExSlot>(kExSlots);
+  w->xrows = alloc_n<ExRow>((size_t)2 * nTri);
   w->F1_3D_a = alloc_n<double>((size_t)nV * nz);
   w->N_b_in = alloc_n<double>(nTri);
   w->dNx_b_in = alloc_n<double>(nTri);
@@ -1224,6 +1242,9 @@ Work *ensure_work(ufe_ctx *ctx) {
   UFE_CUDA(cudaMemsetAsync(w->tau_b, 0, sizeof(double2) * nTri, s));
   UFE_CUDA(cudaMemsetAsync(w->eta_3D_b, 0, sizeof(double) * (size_t)nTri * nz, s));
   UFE_CUDA(cudaMemsetAsync(w->ks, 0, sizeof(KrylovScalars) * 3, s));
+  UFE_CUDA(cudaMemsetAsync(w->gsync, 0, sizeof(GridSync), s));
+  UFE_CUDA(cudaMemsetAsync(w->xrows, 0, sizeof(ExRow) * 2 * (size_t)nTri, s));
+  UFE_CUDA(cudaMemsetAsync(w->xslots, 0, sizeof(ExSlot) * kExSlots, s));
   UFE_CUDA(cudaMemsetAsync(w->err, 0, sizeof(int), s));
   UFE_CUDA(cudaMemsetAsync(w->pred_flag, 0, sizeof(int32_t), s));
   UFE_CUDA(cudaStreamSynchronize(s));
@@ -1245,7 +1266,7 @@ void free_work(ufe_ctx *ctx) {
                   w->eta_3D_b, w->bfc_b, w->F2b1, w->beta_b, w->Hi, w->Hs, w->Avav, w->A_flow, w->beta_sq, w->A_pow,
                   w->alpha_sq, w->effp, w->tys, w->mask_gr, w->N_a, w->beta_a, w->beta_eff_a, w->F2a1,
                   w->eta_3D_a, w->F1_3D_a, w->N_b_in, w->dNx_b_in, w->dNy_b_in, w->beta_b_in, w->ks,
-                  w->ps, w->err, w->ppart, w->gsync, w->sell_off, w->sell_col, w->sell_map, w->sell_blk,
+                  w->ps, w->err, w->ppart, w->gsync, w->xslots, w->xrows, w->halo_pub, w->sell_off, w->sell_col, w->sell_map, w->sell_blk,
                   w->sell_blk32, w->halo_off, w->halo_idx, w->halo_lcol, w->pX, w->pR, w->pRP, w->pS, w->pT,
                   w->pdinv, w->pP[0], w->pP[1], w->pV[0], w->pV[1], w->sell_blkp, w->pair_bad,
                   w->Ti, w->mask_fl, w->fgr_v, w->Hib, w->SL, w->A_rheo, w->tys_ideal, w->cp_ptr, w->cp_idx,
@@ -1354,7 +1375,6 @@ namespace {
 
 __global__ void k_reset_gsync(GridSync *g) {
   g->count = 0u;
-  g->gen = 0u;
   g->err = 0;
 }
 
@@ -1380,6 +1400,9 @@ unsigned persist_blocks(const void *kernel, int64_t lanes_total) {
   nb = std::min<int64_t>(nb, (lanes_total + kPersistThreads - 1) / kPersistThreads);
   return (unsigned)std::max<int64_t>(nb, 1);
 }
+
+// dynamic shared memory of k_bicgstab_resident: 227 KB less its static part
+constexpr size_t kResidentSmem = 216 * 1024;
 
 struct Solver {
   ufe_ctx *ctx;
@@ -1564,35 +1587,59 @@ struct Solver {
     return use_sell() && lanes == 1 && w->halo_G > 0 &&
            (size_t)w->halo_maxlocal * sizeof(float2) <= 160 * 1024 && !getenv("UFE_NO_HALO");
   }
-  void inner_halo() {
-    const size_t smem = (size_t)w->halo_maxlocal * sizeof(float2);
-    static size_t attr = 0;
-    if (smem > attr) {
-      UFE_CUDA(cudaFuncSetAttribute(k_bicgstab_halo<float2, float4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-      attr = smem;
-    }
-    HaloDiffMat m{w->nTri, w->halo_rpb, w->sell_off, w->halo_lcol, w->sell_blk32, w->rowsum32, w->halo_off,
-                  w->halo_idx};
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    UFE_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
-      k_bicgstab_halo<float2, float4><<<w->halo_G, kPersistThreads, smem, s>>>(m, kv_inner(), w->ks + 1, w->ppart,
-                                                                              w->gsync);
-      UFE_CUDA(cudaGetLastError());
-      return;
-    }
+  // One co-resident launch: cooperative outside graphs, plain inside a captured graph (its kernels run one
+  // after another, and the grid never exceeds the co-resident count).
+  template <class... KArgs, class... Args>
+  void launch_coresident(void (*kern)(KArgs...), unsigned threads, size_t smem, Args... args) {
+    UFE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(w->halo_G);
-    cfg.blockDim = dim3(kPersistThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr1[1];
-    attr1[0].id = cudaLaunchAttributeCooperative;
-    attr1[0].val.cooperative = 1;
-    cfg.attrs = attr1;
-    cfg.numAttrs = 1;
-    UFE_CUDA(cudaLaunchKernelEx(&cfg, k_bicgstab_halo<float2, float4>, m, kv_inner(), w->ks + 1, w->ppart, w->gsync));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    UFE_CUDA(cudaStreamIsCapturing(s, &cap));
+    cfg.attrs = at;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+    UFE_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  }
+  // k_bicgstab_resident takes a mesh with at most one row per thread; the shared memory that its vectors leave
+  // holds the first blocks of every row.  False when the patch does not fit.
+  template <class Vec, class Blk>
+  bool launch_resident(const HaloMat<Blk> &m, KV<Vec> v, KrylovScalars *ks) {
+    if (w->halo_rpb > kPersistThreads) return false;
+    ResidentLayout lay;
+    lay.rows = w->halo_rpb;
+    lay.local = w->halo_maxlocal;
+    lay.halo = w->halo_maxhalo;
+    lay.slots = w->halo_maxslots;
+    lay.scratch_bytes = std::is_same<Vec, dw2>::value ? kPersistSlots * 32 * sizeof(float2)
+                                                      : kPersistSlots * sizeof(double) * (size_t)w->halo_rpb;
+    lay.depth = 0;
+    if (lay.bytes() > kResidentSmem) return false;
+    lay.depth = (int)std::min<size_t>((kResidentSmem - lay.bytes()) / (32ull * lay.rows), (size_t)w->halo_maxwidth);
+    auto launch = [&](auto nt) {
+      launch_coresident(k_bicgstab_resident<Vec, Blk, decltype(nt)::value>, decltype(nt)::value, lay.bytes(), m, v, ks,
+                        w->xslots, w->xrows, w->xrows + w->nTri, w->gsync, lay);
+    };
+    // fewer threads leave more registers, and with them more loads in flight, to each
+    if (w->halo_rpb <= 512) launch(std::integral_constant<int, 512>());
+    else if (w->halo_rpb <= 768) launch(std::integral_constant<int, 768>());
+    else launch(std::integral_constant<int, kPersistThreads>());
+    return true;
+  }
+  template <class Vec, class Blk>
+  void launch_halo(const HaloMat<Blk> &m, KV<Vec> v, KrylovScalars *ks) {
+    launch_coresident(k_bicgstab_halo<Vec, Blk>, kPersistThreads, (size_t)w->halo_maxlocal * sizeof(Vec), m, v, ks,
+                      w->xslots, w->gsync);
+  }
+  void inner_halo() {
+    HaloDiffMat m{w->nTri, w->halo_rpb, w->sell_off, w->halo_lcol, w->sell_blk32, w->rowsum32, w->halo_off,
+                  w->halo_idx, w->halo_pub};
+    launch_halo(m, kv_inner(), w->ks + 1);
   }
   // the FP64 solve as one persistent launch with shared-memory patches (the plain FP64 path)
   bool halo64_ok() const {
@@ -1600,36 +1647,11 @@ struct Solver {
            (size_t)w->halo_maxlocal * sizeof(double2) <= 160 * 1024 && !getenv("UFE_NO_HALO");
   }
   void enqueue_outer_halo64() {
-    const size_t smem = (size_t)w->halo_maxlocal * sizeof(double2);
-    static size_t attr = 0;
-    if (smem > attr) {
-      UFE_CUDA(cudaFuncSetAttribute(k_bicgstab_halo<double2, double4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-      attr = smem;
-    }
     HaloMat<double4> m{w->nTri, w->halo_rpb, w->sell_off, w->halo_lcol, w->sell_blk, nullptr, w->halo_off,
-                       w->halo_idx};
+                       w->halo_idx, w->halo_pub};
     k_reset_gsync<<<1, 1, 0, s>>>(w->gsync);
     UFE_CUDA(cudaGetLastError());
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    UFE_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
-      k_bicgstab_halo<double2, double4><<<w->halo_G, kPersistThreads, smem, s>>>(m, kv64(), w->ks, w->ppart,
-                                                                                 w->gsync);
-      UFE_CUDA(cudaGetLastError());
-      return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(w->halo_G);
-    cfg.blockDim = dim3(kPersistThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    UFE_CUDA(cudaLaunchKernelEx(&cfg, k_bicgstab_halo<double2, double4>, m, kv64(), w->ks, w->ppart, w->gsync));
+    if (!launch_resident(m, kv64(), w->ks)) launch_halo(m, kv64(), w->ks);
   }
   // UFE_PREC_FP32_PAIR: the linear solve in double-word arithmetic, one persistent launch with the
   // FP64 solve's shared-memory patches; the FP64 persistent solve runs after it and does the work
@@ -1659,35 +1681,11 @@ struct Solver {
                                         w->pdinv, w->pP[0], w->pV[0], w->ks, w->pair_bad);
     k_pair_decide<<<1, 1, 0, s>>>(w->ks, w->pair_bad);
     UFE_CUDA(cudaGetLastError());
-    const size_t smem = (size_t)w->halo_maxlocal * sizeof(dw2);
-    static size_t attr = 0;
-    if (smem > attr) {
-      UFE_CUDA(cudaFuncSetAttribute(k_bicgstab_halo<dw2, dwblk>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-      attr = smem;
-    }
     HaloMat<dwblk> m{w->nTri, w->halo_rpb, w->sell_off, w->halo_lcol, w->sell_blkp, nullptr, w->halo_off,
-                     w->halo_idx};
+                     w->halo_idx, w->halo_pub};
     k_reset_gsync<<<1, 1, 0, s>>>(w->gsync);
     UFE_CUDA(cudaGetLastError());
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    UFE_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
-      k_bicgstab_halo<dw2, dwblk><<<w->halo_G, kPersistThreads, smem, s>>>(m, kvpair(), w->ks + 2, w->ppart, w->gsync);
-      UFE_CUDA(cudaGetLastError());
-    } else {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(w->halo_G);
-      cfg.blockDim = dim3(kPersistThreads);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = s;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeCooperative;
-      at[0].val.cooperative = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      UFE_CUDA(cudaLaunchKernelEx(&cfg, k_bicgstab_halo<dw2, dwblk>, m, kvpair(), w->ks + 2, w->ppart, w->gsync));
-    }
+    if (!launch_resident(m, kvpair(), w->ks + 2)) launch_halo(m, kvpair(), w->ks + 2);
     k_pair_exit<<<g, kThreads, 0, s>>>(w->nTri, w->pX, w->kv.X, w->ks);
     UFE_CUDA(cudaGetLastError());
   }

@@ -153,8 +153,10 @@ struct Work {
   float4 *sell_blk32 = nullptr;
   // patches of the persistent FP32 solve: block b owns rows [b*halo_rpb, (b+1)*halo_rpb)
   int32_t halo_G = 0, halo_rpb = 0, halo_maxlocal = 0;
+  int32_t halo_maxhalo = 0, halo_maxslots = 0, halo_maxwidth = 0;   // most halo rows and slots of a block; most blocks of a row
   int32_t *halo_off = nullptr;   // halo_G + 1
   int32_t *halo_idx = nullptr;   // halo rows of every block
+  uint8_t *halo_pub = nullptr;   // nTri: 1 where the row is in some block's halo
   int32_t *halo_lcol = nullptr;  // nslots: local index of each slot's column
   // double-word Krylov solve (UFE_PREC_FP32_PAIR), allocated on first use: its vectors, the
   // sliced-ELL blocks in double-word form, and the flag of values outside the FP32 range
@@ -162,9 +164,11 @@ struct Work {
   dw2 *pP[2] = {nullptr, nullptr}, *pV[2] = {nullptr, nullptr};
   dwblk *sell_blkp = nullptr;
   int *pair_bad = nullptr;
-  // persistent Krylov kernel: per-block partial sums of its three phases and its grid barrier
+  // persistent Krylov kernels: per-block partial sums and the counter of k_bicgstab_persist's grid barrier
   double *ppart = nullptr;
   struct GridSync *gsync = nullptr;
+  struct ExSlot *xslots = nullptr;   // stamped slots of its grid-wide sums
+  struct ExRow *xrows = nullptr;     // and of its halo entries: v, then t (nTri each)
   // graphs, and their kernel nodes: in the prologue and in one Picard iteration ([0] SSA, [1] DIVA;
   // -1 where a Picard iteration holds a data-dependent loop)
   cudaGraphExec_t graph_ssa = nullptr, graph_diva = nullptr;
