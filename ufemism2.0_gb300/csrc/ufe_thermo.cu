@@ -317,60 +317,94 @@ __global__ void __launch_bounds__(128) k_heat_columns(In in, ZOps z, Consts c, V
   }
 }
 
-// The dt-halving retries (:161-239), one warp per listed column.  Per column the row
-// coefficients that do not depend on dt or on the current profile (c_ddzeta, c_d2dzeta2, the
-// off-diagonals, the advection and heating terms) are computed once, one row per lane.  Per dt
-// level the matrix part of the Thomas elimination (w = a / b', b' = b - w c) is done once by lane 0:
-// it is the same in every substep, so hoisting it changes no value.  Per substep the two
-// recurrences of the solve -- the forward sweep d'_k = d_k - w_k d'_{k-1} and the back substitution
-// x_k = (d'_k - c_k x_{k+1}) / b'_k -- are first-order affine recurrences, evaluated across the warp
-// as parallel prefix compositions of affine maps y -> a + b y (Kogge-Stone, 5 shuffle steps; rows
-// beyond 32 are composed sequentially inside each lane first).  The back substitution is split as
-// x_k = A_k + B_k x_base, so both basal conditions of a subgrid grounding-line column come from one
-// scan.  Divisions by b'_k and dt become multiplications by reciprocals formed once per dt level
-// (FP64 division is a long dependent sequence on GB300).  The scans reassociate the sums and the
-// reciprocals round differently, so retried columns differ from the sequential recurrence in the
-// last bits (well below 1e-9 K); the lanes then clamp, mix and check the rows in parallel.
-constexpr int kRetryArrays = 16;
-constexpr int kRetryWarps = 1;
+// The dt-halving retries (:161-239), one warp per listed column, R consecutive rows per lane (row k in lane
+// k / R; R = 1, 2, 4 or 8 for up to 32, 64, 128, 256 layers).  Per column the row coefficients that do not
+// depend on dt or on the current profile (the off-diagonals, the advection and heating terms) are computed
+// once, and the matrix part of the Thomas elimination (w = a / b', b' = b - w c) once for all dt levels at
+// the same time, level l in lane l - 2: it is the same in every substep, so hoisting it changes no value.
+//
+// Per substep the two recurrences of the solve -- the forward sweep d'_k = d_k - w_k d'_{k-1} and the back
+// substitution x_k = (d'_k - c_k x_{k+1}) / b'_k -- are first-order affine recurrences, evaluated across the
+// warp as parallel prefix compositions of affine maps y -> a + b y (Kogge-Stone, 5 shuffle steps).  Only the
+// constants `a` change from one substep to the next: the slopes that each step multiplies by are formed once
+// per dt level (Slopes) and a step is one shuffle and one FMA.  The back substitution is carried as
+// x_k = A_k + B_k x_base, so both basal conditions of a subgrid grounding-line column come from one scan.
+// Divisions by b'_k and dt become multiplications by reciprocals formed once per dt level.  The scans
+// reassociate the sums and the reciprocals round differently, so retried columns differ from the sequential
+// recurrence in the last bits (well below 1e-9 K).
+//
+// What bounds it: the chain of dependent FP64 instructions and shuffles of up to 1,022 substeps (65 and 29
+// cycles each on GB300, and an FP64 instruction costs a warp 64 cycles whatever it masks), with few columns
+// (94 of 200k on the large workload) to hide it.  So the substep holds 15 FP64 instructions for up to 32
+// layers: the minimum with the melting point is taken on bit patterns, the stability check runs on the
+// last substep only (the earlier ones' results were overwritten), and the profile stays in registers.
+// Measured on 200k columns x 30 layers (94 columns through all levels): 1.13 ms per time step, 2.76 ms before,
+// when each substep composed the slopes again, compared in FP64 and kept the profile in shared memory.
+constexpr int kRetryLevels = 9;          // dt / 2 ... dt / 512 (:163)
+constexpr int kRetryArrays = 4 + 2 * kRetryLevels;
 constexpr int kRetryBlocks = 4 * 152;
 
-struct Affine {   // y -> a + b y
-  double a, b;
-};
-// g after f
-__device__ __forceinline__ Affine compose(const Affine &g, const Affine &f) {
-  return Affine{fma(g.b, f.a, g.a), g.b * f.b};
+// min(x, limit) for a positive finite limit, as fmin gives it (limit for a NaN x), without FP64 instructions:
+// positive values order as their bits, a negative value's bits are a negative integer.
+__device__ __forceinline__ double min_limit(double x, double limit) {
+  const long long b = __double_as_longlong(x), l = __double_as_longlong(limit);
+  const bool nan = ((unsigned long long)b << 1) > 0xffe0000000000000ull;
+  return (nan || b > l) ? limit : x;
 }
-// Inclusive scan over the lanes in increasing (up = true) or decreasing lane order: lane l gets
-// M_l o M_{l-1} o ... o M_0 (up) or M_l o M_{l+1} o ... o M_31 (down).
-__device__ __forceinline__ Affine warp_scan(Affine m, int lane, bool up) {
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const double qa = up ? __shfl_up_sync(0xffffffffu, m.a, off) : __shfl_down_sync(0xffffffffu, m.a, off);
-    const double qb = up ? __shfl_up_sync(0xffffffffu, m.b, off) : __shfl_down_sync(0xffffffffu, m.b, off);
-    if (up ? lane >= off : lane + off < 32) m = compose(m, Affine{qa, qb});
-  }
-  return m;
-}
+__device__ __forceinline__ double shfl_up_d(double v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double shfl_down_d(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
 
-template <class In>
-__global__ void __launch_bounds__(32 * kRetryWarps) k_heat_retry(In in, ZOps z, Consts c, VertexFields vf,
-                                                                  int64_t nV, double *__restrict__ Ti_next,
-                                                                  Lists lists, Counters *cnt) {
+// Slopes of a warp scan over affine maps, for fixed per-lane slopes b: step[i] multiplies the value received
+// in step i, all is the slope of the lane's composed map, and scan() composes the constants.
+struct Slopes {
+  double step[5], all;
+  __device__ __forceinline__ void up(double b, int lane) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      step[i] = b;
+      const double q = shfl_up_d(b, 1 << i);
+      if (lane >= (1 << i)) b = b * q;
+    }
+    all = b;
+  }
+  __device__ __forceinline__ void down(double b, int lane) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      step[i] = b;
+      const double q = shfl_down_d(b, 1 << i);
+      if (lane + (1 << i) < 32) b = b * q;
+    }
+    all = b;
+  }
+  __device__ __forceinline__ double scan_up(double a, int lane) const {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const double q = shfl_up_d(a, 1 << i);
+      const double f = fma(step[i], q, a);
+      a = lane >= (1 << i) ? f : a;
+    }
+    return a;
+  }
+  __device__ __forceinline__ double scan_down(double a, int lane) const {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const double q = shfl_down_d(a, 1 << i);
+      const double f = fma(step[i], q, a);
+      a = lane + (1 << i) < 32 ? f : a;
+    }
+    return a;
+  }
+};
+
+template <class In, int R>
+__global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, VertexFields vf, int64_t nV,
+                                                   double *__restrict__ Ti_next, Lists lists, Counters *cnt) {
   if (cnt->err) return;
   extern __shared__ double sm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nz = z.nz;
-  const int R = (nz + 31) / 32;                      // rows per lane: [lane*R, lane*R + R)
-  const int k0 = lane * R, k1 = min(k0 + R, nz);
-  double *base = sm + (size_t)warp * kRetryArrays * nz;
-  double *C1 = base, *C2 = C1 + nz, *UDX = C2 + nz, *VDY = UDX + nz, *PHI = VDY + nz, *A = PHI + nz,
-         *Cc = A + nz, *Bp = Cc + nz, *W = Bp + nz, *D = W + nz, *X = D + nz, *PMP = X + nz, *NB = PMP + nz,
-         *XB = NB + nz, *SB = XB + nz, *RB = SB + nz;
+  const int lane = threadIdx.x, nz = z.nz, kb = nz - 1, k0 = lane * R;
+  double *A = sm, *Cc = A + nz, *E1 = Cc + nz, *E2 = E1 + nz, *W = E2 + nz, *Bp = W + kRetryLevels * nz;
   const int32_t n = cnt->n_retry;
-  const int warps_total = gridDim.x * kRetryWarps;
-  for (int32_t j = blockIdx.x * kRetryWarps + warp; j < n; j += warps_total) {
+  for (int32_t j = blockIdx.x; j < n; j += gridDim.x) {
     const int64_t vi = lists.retry[j];
     const double Hi_eff = __ldg(vf.Hi_eff + vi);
     const double Ts = __ldg(vf.T_surf + vi);
@@ -380,126 +414,160 @@ __global__ void __launch_bounds__(32 * kRetryWarps) k_heat_retry(In in, ZOps z, 
     const bool two_solves = mask == UFE_COL_GL_GR && c.glbc == UFE_GLBC_SUBGRID;
     const bool grounded = mask == UFE_COL_GROUNDED || (mask == UFE_COL_GL_GR && c.glbc == UFE_GLBC_GROUNDED);
     const typename In::Col col = in.col(vi);
-    for (int k = lane; k < nz; k += 32) {
+    double X[R], G[R], PMP[R];   // the profile; advection and heating; the melting point
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int k = k0 + r;
+      X[r] = G[r] = PMP[r] = 0.0;
+      if (k >= nz) continue;
       const double zk = __ldg(z.zeta + k);
-      PMP[k] = melting_point(Hi_eff, zk);
-      X[k] = Ti_next[(int64_t)k * nV + vi];   // the profile the full-dt solve left (:222)
-      if (k >= 1 && k < nz - 1) {
+      PMP[r] = melting_point(Hi_eff, zk);
+      X[r] = Ti_next[(int64_t)k * nV + vi];   // the profile the full-dt solve left (:222)
+      double a = 0.0, cc = 0.0;               // boundary rows: AA_ldiag / AA_udiag stay zero (:389-391)
+      if (k >= 1 && k < kb) {
         Layer L;
         in.layer(col, vi, k, zk, L);
         const double Cpi = heat_capacity(c, L.Ti0);
         const double Ki = conductivity(c, L.Ti0);
         const double c1 = L.dzt + (L.u * L.dzx) + (L.v * L.dzy) + (L.w * L.dzz);
         const double c2 = -(Ki / (kIceDensity * Cpi) * (L.dzz * L.dzz));
-        C1[k] = c1;
-        C2[k] = c2;
-        UDX[k] = L.udx;
-        VDY[k] = L.vdy;
-        PHI[k] = L.phi / (kIceDensity * Cpi);
-        A[k] = (c1 * __ldg(z.l1 + k)) + (c2 * __ldg(z.l2 + k));
-        Cc[k] = (c1 * __ldg(z.u1 + k)) + (c2 * __ldg(z.u2 + k));
-      } else {
-        A[k] = 0.0;    // boundary rows: AA_ldiag / AA_udiag stay zero (:389-391)
-        Cc[k] = 0.0;
+        G[r] = L.phi / (kIceDensity * Cpi) - L.udx - L.vdy;
+        a = (c1 * __ldg(z.l1 + k)) + (c2 * __ldg(z.l2 + k));
+        cc = (c1 * __ldg(z.u1 + k)) + (c2 * __ldg(z.u2 + k));
+        E1[k] = c1 * __ldg(z.d1 + k);
+        E2[k] = c2 * __ldg(z.d2 + k);
       }
+      A[k] = a;
+      Cc[k] = cc;
     }
     // basal row inputs (grounded flux condition)
-    const int kb = nz - 1;
     const double pmp_b = melting_point(Hi_eff, __ldg(z.zeta + kb));
     double Ti0b, dzzb;
     in.basal(col, vi, kb, __ldg(z.zeta + kb), Ti0b, dzzb);
-    const double Kb = conductivity(c, Ti0b);
-    const double dzeta_b = __ldg(z.zeta + kb) - __ldg(z.zeta + kb - 1);
+    const double flux_b = (__ldg(z.zeta + kb) - __ldg(z.zeta + kb - 1)) * Q / (dzzb * conductivity(c, Ti0b));
+    __syncwarp();
+    if (lane < kRetryLevels) {
+      // matrix part of the forward elimination, dt level lane + 2
+      const double inv_dt = 1.0 / (c.dt * (1.0 / (double)(2 << lane)));
+      double *Wl = W + lane * nz, *Bl = Bp + lane * nz;
+      double bprev = 1.0, cprev = 0.0;
+      Wl[0] = 0.0;
+      Bl[0] = 1.0;
+      for (int k = 1; k < kb; ++k) {
+        double b = inv_dt + E1[k] + E2[k];
+        const double wgt = A[k] / bprev;
+        b = b - wgt * cprev;
+        Wl[k] = wgt;
+        Bl[k] = b;
+        bprev = b;
+        cprev = Cc[k];
+      }
+      const double wgt = 0.0 / bprev;
+      Wl[kb] = wgt;
+      Bl[kb] = 1.0 - wgt * cprev;
+    }
     __syncwarp();
     bool found = false;
-    for (int it_dt = 2; it_dt <= 10 && !found; ++it_dt) {
-      double half = 1.0;
-      for (int i = 1; i < it_dt; ++i) half *= 0.5;   // 0.5**(it_dt-1), exact
-      const double dt = c.dt * half;
-      const double inv_dt = 1.0 / dt;
-      if (lane == 0) {
-        // matrix part of the forward elimination for this dt
-        double bprev = 1.0, cprev = 0.0;
-        Bp[0] = 1.0;
-        for (int k = 1; k < nz - 1; ++k) {
-          double b = inv_dt + (C1[k] * __ldg(z.d1 + k)) + (C2[k] * __ldg(z.d2 + k));
-          const double wgt = A[k] / bprev;
-          b = b - wgt * cprev;
-          W[k] = wgt;
-          Bp[k] = b;
-          bprev = b;
-          cprev = Cc[k];
-        }
-        const double wgt = 0.0 / bprev;
-        W[kb] = wgt;
-        Bp[kb] = 1.0 - wgt * cprev;
+    for (int it_dt = 2; it_dt <= 1 + kRetryLevels && !found; ++it_dt) {
+      const double *Wl = W + (it_dt - 2) * nz, *Bl = Bp + (it_dt - 2) * nz;
+      const double inv_dt = 1.0 / (c.dt * (1.0 / (double)(1 << (it_dt - 1))));   // 0.5**(it_dt-1), exact
+      // per row for this dt: the forward slope -w_k, 1 / b'_k and the back substitution's slope,
+      // x_k = d'_k / b'_k - (c_k / b'_k) x_{k+1}; rows from the base on are the identity
+      double Wn[R], RB[R], NB[R];
+      double bf = 1.0, bb = 1.0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int k = k0 + r;
+        const bool row = k < kb;
+        Wn[r] = !row ? 1.0 : (k == 0 ? 0.0 : -Wl[k]);
+        RB[r] = row ? 1.0 / Bl[k] : 0.0;
+        NB[r] = row ? -(Cc[k] * RB[r]) : 1.0;
+        bf = r == 0 ? Wn[r] : Wn[r] * bf;
       }
-      __syncwarp();
-      // per row for this dt: 1 / b'_k and the back
-      // substitution's slope, x_k = d'_k / b'_k - (c_k / b'_k) x_{k+1}
-      for (int k = lane; k < nz; k += 32) {
-        const double rb = 1.0 / Bp[k];
-        RB[k] = rb;
-        NB[k] = (k < kb) ? -(Cc[k] * rb) : 0.0;
-      }
-      __syncwarp();
+#pragma unroll
+      for (int r = R - 1; r >= 0; --r) bb = r == R - 1 ? NB[r] : NB[r] * bb;
+      Slopes fwd, bwd;
+      fwd.up(bf, lane);
+      bwd.down(bb, lane);
+      const double w_b = Wl[kb], rb_b = 1.0 / Bl[kb], d_top = fmin(Ts, kT0);
+      const bool unit_b = rb_b == 1.0;
       const int nsub = 1 << (it_dt - 1);
-      bool ok = true;
+#pragma unroll 1
       for (int sub = 0; sub < nsub; ++sub) {
-        // right-hand side (rows 0 .. nz-2) and the basal row's value from the current profile
-        for (int k = lane; k < nz - 1; k += 32)
-          D[k] = (k == 0) ? fmin(Ts, kT0) : X[k] * inv_dt - UDX[k] - VDY[k] + PHI[k];
-        const double d_gr = fmin(pmp_b, X[nz - 2] - dzeta_b * Q / (dzzb * Kb));
-        __syncwarp();
-        // forward sweep over rows 0 .. nz-2: d'_k = D_k - W_k d'_{k-1} (row 0: the constant D_0)
-        Affine mine{0.0, 1.0};
-        for (int k = k0; k < min(k1, kb); ++k)
-          mine = compose(Affine{D[k], k == 0 ? 0.0 : -W[k]}, mine);
-        const Affine pre = warp_scan(mine, lane, true);
-        double y = __shfl_up_sync(0xffffffffu, pre.a, 1);   // d' of the row before this lane's first
-        if (lane == 0) y = 0.0;
-        for (int k = k0; k < min(k1, kb); ++k) {
-          y = (k == 0) ? D[0] : fma(-W[k], y, D[k]);
-          D[k] = y;
+        // right-hand side (rows 0 .. nz-2) and the forward sweep d'_k = D_k - w_k d'_{k-1}
+        double D[R], a = 0.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int k = k0 + r;
+          D[r] = k == 0 ? d_top : (k < kb ? fma(X[r], inv_dt, G[r]) : 0.0);
+          a = r == 0 ? D[r] : fma(Wn[r], a, D[r]);
         }
-        __syncwarp();
-        const double dprev = D[kb - 1];
-        // back substitution over rows nz-2 .. 0 as x_k = XB_k + SB_k x_base: each lane composes its
-        // rows (m_k: x_{k+1} -> x_k), the suffix scan gives the map from x_base to each lane's rows
-        Affine mb{0.0, 1.0};
-        for (int k = min(k1, kb) - 1; k >= k0; --k) mb = compose(Affine{D[k] * RB[k], NB[k]}, mb);
-        const Affine suf = warp_scan(mb, lane, false);
-        double sa = __shfl_down_sync(0xffffffffu, suf.a, 1), sb = __shfl_down_sync(0xffffffffu, suf.b, 1);
-        if (lane == 31) { sa = 0.0; sb = 1.0; }
-        for (int k = min(k1, kb) - 1; k >= k0; --k) {   // (sa, sb): x_base -> x_{k+1}
-          const Affine r = compose(Affine{D[k] * RB[k], NB[k]}, Affine{sa, sb});
-          XB[k] = r.a;
-          SB[k] = r.b;
-          sa = r.a;
-          sb = r.b;
+        a = fwd.scan_up(a, lane);   // d' of the lane's last row (of row nz-2 from there on)
+        if (R == 1) {
+          D[0] = a;
+        } else {
+          double y = shfl_up_d(a, 1);   // d' of the row before this lane's first
+          if (lane == 0) y = 0.0;
+#pragma unroll
+          for (int r = 0; r < R; ++r) D[r] = y = fma(Wn[r], y, D[r]);
         }
-        __syncwarp();
-        // basal values and the rows' solutions, clamped (and mixed for the subgrid condition)
-        const double x_gr = ((grounded ? d_gr : pmp_b) - W[kb] * dprev) * RB[kb];
-        const double x_fl = (pmp_b - W[kb] * dprev) * RB[kb];
-        const double x_sel = two_solves ? (d_gr - W[kb] * dprev) * RB[kb] : x_gr;
-        bool bad = false;
-        for (int k = lane; k < nz; k += 32) {
-          const double xg = (k == kb) ? x_sel : fma(SB[k], x_sel, XB[k]);
-          double v = fmin(xg, PMP[k]);
-          if (two_solves) {
-            const double xf = (k == kb) ? x_fl : fma(SB[k], x_fl, XB[k]);
-            v = fr * v + (1.0 - fr) * fmin(xf, PMP[k]);
+        const double dprev = __shfl_sync(0xffffffffu, a, 31);
+        // back substitution over rows nz-2 .. 0: x_k = A_k + B_k x_base
+        double t = 0.0;
+#pragma unroll
+        for (int r = R - 1; r >= 0; --r) {
+          D[r] = k0 + r < kb ? D[r] * RB[r] : 0.0;
+          t = r == R - 1 ? D[r] : fma(NB[r], t, D[r]);
+        }
+        t = bwd.scan_down(t, lane);
+        // basal values
+        double x_above = X[0];   // row nz-2 of the current profile
+#pragma unroll
+        for (int r = 1; r < R; ++r)
+          if ((nz - 2) % R == r) x_above = X[r];
+        x_above = __shfl_sync(0xffffffffu, x_above, (nz - 2) / R);
+        const double d_gr = min_limit(x_above - flux_b, pmp_b);
+        auto base = [&](double d) {
+          const double x = fma(-w_b, dprev, d);   // w of the base is zero: d, or NaN after an overflow
+          return unit_b ? x : x * rb_b;
+        };
+        const double x_sel = base(grounded || two_solves ? d_gr : pmp_b);
+        const double x_fl = two_solves ? base(pmp_b) : 0.0;
+        // the rows' solutions, clamped (and mixed for the subgrid condition)
+        auto rows = [&](double x_base, double *x) {
+          if (R == 1) {
+            x[0] = k0 == kb ? x_base : fma(bwd.all, x_base, t);
+          } else {
+            const double ta = shfl_down_d(t, 1), tb = shfl_down_d(bwd.all, 1);
+            double y = lane == 31 ? x_base : fma(tb, x_base, ta);   // x of the row after this lane's last
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) {
+              y = k0 + r >= kb ? x_base : fma(NB[r], y, D[r]);
+              x[r] = y;
+            }
           }
-          X[k] = v;
-          bad |= unstable_value(v);
+        };
+        double xg[R];
+        rows(x_sel, xg);
+        if (two_solves) {
+          double xf[R];
+          rows(x_fl, xf);
+#pragma unroll
+          for (int r = 0; r < R; ++r) X[r] = fr * min_limit(xg[r], PMP[r]) + (1.0 - fr) * min_limit(xf[r], PMP[r]);
+        } else {
+#pragma unroll
+          for (int r = 0; r < R; ++r) X[r] = min_limit(xg[r], PMP[r]);
         }
-        ok = !__any_sync(0xffffffffu, bad);
-        __syncwarp();
       }
-      found = ok;
+      bool bad = false;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (k0 + r < nz) bad |= unstable_value(X[r]);
+      found = !__any_sync(0xffffffffu, bad);
     }
-    for (int k = lane; k < nz; k += 32) Ti_next[(int64_t)k * nV + vi] = X[k];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (k0 + r < nz) Ti_next[(int64_t)(k0 + r) * nV + vi] = X[r];
     if (!found && lane == 0) {
       const int32_t u = atomicAdd(&cnt->n_unstable, 1);
       lists.unstable[u] = (int32_t)vi;
@@ -866,22 +934,36 @@ void reset_counters(ufe_ctx *ctx, ThermoWork *t, int64_t nV) {
   UFE_CUDA(cudaMemcpyAsync(t->cnt, t->cnt_host, sizeof(Counters), cudaMemcpyHostToDevice, ctx->stream));
 }
 
+// The retry list is short: a fixed grid of warps (4 per SM) strides over it.
+template <class In, int R>
+void launch_retry_rows(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, const VertexFields &vf, int64_t nV,
+                       double *Ti_next, const Lists &lists, Counters *cnt) {
+  const size_t smem = (size_t)kRetryArrays * z.nz * sizeof(double);
+  UFE_CUDA(cudaFuncSetAttribute(k_heat_retry<In, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_heat_retry<In, R><<<kRetryBlocks, 32, smem, s>>>(in, z, c, vf, nV, Ti_next, lists, cnt);
+  UFE_CUDA(cudaGetLastError());
+}
+template <class In>
+void launch_retry(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, const VertexFields &vf, int64_t nV,
+                  double *Ti_next, const Lists &lists, Counters *cnt) {
+  if (z.nz <= 32) launch_retry_rows<In, 1>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
+  else if (z.nz <= 64) launch_retry_rows<In, 2>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
+  else if (z.nz <= 128) launch_retry_rows<In, 4>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
+  else launch_retry_rows<In, 8>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
+}
+
 template <class In>
 void launch_step(ufe_ctx *ctx, ThermoWork *t, const In &in, const Consts &c, const VertexFields &vf, int64_t nV,
                  const double *Ti_cur, double *Ti_next) {
   const ZOps z = zops_of(t);
   const int T = threads_for(z.nz);
   const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
-  const size_t smem_retry = (size_t)kRetryArrays * z.nz * kRetryWarps * sizeof(double);
   UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  UFE_CUDA(cudaFuncSetAttribute(k_heat_retry<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_retry));
   cudaStream_t s = ctx->stream;
   const unsigned blocks = (unsigned)((nV + T - 1) / T);
   k_heat_columns<In><<<blocks, T, smem, s>>>(in, z, c, vf, nV, Ti_cur, Ti_next, t->lists, t->cnt);
   UFE_CUDA(cudaGetLastError());
-  // the retry list is short: a fixed grid of warps (4 per SM) strides over it
-  k_heat_retry<In><<<kRetryBlocks, 32 * kRetryWarps, smem_retry, s>>>(in, z, c, vf, nV, Ti_next, t->lists, t->cnt);
-  UFE_CUDA(cudaGetLastError());
+  launch_retry(s, in, z, c, vf, nV, Ti_next, t->lists, t->cnt);
   k_heat_finish<<<152, 128, 0, s>>>(z, c, vf, nV, Ti_next, t->lists, t->cnt);
   UFE_CUDA(cudaGetLastError());
   k_heat_close<<<1, 1, 0, s>>>(t->cnt);
@@ -1241,10 +1323,7 @@ extern "C" int32_t ufe_profile_heat_kernels(ufe_ctx *ctx, const ufe_thermo_param
     const ZOps z = zops_of(t);
     const int T = threads_for(z.nz);
     const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
-    const size_t smem_retry = (size_t)kRetryArrays * z.nz * kRetryWarps * sizeof(double);
-    UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<HeatMesh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    UFE_CUDA(cudaFuncSetAttribute(k_heat_retry<HeatMesh>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_retry));
+      UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<HeatMesh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t nV = t->nV;
     const unsigned blocks = (unsigned)((nV + T - 1) / T);
     reset_counters(ctx, t, nV);
@@ -1255,8 +1334,7 @@ extern "C" int32_t ufe_profile_heat_kernels(ufe_ctx *ctx, const ufe_thermo_param
         if (which == 0) {
           k_heat_columns<HeatMesh><<<blocks, T, smem, s>>>(in, z, c, vf, nV, in.Ti0, out, t->lists, t->cnt);
         } else if (which == 1) {
-          k_heat_retry<HeatMesh><<<kRetryBlocks, 32 * kRetryWarps, smem_retry, s>>>(in, z, c, vf, nV, out,
-                                                                                      t->lists, t->cnt);
+          launch_retry(s, in, z, c, vf, nV, out, t->lists, t->cnt);
         } else if (which == 2) {
           k_heat_finish<<<152, 128, 0, s>>>(z, c, vf, nV, out, t->lists, t->cnt);
         } else {
