@@ -128,12 +128,6 @@ __device__ __forceinline__ void stage_weights(uint8_t *dst, const uint16_t *__re
     *reinterpret_cast<uint4 *>(dst + kb * rows * 128 + umma::sw128_chunk(r, c)) = v;
   }
 }
-// Write this thread's row r of 64 floats (BF16) into K block `blk` of a 128-row A tile.
-__device__ __forceinline__ void stage_row64(uint8_t *tile, int r, const float *v) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(tile + umma::sw128_chunk(r, c)) = pack8(v + 8 * c);
-}
-
 struct Sync {
   uint64_t mbar;
   uint32_t tslot;
@@ -173,445 +167,598 @@ __device__ __forceinline__ void sync_teardown(Sync &sy, uint32_t phase, uint32_t
   umma::fence_after();
   if (threadIdx.x < 32) umma::tmem_dealloc(sy.tslot, tmem_cols);
 }
-// this thread's TMEM lane (row 32*warp + lane), 64 columns from `col`
-__device__ __forceinline__ void tmem_row64(uint32_t tmem, int col, float *v) {
-  const uint32_t base = tmem + ((uint32_t)(32 * (threadIdx.x >> 5)) << 16) + col;
-#pragma unroll
-  for (int c = 0; c < 64; c += 16) umma::tmem_ld16(base + c, v + c);
-}
-
 struct Graph {
   int64_t n;                     // nodes
   const int32_t *__restrict__ nbr;   // n x 3, -1: none
 };
 
-// ---- forward -----------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_gnn_encoder(Graph g, const float *__restrict__ x,
-                                                     const uint16_t *__restrict__ wbf, const float *__restrict__ prm,
-                                                     float *__restrict__ h0, int *err) {
+// decoder gradient: dWd [kGnnOut x 64] and dbd
+constexpr int kDecParts = kGnnOut * kC + kGnnOut;
+static_assert(kGnnOut * kC + 64 <= 256, "one thread of a CTA per entry of the decoder's gradient");
+
+// ---- the layer kernels ---------------------------------------------------------------------------
+// What bounds them is memory, not the tensor cores: a layer reads each node's row and its neighbours' rows
+// (256 B each, mostly L2 hits) and writes one, 30 MB per 115k nodes and layer.  So a CTA of 256 threads stays
+// resident, stages the layer's weights once and loops over 128-node tiles; rows are read and written
+// coalesced (16 lanes per row, 16 bytes each, the sums of a column always in the same thread) and pass
+// through swizzled shared memory on their way to and from the tensor cores; the CTAs on an SM overlap one
+// another's loads and MMAs.  Measured (cold caches): a forward layer on 115k nodes 34 us, where one thread per
+// row with 256-byte strides and weights staged for every tile took 118; a layer's backward pass on 60k nodes 54
+// us, where six kernels (transposing stores for the weight gradients, a serial sum of their partials) took 340;
+// the decoder inside the last layer, 32 us before.
+//
+// The backward pass of a layer is one kernel as well.  dh_out is gathered while it is loaded (the mean's
+// backward), and the weight gradients D[features x outputs] += A^T B over the tile's nodes read the same
+// tiles as the data gradients: a [node][64 features] tile is K-major for a product over features and
+// MN-major for a product over nodes (transpose bits in the instruction descriptor), so nothing is
+// transposed.  Their accumulators stay in tensor memory over all tiles of the CTA.
+constexpr int kTile = 128;
+constexpr int kGnnThreads = 256;
+constexpr int kTileBytes = kTile * 128;   // a K block: 128 rows x 64 BF16
+
+struct RowMap {   // coalesced view of a tile: this thread's float4 column and first row (rows rr + 16 m)
+  int c4, rr;
+  __device__ __forceinline__ RowMap() : c4(threadIdx.x & 15), rr(threadIdx.x >> 4) {}
+};
+// four floats as BF16 at (row r, columns 4 c4 ...) of a K block
+__device__ __forceinline__ void stage4(uint8_t *tile, int r, int c4, float4 v) {
+  *reinterpret_cast<uint2 *>(tile + umma::sw128_chunk(r, c4 >> 1) + (c4 & 1) * 8) =
+      make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+}
+// FP32 tile [128][64], float4 columns permuted so that reads by row and by column are free of conflicts
+__device__ __forceinline__ float4 *otile(uint8_t *o, int r, int c4) {
+  return reinterpret_cast<float4 *>(o + r * 256 + ((c4 ^ (r & 15)) << 4));
+}
+__device__ __forceinline__ float4 ld_row(const float *__restrict__ h, int64_t i, int c4) {
+  return __ldg(reinterpret_cast<const float4 *>(h + i * kC) + c4);
+}
+__device__ __forceinline__ float4 f4_zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ void f4_add(float4 &a, float4 b) {
+  a.x += b.x;
+  a.y += b.y;
+  a.z += b.z;
+  a.w += b.w;
+}
+// sum of the neighbours' rows (FP32, neighbour order), and their number
+__device__ __forceinline__ int neighbour_sum(const Graph &g, const float *__restrict__ h, int64_t i, int c4, float4 &a) {
+  int j[kNb], deg = 0;
+  float4 t[kNb];
+#pragma unroll
+  for (int q = 0; q < kNb; ++q) j[q] = __ldg(g.nbr + i * kNb + q);
+#pragma unroll
+  for (int q = 0; q < kNb; ++q)
+    if (j[q] >= 0) t[q] = ld_row(h, j[q], c4);
+#pragma unroll
+  for (int q = 0; q < kNb; ++q)
+    if (j[q] >= 0) {
+      f4_add(a, t[q]);
+      ++deg;
+    }
+  return deg;
+}
+__device__ __forceinline__ float4 neighbour_mean4(const Graph &g, const float *__restrict__ h, int64_t i, int c4) {
+  float4 a = f4_zero();
+  const int deg = neighbour_sum(g, h, i, c4, a);
+  if (deg > 0) {
+    const float inv = 1.0f / (float)deg;
+    a.x *= inv;
+    a.y *= inv;
+    a.z *= inv;
+    a.w *= inv;
+  }
+  return a;
+}
+// 32 TMEM columns from `col` of row 32 (warp % 4) + lane
+__device__ __forceinline__ void tmem_row32(uint32_t tmem, int col, float *v) {
+  const uint32_t base = tmem + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16) + col;
+  umma::tmem_ld16(base, v);
+  umma::tmem_ld16(base + 16, v + 16);
+}
+// the epilogue's view: this thread's row and first column
+struct EpiMap {
+  int r, col;
+  __device__ __forceinline__ EpiMap()
+      : r(32 * ((threadIdx.x >> 5) & 3) + (threadIdx.x & 31)), col(32 * (threadIdx.x >> 7)) {}
+};
+__device__ __forceinline__ void issue_commit(Sync &sy) { umma::commit(umma::smem_u32(&sy.mbar)); }
+
+__global__ void __launch_bounds__(kGnnThreads, 4) k_gnn_encoder(Graph g, const float *__restrict__ x,
+                                                                const uint16_t *__restrict__ wbf,
+                                                                const float *__restrict__ prm, float *__restrict__ h0,
+                                                                int *err) {
   extern __shared__ uint8_t smraw[];
   __shared__ Sync sy;
+  __shared__ float be[kC];
   uint8_t *sm = align1024(smraw);
-  uint8_t *sA = sm, *sB = sm + 128 * 128;
-  const int r = threadIdx.x;
-  const int64_t i = (int64_t)blockIdx.x * 128 + r;
-  float v[64];
-#pragma unroll
-  for (int k = 0; k < 64; ++k) v[k] = 0.f;
-  if (i < g.n)
-    for (int k = 0; k < kFin; ++k) v[k] = x[i * kFin + k];
-  stage_row64(sA, r, v);
+  uint8_t *sA = sm, *sB = sA + kTileBytes, *sO = sB + 64 * 128;
+  const RowMap m;
+  const EpiMap e;
+  // features 16 .. 63 of the tile stay zero
+  for (int i = threadIdx.x; i < kTileBytes / 16; i += kGnnThreads) reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0, 0, 0, 0);
   stage_weights(sB, wbf + kBfWe, kC, 1);
+  if (threadIdx.x < kC) be[threadIdx.x] = prm[kOffBe + threadIdx.x];
   sync_setup(sy, 64);
   uint32_t phase = 0;
-  smem_to_mma();
-  if (threadIdx.x == 0) {
-    umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA), umma::smem_u32(sB), 1, false);
-    umma::commit(umma::smem_u32(&sy.mbar));
-  }
-  const bool ok = mma_done(sy, phase, err);
-  if (ok) {
-    tmem_row64(sy.tslot, 0, v);
-    if (i < g.n)
-      for (int k = 0; k < kC; ++k) h0[i * kC + k] = fmaxf(v[k] + prm[kOffBe + k], 0.f);
+  bool ok = true;
+  for (int64_t i0 = (int64_t)blockIdx.x * kTile; i0 < g.n && ok; i0 += (int64_t)gridDim.x * kTile) {
+    const int rows = (int)min((int64_t)kTile, g.n - i0);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {   // 4 lanes per row of 16 features
+      const int t = threadIdx.x + q * kGnnThreads, r = t >> 2, c4 = t & 3;
+      stage4(sA, r, c4, r < rows ? __ldg(reinterpret_cast<const float4 *>(x + (i0 + r) * kFin) + c4) : f4_zero());
+    }
+    smem_to_mma();
+    if (threadIdx.x == 0) {
+      umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA), umma::smem_u32(sB), 1, false);
+      issue_commit(sy);
+    }
+    ok = mma_done(sy, phase, err);
+    if (!ok) break;
+    float v[32];
+    tmem_row32(sy.tslot, e.col, v);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k] + be[e.col + k], 0.f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      *otile(sO, e.r, e.col / 4 + k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      if (r < rows) reinterpret_cast<float4 *>(h0 + (i0 + r) * kC)[m.c4] = *otile(sO, r, m.c4);
+    }
   }
   sync_teardown(sy, phase, 64, ok);
 }
 
-// mean of the neighbours' rows (FP32, neighbour order), and the degree
-__device__ __forceinline__ int neighbour_mean(const Graph &g, const float *__restrict__ h, int64_t i, float *a) {
-#pragma unroll
-  for (int k = 0; k < kC; ++k) a[k] = 0.f;
-  int deg = 0;
-  for (int q = 0; q < kNb; ++q) {
-    const int32_t j = g.nbr[i * kNb + q];
-    if (j < 0) continue;
-    const float4 *hj = reinterpret_cast<const float4 *>(h + (int64_t)j * kC);
-#pragma unroll
-    for (int k = 0; k < kC / 4; ++k) {
-      const float4 t = hj[k];
-      a[4 * k] += t.x;
-      a[4 * k + 1] += t.y;
-      a[4 * k + 2] += t.z;
-      a[4 * k + 3] += t.w;
-    }
-    ++deg;
-  }
-  if (deg > 0) {
-    const float inv = 1.0f / (float)deg;
-#pragma unroll
-    for (int k = 0; k < kC; ++k) a[k] *= inv;
-  }
-  return deg;
-}
+// The decoder's arguments: y = Wd h + bd of the last layer's output.  With targets (training): the loss (w: per-node
+// weight divided by the batch's total weight, 0 for nodes outside the loss), dy in y's place and the
+// decoder's gradient, per CTA.
+struct DecoderArgs {
+  float *y;
+  const float *target, *w;
+  double *loss_part;
+  float *dpart;
+};
 
-__global__ void __launch_bounds__(128) k_gnn_layer_fwd(Graph g, int layer, const uint16_t *__restrict__ wbf,
-                                                       const float *__restrict__ prm, const float *__restrict__ h_in,
-                                                       float *__restrict__ h_out, uint16_t *__restrict__ t_out,
-                                                       int *err) {
+template <bool kTrain, bool kLast>
+__global__ void __launch_bounds__(kGnnThreads, 2) k_gnn_layer_fwd(Graph g, int layer, const uint16_t *__restrict__ wbf,
+                                                                  const float *__restrict__ prm,
+                                                                  const float *__restrict__ h_in,
+                                                                  float *__restrict__ h_out, uint16_t *__restrict__ t_out,
+                                                                  DecoderArgs dec, int *err) {
   extern __shared__ uint8_t smraw[];
   __shared__ Sync sy;
+  __shared__ float b1[kC], b2[kC], wd[kGnnOut * kC], bd[kGnnOut], sdy[kLast && kTrain ? kTile * kGnnOut : 1];
+  __shared__ double sloss[kLast && kTrain ? 4 : 1];
   uint8_t *sm = align1024(smraw);
-  uint8_t *sA1 = sm;                       // 128 x 128 (2 K blocks)
-  uint8_t *sB1 = sA1 + 2 * 128 * 128;      // 64 x 128
+  uint8_t *sA1 = sm;                       // 128 x 128 (2 K blocks); then the FP32 output tile
+  uint8_t *sB1 = sA1 + 2 * kTileBytes;     // 64 x 128
   uint8_t *sA2 = sB1 + 2 * 64 * 128;       // 128 x 64
-  uint8_t *sB2 = sA2 + 128 * 128;          // 64 x 64
-  const int r = threadIdx.x;
-  const int64_t i = (int64_t)blockIdx.x * 128 + r;
-  float v[64];
-  if (i < g.n) {
-    const float4 *hi = reinterpret_cast<const float4 *>(h_in + i * kC);
-#pragma unroll
-    for (int k = 0; k < kC / 4; ++k) {
-      const float4 t = hi[k];
-      v[4 * k] = t.x; v[4 * k + 1] = t.y; v[4 * k + 2] = t.z; v[4 * k + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kC; ++k) v[k] = 0.f;
-  }
-  stage_row64(sA1, r, v);
-  if (i < g.n) {
-    neighbour_mean(g, h_in, i, v);
-  } else {
-#pragma unroll
-    for (int k = 0; k < kC; ++k) v[k] = 0.f;
-  }
-  stage_row64(sA1 + 128 * 128, r, v);
+  uint8_t *sB2 = sA2 + kTileBytes;         // 64 x 64
+  const RowMap m;
+  const EpiMap e;
   stage_weights(sB1, wbf + bf_W1(layer), kC, 2);
   stage_weights(sB2, wbf + bf_W2(layer), kC, 1);
+  if (threadIdx.x < kC) {
+    b1[threadIdx.x] = prm[off_b1(layer) + threadIdx.x];
+    b2[threadIdx.x] = prm[off_b2(layer) + threadIdx.x];
+  }
+  if (kLast) {
+    if (threadIdx.x < kGnnOut * kC) wd[threadIdx.x] = prm[kOffWd + threadIdx.x];
+    if (threadIdx.x < kGnnOut) bd[threadIdx.x] = prm[kOffBd + threadIdx.x];
+  }
   sync_setup(sy, 128);
   uint32_t phase = 0;
-  smem_to_mma();
-  if (threadIdx.x == 0) {
-    umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA1), umma::smem_u32(sB1), 2, false);
-    umma::commit(umma::smem_u32(&sy.mbar));
-  }
-  bool ok = mma_done(sy, phase, err);
-  if (ok) {
-    tmem_row64(sy.tslot, 0, v);
-    const float *b1 = prm + off_b1(layer);
+  bool ok = true;
+  double loss = 0.0;
+  float dgrad = 0.f;   // kLast && kTrain: this thread's entry of the decoder's gradient
+  for (int64_t i0 = (int64_t)blockIdx.x * kTile; i0 < g.n && ok; i0 += (int64_t)gridDim.x * kTile) {
+    const int rows = (int)min((int64_t)kTile, g.n - i0);
+    float4 own[8];
 #pragma unroll
-    for (int k = 0; k < kC; ++k) v[k] = fmaxf(v[k] + b1[k], 0.f);
-    if (i < g.n) {
-      uint4 *to = reinterpret_cast<uint4 *>(t_out + i * kC);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) to[c] = pack8(v + 8 * c);
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      own[q] = r < rows ? ld_row(h_in, i0 + r, m.c4) : f4_zero();
     }
-    stage_row64(sA2, r, v);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      stage4(sA1, r, m.c4, own[q]);
+      stage4(sA1 + kTileBytes, r, m.c4, r < rows ? neighbour_mean4(g, h_in, i0 + r, m.c4) : f4_zero());
+    }
+    smem_to_mma();
+    if (threadIdx.x == 0) {
+      umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA1), umma::smem_u32(sB1), 2, false);
+      issue_commit(sy);
+    }
+    ok = mma_done(sy, phase, err);
+    if (!ok) break;
+    float v[32];
+    tmem_row32(sy.tslot, e.col, v);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k] + b1[e.col + k], 0.f);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      *reinterpret_cast<uint4 *>(sA2 + umma::sw128_chunk(e.r, e.col / 8 + c)) = pack8(v + 8 * c);
     smem_to_mma();
     if (threadIdx.x == 0) {
       umma::mma_tile<64>(sy.tslot + 64, umma::smem_u32(sA2), umma::smem_u32(sB2), 1, false);
-      umma::commit(umma::smem_u32(&sy.mbar));
+      issue_commit(sy);
     }
-    ok = mma_done(sy, phase, err);
-    if (ok) {
-      tmem_row64(sy.tslot, 64, v);
-      if (i < g.n) {
-        const float *b2 = prm + off_b2(layer);
-        const float *hi = h_in + i * kC;
-        float *ho = h_out + i * kC;
-        for (int k = 0; k < kC; ++k) ho[k] = hi[k] + (v[k] + b2[k]);
+    if (kTrain) {   // t = relu(...) for the backward pass, from the staged tile
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = threadIdx.x + q * kGnnThreads, r = t >> 3, c = t & 7;
+        if (r < rows)
+          reinterpret_cast<uint4 *>(t_out + (i0 + r) * kC)[c] =
+              *reinterpret_cast<const uint4 *>(sA2 + umma::sw128_chunk(r, c));
       }
     }
+    ok = mma_done(sy, phase, err);
+    if (!ok) break;
+    tmem_row32(sy.tslot, 64 + e.col, v);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = v[k] + b2[e.col + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      *otile(sA1, e.r, e.col / 4 + k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      float4 o = *otile(sA1, r, m.c4);
+      o = make_float4(own[q].x + o.x, own[q].y + o.y, own[q].z + o.z, own[q].w + o.w);
+      if (kLast) *otile(sA1, r, m.c4) = o;
+      else if (r < rows) reinterpret_cast<float4 *>(h_out + (i0 + r) * kC)[m.c4] = o;
+    }
+    __syncthreads();   // the tile is staged again, or read by rows
+    if (kLast) {
+      const int r = threadIdx.x;
+      if (r < kTile) {
+        float yo[kGnnOut], sc[kGnnOut];
+#pragma unroll
+        for (int c = 0; c < kGnnOut; ++c) sc[c] = 0.f;
+#pragma unroll 4
+        for (int k = 0; k < kC / 4; ++k) {
+          const float4 hv = *otile(sA1, r, k);
+#pragma unroll
+          for (int c = 0; c < kGnnOut; ++c) {
+            const float *wk = wd + c * kC + 4 * k;
+            sc[c] += wk[0] * hv.x;
+            sc[c] += wk[1] * hv.y;
+            sc[c] += wk[2] * hv.z;
+            sc[c] += wk[3] * hv.w;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kGnnOut; ++c) yo[c] = bd[c] + sc[c];
+        if (kTrain) {
+          const float wi = r < rows ? dec.w[i0 + r] : 0.f;
+#pragma unroll
+          for (int c = 0; c < kGnnOut; ++c) {
+            const float er = r < rows ? yo[c] - dec.target[kGnnOut * (i0 + r) + c] : 0.f;
+            loss += (double)wi * ((double)er * er);
+            yo[c] = 2.f * wi * er;   // dy takes y's place
+            sdy[r * kGnnOut + c] = yo[c];
+          }
+        }
+        if (r < rows)
+#pragma unroll
+          for (int c = 0; c < kGnnOut; ++c) dec.y[kGnnOut * (i0 + r) + c] = yo[c];
+      }
+      __syncthreads();   // the tile is staged again, or read for the decoder's gradient
+      if (kTrain) {
+        const int c = threadIdx.x >> 6, k = threadIdx.x & 63;
+        if (c < kGnnOut) {
+          for (int q = 0; q < rows; ++q)
+            dgrad += sdy[q * kGnnOut + c] * reinterpret_cast<const float *>(otile(sA1, q, k >> 2))[k & 3];
+        } else if (k < kGnnOut) {
+          for (int q = 0; q < rows; ++q) dgrad += sdy[q * kGnnOut + k];
+        }
+        __syncthreads();
+      }
+    }
+  }
+  if (kLast && kTrain) {
+    if (threadIdx.x < kDecParts) dec.dpart[(int64_t)blockIdx.x * kDecParts + threadIdx.x] = dgrad;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kTile) sloss[threadIdx.x >> 5] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) dec.loss_part[blockIdx.x] = (sloss[0] + sloss[1]) + (sloss[2] + sloss[3]);
   }
   sync_teardown(sy, phase, 128, ok);
 }
 
-// y = Wd h + bd; with targets: loss partials, dy and dh = Wd^T dy.  w: per-node loss weight
-// divided by the batch's total weight (0 for nodes outside the loss).
-__global__ void k_gnn_decoder(Graph g, const float *__restrict__ prm, const float *__restrict__ h,
-                              float *__restrict__ y, const float *__restrict__ target, const float *__restrict__ w,
-                              float *__restrict__ dh, double *__restrict__ loss_part) {
-  __shared__ double red[256];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double l = 0.0;
-  if (i < g.n) {
-    const float *hi = h + i * kC;
-    float yo[kGnnOut];
+// ---- backward ------------------------------------------------------------------------------------
+// What a layer's backward pass leaves per node: dh_acc and dA (what each neighbour receives through the mean); the
+// gradient that arrives at a node is dh_acc + the sum of its neighbours' dA (the adjacency is symmetric).
+struct GradIn {
+  const float *dacc, *dA;   // of the layer above; or, for the last layer,
+  const float *dy;          // the decoder's dy (then dacc and dA are null)
+};
+__device__ __forceinline__ float4 grad_row(const Graph &g, const GradIn &in, const float *wd, int64_t i, int c4) {
+  if (in.dy) {
+    float d[kGnnOut];
+#pragma unroll
+    for (int c = 0; c < kGnnOut; ++c) d[c] = __ldg(in.dy + kGnnOut * i + c);
+    float4 a = f4_zero();
 #pragma unroll
     for (int c = 0; c < kGnnOut; ++c) {
-      float sc = 0.f;
-      for (int k = 0; k < kC; ++k) sc += prm[kOffWd + c * kC + k] * hi[k];
-      yo[c] = prm[kOffBd + c] + sc;
-      y[kGnnOut * i + c] = yo[c];
+      const float4 wv = *reinterpret_cast<const float4 *>(wd + c * kC + 4 * c4);
+      f4_add(a, make_float4(wv.x * d[c], wv.y * d[c], wv.z * d[c], wv.w * d[c]));
     }
-    if (target) {
-      const float wi = w[i];
-      float d[kGnnOut];
-#pragma unroll
-      for (int c = 0; c < kGnnOut; ++c) {
-        const float e = yo[c] - target[kGnnOut * i + c];
-        l += (double)wi * ((double)e * e);
-        d[c] = 2.f * wi * e;
-      }
-      float *dhi = dh + i * kC;
-      for (int k = 0; k < kC; ++k) {
-        float a = 0.f;
-#pragma unroll
-        for (int c = 0; c < kGnnOut; ++c) a += prm[kOffWd + c * kC + k] * d[c];
-        dhi[k] = a;
-      }
-#pragma unroll
-      for (int c = 0; c < kGnnOut; ++c) y[kGnnOut * i + c] = d[c];   // dy replaces y when training
-    }
+    return a;
   }
-  if (loss_part) {
-    red[threadIdx.x] = l;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) loss_part[blockIdx.x] = red[0];
+  float4 a = ld_row(in.dacc, i, c4);
+  neighbour_sum(g, in.dA, i, c4, a);
+  return a;
+}
+
+// Weight-gradient partials per CTA: [128 features x 64 outputs] FP32, then the 64 column sums (bias).
+constexpr int kPartW = 128 * kC, kPart = kPartW + kC;
+
+// D[128 x 64] (+)= A^T B over the tile's 128 nodes: A the MN-major view of feature blocks a_stride bytes apart
+// (0: one block, twice), B of one block of 64 outputs.  One thread calls this.
+__device__ __forceinline__ void mma_wgrad(uint32_t tmem_d, uint32_t a, uint32_t a_stride, uint32_t b, bool accumulate) {
+  constexpr uint32_t idesc = umma::idesc_bf16_f32(128, kC) | (1u << 15) | (1u << 16);
+#pragma unroll
+  for (int j = 0; j < kTile / 16; ++j)
+    umma::mma_bf16(tmem_d, umma::desc_sw128_mn(a + j * 2048, a_stride), umma::desc_sw128_mn(b + j * 2048, 0), idesc,
+                   (accumulate || j > 0) ? 1u : 0u);
+}
+// this thread's half row of a weight-gradient accumulator, of the first `features` rows, to the CTA's partial
+__device__ __forceinline__ void store_partial(uint32_t tmem, const EpiMap &e, int features, float *part) {
+  float v[32];
+  tmem_row32(tmem, e.col, v);
+  if (e.r >= features) return;
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    reinterpret_cast<float4 *>(part + e.r * kC + e.col)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+}
+// column sums of the coalesced view (four columns per thread, 16 threads per column) in a fixed order
+__device__ __forceinline__ void store_column_sums(uint8_t *scratch, const RowMap &m, float4 s, float *out) {
+  float4 *red = reinterpret_cast<float4 *>(scratch);
+  __syncthreads();
+  red[m.rr * 16 + m.c4] = s;
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    float4 a = red[threadIdx.x];
+    for (int q = 1; q < 16; ++q) f4_add(a, red[q * 16 + threadIdx.x]);
+    reinterpret_cast<float4 *>(out)[threadIdx.x] = a;
   }
 }
 
-// ---- backward ------------------------------------------------------------------------------------
-// dt = dh_out W2 (masked by t > 0) -> ds; dz = ds W1 -> dh_acc = dh_out + dz[:64],
-// dA = dz[64:] / deg (what each neighbour of i receives through the mean).
-__global__ void __launch_bounds__(128) k_gnn_layer_bwd(Graph g, int layer, const uint16_t *__restrict__ wbf,
-                                                       const float *__restrict__ dh_out,
-                                                       const uint16_t *__restrict__ t_in, float *__restrict__ ds_out,
-                                                       float *__restrict__ dh_acc, float *__restrict__ dA, int *err) {
+// dt = dh_out W2 (masked by t > 0) = ds; dz = ds W1 -> dh_acc = dh_out + dz[:64], dA = dz[64:] / deg; and the
+// partials of dW2 = dh_out^T t, db2, dW1 = ds^T [h, mean], db1.
+__global__ void __launch_bounds__(kGnnThreads, 2) k_gnn_layer_bwd(Graph g, int layer, const uint16_t *__restrict__ wbf,
+                                                                  const float *__restrict__ prm, GradIn in,
+                                                                  const uint16_t *__restrict__ t_in,
+                                                                  const float *__restrict__ h_in,
+                                                                  float *__restrict__ dacc, float *__restrict__ dA,
+                                                                  float *__restrict__ part1, float *__restrict__ part2,
+                                                                  int *err) {
   extern __shared__ uint8_t smraw[];
   __shared__ Sync sy;
+  __shared__ __align__(16) float wd[kGnnOut * kC];
   uint8_t *sm = align1024(smraw);
-  uint8_t *sA = sm;                    // 128 x 64: dh_out
-  uint8_t *sB = sA + 128 * 128;        // 64 x 64: W2^T
-  uint8_t *sA2 = sB + 64 * 128;        // 128 x 64: ds
-  uint8_t *sB2 = sA2 + 128 * 128;      // 128 x 64: W1^T
-  const int r = threadIdx.x;
-  const int64_t i = (int64_t)blockIdx.x * 128 + r;
-  float v[64];
-  if (i < g.n) {
-    for (int k = 0; k < kC; ++k) v[k] = dh_out[i * kC + k];
-  } else {
-    for (int k = 0; k < kC; ++k) v[k] = 0.f;
-  }
-  stage_row64(sA, r, v);
+  uint8_t *sD = sm;                      // dh_out
+  uint8_t *sT = sD + kTileBytes;         // t; with sD the FP32 output tile later
+  uint8_t *sH = sT + kTileBytes;         // h, then the mean
+  uint8_t *sS = sH + 2 * kTileBytes;     // ds
+  uint8_t *sB = sS + kTileBytes;         // 64 x 64: W2^T
+  uint8_t *sB2 = sB + 64 * 128;          // 128 x 64: W1^T
+  const RowMap m;
+  const EpiMap e;
+  const int lane = threadIdx.x & 31;
   stage_weights(sB, wbf + bf_W2T(layer), kC, 1);
   stage_weights(sB2, wbf + bf_W1T(layer), 2 * kC, 1);
+  if (threadIdx.x < kGnnOut * kC) wd[threadIdx.x] = prm[kOffWd + threadIdx.x];
   sync_setup(sy, 256);
+  const uint32_t tD = sy.tslot, tW2 = tD + 128, tW1 = tD + 192;
   uint32_t phase = 0;
-  smem_to_mma();
-  if (threadIdx.x == 0) {
-    umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA), umma::smem_u32(sB), 1, false);
-    umma::commit(umma::smem_u32(&sy.mbar));
-  }
-  bool ok = mma_done(sy, phase, err);
-  if (ok) {
-    tmem_row64(sy.tslot, 0, v);
-    if (i < g.n) {
-      const uint16_t *ti = t_in + i * kC;
-      for (int k = 0; k < kC; ++k) {
-        const float tv = __bfloat162float(__ushort_as_bfloat16(ti[k]));
-        v[k] = tv > 0.f ? v[k] : 0.f;
-        ds_out[i * kC + k] = v[k];
-      }
-    } else {
-      for (int k = 0; k < kC; ++k) v[k] = 0.f;
+  bool ok = true, first = true;
+  float4 bias2 = f4_zero();
+  float bias1 = 0.f;   // column e.col + lane, summed over this warp's rows
+  for (int64_t i0 = (int64_t)blockIdx.x * kTile; i0 < g.n && ok; i0 += (int64_t)gridDim.x * kTile) {
+    const int rows = (int)min((int64_t)kTile, g.n - i0);
+    float4 own[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      own[q] = r < rows ? grad_row(g, in, wd, i0 + r, m.c4) : f4_zero();
+      stage4(sD, r, m.c4, own[q]);
+      f4_add(bias2, own[q]);
     }
-    stage_row64(sA2, r, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int t = threadIdx.x + q * kGnnThreads, r = t >> 3, c = t & 7;
+      *reinterpret_cast<uint4 *>(sT + umma::sw128_chunk(r, c)) =
+          r < rows ? __ldg(reinterpret_cast<const uint4 *>(t_in + (i0 + r) * kC) + c) : make_uint4(0, 0, 0, 0);
+    }
     smem_to_mma();
     if (threadIdx.x == 0) {
-      umma::mma_tile<128>(sy.tslot + 64, umma::smem_u32(sA2), umma::smem_u32(sB2), 1, false);
-      umma::commit(umma::smem_u32(&sy.mbar));
+      umma::mma_tile<64>(tD, umma::smem_u32(sD), umma::smem_u32(sB), 1, false);
+      mma_wgrad(tW2, umma::smem_u32(sT), 0, umma::smem_u32(sD), !first);
+      issue_commit(sy);
+    }
+    // the layer's input and its mean, while the first products run
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      stage4(sH, r, m.c4, r < rows ? ld_row(h_in, i0 + r, m.c4) : f4_zero());
+      stage4(sH + kTileBytes, r, m.c4, r < rows ? neighbour_mean4(g, h_in, i0 + r, m.c4) : f4_zero());
     }
     ok = mma_done(sy, phase, err);
-    if (ok) {   // tcgen05.ld is warp-collective: every thread loads, only real rows store
-      tmem_row64(sy.tslot, 64, v);
-      if (i < g.n)
-        for (int k = 0; k < kC; ++k) dh_acc[i * kC + k] = dh_out[i * kC + k] + v[k];
-      tmem_row64(sy.tslot, 128, v);
-      if (i < g.n) {
-        int deg = 0;
-        for (int q = 0; q < kNb; ++q) deg += g.nbr[i * kNb + q] >= 0;
-        const float inv = deg > 0 ? 1.0f / (float)deg : 0.f;
-        for (int k = 0; k < kC; ++k) dA[i * kC + k] = v[k] * inv;
+    if (!ok) break;
+    float v[32];
+    tmem_row32(tD, e.col, v);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {   // t > 0: a positive BF16's bits lie in 1 .. 0x7f80 (t is never NaN)
+      const uint4 tv = *reinterpret_cast<const uint4 *>(sT + umma::sw128_chunk(e.r, e.col / 8 + c));
+      const uint32_t tw[4] = {tv.x, tv.y, tv.z, tv.w};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float t = __uint_as_float(k & 1 ? tw[k >> 1] & 0xffff0000u : tw[k >> 1] << 16);
+        v[8 * c + k] = t > 0.f ? v[8 * c + k] : 0.f;
+      }
+      *reinterpret_cast<uint4 *>(sS + umma::sw128_chunk(e.r, e.col / 8 + c)) = pack8(v + 8 * c);
+    }
+    smem_to_mma();
+    if (threadIdx.x == 0) {
+      umma::mma_tile<128>(tD, umma::smem_u32(sS), umma::smem_u32(sB2), 1, false);
+      mma_wgrad(tW1, umma::smem_u32(sH), kTileBytes, umma::smem_u32(sS), !first);
+      issue_commit(sy);
+    }
+    // db1: the columns of v over the warp's 32 rows, each lane ends with one column (31 additions)
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      const bool up = lane & w;
+#pragma unroll
+      for (int k = 0; k < w; ++k) {
+        const float keep = up ? v[k + w] : v[k], send = up ? v[k] : v[k + w];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, w);
       }
     }
+    bias1 += v[0];
+    ok = mma_done(sy, phase, err);
+    if (!ok) break;
+    first = false;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {   // dz[:64], then dz[64:], through the FP32 tile (over sD, sT)
+      tmem_row32(tD, 64 * half + e.col, v);
+      if (half) __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        *otile(sD, e.r, e.col / 4 + k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      umma::fence_before();
+      __syncthreads();
+      umma::fence_after();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int r = m.rr + 16 * q;
+        float4 o = *otile(sD, r, m.c4);
+        if (r >= rows) continue;
+        if (half == 0) {
+          o = make_float4(own[q].x + o.x, own[q].y + o.y, own[q].z + o.z, own[q].w + o.w);
+          reinterpret_cast<float4 *>(dacc + (i0 + r) * kC)[m.c4] = o;
+        } else {
+          int deg = 0;
+#pragma unroll
+          for (int j = 0; j < kNb; ++j) deg += __ldg(g.nbr + (i0 + r) * kNb + j) >= 0;
+          const float inv = deg > 0 ? 1.0f / (float)deg : 0.f;
+          reinterpret_cast<float4 *>(dA + (i0 + r) * kC)[m.c4] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+        }
+      }
+    }
+    __syncthreads();   // the FP32 tile is staged again
+  }
+  float *p1 = part1 + (int64_t)blockIdx.x * kPart, *p2 = part2 + (int64_t)blockIdx.x * kPart;
+  if (ok) {   // every CTA has at least one tile
+    store_partial(tW1, e, 2 * kC, p1);
+    store_partial(tW2, e, kC, p2);
+  }
+  store_column_sums(sD, m, bias2, p2 + kPartW);
+  float *red = reinterpret_cast<float *>(sS);
+  red[threadIdx.x] = bias1;
+  __syncthreads();
+  if (threadIdx.x < kC) {   // warps 0-3 hold columns 0-31, warps 4-7 columns 32-63
+    const float *q = red + (threadIdx.x >> 5) * 128 + (threadIdx.x & 31);
+    p1[kPartW + threadIdx.x] = ((q[0] + q[32]) + q[64]) + q[96];
   }
   sync_teardown(sy, phase, 256, ok);
 }
 
-// dh_in[j] = dh_acc[j] + sum over the neighbours i of j of dA[i] (the adjacency is symmetric)
-__global__ void k_gnn_gather_bwd(Graph g, const float *__restrict__ dh_acc, const float *__restrict__ dA,
-                                 float *__restrict__ dh_in) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.n * kC) return;
-  const int64_t j = t / kC;
-  const int k = (int)(t - j * kC);
-  float s = dh_acc[t];
-  for (int q = 0; q < kNb; ++q) {
-    const int32_t i = g.nbr[j * kNb + q];
-    if (i >= 0) s += dA[(int64_t)i * kC + k];
-  }
-  dh_in[t] = s;
-}
-
-// encoder backward: ds_e = dh0 * (h0 > 0) in place
-__global__ void k_gnn_relu_bwd(int64_t total, const float *__restrict__ h0, float *__restrict__ dh0) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < total && !(h0[t] > 0.f)) dh0[t] = 0.f;
-}
-
-// Weight gradients as tensor-core reductions over nodes: D[128 x 64] += A^T B over chunks of 128
-// nodes, A = the layer input rows (up to 128 features, zero-padded), B = the output gradient rows
-// (64).  Both are transposed while staged (feature rows, node columns).  Per CTA: partial D and
-// the column sums of B (bias gradient).
-enum WgradMode { kWgEncoder = 0, kWgW1 = 1, kWgW2 = 2 };
-
-template <int MODE>
-__global__ void __launch_bounds__(128) k_gnn_wgrad(Graph g, const float *__restrict__ in0,
-                                                   const uint16_t *__restrict__ in_bf, const float *__restrict__ gout,
-                                                   float *__restrict__ part, float *__restrict__ bpart, int *err) {
+// encoder backward: ds = (the gradient at h0) * (h0 > 0); partials of dWe = ds^T x and dbe
+__global__ void __launch_bounds__(kGnnThreads, 3) k_gnn_encoder_bwd(Graph g, const float *__restrict__ x, GradIn in,
+                                                                    const float *__restrict__ h0,
+                                                                    float *__restrict__ part, int *err) {
   extern __shared__ uint8_t smraw[];
   __shared__ Sync sy;
   uint8_t *sm = align1024(smraw);
-  uint8_t *sA = sm;                    // 128 features x 128 nodes (2 K blocks of 64 nodes)
-  uint8_t *sB = sA + 2 * 128 * 128;    // 64 outputs x 128 nodes
-  const int r = threadIdx.x;
+  uint8_t *sD = sm, *sX = sD + kTileBytes;
+  const RowMap m;
+  const EpiMap e;
+  for (int i = threadIdx.x; i < kTileBytes / 16; i += kGnnThreads) reinterpret_cast<uint4 *>(sX)[i] = make_uint4(0, 0, 0, 0);
   sync_setup(sy, 64);
   uint32_t phase = 0;
-  float bsum[kC];
-  for (int k = 0; k < kC; ++k) bsum[k] = 0.f;
-  const int64_t nchunks = (g.n + 127) / 128;
-  bool ok = true;
-  bool first = true;
-  for (int64_t ch = blockIdx.x; ch < nchunks && ok; ch += gridDim.x) {
-    const int64_t i = ch * 128 + r;
-    const int kb = r >> 6, kk = r & 63;
-    uint8_t *aBase = sA + kb * 128 * 128;
-    uint8_t *bBase = sB + kb * 64 * 128;
-    float v[64];
-    // A^T column (features of node i)
-    if (MODE == kWgW1) {
-      if (i < g.n) {
-        for (int k = 0; k < kC; ++k) v[k] = in0[i * kC + k];
-      } else {
-        for (int k = 0; k < kC; ++k) v[k] = 0.f;
+  bool ok = true, first = true;
+  float4 bias = f4_zero();
+  for (int64_t i0 = (int64_t)blockIdx.x * kTile; i0 < g.n && ok; i0 += (int64_t)gridDim.x * kTile) {
+    const int rows = (int)min((int64_t)kTile, g.n - i0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = m.rr + 16 * q;
+      float4 d = f4_zero();
+      if (r < rows) {
+        d = grad_row(g, in, nullptr, i0 + r, m.c4);
+        const float4 h = ld_row(h0, i0 + r, m.c4);
+        if (!(h.x > 0.f)) d.x = 0.f;
+        if (!(h.y > 0.f)) d.y = 0.f;
+        if (!(h.z > 0.f)) d.z = 0.f;
+        if (!(h.w > 0.f)) d.w = 0.f;
       }
-      for (int f = 0; f < kC; ++f)
-        *reinterpret_cast<uint16_t *>(aBase + umma::sw128_offset(f, kk)) = bf16_bits(v[f]);
-      if (i < g.n) {
-        neighbour_mean(g, in0, i, v);
-      } else {
-        for (int k = 0; k < kC; ++k) v[k] = 0.f;
-      }
-      for (int f = 0; f < kC; ++f)
-        *reinterpret_cast<uint16_t *>(aBase + umma::sw128_offset(kC + f, kk)) = bf16_bits(v[f]);
-    } else {
-      for (int f = 0; f < 128; ++f) {
-        float x = 0.f;
-        if (i < g.n) {
-          if (MODE == kWgEncoder && f < kFin) x = in0[i * kFin + f];
-          if (MODE == kWgW2 && f < kC) x = __bfloat162float(__ushort_as_bfloat16(in_bf[i * kC + f]));
-        }
-        *reinterpret_cast<uint16_t *>(aBase + umma::sw128_offset(f, kk)) = bf16_bits(x);
-      }
+      stage4(sD, r, m.c4, d);
+      f4_add(bias, d);
     }
-    // B^T column (output gradient of node i)
-    for (int o = 0; o < kC; ++o) {
-      const float gv = i < g.n ? gout[i * kC + o] : 0.f;
-      bsum[o] += gv;
-      *reinterpret_cast<uint16_t *>(bBase + umma::sw128_offset(o, kk)) = bf16_bits(gv);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int t = threadIdx.x + q * kGnnThreads, r = t >> 2, c4 = t & 3;
+      stage4(sX, r, c4, r < rows ? __ldg(reinterpret_cast<const float4 *>(x + (i0 + r) * kFin) + c4) : f4_zero());
     }
     smem_to_mma();
     if (threadIdx.x == 0) {
-      umma::mma_tile<64>(sy.tslot, umma::smem_u32(sA), umma::smem_u32(sB), 2, !first);
-      umma::commit(umma::smem_u32(&sy.mbar));
+      mma_wgrad(sy.tslot, umma::smem_u32(sX), 0, umma::smem_u32(sD), !first);
+      issue_commit(sy);
     }
     ok = mma_done(sy, phase, err);
     first = false;
   }
-  // per-CTA partials: D (row f = input feature, column o = output), bias column sums
-  float *pd = part + (int64_t)blockIdx.x * 128 * kC;
-  if (ok) {
-    float v[64];
-    if (!first) {
-      tmem_row64(sy.tslot, 0, v);
-    } else {
-      for (int k = 0; k < kC; ++k) v[k] = 0.f;
-    }
-    for (int o = 0; o < kC; ++o) pd[(int64_t)r * kC + o] = v[o];
-  }
-  // bias partial: reduce bsum over the CTA's threads in a fixed order through shared memory
-  float *red = reinterpret_cast<float *>(sA);   // 128 x 64 floats = 32 KB, free after the MMAs
-  __syncthreads();
-  for (int o = 0; o < kC; ++o) red[r * kC + o] = bsum[o];
-  __syncthreads();
-  if (r < kC) {
-    float s = 0.f;
-    for (int t = 0; t < 128; ++t) s += red[t * kC + r];
-    bpart[(int64_t)blockIdx.x * kC + r] = s;
-  }
+  float *p = part + (int64_t)blockIdx.x * kPart;
+  if (ok) store_partial(sy.tslot, e, kFin, p);
+  store_column_sums(sD, m, bias, p + kPartW);
   sync_teardown(sy, phase, 64, ok);
 }
 
-// Sum the per-CTA partials in CTA order into the gradient vector.
-//   kWgEncoder: dWe[o][f] (f < 16) and dbe;  kWgW1: dW1[o][f] (f < 128) and db1;  kWgW2: dW2[o][f], db2.
-__global__ void k_gnn_wgrad_reduce(int mode, int layer, int nparts, const float *__restrict__ part,
-                                   const float *__restrict__ bpart, float *__restrict__ grad) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int fin = mode == kWgEncoder ? kFin : (mode == kWgW1 ? 2 * kC : kC);
-  const int wsize = kC * fin;
-  if (t < wsize) {
-    const int o = t / fin, f = t - o * fin;
-    float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += part[(int64_t)p * 128 * kC + f * kC + o];
-    const int off = mode == kWgEncoder ? kOffWe : (mode == kWgW1 ? off_W1(layer) : off_W2(layer));
-    grad[off + o * fin + f] = s;
-  } else if (t < wsize + kC) {
-    const int o = t - wsize;
-    float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += bpart[(int64_t)p * kC + o];
-    const int off = mode == kWgEncoder ? kOffBe : (mode == kWgW1 ? off_b1(layer) : off_b2(layer));
-    grad[off + o] = s;
-  }
-}
-
-// decoder gradient partials: per block, dWd[c][k] = sum_i dy_i[c] h_i[k] and dbd[c] over a fixed
-// node range; one warp per node row (lane k reads h[k], h[k+32]), warps combined in order.
-constexpr int kDecParts = kGnnOut * kC + kGnnOut;
-static_assert(kDecParts <= 256, "the decoder partials are summed by one 256-thread block");
-__global__ void k_gnn_decoder_grad(Graph g, const float *__restrict__ dy, const float *__restrict__ h,
-                                   float *__restrict__ part) {
-  __shared__ float red[8][kDecParts];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float a0[kGnnOut], a1[kGnnOut], b[kGnnOut];
-#pragma unroll
-  for (int c = 0; c < kGnnOut; ++c) a0[c] = a1[c] = b[c] = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * nw + warp; i < g.n; i += (int64_t)gridDim.x * nw) {
-    const float h0 = h[i * kC + lane], h1 = h[i * kC + lane + 32];
-#pragma unroll
-    for (int c = 0; c < kGnnOut; ++c) {
-      const float d = dy[kGnnOut * i + c];
-      a0[c] += d * h0;
-      a1[c] += d * h1;
-      b[c] += d;
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < kGnnOut; ++c) {
-    red[warp][c * kC + lane] = a0[c];
-    red[warp][c * kC + lane + 32] = a1[c];
-    if (lane == 0) red[warp][kGnnOut * kC + c] = b[c];
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < kDecParts) {
-    float s = 0.f;
-    for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
-    part[(int64_t)blockIdx.x * kDecParts + threadIdx.x] = s;
-  }
-}
-
-__global__ void k_gnn_decoder_reduce(int nparts, const float *__restrict__ part, float *__restrict__ grad) {
-  const int t = threadIdx.x;
-  if (t >= kDecParts) return;
+// Sum all CTAs' partials into the gradient vector, in a fixed order: each block takes 32 consecutive entries of one
+// of the nine [128 x 64] + 64 partial sets (0: encoder, 1 + 2l: W1 and b1, 2 + 2l: W2 and b2 of layer l) or of
+// the decoder's, its eight warps every eighth CTA, and adds the warps' sums in order.
+constexpr int kPartSets = 1 + 2 * kLayers;
+constexpr int kReduceBlocks = kPartSets * (kPart / 32) + (kDecParts + 31) / 32;
+__global__ void __launch_bounds__(256) k_gnn_reduce(int nparts, int ndec, const float *__restrict__ part,
+                                                    const float *__restrict__ dpart, float *__restrict__ grad) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int set = blockIdx.x / (kPart / 32);
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += part[(int64_t)p * kDecParts + t];
-  grad[t < kGnnOut * kC ? kOffWd + t : kOffBd + (t - kGnnOut * kC)] = s;
+  int off = -1;
+  if (set < kPartSets) {
+    const int en = (blockIdx.x % (kPart / 32)) * 32 + lane;
+    const int fin = set == 0 ? kFin : (set & 1) ? 2 * kC : kC, layer = (set - 1) >> 1;
+    const int w0 = set == 0 ? kOffWe : (set & 1) ? off_W1(layer) : off_W2(layer);
+    const int b0 = set == 0 ? kOffBe : (set & 1) ? off_b1(layer) : off_b2(layer);
+    const int f = en / kC, o = en % kC;   // en < kPartW: row f, column o
+    off = en >= kPartW ? b0 + en - kPartW : f < fin ? w0 + o * fin + f : -1;
+    const float *p = part + (int64_t)set * nparts * kPart + en;
+    if (off >= 0)
+      for (int c = warp; c < nparts; c += 8) s += __ldg(p + (int64_t)c * kPart);
+  } else {
+    const int en = (blockIdx.x - kPartSets * (kPart / 32)) * 32 + lane;
+    off = en < kGnnOut * kC ? kOffWd + en : en < kDecParts ? kOffBd + en - kGnnOut * kC : -1;
+    if (off >= 0)
+      for (int c = warp; c < ndec; c += 8) s += __ldg(dpart + (int64_t)c * kDecParts + en);
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && off >= 0) {
+    for (int q = 1; q < 8; ++q) s += red[q][lane];
+    grad[off] = s;
+  }
 }
 
 // Adam (FP32) on the flat parameter vector
@@ -716,11 +863,10 @@ struct ufe_gnn {
   int64_t cap = 0;                   // node capacity of the work buffers
   float *h[kLayers + 1] = {};
   uint16_t *t[kLayers] = {};
-  float *ds = nullptr, *dhA = nullptr, *dhB = nullptr, *dacc = nullptr, *dA = nullptr, *ybuf = nullptr;
-  float *part = nullptr, *bpart = nullptr, *dpart = nullptr;
+  float *dacc[2] = {}, *dA[2] = {}, *ybuf = nullptr;   // dacc, dA: of the layer above and of this one, in turn
+  float *part = nullptr, *dpart = nullptr;             // gradient partials per CTA
   double *loss_part = nullptr;
   double *loss_host = nullptr;       // pinned
-  int64_t loss_cap = 0;
   // scratch for explicit graphs and mesh features
   int32_t *gnbr = nullptr;
   float *gx = nullptr, *gy = nullptr, *gw = nullptr, *gmask = nullptr;
@@ -730,20 +876,22 @@ struct ufe_gnn {
 
 namespace {
 
-constexpr int kWgradBlocks = 2 * 152;
-constexpr int kDecBlocks = 152;
-constexpr size_t kSmemEncoder = 48 * 1024;      // caps residency at 4 CTAs/SM (64 TMEM columns each)
-constexpr size_t kSmemLayerFwd = 74 * 1024;     // 3 CTAs/SM x 128 columns
-constexpr size_t kSmemLayerBwd = 100 * 1024;    // 2 CTAs/SM x 256 columns
-constexpr size_t kSmemWgrad = 50 * 1024;        // 4 CTAs/SM x 64 columns
+// resident CTAs per SM, as shared memory allows (TMEM: 64, 128, 256, 64 of 512 columns each)
+constexpr int kSms = 152;
+constexpr size_t kSmemEncoder = kTileBytes + 64 * 128 + 2 * kTileBytes + 1024;
+constexpr size_t kSmemLayerFwd = 3 * kTileBytes + 3 * 64 * 128 + 1024;
+constexpr size_t kSmemLayerBwd = 5 * kTileBytes + 3 * 64 * 128 + 1024;
+constexpr size_t kSmemEncoderBwd = 2 * kTileBytes + 1024;
+constexpr int kFwdBlocks = 2 * kSms, kEncBlocks = 3 * kSms, kBwdBlocks = 2 * kSms;
+unsigned gnn_grid(int64_t n, int most) { return (unsigned)std::min<int64_t>((n + kTile - 1) / kTile, most); }
 
 void gnn_free_buffers(ufe_gnn *g) {
   for (auto &p : g->h) { dev_free(p); p = nullptr; }
   for (auto &p : g->t) { dev_free(p); p = nullptr; }
-  void *ptrs[] = {g->ds, g->dhA, g->dhB, g->dacc, g->dA, g->ybuf, g->loss_part};
-  for (void *p : ptrs) dev_free(p);
-  g->ds = g->dhA = g->dhB = g->dacc = g->dA = g->ybuf = nullptr;
-  g->loss_part = nullptr;
+  for (auto &p : g->dacc) { dev_free(p); p = nullptr; }
+  for (auto &p : g->dA) { dev_free(p); p = nullptr; }
+  dev_free(g->ybuf);
+  g->ybuf = nullptr;
   g->cap = 0;
 }
 
@@ -751,21 +899,11 @@ void gnn_ensure(ufe_gnn *g, int64_t n) {
   if (g->cap >= n) return;
   gnn_free_buffers(g);
   const size_t rows = (size_t)n * kC;
-  for (auto &p : g->h) p = (float *)dev_alloc(rows * 4);
+  for (int l = 0; l < kLayers; ++l) g->h[l] = (float *)dev_alloc(rows * 4);
   for (auto &p : g->t) p = (uint16_t *)dev_alloc(rows * 2);
-  g->ds = (float *)dev_alloc(rows * 4);
-  g->dhA = (float *)dev_alloc(rows * 4);
-  g->dhB = (float *)dev_alloc(rows * 4);
-  g->dacc = (float *)dev_alloc(rows * 4);
-  g->dA = (float *)dev_alloc(rows * 4);
+  for (auto &p : g->dacc) p = (float *)dev_alloc(rows * 4);
+  for (auto &p : g->dA) p = (float *)dev_alloc(rows * 4);
   g->ybuf = (float *)dev_alloc((size_t)n * kGnnOut * 4);
-  const int64_t nb = (n + 255) / 256;
-  g->loss_part = (double *)dev_alloc(sizeof(double) * nb);
-  if (g->loss_cap < nb) {
-    if (g->loss_host) cudaFreeHost(g->loss_host);
-    UFE_CUDA(cudaMallocHost(&g->loss_host, sizeof(double) * nb));
-    g->loss_cap = nb;
-  }
   g->cap = n;
 }
 
@@ -785,72 +923,56 @@ void set_attrs() {
   static bool done = false;
   if (done) return;
   UFE_CUDA(cudaFuncSetAttribute(k_gnn_encoder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemEncoder));
-  UFE_CUDA(cudaFuncSetAttribute(k_gnn_layer_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLayerFwd));
-  UFE_CUDA(cudaFuncSetAttribute(k_gnn_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLayerBwd));
-  UFE_CUDA(cudaFuncSetAttribute(k_gnn_wgrad<kWgEncoder>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kSmemWgrad));
-  UFE_CUDA(cudaFuncSetAttribute(k_gnn_wgrad<kWgW1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemWgrad));
-  UFE_CUDA(cudaFuncSetAttribute(k_gnn_wgrad<kWgW2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemWgrad));
+  auto smem = [](auto kern, size_t bytes) {
+    UFE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  };
+  smem(k_gnn_layer_fwd<false, false>, kSmemLayerFwd);
+  smem(k_gnn_layer_fwd<false, true>, kSmemLayerFwd);
+  smem(k_gnn_layer_fwd<true, false>, kSmemLayerFwd);
+  smem(k_gnn_layer_fwd<true, true>, kSmemLayerFwd);
+  smem(k_gnn_layer_bwd, kSmemLayerBwd);
+  smem(k_gnn_encoder_bwd, kSmemEncoderBwd);
   done = true;
 }
 
-// forward over a graph already on the device; y gets the outputs.  With targets: loss partials,
-// dy (in ybuf) and dh of the last layer (in dhA).
+// forward over a graph already on the device; ybuf gets the outputs.  With targets: loss and decoder-gradient partials,
+// dy (in ybuf) and the activations the backward pass reads.
 void gnn_forward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x, const float *target, const float *w) {
   set_attrs();
   gnn_ensure(g, gr.n);
-  const unsigned tiles = (unsigned)((gr.n + 127) / 128);
-  k_gnn_encoder<<<tiles, 128, kSmemEncoder, s>>>(gr, x, g->wbf, g->prm, g->h[0], g->err);
+  const unsigned G = gnn_grid(gr.n, kFwdBlocks);
+  k_gnn_encoder<<<gnn_grid(gr.n, kEncBlocks), kGnnThreads, kSmemEncoder, s>>>(gr, x, g->wbf, g->prm, g->h[0], g->err);
   UFE_CUDA(cudaGetLastError());
+  const DecoderArgs dec{g->ybuf, target, w, g->loss_part, g->dpart};
   for (int l = 0; l < kLayers; ++l) {
-    k_gnn_layer_fwd<<<tiles, 128, kSmemLayerFwd, s>>>(gr, l, g->wbf, g->prm, g->h[l], g->h[l + 1], g->t[l], g->err);
+    const bool last = l == kLayers - 1;
+    auto kern = target ? (last ? k_gnn_layer_fwd<true, true> : k_gnn_layer_fwd<true, false>)
+                       : (last ? k_gnn_layer_fwd<false, true> : k_gnn_layer_fwd<false, false>);
+    kern<<<G, kGnnThreads, kSmemLayerFwd, s>>>(gr, l, g->wbf, g->prm, g->h[l], last ? nullptr : g->h[l + 1], g->t[l],
+                                               dec, g->err);
     UFE_CUDA(cudaGetLastError());
   }
-  k_gnn_decoder<<<(unsigned)((gr.n + 255) / 256), 256, 0, s>>>(gr, g->prm, g->h[kLayers], g->ybuf, target, w, g->dhA,
-                                                                 target ? g->loss_part : nullptr);
-  UFE_CUDA(cudaGetLastError());
-}
-
-void wgrad(ufe_gnn *g, cudaStream_t s, const Graph &gr, int mode, int layer, const float *in0, const uint16_t *in_bf,
-           const float *gout) {
-  const int64_t nchunks = (gr.n + 127) / 128;
-  const int G = (int)std::min<int64_t>(nchunks, kWgradBlocks);
-  if (mode == kWgEncoder)
-    k_gnn_wgrad<kWgEncoder><<<G, 128, kSmemWgrad, s>>>(gr, in0, in_bf, gout, g->part, g->bpart, g->err);
-  else if (mode == kWgW1)
-    k_gnn_wgrad<kWgW1><<<G, 128, kSmemWgrad, s>>>(gr, in0, in_bf, gout, g->part, g->bpart, g->err);
-  else
-    k_gnn_wgrad<kWgW2><<<G, 128, kSmemWgrad, s>>>(gr, in0, in_bf, gout, g->part, g->bpart, g->err);
-  UFE_CUDA(cudaGetLastError());
-  const int fin = mode == kWgEncoder ? kFin : (mode == kWgW1 ? 2 * kC : kC);
-  k_gnn_wgrad_reduce<<<(kC * fin + kC + 255) / 256, 256, 0, s>>>(mode, layer, G, g->part, g->bpart, g->grad);
-  UFE_CUDA(cudaGetLastError());
 }
 
 // backward after gnn_forward with targets: the full gradient in g->grad
 void gnn_backward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x) {
-  const unsigned tiles = (unsigned)((gr.n + 127) / 128);
-  k_gnn_decoder_grad<<<kDecBlocks, 256, 0, s>>>(gr, g->ybuf, g->h[kLayers], g->dpart);
-  UFE_CUDA(cudaGetLastError());
-  k_gnn_decoder_reduce<<<1, 256, 0, s>>>(kDecBlocks, g->dpart, g->grad);   // kDecParts <= 256
-  UFE_CUDA(cudaGetLastError());
-  float *cur = g->dhA, *nxt = g->dhB;
-  for (int l = kLayers - 1; l >= 0; --l) {
-    k_gnn_layer_bwd<<<tiles, 128, kSmemLayerBwd, s>>>(gr, l, g->wbf, cur, g->t[l], g->ds, g->dacc, g->dA, g->err);
+  const int G = (int)gnn_grid(gr.n, kBwdBlocks), D = (int)gnn_grid(gr.n, kFwdBlocks);
+  auto set = [&](int q) { return g->part + (int64_t)q * G * kPart; };
+  GradIn in{nullptr, nullptr, g->ybuf};
+  for (int l = kLayers - 1, c = 0; l >= 0; --l, c ^= 1) {
+    k_gnn_layer_bwd<<<G, kGnnThreads, kSmemLayerBwd, s>>>(gr, l, g->wbf, g->prm, in, g->t[l], g->h[l], g->dacc[c],
+                                                          g->dA[c], set(1 + 2 * l), set(2 + 2 * l), g->err);
     UFE_CUDA(cudaGetLastError());
-    wgrad(g, s, gr, kWgW2, l, nullptr, g->t[l], cur);
-    wgrad(g, s, gr, kWgW1, l, g->h[l], nullptr, g->ds);
-    k_gnn_gather_bwd<<<(unsigned)((gr.n * kC + 255) / 256), 256, 0, s>>>(gr, g->dacc, g->dA, nxt);
-    UFE_CUDA(cudaGetLastError());
-    std::swap(cur, nxt);
+    in = GradIn{g->dacc[c], g->dA[c], nullptr};
   }
-  k_gnn_relu_bwd<<<(unsigned)((gr.n * kC + 255) / 256), 256, 0, s>>>(gr.n * kC, g->h[0], cur);
+  k_gnn_encoder_bwd<<<G, kGnnThreads, kSmemEncoderBwd, s>>>(gr, x, in, g->h[0], set(0), g->err);
   UFE_CUDA(cudaGetLastError());
-  wgrad(g, s, gr, kWgEncoder, 0, x, nullptr, cur);
+  k_gnn_reduce<<<kReduceBlocks, 256, 0, s>>>(G, D, g->part, g->dpart, g->grad);
+  UFE_CUDA(cudaGetLastError());
 }
 
 double gnn_loss(ufe_gnn *g, cudaStream_t s, int64_t n) {
-  const int64_t nb = (n + 255) / 256;
+  const int64_t nb = gnn_grid(n, kFwdBlocks);
   UFE_CUDA(cudaMemcpyAsync(g->loss_host, g->loss_part, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
   UFE_CUDA(cudaStreamSynchronize(s));
   double l = 0.0;
@@ -925,9 +1047,10 @@ extern "C" int32_t ufe_gnn_create(ufe_ctx *ctx, uint64_t seed, ufe_gnn **out) {
       g->v = (float *)dev_alloc(sizeof(float) * kParams);
       g->wbf = (uint16_t *)dev_alloc(sizeof(uint16_t) * kBfTotal);
       g->err = (int *)dev_alloc(sizeof(int));
-      g->part = (float *)dev_alloc(sizeof(float) * kWgradBlocks * 128 * kC);
-      g->bpart = (float *)dev_alloc(sizeof(float) * kWgradBlocks * kC);
-      g->dpart = (float *)dev_alloc(sizeof(float) * kDecBlocks * kDecParts);
+      g->part = (float *)dev_alloc(sizeof(float) * (size_t)kPartSets * kBwdBlocks * kPart);
+      g->dpart = (float *)dev_alloc(sizeof(float) * kFwdBlocks * kDecParts);
+      g->loss_part = (double *)dev_alloc(sizeof(double) * kFwdBlocks);
+      UFE_CUDA(cudaMallocHost(&g->loss_host, sizeof(double) * kFwdBlocks));
       cudaStream_t s = ctx->stream;
       const std::vector<float> p = init_params(seed);
       UFE_CUDA(cudaMemcpyAsync(g->prm, p.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice, s));
@@ -960,7 +1083,7 @@ extern "C" void ufe_gnn_destroy(ufe_gnn *g) {
     dev_free(m.w);
   }
   gnn_free_buffers(g);
-  void *ptrs[] = {g->prm, g->grad, g->m, g->v, g->wbf, g->err, g->part, g->bpart, g->dpart,
+  void *ptrs[] = {g->prm, g->grad, g->m, g->v, g->wbf, g->err, g->part, g->dpart, g->loss_part,
                   g->gnbr, g->gx, g->gy, g->gw, g->gmask};
   for (void *p : ptrs) dev_free(p);
   if (g->loss_host) cudaFreeHost(g->loss_host);
@@ -1181,10 +1304,10 @@ extern "C" int32_t ufe_gnn_evaluate(ufe_gnn *g, double *mean_loss) {
 // neighbours take the prediction's small-scale noise out first.  With `with_viscosity` the
 // predicted vertically averaged viscosity is stored on the vertices as well and the next solve's
 // first Picard iteration uses it in place of Glen's law (SSA: the viscosity; DIVA: every layer).
-// Kernels one prediction launches: graph, features, encoder, the layers, decoder, velocity store,
+// Kernels one prediction launches: graph, features, encoder, the layers (the last with the decoder), velocity store,
 // two per smoothing pass, and the viscosity store.
 extern "C" int32_t ufe_gnn_predict_kernels(int32_t smooth_passes) {
-  return 1 + 1 + (2 + kLayers) + 1 + 2 * (smooth_passes > 0 ? smooth_passes : 0);
+  return 1 + 1 + (1 + kLayers) + 1 + 2 * (smooth_passes > 0 ? smooth_passes : 0);
 }
 
 extern "C" int32_t ufe_gnn_predict_start(ufe_gnn *g, ufe_ctx *mesh_ctx, int32_t use_prev_velocity,

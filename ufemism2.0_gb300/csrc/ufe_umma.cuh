@@ -45,6 +45,18 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
   return d;
 }
 
+// The same for an MN-major operand: a [K rows][64 elements] tile with the 128-byte swizzle, 8-row groups 1024 B
+// apart (stride byte offset), blocks of 64 elements `block_stride` bytes apart (leading byte offset).
+__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t block_stride) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)((block_stride >> 4) & 0x3FFF) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
 // Instruction descriptor for kind::f16: FP32 accumulator (bits 4-5 = 1), BF16 A and B (bits 7-9,
 // 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
