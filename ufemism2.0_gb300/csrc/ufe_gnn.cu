@@ -135,6 +135,7 @@ struct Sync {
 
 // CTA-wide: make staged shared memory visible to the tensor core and order it before the MMA
 __device__ __forceinline__ void smem_to_mma() {
+  __syncwarp();   // per-row conditions came before
   umma::fence_smem_async();
   umma::fence_before();
   __syncthreads();
@@ -482,21 +483,21 @@ struct GradIn {
   const float *dacc, *dA;   // of the layer above; or, for the last layer,
   const float *dy;          // the decoder's dy (then dacc and dA are null)
 };
-__device__ __forceinline__ float4 grad_row(const Graph &g, const GradIn &in, const float *wd, int64_t i, int c4) {
-  if (in.dy) {
-    float d[kGnnOut];
-#pragma unroll
-    for (int c = 0; c < kGnnOut; ++c) d[c] = __ldg(in.dy + kGnnOut * i + c);
-    float4 a = f4_zero();
-#pragma unroll
-    for (int c = 0; c < kGnnOut; ++c) {
-      const float4 wv = *reinterpret_cast<const float4 *>(wd + c * kC + 4 * c4);
-      f4_add(a, make_float4(wv.x * d[c], wv.y * d[c], wv.z * d[c], wv.w * d[c]));
-    }
-    return a;
-  }
+__device__ __forceinline__ float4 grad_gather(const Graph &g, const GradIn &in, int64_t i, int c4) {
   float4 a = ld_row(in.dacc, i, c4);
   neighbour_sum(g, in.dA, i, c4, a);
+  return a;
+}
+__device__ __forceinline__ float4 grad_decoder(const GradIn &in, const float *wd, int64_t i, int c4) {
+  float d[kGnnOut];
+#pragma unroll
+  for (int c = 0; c < kGnnOut; ++c) d[c] = __ldg(in.dy + kGnnOut * i + c);
+  float4 a = f4_zero();
+#pragma unroll
+  for (int c = 0; c < kGnnOut; ++c) {
+    const float4 wv = *reinterpret_cast<const float4 *>(wd + c * kC + 4 * c4);
+    f4_add(a, make_float4(wv.x * d[c], wv.y * d[c], wv.z * d[c], wv.w * d[c]));
+  }
   return a;
 }
 
@@ -571,7 +572,8 @@ __global__ void __launch_bounds__(kGnnThreads, 2) k_gnn_layer_bwd(Graph g, int l
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int r = m.rr + 16 * q;
-      own[q] = r < rows ? grad_row(g, in, wd, i0 + r, m.c4) : f4_zero();
+      own[q] = f4_zero();
+      if (r < rows) own[q] = in.dy ? grad_decoder(in, wd, i0 + r, m.c4) : grad_gather(g, in, i0 + r, m.c4);
       stage4(sD, r, m.c4, own[q]);
       f4_add(bias2, own[q]);
     }
@@ -631,8 +633,8 @@ __global__ void __launch_bounds__(kGnnThreads, 2) k_gnn_layer_bwd(Graph g, int l
     first = false;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {   // dz[:64], then dz[64:], through the FP32 tile (over sD, sT)
+      if (half) __syncthreads();             // the first half has been read, and the warps are whole again
       tmem_row32(tD, 64 * half + e.col, v);
-      if (half) __syncthreads();
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         *otile(sD, e.r, e.col / 4 + k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
@@ -643,11 +645,10 @@ __global__ void __launch_bounds__(kGnnThreads, 2) k_gnn_layer_bwd(Graph g, int l
       for (int q = 0; q < 8; ++q) {
         const int r = m.rr + 16 * q;
         float4 o = *otile(sD, r, m.c4);
-        if (r >= rows) continue;
-        if (half == 0) {
+        if (r < rows && half == 0) {
           o = make_float4(own[q].x + o.x, own[q].y + o.y, own[q].z + o.z, own[q].w + o.w);
           reinterpret_cast<float4 *>(dacc + (i0 + r) * kC)[m.c4] = o;
-        } else {
+        } else if (r < rows) {
           int deg = 0;
 #pragma unroll
           for (int j = 0; j < kNb; ++j) deg += __ldg(g.nbr + (i0 + r) * kNb + j) >= 0;
@@ -696,7 +697,7 @@ __global__ void __launch_bounds__(kGnnThreads, 3) k_gnn_encoder_bwd(Graph g, con
       const int r = m.rr + 16 * q;
       float4 d = f4_zero();
       if (r < rows) {
-        d = grad_row(g, in, nullptr, i0 + r, m.c4);
+        d = grad_gather(g, in, i0 + r, m.c4);
         const float4 h = ld_row(h0, i0 + r, m.c4);
         if (!(h.x > 0.f)) d.x = 0.f;
         if (!(h.y > 0.f)) d.y = 0.f;

@@ -956,20 +956,22 @@ __device__ __forceinline__ int slot_index(int k, int b, int c) {
 }
 // Waits for this exchange's words, two 16-byte items per thread at a time (one after the other, the second's
 // round trip follows the first's): all blocks' np partials to sp[k * kHaloMaxBlocks + block] (shared memory),
-// and the entries of the nhalo rows hg[] of `rows` to halo[].  False after a timeout.
+// and (kHalo) the entries of the nhalo rows hg[] of `rows` to halo[].  False after a timeout.
+template <bool kHalo>
 __device__ __forceinline__ bool exchange_wait(int np, const ExSlot *slots, double *sp, const ExRow *rows,
                                               const int *hg, int nhalo, double *halo, unsigned int stamp,
                                               GridSync *gs) {
-  const int ns = np * kHaloMaxBlocks, n = ns + 2 * nhalo, G = (int)gridDim.x;
+  const int ns = np * kHaloMaxBlocks, n = kHalo ? ns + 2 * nhalo : ns, G = (int)gridDim.x;
   slots += slot_index(0, 0, (int)blockIdx.x % kReplicas);
   bool ok = true;
   // item t: slot t = k * kHaloMaxBlocks + block, then halo row (t - ns) / 2's halves; null: nothing to wait for
   auto item = [&](int t) -> const void * {
     if (t < ns) return t % kHaloMaxBlocks < G ? (const void *)(slots + t) : nullptr;
+    if (!kHalo) return nullptr;
     return t < n ? (const void *)(rows[hg[(t - ns) >> 1]].w + 2 * ((t - ns) & 1)) : nullptr;
   };
   auto put = [&](int t, unsigned long long a, unsigned long long b) {
-    (t < ns ? sp : halo - ns)[t] = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+    (!kHalo || t < ns ? sp : halo - ns)[t] = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
   };
 #pragma unroll 1
   for (int t = threadIdx.x; t < n; t += 2 * (int)blockDim.x) {
@@ -1344,7 +1346,7 @@ __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> 
       }
       ++stamp;
       block_publish<true>(1, acc, nact, scratch, slotP, stamp);
-      ok = exchange_wait(1, slotP, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
+      ok = exchange_wait<false>(1, slotP, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
       fence_acq_rel_gpu();
       if (!(ok = __syncthreads_and(ok) != 0)) break;
       after_exchange(ph, sp, false);
@@ -1376,7 +1378,7 @@ __global__ void __launch_bounds__(kPersistThreads) k_bicgstab_halo(HaloMat<Blk> 
       }
       ++stamp;
       block_publish<true>(5, acc, nact, scratch, slotS, stamp);
-      ok = exchange_wait(5, slotS, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
+      ok = exchange_wait<false>(5, slotS, sp, nullptr, nullptr, 0, nullptr, stamp, gs);
       fence_acq_rel_gpu();
       if (!(ok = __syncthreads_and(ok) != 0)) break;
       after_exchange(ph, sp, true);
@@ -1613,7 +1615,7 @@ __global__ void __launch_bounds__(NT, 1) k_bicgstab_resident(HaloMat<Blk> m, KV<
     const int np = s_phase ? 5 : 1;
     block_publish<false>(np, acc, own, scratch, s_phase ? slotS : slotP, stamp);
     if (mine && s_phase) x1 = v_axpy(sx[tid], ph.rs()[2], p);   // half of the x update, while the sums travel
-    ok = exchange_wait(np, s_phase ? slotS : slotP, sp, s_phase ? xt : xv, hg, nhalo,
+    ok = exchange_wait<true>(np, s_phase ? slotS : slotP, sp, s_phase ? xt : xv, hg, nhalo,
                        reinterpret_cast<double *>(s_phase ? ht : hv), stamp, gs);
     if (!(ok = __syncthreads_and(ok) != 0)) break;
     after_exchange(ph, sp, s_phase);

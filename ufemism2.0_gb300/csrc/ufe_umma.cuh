@@ -105,17 +105,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
 
 // TMEM allocation by one full warp; the base address is written to *slot (shared memory)
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
+  __syncwarp();   // warp-collective, as the load below
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane (warp w reads lanes 32(w%4) .. +31)
+// 16 consecutive FP32 columns of this thread's TMEM lane (warp w reads lanes 32(w%4) .. +31).  The load is
+// warp-collective (.sync.aligned): executed by a diverged warp it is an illegal instruction, so the lanes are
+// brought together first, whatever per-row conditions came before.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
