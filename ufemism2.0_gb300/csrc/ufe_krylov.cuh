@@ -1637,3 +1637,264 @@ __global__ void __launch_bounds__(NT, 1) k_bicgstab_resident(HaloMat<Blk> m, KV<
   }
   persist_close(ph.s, ok, ks, gs, stamp);
 }
+
+// ---- scalar CSR systems (solve_matrix_equation_CSR_PETSc, the ice-thickness step) --------------------------
+// BiCGStab for a caller's matrix as one persistent launch.  There are no patches here, so p and s travel as
+// stamped words (ExSlot) that the products' gathers wait for one by one: no barrier stands between forming a
+// vector and multiplying by it, and no fence.  An iteration waits for its three sums only.
+//
+// The sums have the order of the kernels this replaces (k_p_spmv, k_s_spmv, k_xr with their last-block sums), so
+// the iterates are the same to the bit: the rows belong to `nvirt` virtual blocks of 256 threads, row
+// 256 b + t (+ 256 nvirt k) to thread t of virtual block b; 256 values are summed as warp butterflies, then a
+// butterfly over the eight warps; the virtual blocks' sums are summed as values t, t + 256, ... of 256 threads
+// in the same way.  A block of 256 q threads runs q virtual blocks at a time.
+//
+// What bounds it: latency (three exchanges of ~3,000 cycles, two gathers, the FP64 sums and scalars), and the
+// FP64 pipe for large systems.  A whole ufe_solve_csr of 60,000 rows of five entries: 3.1 ms, 5.8 ms with five
+// kernels an iteration (each ends in a last block's serial sums, 10 to 16 us however small the system) and a host
+// check every eight; the thickness step on 1.05M vertices: 2.58 ms, 2.83 ms with the kernels in a graph.
+constexpr int kMaxVirt = 8 * 152;
+constexpr int kCsrSums = 3;
+constexpr size_t kCsrSet = (size_t)kReplicas * kCsrSums * kMaxVirt;   // slots of one exchange; two sets in turn
+
+__device__ __forceinline__ ExSlot *csr_slot(ExSlot *set, int k, int b, int c) {
+  return set + ((size_t)c * kCsrSums + k) * kMaxVirt + b;
+}
+// The sums of up to three values over the 256 threads of this thread's virtual block, as 8-lane groups of its first
+// warp: lane 8 k + w of it returns value k's sum, for every w.  red: 32 doubles per virtual block of the block.
+__device__ __forceinline__ double virt_sum(int np, double a, double b, double c, double *red) {
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 7, sub = threadIdx.x >> 8;
+  double v;
+  if (np == 1) {
+    v = a + __shfl_xor_sync(0xffffffffu, a, 16);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+  } else {
+    // two or three butterflies in one: after these steps lanes 0-7 carry a, 16-23 b and, of three, 8-15 and 24-31 c
+    const bool up = lane & 16, mid = lane & 8;
+    v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+    if (np == 3) {
+      const double x = c + __shfl_xor_sync(0xffffffffu, c, 16);
+      v = (mid ? x : v) + __shfl_xor_sync(0xffffffffu, mid ? v : x, 8);
+    } else {
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+    }
+  }
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  double *r = red + 32 * sub;
+  if (lane == 0) r[w] = v;
+  if (np > 1 && lane == 16) r[8 + w] = v;
+  if (np == 3 && lane == 8) r[16 + w] = v;
+  asm volatile("bar.sync %0, 256;" ::"r"(1 + sub) : "memory");   // the virtual block's warps
+  double t = 0.0;
+  if (w == 0) {
+    t = r[lane];   // (lanes of values that are not asked for: unused)
+    t += __shfl_xor_sync(0xffffffffu, t, 4);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+  }
+  return t;
+}
+// Waits for all virtual blocks' np sums and leaves the totals in tot[0 .. np); false (block-uniform) on a timeout.
+__device__ __forceinline__ bool csr_exchange(int np, int nvirt, ExSlot *set, unsigned int stamp, GridSync *gs,
+                                             double *sp, double *red, double *tot) {
+  bool ok = true;
+  const ExSlot *mine = csr_slot(set, 0, 0, (int)blockIdx.x % kReplicas);
+  const int n = np * nvirt;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const int k = t / nvirt, b = t - k * nvirt;
+    unsigned long long lo, hi;
+    unsigned int polls = 0;
+    for (;;) {
+      ld_words(mine + k * kMaxVirt + b, lo, hi);
+      if (stamped(lo, stamp) && stamped(hi, stamp)) break;
+      if (poll_expired(polls, gs)) {
+        ok = false;
+        break;
+      }
+    }
+    sp[k * kMaxVirt + b] = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
+  }
+  if (!__syncthreads_and(ok)) return false;
+  if (threadIdx.x < 256) {
+    double v[kCsrSums] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int b = threadIdx.x; b < ((nvirt + 255) & ~255); b += 256)
+#pragma unroll
+      for (int k = 0; k < kCsrSums; ++k)
+        if (k < np) v[k] = b < nvirt ? v[k] + sp[k * kMaxVirt + b] : v[k];
+    const double t = virt_sum(np, v[0], v[1], v[2], red);
+    if (threadIdx.x < 8 * np && (threadIdx.x & 7) == 0) tot[threadIdx.x >> 3] = t;
+  }
+  __syncthreads();
+  return true;
+}
+
+// Row i times the vector of stamped words `in`, in storage order, four gathers in flight.
+__device__ __forceinline__ double csr_row(const CsrMat &mat, int i, const ExSlot *in, unsigned int stamp, GridSync *gs,
+                                          bool &ok) {
+  double y = 0.0;
+  const int k2 = __ldg(mat.ptr + i + 1);
+#pragma unroll 1
+  for (int k = __ldg(mat.ptr + i); k < k2; k += 4) {
+    unsigned long long lo[4], hi[4];
+    double a[4];
+    int c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int q = min(k + j, k2 - 1);
+      c[j] = __ldg(mat.col + q);
+      a[j] = __ldg(mat.val + q);
+    }
+    unsigned int polls = 0;
+    for (;;) {
+      bool all = true;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ld_words(in + c[j], lo[j], hi[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) all = all && stamped(lo[j], stamp) && stamped(hi[j], stamp);
+      if (all) break;
+      if (poll_expired(polls, gs)) {
+        ok = false;
+        break;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k + j < k2) y = fma(a[j], __longlong_as_double((long long)((lo[j] & 0xffffffffull) | (hi[j] << 32))), y);
+  }
+  return y;
+}
+
+template <class M>
+__global__ void __launch_bounds__(kPersistThreads) k_csr_persist(M mat, int nvirt, KV<typename M::Vec> v,
+                                                                 KrylovScalars *ks, ExSlot *pw, ExSlot *sw,
+                                                                 ExSlot *slots, GridSync *gs) {
+  __shared__ PhaseScalars<double> ph;
+  __shared__ double sp[kCsrSums * kMaxVirt];
+  __shared__ double red[32 * kPersistThreads / 256];
+  if (threadIdx.x == 0) ph.open(ks);
+  __syncthreads();
+  if (!ph.s.active) return;
+  unsigned int stamp = *((volatile unsigned int *)&gs->gen);
+  const int lane = threadIdx.x & 31, q = blockDim.x >> 8, sub = threadIdx.x >> 8;
+  const int64_t gstride = (int64_t)nvirt * 256;
+  double *P = v.P[0], *V = v.V[0];
+  bool ok = true;
+  int phase = 0;   // 0: p, v, alpha;  1: s, t, omega;  2: x, r, rho
+  // every row of every virtual block of this block: body(row); once per virtual block afterwards: done(index)
+  auto each_row = [&](auto &&body, auto &&done) {
+#pragma unroll 1
+    for (int b0 = blockIdx.x * q; b0 < nvirt; b0 += gridDim.x * q) {
+      const int b = b0 + sub;
+      if (b < nvirt)
+#pragma unroll 1
+        for (int64_t i = (int64_t)b * 256 + (threadIdx.x & 255); i < mat.items; i += gstride) body((int)i);
+      done(b);
+    }
+  };
+#pragma unroll 1
+  for (;;) {
+    ++stamp;
+    ExSlot *set = slots + (stamp & 1u) * kCsrSet;
+    const double beta = ph.rs()[0], bw = ph.rs()[1], alpha = ph.rs()[2], omega = ph.rs()[3];
+    const int np = phase == 0 ? 1 : phase == 1 ? 3 : 2;
+    if (phase < 2)
+      each_row(
+          [&](int i) {
+            double x;
+            if (phase == 0) {
+              x = v_pupd(v.R[i], bw, V[i], beta, P[i]);
+              P[i] = x;
+            } else {
+              x = v_sub_scaled(v.R[i], alpha, V[i]);
+              v.S[i] = x;
+            }
+            slot_publish((phase == 0 ? pw : sw) + i, x, stamp);
+          },
+          [](int) {});
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    each_row(
+        [&](int i) {
+          if (phase == 0) {
+            const double vn = v_mul(v.dinv[i], csr_row(mat, i, pw, stamp, gs, ok));
+            V[i] = vn;
+            a0 += v_dot(vn, v.RP[i]);
+          } else if (phase == 1) {
+            const double si = v.S[i], ti = v_mul(v.dinv[i], csr_row(mat, i, sw, stamp, gs, ok));
+            v.T[i] = ti;
+            a0 += v_dot(si, ti);
+            a1 += v_dot(ti, ti);
+            a2 += v_dot(si, si);
+          } else {
+            const double si = v.S[i], ri = v_sub_scaled(si, omega, v.T[i]);
+            v.X[i] = v_xupd(v.X[i], alpha, P[i], omega, si);
+            v.R[i] = ri;
+            a0 += v_dot(ri, v.RP[i]);
+            a1 += v_dot(ri, ri);
+          }
+        },
+        [&](int b) {
+          const double t = virt_sum(np, a0, a1, a2, red);
+          if (((threadIdx.x >> 5) & 7) == 0 && lane < 8 * np && b < nvirt)
+            slot_publish(csr_slot(set, lane >> 3, b, lane & 7), t, stamp);
+          a0 = a1 = a2 = 0.0;
+          __syncthreads();   // red is used again
+        });
+    if (!(ok = __syncthreads_and(ok) != 0)) break;
+    if (!(ok = csr_exchange(np, nvirt, set, stamp, gs, sp, red, ph.tot))) break;
+    if (warp_index() == 0) {
+      KrylovScalars &s = ph.s;
+      const double t0 = ph.tot[0], t1 = ph.tot[1], t2 = ph.tot[2];
+      if (phase == 0) {
+        const bool nan = bits_nan(t0), stop = nan || bits_zero(t0);
+        const double al = fp64_div(s.rho, t0);
+        if (lane == 0) {
+          if (stop) {
+            s.status = nan ? UFE_ERR_NAN : UFE_ERR_DIVERGED;
+            s.active = 0;
+          } else {
+            s.alpha = al;
+            ph.rs()[2] = al;
+          }
+        }
+      } else if (phase == 1) {
+        const bool zero = bits_zero(t1), nan = bits_nan(t1), fail = (zero && !bits_zero(t2)) || nan;
+        const double om = zero ? 0.0 : fp64_div(t0, t1);
+        if (lane == 0) {
+          if (fail) {
+            s.status = zero ? UFE_ERR_DIVERGED : UFE_ERR_NAN;
+            s.active = 0;
+          } else {
+            s.omega = om;
+            s.tbreak = zero;
+            ph.rs()[3] = om;
+          }
+        }
+      } else {
+        const double quo = fp64_div(lane == 0 ? t0 : s.alpha, lane == 0 ? s.rho : omega);
+        const double be = __shfl_sync(0xffffffffu, quo, 0) * __shfl_sync(0xffffffffu, quo, 1);
+        if (lane == 0) {
+          s.it += 1;
+          s.total_its += 1;
+          s.rhoold = s.rho;
+          s.omegaold = omega;
+          s.rho = t0;
+          ph.res2 = t1;
+          if (s.tbreak || s.it >= s.max_it || bits_zero(t0) || bits_le(t1, ph.lo2) || bits_le(ph.hi2, t1))
+            stop_tests(ph, t1, t0, s.tbreak != 0);
+          s.beta = be;
+          ph.rs()[0] = be;
+          ph.rs()[1] = be * omega;
+        }
+      }
+    }
+    __syncthreads();
+    if (!ph.s.active) break;
+    phase = phase == 2 ? 0 : phase + 1;
+  }
+  if (threadIdx.x == 0 && ok && phase < 2 && ph.s.it > 0) ph.s.dp = sqrt(ph.res2);   // stopped between two norms
+  persist_close(ph.s, ok, ks, gs, stamp);
+}

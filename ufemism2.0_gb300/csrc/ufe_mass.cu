@@ -343,7 +343,7 @@ MassWork *mass_work(ufe_ctx *ctx) {
 template <class T>
 T *alloc_n(size_t n) { return (T *)dev_alloc(sizeof(T) * (n ? n : 1)); }
 
-void alloc_fields(MassWork *w) {
+void alloc_fields(MassWork *w, cudaStream_t s) {
   const size_t nV = w->nV, nT = w->nTri;
   double **vs[] = {&w->Hi, &w->Hb, &w->SL, &w->SMB, &w->BMB, &w->LMB, &w->fm, &w->target, &w->prHi, &w->dprev,
                    &w->dHdt, &w->Hit, &w->divQ, &w->AMB, &w->dex, &w->Hex, &w->qex, &w->aex, &w->Hs, &w->Hs_tot,
@@ -359,7 +359,7 @@ void alloc_fields(MassWork *w) {
   w->flag = alloc_n<int32_t>(1);
   w->valM = alloc_n<double>(w->nnz);
   w->valA = alloc_n<double>(w->nnz);
-  csr_scratch_alloc(w->krylov, w->nV);
+  csr_scratch_alloc(w->krylov, w->nV, s);
   w->stage = alloc_n<double>(std::max(nV, nT));
   w->stagei = alloc_n<int32_t>(nV);
 }
@@ -552,7 +552,7 @@ extern "C" int32_t ufe_mesh_voronoi_upload(ufe_ctx *ctx, const double *A, const 
     w->ind = alloc_n<int32_t>(w->nnz);
     UFE_CUDA(cudaMemcpyAsync(w->ptr, ptr.data(), sizeof(int32_t) * (w->nV + 1), cudaMemcpyHostToDevice, s));
     UFE_CUDA(cudaMemcpyAsync(w->ind, ind.data(), sizeof(int32_t) * w->nnz, cudaMemcpyHostToDevice, s));
-    alloc_fields(w);
+    alloc_fields(w, s);
     UFE_CUDA(cudaStreamSynchronize(s));
     return UFE_OK;
   });

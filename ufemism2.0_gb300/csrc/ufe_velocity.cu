@@ -2964,14 +2964,8 @@ extern "C" int32_t ufe_profile_krylov_kernels(ufe_ctx *ctx, int32_t precision, i
   });
 }
 
-// General CSR matrix-equation solve (solve_matrix_equation_CSR_PETSc): same BiCGStab kernels on
-// scalar rows, host-checked every few iterations.
-static uint64_t bits_of_double(double d) {
-  uint64_t u;
-  memcpy(&u, &d, sizeof(u));
-  return u;
-}
-
+// General CSR matrix-equation solve (solve_matrix_equation_CSR_PETSc): BiCGStab on scalar rows as one persistent
+// launch (k_csr_persist); with UFE_NO_PERSIST=1 five kernels per iteration, host-checked every eight.
 // inverse diagonal of a CSR matrix: the row's diagonal entries summed in storage order
 __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const double *val, double *dinv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2982,17 +2976,22 @@ __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const 
   dinv[i] = d != 0.0 ? 1.0 / d : 1.0;
 }
 
-void csr_scratch_alloc(CsrSolveScratch &scr, int64_t m) {
+void csr_scratch_alloc(CsrSolveScratch &scr, int64_t m, cudaStream_t s) {
   scr.vec = (double *)dev_alloc(sizeof(double) * (size_t)m * 10);
   scr.ks = (KrylovScalars *)dev_alloc(sizeof(KrylovScalars));
+  scr.slots = (ExSlot *)dev_alloc(sizeof(ExSlot) * (2 * kCsrSet + 2 * (size_t)m));
+  scr.gsync = (GridSync *)dev_alloc(sizeof(GridSync));
+  UFE_CUDA(cudaMemsetAsync(scr.slots, 0, sizeof(ExSlot) * (2 * kCsrSet + 2 * (size_t)m), s));
+  UFE_CUDA(cudaMemsetAsync(scr.gsync, 0, sizeof(GridSync), s));
   UFE_CUDA(cudaMallocHost(&scr.hks, sizeof(KrylovScalars)));
   scr.cap = m;
 }
 
 void csr_scratch_free(CsrSolveScratch &scr) {
-  if (scr.graph) cudaGraphExecDestroy(scr.graph);
   dev_free(scr.vec);
   dev_free(scr.ks);
+  dev_free(scr.slots);
+  dev_free(scr.gsync);
   if (scr.hks) cudaFreeHost(scr.hks);
   scr = CsrSolveScratch{};
 }
@@ -3003,7 +3002,7 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
   const int m = A.m;
   CsrSolveScratch own;
   const bool owned = !(scratch && scratch->cap >= m);
-  if (owned) csr_scratch_alloc(own, m);
+  if (owned) csr_scratch_alloc(own, m, s);
   CsrSolveScratch &scr = owned ? own : *scratch;
   double *vec = scr.vec;
   KrylovScalars *ks = scr.ks;
@@ -3012,63 +3011,6 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
   try {
     double *dinv = vec, *R = vec + m, *RP = R + m, *S = RP + m, *T = S + m, *P0 = T + m, *P1 = P0 + m,
            *V0 = P1 + m, *V1 = V0 + m;
-    const char *ng = getenv("UFE_NO_GRAPH");
-    if (!owned && !(ng && *ng && *ng != '0')) {
-      // a caller that solves repeatedly on the same buffers: the whole solve as one graph, its
-      // iteration loop a conditional while-node that k_xr keeps open (built once per buffers,
-      // sizes and tolerances; the host waits once, at the end)
-      uint64_t key = 1469598103934665603ull;
-      const uint64_t parts[] = {(uint64_t)(uintptr_t)A.ptr, (uint64_t)(uintptr_t)A.ind, (uint64_t)(uintptr_t)A.val,
-                                (uint64_t)(uintptr_t)b, (uint64_t)(uintptr_t)x, (uint64_t)m, (uint64_t)A.nnz,
-                                (uint64_t)bits_of_double(rtol), (uint64_t)bits_of_double(abstol),
-                                (uint64_t)max_it};
-      for (uint64_t q : parts) { key ^= q; key *= 1099511628211ull; }
-      if (!scr.graph || scr.key != key) {
-        if (scr.graph) { cudaGraphExecDestroy(scr.graph); scr.graph = nullptr; }
-        cudaGraph_t g;
-        UFE_CUDA(cudaGraphCreate(&g, 0));
-        try {
-          cudaGraphConditionalHandle h;
-          UFE_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
-          const CondArg cond{h, 1};
-          using M1 = CsrMat;
-          M1 mat{m, A.ptr, A.ind, A.val};
-          KV<double> v;
-          v.X = x; v.R = R; v.RP = RP; v.S = S; v.T = T; v.B = const_cast<double *>(b); v.dinv = dinv;
-          v.P[0] = P0; v.P[1] = P1; v.V[0] = V0; v.V[1] = V1;
-          const unsigned gk = krylov_grid(mat, kThreads, max_grid(ctx));
-          auto deps = capture_into(s, g, {}, [&]() {
-            k_csr_dinv<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, A.ptr, A.ind, A.val, dinv);
-            UFE_CUDA(cudaMemsetAsync(ks, 0, sizeof(KrylovScalars), s));
-            k_krylov_init<M1><<<gk, kThreads, 0, s>>>(mat, v, ks, rtol, abstol, max_it, 0, ctx->red.partials,
-                                                      ctx->red.tickets, cond);
-            UFE_CUDA(cudaGetLastError());
-          });
-          cudaGraph_t body;
-          add_while(g, deps, h, &body);
-          const unsigned gu = (unsigned)pick_blocks(m, kThreads, kMaxReduceBlocks);
-          capture_into(s, body, {}, [&]() {   // p and s row by row, then the SpMVs gather them
-            k_p_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
-            k_p_spmv<M1><<<gk, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
-            k_s_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
-            k_s_spmv<M1><<<gk, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
-            k_xr<M1><<<gk, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, cond);
-            UFE_CUDA(cudaGetLastError());
-          });
-          UFE_CUDA(cudaGraphInstantiate(&scr.graph, g, 0));
-        } catch (...) {
-          cudaGraphDestroy(g);
-          throw;
-        }
-        UFE_CUDA(cudaGraphDestroy(g));
-        scr.key = key;
-      }
-      UFE_CUDA(cudaGraphLaunch(scr.graph, s));
-      UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
-      UFE_CUDA(cudaStreamSynchronize(s));
-      *its = hks->it;
-      return hks->status;
-    }
     // Jacobi diagonal (PCJACOBI: 1 where the diagonal is zero)
     k_csr_dinv<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, A.ptr, A.ind, A.val, dinv);
     UFE_CUDA(cudaMemsetAsync(ks, 0, sizeof(KrylovScalars), s));
@@ -3081,20 +3023,40 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
     k_krylov_init<CsrMat><<<krylov_grid(mat, kThreads, grid), kThreads, 0, s>>>(
         mat, v, ks, rtol, abstol, max_it, 0, ctx->red.partials, ctx->red.tickets, none);
     UFE_CUDA(cudaGetLastError());
-    for (;;) {
-      const unsigned gu = (unsigned)pick_blocks(m, kThreads, kMaxReduceBlocks);
-      for (int c = 0; c < 8; ++c) {
-        unsigned g = krylov_grid(mat, kThreads, grid);
-        k_p_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
-        k_p_spmv<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
-        k_s_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
-        k_s_spmv<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
-        k_xr<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, none);
-      }
-      UFE_CUDA(cudaGetLastError());
+    if (persistent_krylov()) {
+      // the virtual blocks of the kernels' launch, up to four per block, one block per SM at most
+      const int nvirt = std::min((int)krylov_grid(mat, 256, grid), kMaxVirt), sms = sm_count(ctx);
+      const int q = std::max(1, std::min(4, (nvirt + sms - 1) / sms));
+      k_reset_gsync<<<1, 1, 0, s>>>(scr.gsync);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(std::min(sms, (nvirt + q - 1) / q));
+      cfg.blockDim = dim3(256 * q);
+      cfg.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      UFE_CUDA(cudaLaunchKernelEx(&cfg, k_csr_persist<CsrMat>, mat, nvirt, v, ks, scr.slots + 2 * kCsrSet,
+                                  scr.slots + 2 * kCsrSet + m, scr.slots, scr.gsync));
       UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
       UFE_CUDA(cudaStreamSynchronize(s));
-      if (!hks->active) break;
+    } else {
+      for (;;) {
+        const unsigned gu = (unsigned)pick_blocks(m, kThreads, kMaxReduceBlocks);
+        for (int c = 0; c < 8; ++c) {
+          unsigned g = krylov_grid(mat, kThreads, grid);
+          k_p_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
+          k_p_spmv<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
+          k_s_update<double><<<gu, kThreads, 0, s>>>(m, v, ks);
+          k_s_spmv<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, 1);
+          k_xr<CsrMat><<<g, kThreads, 0, s>>>(mat, v, ks, ctx->red.partials, ctx->red.tickets, none);
+        }
+        UFE_CUDA(cudaGetLastError());
+        UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
+        UFE_CUDA(cudaStreamSynchronize(s));
+        if (!hks->active) break;
+      }
     }
     *its = hks->it;
     status = hks->status;
