@@ -16,6 +16,57 @@ void dev_free(void *p) {
   if (p) cudaFree(p);
 }
 
+void *temp_alloc(ufe_ctx *ctx, size_t bytes) {
+  std::vector<TempPool::Block> &bl = ctx->temps.blocks;
+  int best = -1;
+  for (int i = 0; i < (int)bl.size(); ++i)
+    if (!bl[i].used && bl[i].bytes >= bytes && bl[i].bytes / 4 <= bytes + (1 << 16) &&
+        (best < 0 || bl[i].bytes < bl[best].bytes))
+      best = i;
+  if (best < 0) {
+    const size_t size = (bytes + 65535) / 65536 * 65536 + (bytes == 0 ? 65536 : 0);
+    void *p = nullptr;
+    if (cudaMalloc(&p, size) != cudaSuccess) {
+      cudaGetLastError();
+      temp_trim(ctx, 0);
+      UFE_CUDA(cudaMalloc(&p, size));
+    }
+    bl.push_back({p, size, false});
+    best = (int)bl.size() - 1;
+  }
+  bl[best].used = true;
+  return bl[best].p;
+}
+
+void temp_free(ufe_ctx *ctx, void *p) {
+  if (!p) return;
+  for (auto &b : ctx->temps.blocks)
+    if (b.p == p) b.used = false;
+  temp_trim(ctx, kTempKeep);
+}
+
+void temp_trim(ufe_ctx *ctx, size_t keep) {
+  std::vector<TempPool::Block> &bl = ctx->temps.blocks;
+  for (;;) {
+    size_t total = 0;
+    int big = -1;
+    for (int i = 0; i < (int)bl.size(); ++i)
+      if (!bl[i].used) {
+        total += bl[i].bytes;
+        if (big < 0 || bl[i].bytes > bl[big].bytes) big = i;
+      }
+    if (big < 0 || total <= keep) return;
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    dev_free(bl[big].p);
+    bl.erase(bl.begin() + big);
+  }
+}
+
+void temp_drop(ufe_ctx *ctx) {
+  if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  temp_trim(ctx, 0);
+}
+
 void free_operators(ufe_ctx *ctx) {
   for (void *p : ctx->op_allocs) dev_free(p);
   ctx->op_allocs.clear();
@@ -46,6 +97,7 @@ static void free_mesh(ufe_ctx *ctx) {
   ctx->V = ctx->TriGC = ctx->zeta = nullptr;
   ctx->nC = ctx->C = ctx->niTri = ctx->iTri = ctx->VBI = ctx->Tri = ctx->TriC = ctx->TriBI = nullptr;
   free_layout(ctx);
+  temp_trim(ctx, 0);
   ctx->has_mesh = false;
 }
 
@@ -143,6 +195,9 @@ extern "C" void ufe_ctx_destroy(ufe_ctx *ctx) {
   free_mesh(ctx);
   dev_free(ctx->red.partials);
   dev_free(ctx->red.tickets);
+  if (ctx->csr) csr_scratch_free(*ctx->csr);
+  delete ctx->csr;
+  temp_trim(ctx, 0);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -356,15 +411,21 @@ extern "C" int32_t ufe_apply_operator(ufe_ctx *ctx, int32_t op, const double *x,
                             op == UFE_OP_DDX_A_A || op == UFE_OP_DDY_A_A);
     const bool cols_tri = !(op == UFE_OP_MAP_A_B || op == UFE_OP_DDX_A_B || op == UFE_OP_DDY_A_B ||
                             op == UFE_OP_DDX_A_A || op == UFE_OP_DDY_A_A);
-    double *dx = (double *)dev_alloc(sizeof(double) * (size_t)A.n * ncols);
-    double *dy = (double *)dev_alloc(sizeof(double) * (size_t)A.m * ncols);
+    Temp<double> dx(ctx, (size_t)A.n * ncols), dy(ctx, (size_t)A.m * ncols);
     to_internal(ctx, dx, x, cols_tri, ncols);
     launch_csr_spmv(s, A, dx, dy, ncols);
     to_external(ctx, y, dy, rows_tri, ncols);
-    dev_free(dx);
-    dev_free(dy);
     return UFE_OK;
   });
+}
+
+// A caller's array in a pool buffer, added to `owned`.
+template <class T>
+static T *upload_temp(ufe_ctx *ctx, const T *h, size_t n, std::vector<void *> &owned) {
+  T *d = (T *)temp_alloc(ctx, sizeof(T) * n);
+  owned.push_back(d);
+  if (n) UFE_CUDA(cudaMemcpyAsync(d, h, sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
+  return d;
 }
 
 // Validate and upload a caller CSR matrix as a 0-based device matrix.
@@ -374,23 +435,32 @@ static DevCSR upload_csr(ufe_ctx *ctx, int32_t m, int32_t n, int64_t nnz, const 
   UFE_REQUIRE(m >= 1 && n >= 1 && nnz >= 0, UFE_ERR_INVALID, "bad matrix sizes");
   UFE_REQUIRE(ptr && ind && val, UFE_ERR_INVALID, "null CSR array");
   UFE_REQUIRE(index_base == 0 || index_base == 1, UFE_ERR_INVALID, "index_base must be 0 or 1");
-  std::vector<int32_t> hp(m + 1), hi((size_t)nnz);
-  for (int32_t i = 0; i <= m; ++i) hp[i] = ptr[i] - index_base;
-  UFE_REQUIRE(hp[0] == 0 && hp[m] == nnz, UFE_ERR_INVALID, "CSR ptr does not span nnz");
-  for (int32_t i = 0; i < m; ++i) UFE_REQUIRE(hp[i] <= hp[i + 1], UFE_ERR_INVALID, "CSR ptr not monotone");
-  for (int64_t k = 0; k < nnz; ++k) {
-    hi[k] = ind[k] - index_base;
-    UFE_REQUIRE(hi[k] >= 0 && hi[k] < n, UFE_ERR_INVALID, "CSR column index out of range");
-  }
+  UFE_REQUIRE(ptr[0] == index_base && ptr[m] - (int64_t)index_base == nnz, UFE_ERR_INVALID, "CSR ptr does not span nnz");
+  bool falls = false, outside = false;   // branch-free loops
+  for (int32_t i = 0; i < m; ++i) falls |= ptr[i] > ptr[i + 1];
+  UFE_REQUIRE(!falls, UFE_ERR_INVALID, "CSR ptr not monotone");
+  for (int64_t k = 0; k < nnz; ++k) outside |= ind[k] < index_base || ind[k] - (int64_t)index_base >= n;
+  UFE_REQUIRE(!outside, UFE_ERR_INVALID, "CSR column index out of range");
   cudaStream_t s = ctx->stream;
   DevCSR A;
   A.m = m; A.n = n; A.nnz = nnz;
-  A.ptr = upload(hp.data(), hp.size(), s);
-  A.ind = upload(hi.data(), hi.size() ? hi.size() : 1, s);
-  A.val = upload(val, nnz ? (size_t)nnz : 1, s);
-  owned.push_back(A.ptr);
-  owned.push_back(A.ind);
-  owned.push_back(A.val);
+  std::vector<int32_t> hp, hi;   // a 1-based matrix, shifted
+  struct Wait {
+    cudaStream_t s;
+    bool on;
+    ~Wait() { if (on) cudaStreamSynchronize(s); }
+  } copied{s, index_base == 1};   // before hp and hi go
+  if (index_base == 1) {
+    hp.resize(m + 1);
+    hi.resize((size_t)nnz);
+    for (int32_t i = 0; i <= m; ++i) hp[i] = ptr[i] - 1;
+    for (int64_t k = 0; k < nnz; ++k) hi[k] = ind[k] - 1;
+    ptr = hp.data();
+    ind = hi.data();
+  }
+  A.ptr = upload_temp(ctx, ptr, (size_t)m + 1, owned);
+  A.ind = upload_temp(ctx, ind, (size_t)nnz, owned);
+  A.val = upload_temp(ctx, val, (size_t)nnz, owned);
   return A;
 }
 
@@ -403,17 +473,14 @@ extern "C" int32_t ufe_csr_spmv(ufe_ctx *ctx, int32_t m, int32_t n, int64_t nnz,
     UFE_CUDA(cudaSetDevice(ctx->device));
     DevCSR A = upload_csr(ctx, m, n, nnz, ptr, ind, val, index_base, owned);
     cudaStream_t s = ctx->stream;
-    double *dx = upload(x, (size_t)n * ncols, s);
-    owned.push_back(dx);
-    double *dy = (double *)dev_alloc(sizeof(double) * (size_t)m * ncols);
-    owned.push_back(dy);
+    double *dx = upload_temp(ctx, x, (size_t)n * ncols, owned);
+    Temp<double> dy(ctx, (size_t)m * ncols);
     launch_csr_spmv(s, A, dx, dy, ncols);
     UFE_CUDA(cudaMemcpyAsync(y, dy, sizeof(double) * (size_t)m * ncols, cudaMemcpyDeviceToHost, s));
     UFE_CUDA(cudaStreamSynchronize(s));
     return UFE_OK;
   });
-  if (ctx) cudaStreamSynchronize(ctx->stream);
-  for (void *p : owned) dev_free(p);
+  for (void *p : owned) temp_free(ctx, p);
   return rc;
 }
 
@@ -428,10 +495,8 @@ extern "C" int32_t ufe_solve_csr(ufe_ctx *ctx, int32_t m, int64_t nnz, const int
     UFE_CUDA(cudaSetDevice(ctx->device));
     DevCSR A = upload_csr(ctx, m, m, nnz, ptr, ind, val, index_base, owned);
     cudaStream_t s = ctx->stream;
-    double *db = upload(bb, (size_t)m, s);
-    owned.push_back(db);
-    double *dx = upload(xx, (size_t)m, s);
-    owned.push_back(dx);
+    double *db = upload_temp(ctx, bb, (size_t)m, owned);
+    double *dx = upload_temp(ctx, xx, (size_t)m, owned);
     int32_t its = 0;
     int32_t st = solve_csr_device(ctx, A, db, dx, rtol, abstol, max_it, &its);
     UFE_CUDA(cudaMemcpyAsync(xx, dx, sizeof(double) * m, cudaMemcpyDeviceToHost, s));
@@ -439,7 +504,6 @@ extern "C" int32_t ufe_solve_csr(ufe_ctx *ctx, int32_t m, int64_t nnz, const int
     if (n_Axb_its) *n_Axb_its = its;
     return st;
   });
-  if (ctx) cudaStreamSynchronize(ctx->stream);
-  for (void *p : owned) dev_free(p);
+  for (void *p : owned) temp_free(ctx, p);
   return rc;
 }

@@ -160,24 +160,21 @@ template <class T>
 void to_internal_t(ufe_ctx *ctx, T *d_dst, const T *h_src, bool tri, int ncols) {
   const int64_t n = tri ? ctx->nTri : ctx->nV;
   cudaStream_t s = ctx->stream;
-  T *tmp = (T *)dev_alloc(sizeof(T) * n * ncols);
+  Temp<T> tmp(ctx, (size_t)n * ncols);
   UFE_CUDA(cudaMemcpyAsync(tmp, h_src, sizeof(T) * n * ncols, cudaMemcpyHostToDevice, s));
-  k_gather_cols<T><<<blocks_for(n * ncols), 256, 0, s>>>(n, ncols, tmp, perm_of(ctx, tri), d_dst);
+  k_gather_cols<T><<<blocks_for(n * ncols), 256, 0, s>>>(n, ncols, tmp.p, perm_of(ctx, tri), d_dst);
   UFE_CUDA(cudaGetLastError());
-  UFE_CUDA(cudaStreamSynchronize(s));
-  dev_free(tmp);
 }
 
 template <class T>
 void to_external_t(ufe_ctx *ctx, T *h_dst, const T *d_src, bool tri, int ncols) {
   const int64_t n = tri ? ctx->nTri : ctx->nV;
   cudaStream_t s = ctx->stream;
-  T *tmp = (T *)dev_alloc(sizeof(T) * n * ncols);
-  k_gather_cols<T><<<blocks_for(n * ncols), 256, 0, s>>>(n, ncols, d_src, iperm_of(ctx, tri), tmp);
+  Temp<T> tmp(ctx, (size_t)n * ncols);
+  k_gather_cols<T><<<blocks_for(n * ncols), 256, 0, s>>>(n, ncols, d_src, iperm_of(ctx, tri), tmp.p);
   UFE_CUDA(cudaGetLastError());
   UFE_CUDA(cudaMemcpyAsync(h_dst, tmp, sizeof(T) * n * ncols, cudaMemcpyDeviceToHost, s));
   UFE_CUDA(cudaStreamSynchronize(s));
-  dev_free(tmp);
 }
 
 void to_internal(ufe_ctx *ctx, double *d_dst, const double *h_src, bool tri, int ncols) {
@@ -194,27 +191,22 @@ void to_external(ufe_ctx *ctx, double *h_dst, const double *d_src, bool tri, int
 void pair_to_internal(ufe_ctx *ctx, double2 *d_dst, const double *h_a, const double *h_b) {
   const int64_t n = ctx->nTri;
   cudaStream_t s = ctx->stream;
-  double *ta = (double *)dev_alloc(sizeof(double) * n), *tb = (double *)dev_alloc(sizeof(double) * n);
+  Temp<double> ta(ctx, n), tb(ctx, n);
   if (h_a) UFE_CUDA(cudaMemcpyAsync(ta, h_a, sizeof(double) * n, cudaMemcpyHostToDevice, s));
   if (h_b) UFE_CUDA(cudaMemcpyAsync(tb, h_b, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  k_gather_pair<<<blocks_for(n), 256, 0, s>>>(n, h_a ? ta : nullptr, h_b ? tb : nullptr, ctx->perm_t, d_dst);
+  k_gather_pair<<<blocks_for(n), 256, 0, s>>>(n, h_a ? ta.p : nullptr, h_b ? tb.p : nullptr, ctx->perm_t, d_dst);
   UFE_CUDA(cudaGetLastError());
-  UFE_CUDA(cudaStreamSynchronize(s));
-  dev_free(ta);
-  dev_free(tb);
 }
 
 void pair_to_external(ufe_ctx *ctx, double *h_a, double *h_b, const double2 *d_src) {
   const int64_t n = ctx->nTri;
   cudaStream_t s = ctx->stream;
-  double *ta = (double *)dev_alloc(sizeof(double) * n), *tb = (double *)dev_alloc(sizeof(double) * n);
+  Temp<double> ta(ctx, n), tb(ctx, n);
   k_scatter_pair<<<blocks_for(n), 256, 0, s>>>(n, d_src, ctx->iperm_t, ta, tb);
   UFE_CUDA(cudaGetLastError());
   if (h_a) UFE_CUDA(cudaMemcpyAsync(h_a, ta, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   if (h_b) UFE_CUDA(cudaMemcpyAsync(h_b, tb, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   UFE_CUDA(cudaStreamSynchronize(s));
-  dev_free(ta);
-  dev_free(tb);
 }
 
 // Row/column maps of an operator between internal and caller numbering.

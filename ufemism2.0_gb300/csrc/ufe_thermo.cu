@@ -1165,25 +1165,19 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     } else {
       // the inputs go up in the caller's order; the kernel gathers them while it computes
       const size_t nl = (size_t)nV * nz;
-      double *buf = (double *)dev_alloc(sizeof(double) * (nl * 10 + nV));
-      try {
-        const double *src[] = {f->A_flow, f->du_dx_3D, f->du_dy_3D, f->du_dz_3D, f->dv_dx_3D, f->dv_dy_3D,
-                               f->dv_dz_3D, f->dw_dx_3D, f->dw_dy_3D, f->dw_dz_3D};
-        for (int q = 0; q < 10; ++q)
-          UFE_CUDA(cudaMemcpyAsync(buf + q * nl, src[q], sizeof(double) * nl, cudaMemcpyHostToDevice, s));
-        UFE_CUDA(cudaMemcpyAsync(buf + 10 * nl, f->Hi, sizeof(double) * nV, cudaMemcpyHostToDevice, s));
-        StrainRates e{buf + nl, buf + 2 * nl, buf + 3 * nl, buf + 4 * nl, buf + 5 * nl, buf + 6 * nl, buf + 7 * nl,
-                      buf + 8 * nl, buf + 9 * nl};
-        k_strain_heating<<<(unsigned)std::min<int64_t>((nl + 255) / 256, 65535), 256, 0, s>>>(
-            nV, nz, buf + 10 * nl, buf, e, f->Glens_flow_law_exponent > 0.0 ? f->Glens_flow_law_exponent : 3.0, ctx->perm_v,
-            t->phi);
-        UFE_CUDA(cudaGetLastError());
-        UFE_CUDA(cudaStreamSynchronize(s));
-      } catch (...) {
-        dev_free(buf);
-        throw;
-      }
-      dev_free(buf);
+      Temp<double> tmp(ctx, nl * 10 + nV);
+      double *buf = tmp;
+      const double *src[] = {f->A_flow, f->du_dx_3D, f->du_dy_3D, f->du_dz_3D, f->dv_dx_3D, f->dv_dy_3D,
+                             f->dv_dz_3D, f->dw_dx_3D, f->dw_dy_3D, f->dw_dz_3D};
+      for (int q = 0; q < 10; ++q)
+        UFE_CUDA(cudaMemcpyAsync(buf + q * nl, src[q], sizeof(double) * nl, cudaMemcpyHostToDevice, s));
+      UFE_CUDA(cudaMemcpyAsync(buf + 10 * nl, f->Hi, sizeof(double) * nV, cudaMemcpyHostToDevice, s));
+      StrainRates e{buf + nl, buf + 2 * nl, buf + 3 * nl, buf + 4 * nl, buf + 5 * nl, buf + 6 * nl, buf + 7 * nl,
+                    buf + 8 * nl, buf + 9 * nl};
+      k_strain_heating<<<(unsigned)std::min<int64_t>((nl + 255) / 256, 65535), 256, 0, s>>>(
+          nV, nz, buf + 10 * nl, buf, e, f->Glens_flow_law_exponent > 0.0 ? f->Glens_flow_law_exponent : 3.0, ctx->perm_v,
+          t->phi);
+      UFE_CUDA(cudaGetLastError());
     }
     double *vt = t->vert;
     // slots: 0 gHs_x, 1 gHi_x, 2 gHs_y, 3 gHi_y, 4 dHs_dt, 5 dHi_dt, 6 Hc, 7 Hi_eff, 8 T_surf, 9 Q,
@@ -1199,60 +1193,46 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     else
       UFE_CUDA(cudaMemsetAsync(vt + 10 * nV, 0, sizeof(double) * nV, s));
     // temporaries: Hi, Hs, u_vav, v_vav, frictional heating, T2m, u_3D_b, v_3D_b
-    double *Hi = (double *)dev_alloc(sizeof(double) * nV * 5);
-    double *Hs = Hi + nV, *uv = Hi + 2 * nV, *vv = Hi + 3 * nV, *fric = Hi + 4 * nV;
-    double *T2m = (double *)dev_alloc(sizeof(double) * nV * f->n_months);
-    double *ubt = (double *)dev_alloc(sizeof(double) * nTri * nz * 2);
-    double *vbt = ubt + nTri * nz;
-    int32_t *err = (int32_t *)dev_alloc(sizeof(int32_t));
+    Temp<double> vtmp(ctx, (size_t)nV * 5), T2m(ctx, (size_t)nV * f->n_months), btmp(ctx, (size_t)nTri * nz * 2);
+    Temp<int32_t> err(ctx, 1);
+    double *Hi = vtmp, *Hs = Hi + nV, *uv = Hi + 2 * nV, *vv = Hi + 3 * nV, *fric = Hi + 4 * nV;
+    double *ubt = btmp, *vbt = ubt + nTri * nz;
     int32_t herr = 0;
-    try {
-      to_internal(ctx, Hi, f->Hi, false, 1);
-      to_internal(ctx, Hs, f->Hs, false, 1);
-      to_internal(ctx, uv, f->u_vav, false, 1);
-      to_internal(ctx, vv, f->v_vav, false, 1);
-      if (!friction) {
-        to_internal(ctx, fric, f->frictional_heating, false, 1);
-      } else {
-        double *bfc = ubt, *uab = ubt + nV;   // ubt is filled below; use it as scratch first
-        to_internal(ctx, bfc, f->basal_friction_coefficient, false, 1);
-        to_internal(ctx, uab, f->uabs_base, false, 1);
-        k_frictional_heating<<<(unsigned)((nV + 255) / 256), 256, 0, s>>>(nV, bfc, uab, t->mask, f->no_sliding,
-                                                                          fric);
-        UFE_CUDA(cudaGetLastError());
-      }
-      to_internal(ctx, T2m, f->T2m, false, f->n_months);
-      to_internal(ctx, ubt, f->u_3D_b, true, nz);
-      to_internal(ctx, vbt, f->v_3D_b, true, nz);
-      // calc_zeta_gradients: ddx_a_a / ddy_a_a of Hi and Hs
-      launch_csr_spmv(s, ctx->ops[UFE_OP_DDX_A_A], Hs, vt + 0 * nV, 1);
-      launch_csr_spmv(s, ctx->ops[UFE_OP_DDX_A_A], Hi, vt + 1 * nV, 1);
-      launch_csr_spmv(s, ctx->ops[UFE_OP_DDY_A_A], Hs, vt + 2 * nV, 1);
-      launch_csr_spmv(s, ctx->ops[UFE_OP_DDY_A_A], Hi, vt + 3 * nV, 1);
-      const unsigned bv = (unsigned)((nV + 255) / 256);
-      k_vertex_prelude<<<bv, 256, 0, s>>>(nV, f->n_months, Hi, T2m, fric, vt + 11 * nV, vt + 6 * nV, vt + 8 * nV,
-                                          vt + 9 * nV);
+    to_internal(ctx, Hi, f->Hi, false, 1);
+    to_internal(ctx, Hs, f->Hs, false, 1);
+    to_internal(ctx, uv, f->u_vav, false, 1);
+    to_internal(ctx, vv, f->v_vav, false, 1);
+    if (!friction) {
+      to_internal(ctx, fric, f->frictional_heating, false, 1);
+    } else {
+      double *bfc = ubt, *uab = ubt + nV;   // ubt is filled below; use it as scratch first
+      to_internal(ctx, bfc, f->basal_friction_coefficient, false, 1);
+      to_internal(ctx, uab, f->uabs_base, false, 1);
+      k_frictional_heating<<<(unsigned)((nV + 255) / 256), 256, 0, s>>>(nV, bfc, uab, t->mask, f->no_sliding,
+                                                                        fric);
       UFE_CUDA(cudaGetLastError());
-      UFE_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
-      k_upwind_triangle<<<bv, 256, 0, s>>>(nV, nTri, ctx->V, ctx->niTri, ctx->iTri, ctx->Tri, Hi, uv, vv, t->ti_up,
-                                           err);
-      UFE_CUDA(cudaGetLastError());
-      k_gather_upwind<<<(unsigned)((nV * nz + 255) / 256), 256, 0, s>>>(nV, nTri, nz, t->ti_up, ubt, vbt, t->ub,
-                                                                        t->vb);
-      UFE_CUDA(cudaGetLastError());
-      UFE_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      UFE_CUDA(cudaStreamSynchronize(s));
-    } catch (...) {
-      dev_free(Hi);
-      dev_free(T2m);
-      dev_free(ubt);
-      dev_free(err);
-      throw;
     }
-    dev_free(Hi);
-    dev_free(T2m);
-    dev_free(ubt);
-    dev_free(err);
+    to_internal(ctx, T2m, f->T2m, false, f->n_months);
+    to_internal(ctx, ubt, f->u_3D_b, true, nz);
+    to_internal(ctx, vbt, f->v_3D_b, true, nz);
+    // calc_zeta_gradients: ddx_a_a / ddy_a_a of Hi and Hs
+    launch_csr_spmv(s, ctx->ops[UFE_OP_DDX_A_A], Hs, vt + 0 * nV, 1);
+    launch_csr_spmv(s, ctx->ops[UFE_OP_DDX_A_A], Hi, vt + 1 * nV, 1);
+    launch_csr_spmv(s, ctx->ops[UFE_OP_DDY_A_A], Hs, vt + 2 * nV, 1);
+    launch_csr_spmv(s, ctx->ops[UFE_OP_DDY_A_A], Hi, vt + 3 * nV, 1);
+    const unsigned bv = (unsigned)((nV + 255) / 256);
+    k_vertex_prelude<<<bv, 256, 0, s>>>(nV, f->n_months, Hi, T2m, fric, vt + 11 * nV, vt + 6 * nV, vt + 8 * nV,
+                                        vt + 9 * nV);
+    UFE_CUDA(cudaGetLastError());
+    UFE_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
+    k_upwind_triangle<<<bv, 256, 0, s>>>(nV, nTri, ctx->V, ctx->niTri, ctx->iTri, ctx->Tri, Hi, uv, vv, t->ti_up,
+                                         err);
+    UFE_CUDA(cudaGetLastError());
+    k_gather_upwind<<<(unsigned)((nV * nz + 255) / 256), 256, 0, s>>>(nV, nTri, nz, t->ti_up, ubt, vbt, t->ub,
+                                                                      t->vb);
+    UFE_CUDA(cudaGetLastError());
+    UFE_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    UFE_CUDA(cudaStreamSynchronize(s));
     UFE_REQUIRE(herr == 0, UFE_ERR_INVALID, "heat upload: could not find upwind triangle for a vertex with ice");
     t->mesh_ready = true;
     return UFE_OK;
@@ -1400,8 +1380,9 @@ extern "C" int32_t ufe_tridiagonal_solve(ufe_ctx *ctx, int32_t n, int32_t nsys, 
     UFE_CUDA(cudaSetDevice(ctx->device));
     const int64_t N = (int64_t)n * nsys;
     cudaStream_t s = ctx->stream;
-    double *buf = (double *)dev_alloc(sizeof(double) * N * 7);
-    try {
+    Temp<double> tmp(ctx, (size_t)N * 7);
+    double *buf = tmp;
+    {
       double *da = buf, *db = buf + N, *dc = buf + 2 * N, *dd = buf + 3 * N, *bw = buf + 4 * N, *dw = buf + 5 * N,
              *dx = buf + 6 * N;
       UFE_CUDA(cudaMemcpyAsync(da, a, sizeof(double) * N, cudaMemcpyHostToDevice, s));
@@ -1412,11 +1393,7 @@ extern "C" int32_t ufe_tridiagonal_solve(ufe_ctx *ctx, int32_t n, int32_t nsys, 
       UFE_CUDA(cudaGetLastError());
       UFE_CUDA(cudaMemcpyAsync(x, dx, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
       UFE_CUDA(cudaStreamSynchronize(s));
-    } catch (...) {
-      dev_free(buf);
-      throw;
     }
-    dev_free(buf);
     return UFE_OK;
   });
 }
