@@ -31,3 +31,29 @@ def test_retried_columns_match_oracle(pkg, oracle_mod, gpu_lib, nz, glbc):
         got, n = s.thermo_step(p, zeta, cols)
     assert n == n_ref
     assert np.abs(got - ref).max() < 1e-8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("glbc", [0, 1])
+@pytest.mark.parametrize("nz", [3, 8, 30, 32])
+@pytest.mark.parametrize("n", [1, 304, 305, 700])
+def test_short_and_long_lists_match_oracle(pkg, oracle_mod, gpu_lib, n, nz, glbc):
+    """Up to 304 listed columns of up to 32 layers are retried by four warps each, longer lists by one: both against
+    the oracle, 1e-8 K as above (the inverse's sums are of at most 32 terms of the profile's size per substep)."""
+    p = pkg.abi.default_thermo_params(dt=10.0)
+    p.choice_GL_temperature_BC = glbc
+    zeta, cols = pkg.geometry.random_columns(6000, nz, seed=nz, stiff_frac=0.6, stiffness=3000.0)
+    rng = np.random.default_rng(nz)
+    cols["w_3D"] *= np.where(rng.random(6000) < 0.5, 1.0, 10.0 ** rng.uniform(0.0, 2.0, 6000))[:, None]
+    flags = np.asarray(oracle_mod.thermo_step(p, zeta, cols)[3])
+    listed = np.flatnonzero(flags == 2)
+    if len(listed) == 0:
+        pytest.skip("no column recovers at this layer count")
+    pick = np.r_[np.resize(listed, n), np.flatnonzero(flags == 0)[:50]]
+    cols = {k: np.asfortranarray(v[pick]) for k, v in cols.items()}
+    ref, n_ref, status, flags = oracle_mod.thermo_step(p, zeta, cols)
+    assert status == pkg.abi.UFE_OK and (np.asarray(flags) > 0).sum() == n
+    with pkg.ColumnSolver() as s:
+        got, n_got = s.thermo_step(p, zeta, cols)
+    assert n_got == n_ref
+    assert np.abs(got - ref).max() < 1e-8

@@ -339,7 +339,8 @@ __global__ void __launch_bounds__(128) k_heat_columns(In in, ZOps z, Consts c, V
 // layers: the minimum with the melting point is taken on bit patterns, the stability check runs on the
 // last substep only (the earlier ones' results were overwritten), and the profile stays in registers.
 // Measured on 200k columns x 30 layers (94 columns through all levels): 1.13 ms per time step, 2.76 ms before,
-// when each substep composed the slopes again, compared in FP64 and kept the profile in shared memory.
+// when each substep composed the slopes again, compared in FP64 and kept the profile in shared memory.  Lists of at
+// most 304 columns of at most 32 layers are k_heat_retry_team's (below).
 constexpr int kRetryLevels = 9;          // dt / 2 ... dt / 512 (:163)
 constexpr int kRetryArrays = 4 + 2 * kRetryLevels;
 constexpr int kRetryBlocks = 4 * 152;
@@ -396,6 +397,66 @@ struct Slopes {
   }
 };
 
+constexpr int kTeamRows = 32;           // k_heat_retry_team takes lists of up to kTeamColumns columns of up to
+constexpr int kTeamColumns = 152 * 2;   // kTeamRows layers
+// Row k of a listed column: the coefficients that do not depend on dt or on the current profile (the off-diagonals a
+// and c, the two parts e1 and e2 of the diagonal, the advection and heating term g).  Boundary rows keep zeros
+// (AA_ldiag / AA_udiag, :389-391).
+struct RetryRow {
+  double a = 0.0, c = 0.0, e1 = 0.0, e2 = 0.0, g = 0.0;
+};
+template <class In>
+__device__ __forceinline__ RetryRow retry_row(const In &in, const typename In::Col &col, const ZOps &z, const Consts &cs,
+                                              int64_t vi, int k, double zk) {
+  RetryRow r;
+  if (k >= 1 && k < z.nz - 1) {
+    Layer L;
+    in.layer(col, vi, k, zk, L);
+    const double Cpi = heat_capacity(cs, L.Ti0);
+    const double Ki = conductivity(cs, L.Ti0);
+    const double c1 = L.dzt + (L.u * L.dzx) + (L.v * L.dzy) + (L.w * L.dzz);
+    const double c2 = -(Ki / (kIceDensity * Cpi) * (L.dzz * L.dzz));
+    r.g = L.phi / (kIceDensity * Cpi) - L.udx - L.vdy;
+    r.a = (c1 * __ldg(z.l1 + k)) + (c2 * __ldg(z.l2 + k));
+    r.c = (c1 * __ldg(z.u1 + k)) + (c2 * __ldg(z.u2 + k));
+    r.e1 = c1 * __ldg(z.d1 + k);
+    r.e2 = c2 * __ldg(z.d2 + k);
+  }
+  return r;
+}
+// The basal row's flux term (grounded flux condition).
+template <class In>
+__device__ __forceinline__ double retry_flux(const In &in, const typename In::Col &col, const ZOps &z, const Consts &cs,
+                                             int64_t vi, double Q) {
+  const int kb = z.nz - 1;
+  double Ti0b, dzzb;
+  in.basal(col, vi, kb, __ldg(z.zeta + kb), Ti0b, dzzb);
+  return (__ldg(z.zeta + kb) - __ldg(z.zeta + kb - 1)) * Q / (dzzb * conductivity(cs, Ti0b));
+}
+// Matrix part of the forward elimination, dt level lane + 2 in each of the first kRetryLevels lanes.
+__device__ __forceinline__ void retry_eliminate(const double *A, const double *Cc, const double *E1, const double *E2,
+                                                double *W, double *Bp, int nz, int kb, double dt, int lane) {
+  if (lane < kRetryLevels) {
+    const double inv_dt = 1.0 / (dt * (1.0 / (double)(2 << lane)));
+    double *Wl = W + lane * nz, *Bl = Bp + lane * nz;
+    double bprev = 1.0, cprev = 0.0;
+    Wl[0] = 0.0;
+    Bl[0] = 1.0;
+    for (int k = 1; k < kb; ++k) {
+      double b = inv_dt + E1[k] + E2[k];
+      const double wgt = A[k] / bprev;
+      b = b - wgt * cprev;
+      Wl[k] = wgt;
+      Bl[k] = b;
+      bprev = b;
+      cprev = Cc[k];
+    }
+    const double wgt = 0.0 / bprev;
+    Wl[kb] = wgt;
+    Bl[kb] = 1.0 - wgt * cprev;
+  }
+}
+
 template <class In, int R>
 __global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, VertexFields vf, int64_t nV,
                                                    double *__restrict__ Ti_next, Lists lists, Counters *cnt) {
@@ -404,6 +465,7 @@ __global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, Vert
   const int lane = threadIdx.x, nz = z.nz, kb = nz - 1, k0 = lane * R;
   double *A = sm, *Cc = A + nz, *E1 = Cc + nz, *E2 = E1 + nz, *W = E2 + nz, *Bp = W + kRetryLevels * nz;
   const int32_t n = cnt->n_retry;
+  if (nz <= kTeamRows && n <= kTeamColumns) return;   // k_heat_retry_team's
   for (int32_t j = blockIdx.x; j < n; j += gridDim.x) {
     const int64_t vi = lists.retry[j];
     const double Hi_eff = __ldg(vf.Hi_eff + vi);
@@ -423,49 +485,17 @@ __global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, Vert
       const double zk = __ldg(z.zeta + k);
       PMP[r] = melting_point(Hi_eff, zk);
       X[r] = Ti_next[(int64_t)k * nV + vi];   // the profile the full-dt solve left (:222)
-      double a = 0.0, cc = 0.0;               // boundary rows: AA_ldiag / AA_udiag stay zero (:389-391)
-      if (k >= 1 && k < kb) {
-        Layer L;
-        in.layer(col, vi, k, zk, L);
-        const double Cpi = heat_capacity(c, L.Ti0);
-        const double Ki = conductivity(c, L.Ti0);
-        const double c1 = L.dzt + (L.u * L.dzx) + (L.v * L.dzy) + (L.w * L.dzz);
-        const double c2 = -(Ki / (kIceDensity * Cpi) * (L.dzz * L.dzz));
-        G[r] = L.phi / (kIceDensity * Cpi) - L.udx - L.vdy;
-        a = (c1 * __ldg(z.l1 + k)) + (c2 * __ldg(z.l2 + k));
-        cc = (c1 * __ldg(z.u1 + k)) + (c2 * __ldg(z.u2 + k));
-        E1[k] = c1 * __ldg(z.d1 + k);
-        E2[k] = c2 * __ldg(z.d2 + k);
-      }
-      A[k] = a;
-      Cc[k] = cc;
+      const RetryRow row = retry_row(in, col, z, c, vi, k, zk);
+      A[k] = row.a;
+      Cc[k] = row.c;
+      E1[k] = row.e1;
+      E2[k] = row.e2;
+      G[r] = row.g;
     }
-    // basal row inputs (grounded flux condition)
     const double pmp_b = melting_point(Hi_eff, __ldg(z.zeta + kb));
-    double Ti0b, dzzb;
-    in.basal(col, vi, kb, __ldg(z.zeta + kb), Ti0b, dzzb);
-    const double flux_b = (__ldg(z.zeta + kb) - __ldg(z.zeta + kb - 1)) * Q / (dzzb * conductivity(c, Ti0b));
+    const double flux_b = retry_flux(in, col, z, c, vi, Q);
     __syncwarp();
-    if (lane < kRetryLevels) {
-      // matrix part of the forward elimination, dt level lane + 2
-      const double inv_dt = 1.0 / (c.dt * (1.0 / (double)(2 << lane)));
-      double *Wl = W + lane * nz, *Bl = Bp + lane * nz;
-      double bprev = 1.0, cprev = 0.0;
-      Wl[0] = 0.0;
-      Bl[0] = 1.0;
-      for (int k = 1; k < kb; ++k) {
-        double b = inv_dt + E1[k] + E2[k];
-        const double wgt = A[k] / bprev;
-        b = b - wgt * cprev;
-        Wl[k] = wgt;
-        Bl[k] = b;
-        bprev = b;
-        cprev = Cc[k];
-      }
-      const double wgt = 0.0 / bprev;
-      Wl[kb] = wgt;
-      Bl[kb] = 1.0 - wgt * cprev;
-    }
+    retry_eliminate(A, Cc, E1, E2, W, Bp, nz, kb, c.dt, lane);
     __syncwarp();
     bool found = false;
     for (int it_dt = 2; it_dt <= 1 + kRetryLevels && !found; ++it_dt) {
@@ -576,7 +606,203 @@ __global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, Vert
   }
 }
 
-// replace_Ti_with_robin_solution for the listed columns, or the step's error.
+// The same retries for short lists, four warps per column (up to 32 layers).  Alone on its scheduler a warp waits
+// out every instruction of the two scans above (1,900 cycles a substep, half of them on shuffles and selects), and the
+// substeps are a chain: each level goes on from the last one's profile.  Here the inverse of each level's matrix is
+// formed once, from the same elimination, and a substep is its product with the right-hand side: warp w, lane l holds
+// row 8 w + l % 8 against columns 8 (l / 8) + i, eight FMAs in registers on each of the four FP64 pipes, two shuffles
+// to sum, and one barrier for the new right-hand side.
+//
+// Unstable columns grow until they overflow, and what is left of such a column is decided by which of its sums become
+// infinite or undefined, so from kTeamLimit on (far enough below for the product's sums to stay finite) a substep is
+// the scans' of k_heat_retry, on the first warp; so is a level whose inverse holds an entry of 2^14 or more.
+//
+// That is three times the scans' FP64 instructions, so it is for lists that leave the schedulers idle otherwise: two
+// columns an SM.  All 1,022 substeps at 30 layers take 0.61 ms for up to 100 columns and 0.86 ms for 152 to 304; the
+// scans take 1.06 ms for up to 304 and 1.10 ms for 600, where the teams' second wave would end at 1.7 ms.
+constexpr int kTeamPad = 10;   // slots j at (j / 8) * 10 + j % 8: the four groups in different banks
+constexpr int kTeamLimit = (1023 + 1004) << 20;   // high words of 2^1004 and 2^14: 32 products stay below 2^1024
+constexpr int kTeamEntry = (1023 + 14) << 20;
+struct TeamShared {
+  double M[kRetryLevels][kTeamRows * kTeamRows];
+  double A[kTeamRows], C[kTeamRows], E1[kTeamRows], E2[kTeamRows];
+  double W[kRetryLevels * kTeamRows], B[kRetryLevels * kTeamRows];
+  double D[2][4 * kTeamPad];   // right-hand sides
+  double d_gr[2];              // the basal one of the grounded flux condition
+  double x[kTeamRows], fwd[5][kTeamRows], bwd[5][kTeamRows], all[kTeamRows];   // the scans' substep
+};
+__device__ __forceinline__ int team_slot(int j) { return (j >> 3) * kTeamPad + (j & 7); }
+
+// Slopes of the scans for dt level l (as k_heat_retry forms them with one row per lane).
+__device__ __noinline__ void team_slopes(TeamShared &sh, int l, int nz, int kb, int lane) {
+  const bool row = lane < kb;
+  const double rb = row ? 1.0 / sh.B[l * nz + lane] : 0.0;
+  Slopes f, b;
+  f.up(!row ? 1.0 : (lane == 0 ? 0.0 : -sh.W[l * nz + lane]), lane);
+  b.down(row ? -(sh.C[lane] * rb) : 1.0, lane);
+  for (int i = 0; i < 5; ++i) {
+    sh.fwd[i][lane] = f.step[i];
+    sh.bwd[i][lane] = b.step[i];
+  }
+  sh.all[lane] = b.all;
+}
+// One substep with the scans; the unclamped profiles of both basal conditions go out.
+__device__ __noinline__ void team_scan(const TeamShared &sh, int buf, int l, int nz, int kb, int lane, double pmp_b,
+                                       bool flux, double &x_sel, double &x_fl) {
+  const bool row = lane < kb;
+  double d = row ? sh.D[buf][team_slot(lane)] : 0.0;
+  for (int i = 0; i < 5; ++i) {
+    const double q = shfl_up_d(d, 1 << i);
+    if (lane >= (1 << i)) d = fma(sh.fwd[i][lane], q, d);
+  }
+  const double dprev = __shfl_sync(0xffffffffu, d, 31);
+  double t = row ? d * (1.0 / sh.B[l * nz + lane]) : 0.0;
+  for (int i = 0; i < 5; ++i) {
+    const double q = shfl_down_d(t, 1 << i);
+    if (lane + (1 << i) < 32) t = fma(sh.bwd[i][lane], q, t);
+  }
+  const double w_b = sh.W[l * nz + kb], rb_b = 1.0 / sh.B[l * nz + kb];
+  const double b_sel = fma(-w_b, dprev, flux ? sh.d_gr[buf] : pmp_b) * rb_b, b_fl = fma(-w_b, dprev, pmp_b) * rb_b;
+  x_sel = lane == kb ? b_sel : fma(sh.all[lane], b_sel, t);
+  x_fl = lane == kb ? b_fl : fma(sh.all[lane], b_fl, t);
+}
+
+template <class In>
+__global__ void __launch_bounds__(128) k_heat_retry_team(In in, ZOps z, Consts c, VertexFields vf, int64_t nV,
+                                                         double *__restrict__ Ti_next, Lists lists, Counters *cnt) {
+  if (cnt->err) return;
+  const int32_t n = cnt->n_retry;
+  if (n > kTeamColumns || (int32_t)blockIdx.x >= n) return;
+  extern __shared__ double2 team_raw[];
+  TeamShared &sh = *reinterpret_cast<TeamShared *>(team_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nz = z.nz, kb = nz - 1;
+  const int row = 8 * warp + (lane & 7), group = lane >> 3;
+  const int64_t vi = lists.retry[blockIdx.x];
+  const double Hi_eff = __ldg(vf.Hi_eff + vi);
+  const double d_top = fmin(__ldg(vf.T_surf + vi), kT0);
+  const int32_t mask = __ldg(vf.mask + vi);
+  const double fr = (c.glbc == UFE_GLBC_SUBGRID) ? __ldg(vf.fr + vi) : 0.0;
+  const bool two_solves = mask == UFE_COL_GL_GR && c.glbc == UFE_GLBC_SUBGRID;
+  const bool grounded = mask == UFE_COL_GROUNDED || (mask == UFE_COL_GL_GR && c.glbc == UFE_GLBC_GROUNDED);
+  const typename In::Col col = in.col(vi);
+  const double pmp_b = melting_point(Hi_eff, __ldg(z.zeta + kb));
+  const double flux_b = retry_flux(in, col, z, c, vi, __ldg(vf.Q + vi));
+  const double pmp = row < nz ? melting_point(Hi_eff, __ldg(z.zeta + row)) : kT0;
+  double x = row < nz ? Ti_next[(int64_t)row * nV + vi] : 0.0;   // the profile the full-dt solve left (:222)
+  if (warp == 0 && lane < nz) {
+    const RetryRow r = retry_row(in, col, z, c, vi, lane, __ldg(z.zeta + lane));
+    sh.A[lane] = r.a;
+    sh.C[lane] = r.c;
+    sh.E1[lane] = r.e1;
+    sh.E2[lane] = r.e2;
+    sh.x[lane] = r.g;
+  }
+  if (threadIdx.x < 2 * 4 * kTeamPad) (&sh.D[0][0])[threadIdx.x] = 0.0;
+  __syncthreads();
+  const double g = row < nz ? sh.x[row] : 0.0;
+  if (threadIdx.x < 2) sh.D[threadIdx.x][team_slot(0)] = d_top;
+  if (warp == 0) retry_eliminate(sh.A, sh.C, sh.E1, sh.E2, sh.W, sh.B, nz, kb, c.dt, lane);
+  __syncthreads();
+  // the inverses, column `lane` per lane: forward sweep of the unit vector, back substitution
+  for (int l = warp; l < kRetryLevels; l += 4) {
+    double *M = sh.M[l] + lane;
+    const double *W = sh.W + l * nz, *B = sh.B + l * nz;
+    const double rb = lane < nz ? 1.0 / B[lane] : 0.0;
+    double y = 0.0;
+#pragma unroll 2
+    for (int k = 0; k < nz; ++k) {
+      y = fma(-W[k], y, k == lane ? 1.0 : 0.0);
+      M[k * kTeamRows] = y;
+    }
+    double v = 0.0;
+#pragma unroll 2
+    for (int k = kb; k >= 0; --k) {
+      const double r = __shfl_sync(0xffffffffu, rb, k);
+      v = (k < kb ? fma(-sh.C[k], v, M[k * kTeamRows]) : M[k * kTeamRows]) * r;
+      M[k * kTeamRows] = v;
+    }
+  }
+  const bool interior = group == 0 && row >= 1 && row < kb, above = group == 0 && row == kb - 1;
+  double inv_dt = 0.0;
+  // the next substep's right-hand side; true when a value nears the overflow
+  auto publish = [&](int buf) -> bool {
+    int hi = 0;
+    if (interior) {
+      const double d = fma(x, inv_dt, g);
+      sh.D[buf][team_slot(row)] = d;
+      hi = __double2hiint(d) & 0x7fffffff;
+    }
+    if (above) {
+      const double d_gr = min_limit(x - flux_b, pmp_b);
+      sh.D[buf][team_slot(kb)] = two_solves ? 0.0 : (grounded ? d_gr : pmp_b);
+      sh.d_gr[buf] = d_gr;
+    }
+    return hi >= kTeamLimit;
+  };
+  bool found = false;
+  int buf = 0, slopes = -1;
+  for (int l = 0; l < kRetryLevels && !found; ++l) {
+    inv_dt = 1.0 / (c.dt * (1.0 / (double)(2 << l)));   // 0.5**(it_dt-1), exact
+    bool big = publish(buf);
+    __syncthreads();
+    double m[8];
+    int m_hi = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      m[i] = row < nz && 8 * group + i < nz ? sh.M[l][row * kTeamRows + 8 * group + i] : 0.0;
+      m_hi = max(m_hi, __double2hiint(m[i]) & 0x7fffffff);
+    }
+    const bool scans = __syncthreads_or(m_hi >= kTeamEntry);   // of this level throughout
+    big = __syncthreads_or(scans || big);
+    const double m_b = row < nz ? sh.M[l][row * kTeamRows + kb] : 0.0;
+    const int nsub = 2 << l;
+#pragma unroll 1
+    for (int sub = 0; sub < nsub; ++sub) {
+      double x_sel, x_fl = 0.0;
+      if (!big) {
+        const double2 *ds = reinterpret_cast<const double2 *>(sh.D[buf] + group * kTeamPad);
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double2 v = ds[i];
+          s = i == 0 ? m[0] * v.x : fma(m[2 * i], v.x, s);
+          s = fma(m[2 * i + 1], v.y, s);
+        }
+        s = s + __shfl_xor_sync(0xffffffffu, s, 8);
+        x_sel = s + __shfl_xor_sync(0xffffffffu, s, 16);
+        if (two_solves) {
+          x_fl = fma(m_b, pmp_b, x_sel);
+          x_sel = fma(m_b, sh.d_gr[buf], x_sel);
+        }
+      } else {
+        if (warp == 0) {
+          if (slopes != l) team_slopes(sh, l, nz, kb, lane);
+          __syncwarp();
+          double u, v;
+          team_scan(sh, buf, l, nz, kb, lane, pmp_b, grounded || two_solves, u, v);
+          sh.x[lane] = u;
+          sh.E1[lane] = v;   // the diagonal's parts are not needed any more
+        }
+        slopes = l;
+        __syncthreads();
+        x_sel = sh.x[row];
+        x_fl = sh.E1[row];
+      }
+      x = two_solves ? fr * min_limit(x_sel, pmp) + (1.0 - fr) * min_limit(x_fl, pmp) : min_limit(x_sel, pmp);
+      buf ^= 1;
+      big = __syncthreads_or(publish(buf) || scans);
+    }
+    found = !__syncthreads_or(row < nz && unstable_value(x));
+  }
+  if (group == 0 && row < nz) Ti_next[(int64_t)row * nV + vi] = x;
+  if (!found && threadIdx.x == 0) {
+    const int32_t u = atomicAdd(&cnt->n_unstable, 1);
+    lists.unstable[u] = (int32_t)vi;
+  }
+}
+
+// replace_Ti_with_robin_solution for the listed columns, a thread per layer (a thread per column: 97 us for 94 columns
+// of 30 layers, a chain of square roots and error functions).
 __global__ void k_heat_finish(ZOps z, Consts c, VertexFields vf, int64_t nV, double *__restrict__ Ti_next,
                               Lists lists, Counters *cnt) {
   if (cnt->err) return;
@@ -584,35 +810,35 @@ __global__ void k_heat_finish(ZOps z, Consts c, VertexFields vf, int64_t nV, dou
   if (cnt->bad_mask > 0 || n >= cnt->threshold) return;   // k_heat_close records the error
   const double K_R = 9.828 * kSecPerYear * exp(-(0.0057 * kT0));
   const double kappa_R = K_R / (kIceDensity * 2127.5);
-  for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const int64_t vi = lists.unstable[j];
+  const int64_t rows = (int64_t)n * z.nz;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < rows; e += (int64_t)gridDim.x * blockDim.x) {
+    const int k = (int)(e % z.nz);
+    const int64_t vi = lists.unstable[e / z.nz];
     const double Hi_eff = vf.Hi_eff[vi];
     const int32_t mask = vf.mask[vi];
     const double Ts = fmin(kT0, vf.T_surf[vi]);
     const double grad = -(1.0 * vf.geo[vi] / K_R);
     const double SMB = vf.SMB[vi];
     const double pmp_b = melting_point(Hi_eff, z.zeta[z.nz - 1]);
-    for (int k = 0; k < z.nz; ++k) {
-      const double zk = z.zeta[k];
-      double T = Ti_next[(int64_t)k * nV + vi];
-      if (Hi_eff > c.Hi_min) {
-        if (mask == UFE_COL_GROUNDED || mask == UFE_COL_GL_GR) {
-          if (SMB > 0.0) {
-            const double L = sqrt(2.0 * kappa_R * Hi_eff / SMB);
-            const double erf1 = erf((1.0 - zk) * Hi_eff / L);
-            const double erf2 = erf(Hi_eff / L);
-            T = Ts + sqrt(kPi) / 2.0 * L * grad * (erf1 - erf2);
-          } else {
-            T = Ts + ((kT0 - kCCGradient * Hi_eff) - Ts) * zk;
-          }
-        } else if (mask == UFE_COL_FLOATING) {
-          T = Ts + zk * (pmp_b - Ts);
+    const double zk = z.zeta[k];
+    double T = Ti_next[(int64_t)k * nV + vi];
+    if (Hi_eff > c.Hi_min) {
+      if (mask == UFE_COL_GROUNDED || mask == UFE_COL_GL_GR) {
+        if (SMB > 0.0) {
+          const double L = sqrt(2.0 * kappa_R * Hi_eff / SMB);
+          const double erf1 = erf((1.0 - zk) * Hi_eff / L);
+          const double erf2 = erf(Hi_eff / L);
+          T = Ts + sqrt(kPi) / 2.0 * L * grad * (erf1 - erf2);
+        } else {
+          T = Ts + ((kT0 - kCCGradient * Hi_eff) - Ts) * zk;
         }
-      } else {
-        T = Ts;
+      } else if (mask == UFE_COL_FLOATING) {
+        T = Ts + zk * (pmp_b - Ts);
       }
-      Ti_next[(int64_t)k * nV + vi] = fmin(T, melting_point(Hi_eff, zk));
+    } else {
+      T = Ts;
     }
+    Ti_next[(int64_t)k * nV + vi] = fmin(T, melting_point(Hi_eff, zk));
   }
 }
 
@@ -946,6 +1172,12 @@ void launch_retry_rows(cudaStream_t s, const In &in, const ZOps &z, const Consts
 template <class In>
 void launch_retry(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, const VertexFields &vf, int64_t nV,
                   double *Ti_next, const Lists &lists, Counters *cnt) {
+  if (z.nz <= kTeamRows) {   // one of the two finds work: the list's length is known on the device only
+    UFE_CUDA(cudaFuncSetAttribute(k_heat_retry_team<In>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(TeamShared)));
+    k_heat_retry_team<In><<<kTeamColumns, 128, sizeof(TeamShared), s>>>(in, z, c, vf, nV, Ti_next, lists, cnt);
+    UFE_CUDA(cudaGetLastError());
+  }
   if (z.nz <= 32) launch_retry_rows<In, 1>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
   else if (z.nz <= 64) launch_retry_rows<In, 2>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
   else if (z.nz <= 128) launch_retry_rows<In, 4>(s, in, z, c, vf, nV, Ti_next, lists, cnt);
