@@ -4,15 +4,16 @@
 // (src/UFEMISM/ice_dynamics/conservation_of_momentum/SSA_DIVA/SSA_main.f90:165-234,
 //  DIVA_main.f90:170-251) is a handful of fused kernels:
 //
-//   k_vertex_{ssa,diva}  one thread per vertex: the b->a operator row (strain rates, velocities
+//   k_vertex_{ssa,diva}  a lane per vertex, the work split over warps: the b->a operator row (strain rates, velocities
 //                        on vertices, DIVA vertical shear), Glen viscosity, N = eta H, the
 //                        sliding law (and DIVA's F-integral and beta_eff)
-//   k_assemble<MODE>     one thread per triangle: the a->b operator row (N_b, dN/dx, dN/dy,
-//                        beta_b), the 2x2-block stiffness row on the 2nd-order b_b pattern
-//                        (solve_linearised_SSA_DIVA.f90:180-641), the Jacobi diagonal, the FP32
-//                        copy, and the Krylov initial residual
+//   k_assemble_rows<MODE> the a->b operator row (N_b, dN/dx, dN/dy, beta_b), the 2x2-block
+//                        stiffness row on the 2nd-order b_b pattern
+//                        (solve_linearised_SSA_DIVA.f90:180-641) and its copies in the solves'
+//                        layouts and precisions, the Jacobi diagonal, the Krylov initial residual
+//   k_assemble_norms     its norm and the right-hand side's, the Krylov solve's scalars
 //   Krylov               ufe_krylov.cuh, three kernels per BiCGStab iteration
-//   k_finalize_{ssa,diva} velocity limits, relaxation, (DIVA basal velocity and stress), the
+//   k_finalize<DIVA>     velocity limits, relaxation, (DIVA basal velocity and stress), the
 //                        Picard L2 norm and divergence control (SSA_DIVA_utilities.f90:84-184)
 //
 // The whole solve is one CUDA graph: a conditional while-node for the Picard loop holds a
@@ -93,24 +94,32 @@ PhysParams make_phys(const ufe_solver_params &p, int has_bc) {
 // e^((1-n)/(2n)), the strain-rate power of Glen's law.  For the usual n = 3 the exponent is -1/3 and
 // the reciprocal cube root replaces the general power (several times fewer FP64 instructions, which
 // bound the viscosity passes on this GPU); n = 1 gives 1.  Both agree with pow to within an ulp or so.
+__device__ __noinline__ double glen_general_pow(double e, double n) { return pow(e, (1.0 - n) / (2.0 * n)); }
 __device__ __forceinline__ double glen_epow(double e, double n) {
   if (n == 3.0) return rcbrt(e);
   if (n == 1.0) return 1.0;
-  return pow(e, (1.0 - n) / (2.0 * n));
+  return glen_general_pow(e, n);
 }
 
 // calc_effective_viscosity_Glen_2D / _3D_uv_only (constitutive_equation.f90:25-80)
-// Glen's flow law, 3-D (constitutive_equation.f90:25-80), with A^(-1/n) evaluated beforehand:
-// 0.5 A^(-1/n) (eps^2 + eps0^2)^((1-n)/(2n))
-__device__ __forceinline__ double glen_apow(double eps0, double ux, double uy, double vx, double vy,
-                                            double uz, double vz, double A_pow, double n) {
-  double e = ux * ux + vy * vy + ux * vy + 0.25 * ((uy + vx) * (uy + vx)) + 0.25 * (uz * uz + vz * vz) + eps0;
-  return 0.5 * A_pow * glen_epow(e, n);
+// Glen's flow law, 3-D (constitutive_equation.f90:25-80):
+// 0.5 A^(-1/n) (eps^2 + eps0^2)^((1-n)/(2n)), with 0.5 A^(-1/n) evaluated beforehand and the horizontal part of eps^2,
+// glen_horizontal, once for all layers
+__device__ __forceinline__ double glen_horizontal(double ux, double uy, double vx, double vy) {
+  return ux * ux + vy * vy + ux * vy + 0.25 * ((uy + vx) * (uy + vx));
+}
+__device__ __forceinline__ double glen_apow(double eps0, double horizontal, double uz, double vz, double A_pow, double n) {
+  const double e = fma(0.25, uz * uz + vz * vz, horizontal) + eps0;   // 0.25 is exact: the sum's rounding is unchanged
+  return A_pow * glen_epow(e, n);
+}
+// 0.5 A^(-1/n)
+__device__ __forceinline__ double glen2d_flow(double A, double n) {
+  return 0.5 * (n == 3.0 ? rcbrt(A) : pow(A, -1.0 / n));
 }
 __device__ __forceinline__ double glen2d(double eps0, double ux, double uy, double vx, double vy,
-                                         double A, double n) {
-  double e = ux * ux + vy * vy + ux * vy + 0.25 * ((uy + vx) * (uy + vx)) + eps0;
-  return 0.5 * (n == 3.0 ? rcbrt(A) : pow(A, -1.0 / n)) * glen_epow(e, n);
+                                         double A_flow, double n) {
+  const double e = glen_horizontal(ux, uy, vx, vy) + eps0;
+  return A_flow * glen_epow(e, n);
 }
 
 struct SlidingIn {
@@ -189,10 +198,10 @@ __global__ void k_prologue(int nV, int nTri, int nz, OpRow ab, const double *Hi,
         a = a + 0.5 * (A_flow[(int64_t)k * nV + v] + A_flow[(int64_t)(k - 1) * nV + v]) * (zeta[k] - zeta[k - 1]);
       Avav[v] = a;
     }
-  // DIVA: A^(-1/n) per vertex and layer, constant over the Picard iterations of a solve
+  // DIVA: 0.5 A^(-1/n) per vertex and layer, constant over the Picard iterations of a solve
   if (A_pow)
     for (int64_t ix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ix < (int64_t)nV * nz; ix += stride)
-      A_pow[ix] = pow(A_flow[ix], -1.0 / n_glen);
+      A_pow[ix] = 0.5 * pow(A_flow[ix], -1.0 / n_glen);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     PicardScalars &p = *ps;
     p.L2 = 1e9;
@@ -266,18 +275,18 @@ __global__ void k_icestream_yield(int nV, const double *Vy, double H, double tan
 // kernel's b->a sums then read them) rather than once per vertex row entry, as tau (zeta / eta):
 // one FP64 division per layer instead of two (the reference's (tau zeta) / eta rounds differently
 // by an ulp or so).
-__device__ __forceinline__ void diva_shear_b(int64_t t, int nTri, int nz, double2 tb, const double *eta_3D_b,
-                                             const double *zeta, double visc_eff_min, double2 *duz_b) {
-  for (int l = 0; l < nz; ++l) {
-    const double f = zeta[l] / fmax(visc_eff_min, eta_3D_b[(int64_t)l * nTri + t]);
-    duz_b[(int64_t)l * nTri + t] = make_double2(tb.x * f, tb.y * f);
-  }
-}
+// A thread per triangle and layer: the division is a chain of its own (in k_finalize, a thread per triangle over all
+// layers, 15.6k triangles x 15 layers took 24 us; the two
+// kernels take 13 and 7).
 __global__ void k_diva_shear_b(int nTri, int nz, const double2 *tau_b, const double *eta_3D_b, const double *zeta,
                                double visc_eff_min, double2 *duz_b) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nTri; t += stride)
-    diva_shear_b(t, nTri, nz, tau_b[t], eta_3D_b, zeta, visc_eff_min, duz_b);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, n = (int64_t)nTri * nz;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const int l = (int)(e / nTri);
+    const double2 tb = tau_b[e - (int64_t)l * nTri];
+    const double f = zeta[l] / fmax(visc_eff_min, eta_3D_b[e]);
+    duz_b[e] = make_double2(tb.x * f, tb.y * f);
+  }
 }
 
 // ---- SSA vertex kernel ----------------------------------------------------------------------
@@ -286,28 +295,55 @@ __global__ void k_diva_shear_b(int nTri, int nz, const double2 *tau_b, const dou
 // (sliding_laws.f90:25-81): all from one pass over the b->a operator row.
 // eta_pred: the learned start's predicted viscosity, which replaces Glen's law in the first
 // iteration of a solve that the prediction armed (no reference counterpart).
-__global__ void k_vertex_ssa(int nV, OpRow ba, const double2 *uv, const double *Avav, const double *Hi,
-                             SlidingIn sl, PhysParams q, const PicardScalars *ps, const double *eta_pred,
-                             double *N_a, double *beta_a) {
+//
+// Four warps per 32 vertices: the velocity gradients in two of them, the basal friction and the flow factor's power in
+// the others.  A warp's FP64 instruction takes its scheduler 64 cycles whatever it masks, so what counts on a mesh of a
+// few thousand vertices is the length of one warp's chain and that every scheduler has one: 8.4k vertices took 27 us
+// with a thread per vertex in blocks of 256 (33 of 152 SMs, two warps a scheduler), 11.7 us like this.
+constexpr int kVertexSsaWarps = 4;
+__global__ void __launch_bounds__(32 * kVertexSsaWarps) k_vertex_ssa(int nV, OpRow ba, const double2 *uv,
+                                                                     const double *Avav, const double *Hi, SlidingIn sl,
+                                                                     PhysParams q, const PicardScalars *ps,
+                                                                     const double *eta_pred, double *N_a,
+                                                                     double *beta_a) {
+  __shared__ double part[3][32];   // vx, vy; 0.5 A^(-1/n)
   const double eps0 = ps->eps0, eta_max = ps->eta_max;
   const bool pred = ps->use_pred != 0 && ps->it == 0;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t vi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vi < nV; vi += stride) {
-    double ux = 0, uy = 0, vx = 0, vy = 0, ua = 0, va = 0;
-    for (int k = ba.ptr[vi]; k < ba.ptr[vi + 1]; ++k) {
-      double2 w = uv[ba.ind[k]];
-      double m = ba.v0[k], dx = ba.v1[k], dy = ba.v2[k];
-      ux = ux + dx * w.x;
-      uy = uy + dy * w.x;
-      vx = vx + dx * w.y;
-      vy = vy + dy * w.y;
-      ua = ua + m * w.x;
-      va = va + m * w.y;
+  const int lane = threadIdx.x & 31, warp = warp_index();
+  const int vi = (int)blockIdx.x * 32 + lane;
+  const bool live = vi < nV;
+  double gx = 0.0, gy = 0.0;   // d/dx and d/dy of u (warp 0) or v (warp 1)
+  if (live) {
+    if (warp < 2) {
+      if (!pred)
+        for (int k = ba.ptr[vi]; k < ba.ptr[vi + 1]; ++k) {
+          const double2 uvk = uv[ba.ind[k]];
+          const double w = warp == 0 ? uvk.x : uvk.y;
+          gx = gx + ba.v1[k] * w;
+          gy = gy + ba.v2[k] * w;
+        }
+      if (warp == 1) {
+        part[0][lane] = gx;
+        part[1][lane] = gy;
+      }
+    } else if (warp == 2) {
+      double ua = 0.0, va = 0.0;
+      for (int k = ba.ptr[vi]; k < ba.ptr[vi + 1]; ++k) {
+        const double2 w = uv[ba.ind[k]];
+        const double m = ba.v0[k];
+        ua = ua + m * w.x;
+        va = va + m * w.y;
+      }
+      beta_a[vi] = sliding_beta(q, sl, vi, ua, va);
+    } else if (!pred) {
+      part[2][lane] = glen2d_flow(Avav[vi], q.n_glen);
     }
-    double eta = pred ? eta_pred[vi] : glen2d(eps0, ux, uy, vx, vy, Avav[vi], q.n_glen);
+  }
+  __syncthreads();
+  if (warp == 0 && live) {
+    double eta = pred ? eta_pred[vi] : glen2d(eps0, gx, gy, part[0][lane], part[1][lane], part[2][lane], q.n_glen);
     eta = fmin(fmax(eta, q.visc_eff_min), eta_max);
     N_a[vi] = eta * fmax(0.1, Hi[vi]);
-    beta_a[vi] = sliding_beta(q, sl, (int)vi, ua, va);
   }
 }
 
@@ -315,48 +351,62 @@ __global__ void k_vertex_ssa(int nV, OpRow ba, const double2 *uv, const double *
 // calc_horizontal_strain_rates, calc_vertical_shear_strain_rates (DIVA_main.f90:375-410),
 // calc_effective_viscosity (:412-479), the surface value of calc_F_integrals' F2 (:481-520) and
 // the vertex part of calc_effective_basal_friction_coefficient (:522-574).
-// One thread per vertex, the layers in a loop.  The FP64 pipe issues a warp instruction at the
-// same cost whatever its active mask, so this pass -- bound by that pipe (the layers' powers, the
-// divisions of F2 and the sliding law) -- keeps every lane busy on its own vertex; per-layer loads
-// and stores of the [layer][vertex] fields stay coalesced across the warp.  du/dz and dv/dz on the
-// triangles come in precomputed (duz_b, formed once per triangle).  The vertical average is summed
-// on the fly in the reference's order (zeta increasing); the F2 integral runs from the base up, so
-// its per-layer terms wait in shared memory, layer-major with one column per thread.
+// A lane per vertex.  The FP64 pipe issues a warp instruction at the same cost whatever its active mask, so this
+// pass -- bound by that pipe (the layers' powers, the divisions of F2 and the sliding law) -- keeps every lane busy on
+// its own vertex; per-layer loads and stores of the [layer][vertex] fields stay coalesced across the warp.  du/dz and dv/dz on the
+// triangles come in precomputed (duz_b, formed once per triangle).  The layers' viscosities
+// and F2 terms wait in shared memory, layer-major with one column per lane, for the vertical average (summed in the
+// reference's order, zeta increasing) and the F2 integral (from the base up).
 // In the first iteration of a solve the learned start armed, every layer takes the predicted
 // vertically averaged viscosity eta_pred instead (a depth-uniform first viscosity).
 // Dynamic shared memory: (kMaxNz + nz * blockDim.x) doubles.
-__global__ void __launch_bounds__(128, 4) k_vertex_diva(int nV, int nTri, int nz, OpRow ba, const double2 *uv,
-                                                        const double2 *uv_base, const double2 *duz_b,
-                                                        const double *A_pow, const double *Hi, const double *zeta_g,
-                                                        SlidingIn sl, PhysParams q, const PicardScalars *ps,
-                                                        const double *eta_pred, double *eta_3D_a, double *N_a,
-                                                        double *F2a1, double *beta_a, double *beta_eff_a) {
+// Six warps per 32 vertices, the layers in turn: as in k_vertex_ssa, one warp's chain of FP64 instructions is what a
+// small mesh waits for, and a large one is evenly spread.  The sums over a row of the b->a operator are split over the
+// warps, the two integrals over the column and the friction go to one warp each.  7.8k vertices x 15 layers: 75 us with
+// a thread per vertex, 34 like this (5, 8 and 16 warps: 36, 35, 36); 58k vertices, where the FP64 pipes are busy either
+// way: 176 and 176 us.
+constexpr int kVertexDivaWarps = 6;
+__global__ void __launch_bounds__(32 * kVertexDivaWarps) k_vertex_diva(
+    int nV, int nTri, int nz, OpRow ba, const double2 *uv, const double2 *uv_base, const double2 *duz_b,
+    const double *A_pow, const double *Hi, const double *zeta_g, SlidingIn sl, PhysParams q, const PicardScalars *ps,
+    const double *eta_pred, double *eta_3D_a, double *N_a, double *F2a1, double *beta_a, double *beta_eff_a) {
   extern __shared__ double vsm[];
-  double *zeta = vsm, *f2 = vsm + kMaxNz + threadIdx.x;
-  for (int k = threadIdx.x; k < nz; k += blockDim.x) zeta[k] = zeta_g[k];
-  __syncthreads();
+  __shared__ double part[5][32];   // ux, uy, vx, vy, F2
+  const int lane = threadIdx.x & 31, warp = warp_index();
+  // zeta^2 and half the layers' spacing: 0.5 (a + b) dz = (a + b) (0.5 dz), the factor being exact
+  double *zeta2 = vsm, *half = vsm + kMaxNz, *es = vsm + 2 * kMaxNz + lane, *f2 = es + nz * 32;
+  for (int k = threadIdx.x; k < nz; k += blockDim.x) {
+    zeta2[k] = zeta_g[k] * zeta_g[k];
+    half[k] = k > 0 ? 0.5 * (zeta_g[k] - zeta_g[k - 1]) : 0.0;
+  }
   const double eps0 = ps->eps0, eta_max = ps->eta_max;
   const bool pred = ps->use_pred != 0 && ps->it == 0;
   const float h_floor_sp = 0.1f;  // max(0.1, Hi) with a default-real literal (DIVA_main.f90:468)
-  const int bd = blockDim.x;
-  const int64_t stride = (int64_t)gridDim.x * bd;
-  for (int64_t vi = (int64_t)blockIdx.x * bd + threadIdx.x; vi < nV; vi += stride) {
-    const int k1 = ba.ptr[vi], k2 = ba.ptr[vi + 1];
-    double ux = 0, uy = 0, vx = 0, vy = 0, ua = 0, va = 0;
+  const int vi = (int)blockIdx.x * 32 + lane;
+  const bool live = vi < nV;
+  const int k1 = live ? ba.ptr[vi] : 0, k2 = live ? ba.ptr[vi + 1] : 0;
+  double ua = 0.0, va = 0.0;   // warp 4
+  if (warp < 4) {
+    const double *g = (warp & 1) ? ba.v2 : ba.v1;
+    double sum = 0.0;
     for (int k = k1; k < k2; ++k) {
-      const int t = ba.ind[k];
-      const double2 w = uv[t], wb = uv_base[t];
-      const double m = ba.v0[k], dx = ba.v1[k], dy = ba.v2[k];
-      ux = ux + dx * w.x;
-      uy = uy + dy * w.x;
-      vx = vx + dx * w.y;
-      vy = vy + dy * w.y;
+      const double2 w = uv[ba.ind[k]];
+      sum = sum + g[k] * (warp < 2 ? w.x : w.y);
+    }
+    part[warp][lane] = sum;
+  } else if (warp == 4) {
+    for (int k = k1; k < k2; ++k) {
+      const double2 wb = uv_base[ba.ind[k]];
+      const double m = ba.v0[k];
       ua = ua + m * wb.x;
       va = va + m * wb.y;
     }
-    double vav = 0.0, e_prev = 0.0;
+  }
+  __syncthreads();
+  if (live) {
+    const double horizontal = glen_horizontal(part[0][lane], part[1][lane], part[2][lane], part[3][lane]);
     const double e_pred = pred ? eta_pred[vi] : 0.0;
-    for (int l = 0; l < nz; ++l) {
+    for (int l = warp; l < nz; l += kVertexDivaWarps) {
       const int64_t ix = (int64_t)l * nV + vi;
       double e = e_pred;
       if (!pred) {
@@ -368,24 +418,67 @@ __global__ void __launch_bounds__(128, 4) k_vertex_diva(int nV, int nTri, int nz
           duz = duz + m * d.x;
           dvz = dvz + m * d.y;
         }
-        e = glen_apow(eps0, ux, uy, vx, vy, duz, dvz, A_pow[ix], q.n_glen);
+        e = glen_apow(eps0, horizontal, duz, dvz, A_pow[ix], q.n_glen);
       }
       e = fmin(fmax(e, q.visc_eff_min), eta_max);
       eta_3D_a[ix] = e;
-      f2[l * bd] = zeta[l] * zeta[l] / e;
-      if (l > 0) vav = vav + 0.5 * (e + e_prev) * (zeta[l] - zeta[l - 1]);
-      e_prev = e;
+      es[l * 32] = e;
+      f2[l * 32] = zeta2[l] / e;
     }
-    N_a[vi] = vav * fmax((double)h_floor_sp, Hi[vi]);
-    // F2 at the surface: integrate zeta^2/eta from the base (zeta = 1) up to zeta(1) = 0
-    double intg = 0.0;
-    for (int l = nz - 1; l >= 1; --l) intg = intg - 0.5 * (f2[l * bd] + f2[(l - 1) * bd]) * (zeta[l] - zeta[l - 1]);
-    const double F2 = -fmax(0.1, Hi[vi]) * intg;
-    F2a1[vi] = F2;
-    const double b = sliding_beta(q, sl, (int)vi, ua, va);
-    beta_a[vi] = b;
+  }
+  __syncthreads();
+  double b = 0.0;
+  if (live) {
+    if (warp == 0) {
+      double vav = 0.0;
+      for (int l = 1; l < nz; ++l) vav = vav + (es[l * 32] + es[(l - 1) * 32]) * half[l];
+      N_a[vi] = vav * fmax((double)h_floor_sp, Hi[vi]);
+    } else if (warp == 1) {
+      // F2 at the surface: integrate zeta^2/eta from the base (zeta = 1) up to zeta(1) = 0
+      double intg = 0.0;
+      for (int l = nz - 1; l >= 1; --l) intg = intg - (f2[l * 32] + f2[(l - 1) * 32]) * half[l];
+      const double F2 = -fmax(0.1, Hi[vi]) * intg;
+      F2a1[vi] = F2;
+      part[4][lane] = F2;
+    } else if (warp == 4) {
+      b = sliding_beta(q, sl, vi, ua, va);
+      beta_a[vi] = b;
+    }
+  }
+  __syncthreads();
+  if (warp == 4 && live) {
+    const double F2 = part[4][lane];
     beta_eff_a[vi] = (q.sliding_law == UFE_SLIDING_NO_SLIDING) ? 1.0 / F2 : b / (1.0 + b * F2);
   }
+}
+
+// Entries a double-word copy cannot carry: beyond the FP32 range, not finite, or so small
+// (below 1e-30) that the low word would leave the normal FP32 range.
+// On bit patterns (positive numbers order as their bits, NaN and infinity above all): three comparisons per value
+// were a third of the FP64 instructions that an entry's double-word copy took.
+__device__ __forceinline__ bool pair_unsafe(double a, bool tiny_matters) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+  return b > (unsigned long long)__double_as_longlong(1e36) ||
+         (tiny_matters && b != 0 && b < (unsigned long long)__double_as_longlong(1e-30));
+}
+
+// The double-word form of a block that is not pair_unsafe, as to_dwblk gives it.  The high word is the value rounded to
+// 24 bits, to nearest and ties to even, which needs no FP64 conversion either way.
+__device__ __forceinline__ void pair_words(double x, float &hi, float &lo) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long r = (u + 0x0fffffffull + ((u >> 29) & 1ull)) & ~0x1fffffffull;
+  const unsigned int sign = (unsigned int)(r >> 32) & 0x80000000u;
+  const unsigned long long mag = (r & 0x7fffffffffffffffull) >> 29;   // 11 bits of exponent, 23 of mantissa
+  hi = __uint_as_float(sign | (unsigned int)(mag ? mag - (896ull << 23) : 0ull));   // exponent bias 1023 -> 127
+  lo = (float)(x - __longlong_as_double((long long)r));
+}
+__device__ __forceinline__ dwblk pair_block(double4 b) {
+  dwblk o;
+  pair_words(b.x, o.hi.x, o.lo.x);
+  pair_words(b.y, o.hi.y, o.lo.y);
+  pair_words(b.z, o.hi.z, o.lo.z);
+  pair_words(b.w, o.hi.w, o.lo.w);
+  return o;
 }
 
 // ---- assembly -----------------------------------------------------------------------------
@@ -411,6 +504,11 @@ struct AssembleArgs {
   // outputs
   double4 *blk;
   float4 *blk32, *rowsum32;
+  const int32_t *sell_map;  // the sliced-ELL copies (sell_blk null: none)
+  double4 *sell_blk;
+  float4 *sell_blk32;
+  dwblk *sell_blkp;
+  int *pair_bad;
   double2 *rhs, *dinv, *X, *R, *RP, *P0, *V0;
   float2 *dinv32;
   double *beta_b_out, *bfc_b, *F2b1, *eta_3D_b;
@@ -430,57 +528,86 @@ __device__ __forceinline__ int find_col(const int32_t *ind, int k1, int k2, int 
   return -1;
 }
 
+// Four warps per 32 triangles.  FP64 instructions bound it (a warp's takes its scheduler 64 cycles whatever it masks),
+// so the lanes are kept full and the warps even: of the sums over the a->b rows each warp forms one for all 32 triangles
+// (N, dN/dx, dN/dy, friction) and a share of the layers, then the triangles' matrix entries, which are consecutive, go
+// round the block's threads, each thread looking its row up; the terms of the row's product with the initial guess wait
+// in shared memory for a lane per triangle to add them up in storage order, a warp for each component.  Products are
+// shared between the four entries of a block (scaling by two and by four is exact, so each keeps its value): 17
+// instructions a free row's entry instead of 24.  A thread per triangle in blocks of 256, the norms in the same kernel
+// and the sliced copy in another, took 52 us on 16.7k triangles (65 of 152 SMs) and 203 us on 115k (DIVA, double-word);
+// this kernel takes 23 and 129 us, k_assemble_norms 10 and 15.
+constexpr int kRowThreads = 128, kRowChunk = 384;
 template <int MODE>
-__global__ void k_assemble(AssembleArgs a, PhysParams q, CondArg cond) {
-  double acc[2] = {0.0, 0.0};
-  const int nTri = a.nTri;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t64 < nTri; t64 += stride) {
-    const int t = (int)t64;
-    // -- coefficients of this triangle
-    double N, dNx, dNy, beta;
-    if (MODE == kFromTriangles) {
-      N = a.N_b[t]; dNx = a.dNx_b[t]; dNy = a.dNy_b[t]; beta = a.beta_b_in[t];
-    } else {
-      N = 0.0; dNx = 0.0; dNy = 0.0; beta = 0.0;
-      double bfc = 0.0, f2 = 0.0;
-      const double *bsrc = (MODE == kFromSSA) ? a.beta_a : a.beta_eff_a;
-      for (int k = a.ab.ptr[t]; k < a.ab.ptr[t + 1]; ++k) {
-        int v = a.ab.ind[k];
-        double m = a.ab.v0[k], na = a.N_a[v];
-        N = N + m * na;
-        dNx = dNx + a.ab.v1[k] * na;
-        dNy = dNy + a.ab.v2[k] * na;
-        beta = beta + m * bsrc[v];
-        if (MODE == kFromDIVA) {
-          bfc = bfc + m * a.beta_a[v];
-          f2 = f2 + m * a.F2a1[v];
-        }
+__global__ void __launch_bounds__(kRowThreads) k_assemble_rows(AssembleArgs a, PhysParams q) {
+  __shared__ double coef[4][32];     // N, dN/dx, dN/dy, beta
+  __shared__ double rhs_sm[2][32], diag_sm[2][32];
+  __shared__ double2 terms[kRowChunk];
+  __shared__ int ptr_sm[33], kd_sm[32];
+  __shared__ bool special_sm[32];
+  const int nTri = a.nTri, lane = threadIdx.x & 31, warp = warp_index();
+  const int t0 = blockIdx.x * 32, t = t0 + lane;
+  const bool live = t < nTri;
+  if (threadIdx.x <= 32) ptr_sm[threadIdx.x] = a.m2_ptr[min(t0 + (int)threadIdx.x, nTri)];
+  if (warp == 3) {
+    kd_sm[lane] = INT_MAX;
+    special_sm[lane] = live && ((q.has_bc && a.bc_mask[t] == 1) || a.TriBI[t] > 0);
+  }
+  // -- coefficients of the triangles
+  if (MODE == kFromTriangles) {
+    const double *src = warp == 0 ? a.N_b : warp == 1 ? a.dNx_b : warp == 2 ? a.dNy_b : a.beta_b_in;
+    coef[warp][lane] = live ? src[t] : 0.0;
+  } else {
+    const double *bsrc = (MODE == kFromSSA) ? a.beta_a : a.beta_eff_a;
+    const double *w = warp == 1 ? a.ab.v1 : warp == 2 ? a.ab.v2 : a.ab.v0, *src = warp == 3 ? bsrc : a.N_a;
+    const int e1 = live ? a.ab.ptr[t] : 0, e2 = live ? a.ab.ptr[t + 1] : 0;
+    double sum = 0.0;
+    for (int k = e1; k < e2; ++k) sum = sum + w[k] * src[a.ab.ind[k]];
+    if (MODE == kFromDIVA) {
+      if (warp < 2) {
+        const double *src2 = warp == 0 ? a.beta_a : a.F2a1;
+        double s2 = 0.0;
+        for (int k = e1; k < e2; ++k) s2 = s2 + a.ab.v0[k] * src2[a.ab.ind[k]];
+        if (live) (warp == 0 ? a.bfc_b : a.F2b1)[t] = s2;
       }
-      if (q.gl_subgrid) {   // f_gr^p; the default p = 2 as a product
-        const double f = a.fgr_b[t];
-        beta = beta * (q.fgr_exp == 2.0 ? f * f : q.fgr_exp == 1.0 ? f : pow(f, q.fgr_exp));
-      }
-      if (MODE == kFromDIVA) {
-        a.bfc_b[t] = bfc;
-        a.F2b1[t] = f2;
-        for (int l = 0; l < a.nz; ++l) {
+      if (live)
+        for (int l = warp; l < a.nz; l += 4) {
           double e = 0.0;
-          for (int k = a.ab.ptr[t]; k < a.ab.ptr[t + 1]; ++k)
-            e = e + a.ab.v0[k] * a.eta_3D_a[(int64_t)l * a.nV + a.ab.ind[k]];
+          for (int k = e1; k < e2; ++k) e = e + a.ab.v0[k] * a.eta_3D_a[(int64_t)l * a.nV + a.ab.ind[k]];
           a.eta_3D_b[(int64_t)l * nTri + t] = e;
         }
-      }
-      a.beta_b_out[t] = beta;
     }
-    // -- block row on the 2nd-order b_b pattern
-    const int k1 = a.m2_ptr[t], k2 = a.m2_ptr[t + 1];
-    const int kd = find_col(a.m2_ind, k1, k2, t);
-    if (kd < 0) { atomicOr(a.err, kErrNoDiag); continue; }
-    double2 rhs;
-    const int bcm = q.has_bc ? a.bc_mask[t] : 0;
-    const int tbi = a.TriBI[t];
-    if (bcm == 1 || tbi > 0) {
+    if (warp == 3 && live) {
+      if (q.gl_subgrid) {   // f_gr^p; the default p = 2 as a product
+        const double f = a.fgr_b[t];
+        sum = sum * (q.fgr_exp == 2.0 ? f * f : q.fgr_exp == 1.0 ? f : pow(f, q.fgr_exp));
+      }
+      a.beta_b_out[t] = sum;
+    }
+    coef[warp][lane] = sum;
+  }
+  __syncthreads();
+  // -- block rows on the 2nd-order b_b pattern: the first diagonal entry of each
+  const int c_begin = ptr_sm[0], c_end = ptr_sm[32];
+  auto row_of = [&](int k) {   // the row that holds entry k
+    int r = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (ptr_sm[r + step] <= k) r += step;
+    return r;
+  };
+  for (int k = c_begin + threadIdx.x; k < c_end; k += kRowThreads) {
+    const int r = row_of(k);
+    if (a.m2_ind[k] == t0 + r) atomicMin(&kd_sm[r], k);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int k1 = ptr_sm[lane], k2 = ptr_sm[lane + 1], kd = kd_sm[lane];
+    const int tbi = live ? a.TriBI[t] : 0, bcm = live && q.has_bc ? a.bc_mask[t] : 0;
+    double2 rhs = make_double2(0.0, 0.0);
+    if (live && kd == INT_MAX) {
+      atomicOr(a.err, kErrNoDiag);
+    } else if (special_sm[lane]) {
       for (int k = k1; k < k2; ++k) a.blk[k] = make_double4(0.0, 0.0, 0.0, 0.0);
       double *bd = reinterpret_cast<double *>(a.blk);
       if (bcm == 1) {
@@ -521,64 +648,118 @@ __global__ void k_assemble(AssembleArgs a, PhysParams q, CondArg cond) {
           }
         }
       }
-    } else {
-      // free rows (calc_SSA_DIVA_stiffness_matrix_row_free :180-329, sans variant :331-479)
-      for (int k = k1; k < k2; ++k) {
-        const int tj = a.m2_ind[k];
-        const double x_ = a.m2_x[k], y_ = a.m2_y[k], xx = a.m2_xx[k], xy = a.m2_xy[k], yy = a.m2_yy[k];
-        double uAu, uAv, vAu, vAv;
-        if (q.crossterms) {
-          uAu = 4.0 * N * xx + 4.0 * dNx * x_ + N * yy + dNy * y_;
-          uAv = 3.0 * N * xy + 2.0 * dNx * y_ + dNy * x_;
-          vAv = 4.0 * N * yy + 4.0 * dNy * y_ + N * xx + dNx * x_;
-          vAu = 3.0 * N * xy + 2.0 * dNy * x_ + dNx * y_;
-          if (tj == t) { uAu = uAu - beta; vAv = vAv - beta; }
-        } else {
-          uAu = 4.0 * xx + yy;
-          uAv = 3.0 * xy;
-          vAv = 4.0 * yy + xx;
-          vAu = 3.0 * xy;
-          if (tj == t) { uAu = uAu - beta / N; vAv = vAv - beta / N; }
-        }
-        a.blk[k] = make_double4(uAu, uAv, vAu, vAv);
-      }
-      double2 td = a.tau_d[t];
+    } else if (live) {
+      const double2 td = a.tau_d[t];
+      const double N = coef[0][lane];
       rhs = q.crossterms ? make_double2(-td.x, -td.y) : make_double2(-td.x / N, -td.y / N);
     }
-    // -- Jacobi diagonal (PCJACOBI; a zero diagonal entry is replaced by one)
-    const double4 dg = a.blk[kd];
-    const double2 di = make_double2(dg.x != 0.0 ? 1.0 / dg.x : 1.0, dg.w != 0.0 ? 1.0 / dg.w : 1.0);
-    a.dinv[t] = di;
-    a.rhs[t] = rhs;
-    if (a.blk32) {
-      double4 rs = make_double4(0.0, 0.0, 0.0, 0.0);
-      for (int k = k1; k < k2; ++k) {
-        double4 b = a.blk[k];
-        a.blk32[k] = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
-        rs.x += b.x; rs.y += b.y; rs.z += b.z; rs.w += b.w;
+    rhs_sm[0][lane] = rhs.x;
+    rhs_sm[1][lane] = rhs.y;
+  }
+  __syncthreads();
+  double ax = 0.0;   // the row's product with the initial guess: component `warp` of triangle `lane`
+  for (int c0 = c_begin; c0 < c_end; c0 += kRowChunk) {
+    const int c1 = min(c0 + kRowChunk, c_end);
+    for (int k = c0 + threadIdx.x; k < c1; k += kRowThreads) {
+      const int r = row_of(k), tj = a.m2_ind[k];
+      double4 b;
+      if (special_sm[r]) {
+        b = a.blk[k];
+      } else {
+        // free rows (calc_SSA_DIVA_stiffness_matrix_row_free :180-329, sans variant :331-479)
+        const double x_ = a.m2_x[k], y_ = a.m2_y[k], xx = a.m2_xx[k], xy = a.m2_xy[k], yy = a.m2_yy[k];
+        const double N = coef[0][r];
+        if (q.crossterms) {
+          //   uu = 4 N xx + 4 dNx x + N yy + dNy y     uv = 3 N xy + 2 dNx y + dNy x
+          //   vv = 4 N yy + 4 dNy y + N xx + dNx x     vu = 3 N xy + 2 dNy x + dNx y
+          const double dNx = coef[1][r], dNy = coef[2][r];
+          const double nxx = N * xx, nyy = N * yy, dxx = dNx * x_, dyy = dNy * y_, dxy = dNx * y_, dyx = dNy * x_;
+          const double n3 = 3.0 * N * xy;
+          b.x = fma(4.0, nxx + dxx, nyy) + dyy;
+          b.y = fma(2.0, dxy, n3) + dyx;
+          b.w = fma(4.0, nyy + dyy, nxx) + dxx;
+          b.z = fma(2.0, dyx, n3) + dxy;
+          if (tj == t0 + r) {
+            const double beta = coef[3][r];
+            b.x = b.x - beta;
+            b.w = b.w - beta;
+          }
+        } else {
+          b.x = 4.0 * xx + yy;
+          b.y = 3.0 * xy;
+          b.w = 4.0 * yy + xx;
+          b.z = 3.0 * xy;
+          if (tj == t0 + r) {
+            const double bN = coef[3][r] / N;
+            b.x = b.x - bN;
+            b.w = b.w - bN;
+          }
+        }
+        a.blk[k] = b;
       }
-      a.rowsum32[t] = make_float4((float)rs.x, (float)rs.y, (float)rs.z, (float)rs.w);
-      a.dinv32[t] = make_float2((float)di.x, (float)di.y);
-    }
-    // -- Krylov initial residual r = D^-1 (b - A x0)
-    double2 ax = make_double2(0.0, 0.0);
-    double2 x0t = make_double2(0.0, 0.0);
-    if (a.x0) {
-      x0t = a.x0[t];
-      for (int k = k1; k < k2; ++k) {
-        double4 b = a.blk[k];
-        double2 xj = a.x0[a.m2_ind[k]];
-        ax.x += b.x * xj.x + b.y * xj.y;
-        ax.y += b.z * xj.x + b.w * xj.y;
+      if (k == kd_sm[r]) {
+        diag_sm[0][r] = b.x;
+        diag_sm[1][r] = b.w;
+      }
+      if (a.sell_blk) {
+        const int32_t slot = a.sell_map[k];
+        a.sell_blk[slot] = b;
+        if (a.sell_blkp) {
+          if (pair_unsafe(b.x, true) || pair_unsafe(b.y, true) || pair_unsafe(b.z, true) || pair_unsafe(b.w, true))
+            atomicOr(a.pair_bad, 1);   // the double-word solve is not taken
+          else
+            a.sell_blkp[slot] = pair_block(b);
+        }
+      }
+      if (a.blk32) {
+        const float4 f = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
+        a.blk32[k] = f;
+        if (a.sell_blk) a.sell_blk32[a.sell_map[k]] = f;
+      }
+      if (a.x0) {
+        const double2 xj = a.x0[tj];
+        terms[k - c0] = make_double2(b.x * xj.x + b.y * xj.y, b.z * xj.x + b.w * xj.y);
       }
     }
-    a.X[t] = x0t;
-    double2 r = make_double2(di.x * (rhs.x - ax.x), di.y * (rhs.y - ax.y));
-    double2 db = make_double2(di.x * rhs.x, di.y * rhs.y);
-    a.R[t] = r;
-    a.RP[t] = r;
+    __syncthreads();
+    if (a.x0 && warp < 2) {
+      const int k2 = min(ptr_sm[lane + 1], c1);
+      for (int k = max(ptr_sm[lane], c0); k < k2; ++k) ax += reinterpret_cast<const double *>(terms + (k - c0))[warp];
+    }
+    if (c1 < c_end) __syncthreads();
+  }
+  if (!live || kd_sm[lane] == INT_MAX) return;
+  if (warp < 2) {
+    // -- Jacobi diagonal (PCJACOBI; a zero diagonal entry is replaced by one), Krylov initial residual
+    //    r = D^-1 (b - A x0)
+    const double d = diag_sm[warp][lane], rc = rhs_sm[warp][lane];
+    const double di = d != 0.0 ? 1.0 / d : 1.0, r = di * (rc - ax);
+    const int64_t o = 2 * (int64_t)t + warp;
+    reinterpret_cast<double *>(a.dinv)[o] = di;
+    reinterpret_cast<double *>(a.rhs)[o] = rc;
+    reinterpret_cast<double *>(a.R)[o] = r;
+    reinterpret_cast<double *>(a.RP)[o] = r;
+    if (a.blk32) reinterpret_cast<float *>(a.dinv32)[o] = (float)di;
+  } else if (warp == 2) {
+    a.X[t] = a.x0 ? a.x0[t] : make_double2(0.0, 0.0);
+  } else {
     a.P0[t] = make_double2(0.0, 0.0);
     a.V0[t] = make_double2(0.0, 0.0);
+  }
+  if (a.blk32) {   // the FP32 inner solve's row sums, component `warp`
+    double rs = 0.0;
+    for (int k = ptr_sm[lane]; k < ptr_sm[lane + 1]; ++k) rs += reinterpret_cast<const double *>(a.blk + k)[warp];
+    reinterpret_cast<float *>(a.rowsum32)[4 * (int64_t)t + warp] = (float)rs;
+  }
+}
+
+// The norms of the initial residual and right-hand side, and the Krylov solve's starting scalars.
+__global__ void k_assemble_norms(AssembleArgs a, CondArg cond) {
+  double acc[2] = {0.0, 0.0};
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.nTri; t += stride) {
+    const double2 di = a.dinv[t], rhs = a.rhs[t], r = a.R[t];
+    const double2 db = make_double2(di.x * rhs.x, di.y * rhs.y);
     acc[0] += r.x * r.x + r.y * r.y;
     acc[1] += db.x * db.x + db.y * db.y;
   }
@@ -794,8 +975,7 @@ template <bool DIVA>
 __global__ void k_finalize(int nTri, const double2 *X, double2 *uv, PhysParams q, PicardScalars *ps,
                            KrylovScalars *ks, const double *beta_eff_b, const double *bfc_b, const double *F2b1,
                            double2 *uv_base, double2 *tau_b, double *partials, unsigned int *tickets,
-                           CondArg cond, int nz = 0, const double *eta_3D_b = nullptr,
-                           const double *zeta = nullptr, double2 *duz_b = nullptr) {
+                           CondArg cond) {
   const double r = ps->relax;
   double acc[2] = {0.0, 0.0};
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -814,9 +994,7 @@ __global__ void k_finalize(int nTri, const double2 *X, double2 *uv, PhysParams q
         uv_base[t] = make_double2(u / den, v / den);
       }
       double be = beta_eff_b[t];
-      const double2 tb = make_double2(u * be, v * be);
-      tau_b[t] = tb;
-      diva_shear_b(t, nTri, nz, tb, eta_3D_b, zeta, q.visc_eff_min, duz_b);   // for the next iteration
+      tau_b[t] = make_double2(u * be, v * be);
     }
     acc[0] += (u - o.x) * (u - o.x) + (v - o.y) * (v - o.y);
     acc[1] += (u + o.x) * (u + o.x) + (v + o.y) * (v + o.y);
@@ -983,29 +1161,6 @@ static void check_operators(ufe_ctx *ctx) {
 }
 
 // The sliced-ELL layout of the stiffness pattern (the 2nd-order b_b operators' pattern).
-// Entries a double-word copy cannot carry: beyond the FP32 range, not finite, or so small
-// (below 1e-30) that the low word would leave the normal FP32 range.
-__device__ __forceinline__ bool pair_unsafe(double a, bool tiny_matters) {
-  const double m = fabs(a);
-  return !(m <= 1e36) || (tiny_matters && m != 0.0 && m < 1e-30);
-}
-
-__global__ void k_sell_fill(int64_t nnzb, const int32_t *__restrict__ map, const double4 *__restrict__ blk,
-                            const float4 *__restrict__ blk32, double4 *__restrict__ sblk, float4 *__restrict__ sblk32,
-                            dwblk *__restrict__ sblkp, int *pair_bad) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nnzb) return;
-  const int32_t slot = map[k];
-  const double4 b = blk[k];
-  sblk[slot] = b;
-  sblk32[slot] = blk32[k];
-  if (sblkp) {
-    sblkp[slot] = to_dwblk(b);
-    if (pair_unsafe(b.x, true) || pair_unsafe(b.y, true) || pair_unsafe(b.z, true) || pair_unsafe(b.w, true))
-      atomicOr(pair_bad, 1);
-  }
-}
-
 // UFE_PREC_FP32_PAIR, around the persistent double-word BiCGStab.  One round:
 //   k_pair_enter  the FP64 start (x, r, r^, D^-1; p = v = 0) in double-word form
 //   k_pair_decide the double-word solve takes the linear solve ([0] -> [2], [0] inactive) unless a
@@ -1483,6 +1638,11 @@ struct Solver {
     a.blk = w->blk;
     a.blk32 = (p.precision == UFE_PREC_FP32_REFINE) ? w->blk32 : nullptr;
     a.rowsum32 = w->rowsum32;
+    a.sell_map = w->sell_map;
+    a.sell_blk = use_sell() ? w->sell_blk : nullptr;
+    a.sell_blk32 = w->sell_blk32;
+    a.sell_blkp = pair_ok() ? w->sell_blkp : nullptr;
+    a.pair_bad = w->pair_bad;
     a.rhs = w->kv.B; a.dinv = w->kv.dinv; a.X = w->kv.X; a.R = w->kv.R; a.RP = w->kv.RP;
     a.P0 = w->kv.P[0]; a.V0 = w->kv.V[0]; a.dinv32 = w->kv.dinv32;
     a.beta_b_out = w->beta_b; a.bfc_b = w->bfc_b; a.F2b1 = w->F2b1; a.eta_3D_b = w->eta_3D_b;
@@ -1500,17 +1660,13 @@ struct Solver {
 
   void enqueue_assemble(int mode, bool x0_current, CondArg c) {
     AssembleArgs a = assemble_args(x0_current ? w->uv : nullptr, mode);
-    int g = eblocks(w->nTri);
-    if (mode == kFromTriangles) k_assemble<kFromTriangles><<<g, kThreads, 0, s>>>(a, q, c);
-    else if (mode == kFromSSA) k_assemble<kFromSSA><<<g, kThreads, 0, s>>>(a, q, c);
-    else k_assemble<kFromDIVA><<<g, kThreads, 0, s>>>(a, q, c);
+    const unsigned g = (unsigned)((w->nTri + 31) / 32);
+    if (mode == kFromTriangles) k_assemble_rows<kFromTriangles><<<g, kRowThreads, 0, s>>>(a, q);
+    else if (mode == kFromSSA) k_assemble_rows<kFromSSA><<<g, kRowThreads, 0, s>>>(a, q);
+    else k_assemble_rows<kFromDIVA><<<g, kRowThreads, 0, s>>>(a, q);
     UFE_CUDA(cudaGetLastError());
-    if (use_sell()) {
-      k_sell_fill<<<(unsigned)((w->nnzb + 255) / 256), 256, 0, s>>>(
-          w->nnzb, w->sell_map, w->blk, w->blk32, w->sell_blk, w->sell_blk32, pair_ok() ? w->sell_blkp : nullptr,
-          w->pair_bad);
-      UFE_CUDA(cudaGetLastError());
-    }
+    k_assemble_norms<<<eblocks(w->nTri), kThreads, 0, s>>>(a, c);
+    UFE_CUDA(cudaGetLastError());
   }
 
   template <class M>
@@ -1800,34 +1956,39 @@ struct Solver {
         w->nV, w->nTri, w->nz, ab, w->Hi, w->Hs, A_src(), ctx->zeta, w->tau_d, diva ? nullptr : w->Avav,
         diva ? w->A_pow : nullptr, w->ps, w->ks, p.visc_it_relax, p.Glens_flow_law_epsilon_sq_0,
         p.Glens_flow_law_exponent, w->pred_flag);
-    if (diva)
-      k_diva_shear_b<<<eblocks(w->nTri), kThreads, 0, s>>>(w->nTri, w->nz, w->tau_b, w->eta_3D_b, ctx->zeta,
-                                                           p.visc_eff_min, w->duz_b);
+    if (diva) enqueue_shear();
     UFE_CUDA(cudaMemsetAsync(w->ks + 1, 0, sizeof(KrylovScalars), s));
     UFE_CUDA(cudaGetLastError());
   }
 
   void enqueue_picard_pre(bool diva, CondArg inner) {
     if (diva) {
-      const int tpb = w->nz <= 40 ? 128 : 64;
-      const size_t smem = (size_t)(kMaxNz + w->nz * tpb) * sizeof(double);
-      k_vertex_diva<<<pick_blocks(w->nV, tpb, 1 << 20), tpb, smem, s>>>(
+      const size_t smem = (size_t)(2 * kMaxNz + 2 * w->nz * 32) * sizeof(double);
+      UFE_CUDA(cudaFuncSetAttribute(k_vertex_diva, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k_vertex_diva<<<(w->nV + 31) / 32, 32 * kVertexDivaWarps, smem, s>>>(
           w->nV, w->nTri, w->nz, ba, w->uv, w->uv_base, w->duz_b, w->A_pow, w->Hi, ctx->zeta,
           sliding(), q, w->ps, w->eta_pred_a, w->eta_3D_a, w->N_a, w->F2a1, w->beta_a, w->beta_eff_a);
     } else {
-      k_vertex_ssa<<<eblocks(w->nV), kThreads, 0, s>>>(w->nV, ba, w->uv, w->Avav, w->Hi, sliding(), q, w->ps,
-                                                       w->eta_pred_a, w->N_a, w->beta_a);
+      k_vertex_ssa<<<(w->nV + 31) / 32, 32 * kVertexSsaWarps, 0, s>>>(w->nV, ba, w->uv, w->Avav, w->Hi, sliding(), q,
+                                                                     w->ps, w->eta_pred_a, w->N_a, w->beta_a);
     }
     UFE_CUDA(cudaGetLastError());
     enqueue_assemble(diva ? kFromDIVA : kFromSSA, p.krylov_initial_guess == UFE_X0_CURRENT, inner);
   }
 
+  // the shear rates of the basal stress and viscosity, for the vertex kernel
+  void enqueue_shear() {
+    k_diva_shear_b<<<eblocks((int64_t)w->nTri * w->nz), kThreads, 0, s>>>(w->nTri, w->nz, w->tau_b, w->eta_3D_b,
+                                                                         ctx->zeta, p.visc_eff_min, w->duz_b);
+  }
   void enqueue_picard_post(bool diva, CondArg outer) {
-    if (diva)
+    if (diva) {
       k_finalize<true><<<eblocks(w->nTri), kThreads, 0, s>>>(w->nTri, w->kv.X, w->uv, q, w->ps, w->ks, w->beta_b,
                                                              w->bfc_b, w->F2b1, w->uv_base, w->tau_b,
-                                                             ctx->red.partials, ctx->red.tickets, outer, w->nz,
-                                                             w->eta_3D_b, ctx->zeta, w->duz_b);
+                                                             ctx->red.partials, ctx->red.tickets, outer);
+      UFE_CUDA(cudaGetLastError());
+      enqueue_shear();
+    }
     else
       k_finalize<false><<<eblocks(w->nTri), kThreads, 0, s>>>(w->nTri, w->kv.X, w->uv, q, w->ps, w->ks, nullptr,
                                                               nullptr, nullptr, nullptr, nullptr,
