@@ -45,7 +45,6 @@ constexpr double kIceDensity = 910.0;
 constexpr double kShapeQ = 1.5;
 
 constexpr int kMaxNz = 256;
-constexpr int kSmemBudget = 200 * 1024;
 
 // Zeta operators in tridiagonal form (device): zeta, then d/dzeta l/d/u, then d2/dzeta2 l/d/u.
 struct ZOps {
@@ -90,7 +89,20 @@ __device__ __forceinline__ double conductivity(const Consts &c, double T) {
 __device__ __forceinline__ double melting_point(double Hi_eff, double zeta) {
   return kT0 - kCCGradient * Hi_eff * zeta;
 }
-__device__ __forceinline__ bool unstable_value(double T) { return T != T || T < 180.0 || T > kT0; }
+// NaN, below 180 K or above T0, on bit patterns (positive numbers order as their bits; the sign bit makes a negative
+// one larger than all of them): no FP64 instructions, which bound the column passes.
+__device__ __forceinline__ bool unstable_value(double T) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(T);
+  return b - (unsigned long long)__double_as_longlong(180.0) >
+         (unsigned long long)__double_as_longlong(kT0) - (unsigned long long)__double_as_longlong(180.0);
+}
+// min(x, limit) for a positive finite limit, as fmin gives it (limit for a NaN x), without FP64 instructions:
+// positive values order as their bits, a negative value's bits are a negative integer.
+__device__ __forceinline__ double min_limit(double x, double limit) {
+  const long long b = __double_as_longlong(x), l = __double_as_longlong(limit);
+  const bool nan = ((unsigned long long)b << 1) > 0xffe0000000000000ull;
+  return (nan || b > l) ? limit : x;
+}
 
 // ---- row inputs --------------------------------------------------------------------------
 struct Layer {
@@ -212,11 +224,12 @@ __device__ bool solve_column(const In &in, const typename In::Col &col, const ZO
     const double Cpi = heat_capacity(cs_, L.Ti0);
     const double Ki = conductivity(cs_, L.Ti0);
     const double c1 = L.dzt + (L.u * L.dzx) + (L.v * L.dzy) + (L.w * L.dzz);
-    const double c2 = -(Ki / (kIceDensity * Cpi) * (L.dzz * L.dzz));
+    const double rc = kIceDensity * Cpi, r_rc = 1.0 / rc;
+    const double c2 = -(div_by(Ki, rc, r_rc) * (L.dzz * L.dzz));
     const double a = (c1 * __ldg(z.l1 + k)) + (c2 * __ldg(z.l2 + k));
     double b = inv_dt + (c1 * __ldg(z.d1 + k)) + (c2 * __ldg(z.d2 + k));
     const double c = (c1 * __ldg(z.u1 + k)) + (c2 * __ldg(z.u2 + k));
-    double d = Tc / dt - L.udx - L.vdy + L.phi / (kIceDensity * Cpi);
+    double d = div_by(Tc, dt, inv_dt) - L.udx - L.vdy + div_by(L.phi, rc, r_rc);
     // Thomas forward elimination
     const double wgt = a / bprev;
     b = b - wgt * cprev;
@@ -251,14 +264,14 @@ __device__ bool solve_column(const In &in, const typename In::Col &col, const ZO
   bool stable = true;
   double x = d_b / bprev;
   {
-    double v = fmin(x, pmp_b);
+    double v = min_limit(x, pmp_b);
     if (combine) v = fr * v + (1.0 - fr) * out[(int64_t)kb * os];
     out[(int64_t)kb * os] = v;
     stable &= !unstable_value(v);
   }
   for (int k = nz - 2; k >= 0; --k) {
     x = (Ds[k * T] - Cs[k * T] * x) / Bs[k * T];
-    double v = fmin(x, melting_point(Hi_eff, __ldg(z.zeta + k)));
+    double v = min_limit(x, melting_point(Hi_eff, __ldg(z.zeta + k)));
     if (combine) v = fr * v + (1.0 - fr) * out[(int64_t)k * os];
     out[(int64_t)k * os] = v;
     stable &= !unstable_value(v);
@@ -286,8 +299,14 @@ __device__ bool column_substep(const In &in, const ZOps &z, const Consts &c, int
 }
 
 // ---- the three passes ------------------------------------------------------------------------
+// A thread per column, bound by FP64 instructions (85% of the pipes' cycles).  So the quotients that share a divisor
+// share its reciprocal, and minima and the stability check work on bit patterns: 101 FP64 instructions a row instead of
+// 115, all values the same to the bit.  Blocks of one warp: the columns' shared memory (3 x 8 bytes a layer) lets nine
+// of them on an SM at 30 layers, against two blocks of four, and the last wave is short.  200k columns x 30 layers:
+// 1.24 ms a step (blocks of 64 and 128: 1.27 and 1.32), 1.49 before.
+constexpr int kColumnThreads = 32;
 template <class In>
-__global__ void __launch_bounds__(128) k_heat_columns(In in, ZOps z, Consts c, VertexFields vf, int64_t nV,
+__global__ void __launch_bounds__(kColumnThreads) k_heat_columns(In in, ZOps z, Consts c, VertexFields vf, int64_t nV,
                                                       const double *__restrict__ Ti_cur, double *__restrict__ Ti_next,
                                                       Lists lists, Counters *cnt) {
   if (cnt->err) return;
@@ -345,13 +364,6 @@ constexpr int kRetryLevels = 9;          // dt / 2 ... dt / 512 (:163)
 constexpr int kRetryArrays = 4 + 2 * kRetryLevels;
 constexpr int kRetryBlocks = 4 * 152;
 
-// min(x, limit) for a positive finite limit, as fmin gives it (limit for a NaN x), without FP64 instructions:
-// positive values order as their bits, a negative value's bits are a negative integer.
-__device__ __forceinline__ double min_limit(double x, double limit) {
-  const long long b = __double_as_longlong(x), l = __double_as_longlong(limit);
-  const bool nan = ((unsigned long long)b << 1) > 0xffe0000000000000ull;
-  return (nan || b > l) ? limit : x;
-}
 __device__ __forceinline__ double shfl_up_d(double v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ double shfl_down_d(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
 
@@ -1064,12 +1076,6 @@ void validate_thermo_params(const ufe_thermo_params *p) {
               UFE_ERR_INVALID, "unknown choice_GL_temperature_BC");
 }
 
-int threads_for(int nz) {
-  int T = 128;
-  while (T > 32 && (size_t)3 * nz * T * sizeof(double) > (size_t)kSmemBudget) T /= 2;
-  return T;
-}
-
 }  // namespace
 
 // ---- work area -------------------------------------------------------------------------------
@@ -1188,7 +1194,7 @@ template <class In>
 void launch_step(ufe_ctx *ctx, ThermoWork *t, const In &in, const Consts &c, const VertexFields &vf, int64_t nV,
                  const double *Ti_cur, double *Ti_next) {
   const ZOps z = zops_of(t);
-  const int T = threads_for(z.nz);
+  const int T = kColumnThreads;
   const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
   UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaStream_t s = ctx->stream;
@@ -1533,7 +1539,7 @@ extern "C" int32_t ufe_profile_heat_kernels(ufe_ctx *ctx, const ufe_thermo_param
     const HeatMesh in = heat_mesh_inputs(ctx, t, t->Ti[t->cur]);
     double *out = t->Ti[t->cur ^ 1];
     const ZOps z = zops_of(t);
-    const int T = threads_for(z.nz);
+    const int T = kColumnThreads;
     const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
       UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<HeatMesh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t nV = t->nV;
