@@ -7,7 +7,7 @@
 // arrays; every row keeps the reference's add_entry layout -- the diagonal, then the connections
 // C(vi, 1:nC) in the caller's order, which the renumbering keeps -- so the values are those of
 // the caller's numbering and an export only renames rows and columns.  Fields cross the ABI
-// through a staging buffer and one gather per array.  One thread per vertex row:
+// through staging buffers and one gather launch each way.  One thread per vertex row:
 //   k_divq_matrix   M_divQ (calc_ice_flux_divergence_matrix_upwind, conservation_of_mass_utilities.f90:22-132),
 //                   the edge velocity of map_velocities_from_b_to_c_2D (map_velocities_to_c_grid.f90:17-69)
 //                   read through the precomputed triangle pair of each connection;
@@ -37,7 +37,7 @@ struct MassWork {
   int64_t nnz = 0;
   double *A = nullptr, *Cw = nullptr;          // Voronoi areas, connection widths (nV x nC_mem)
   int2 *ct = nullptr;                           // triangles of each connection's edge (nV x nC_mem)
-  double *Dc = nullptr;                         // connection lengths D (nV x nC_mem), once per mesh
+  double *Dc = nullptr, *rDc = nullptr;         // connection lengths D and 1 / D (nV x nC_mem), once per mesh
   int32_t *ptr = nullptr, *ind = nullptr;       // M_divQ pattern, 0-based
   double *valM = nullptr, *valA = nullptr;
   // inputs (nV unless noted)
@@ -47,15 +47,13 @@ struct MassWork {
   int32_t *noice = nullptr, *prmask = nullptr;
   // outputs and scratch
   double *dHdt = nullptr, *Hit = nullptr, *divQ = nullptr, *AMB = nullptr;
-  double *dex = nullptr, *Hex = nullptr, *qex = nullptr, *aex = nullptr;
-  double *Hs = nullptr, *Hs_tot = nullptr, *bb = nullptr;
+  double *dex = nullptr, *Hex = nullptr, *aex = nullptr;
+  double *Hs = nullptr, *bb = nullptr;
   int32_t *nint = nullptr;
-  double *dt = nullptr;                         // [0] dt of the scheme, [1] the explicit part's
+  double *dt = nullptr;                         // [0] dt of the scheme, [1] the explicit part's; [2] holds flag
   unsigned long long *dtlim = nullptr;          // [0], [1]: bit patterns of the limits
-  int32_t *flag = nullptr;                      // negative thickness found
+  int32_t *flag = nullptr;                      // negative thickness found (in dt[2])
   CsrSolveScratch krylov;                       // the semi-implicit solve's work vectors
-  double *stage = nullptr;                      // max(nV, nTri): fields in the caller's order
-  int32_t *stagei = nullptr;                    // nV
 };
 
 namespace {
@@ -72,6 +70,27 @@ __global__ void k_permute(int64_t n, int ncols, const T *__restrict__ src, const
   dst[e] = src[c * n + map[i]];
 }
 
+// The same for a list of fields in one launch (a field per blockIdx.y): the gathers of one field leave the memory
+// system idle (7 us each at 260k vertices, 14 fields a step).
+struct PermuteList {
+  struct Field {
+    const void *src;
+    void *dst;
+    const int32_t *map;
+    int64_t n;
+    bool wide;   // double, else int32_t
+  } f[16];
+  int count = 0;
+  void add(const void *src, void *dst, const int32_t *map, int64_t n, bool wide) { f[count++] = {src, dst, map, n, wide}; }
+};
+__global__ void k_permute_list(PermuteList l) {
+  const PermuteList::Field &f = l.f[blockIdx.y];
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= f.n) return;
+  if (f.wide) ((double *)f.dst)[i] = ((const double *)f.src)[f.map[i]];
+  else ((int32_t *)f.dst)[i] = ((const int32_t *)f.src)[f.map[i]];
+}
+
 __device__ __forceinline__ double surface_elevation(double Hi, double Hb, double SL) {
   return Hi + fmax(SL - kIceDensityM / kSeawaterDensityM * Hi, Hb);   // ice_geometry_basics.f90:28-41
 }
@@ -85,7 +104,8 @@ __device__ __forceinline__ double thickness_from_surface(double Hb, double Hs, d
 // the triangles of the edge from vi to each neighbour (the ones among iTri(vi, :) holding vj),
 // and the connection length D = sqrt(D_x^2 + D_y^2) (mesh_secondary.f90:333-339)
 __global__ void k_conn_tris(int nV, int nTri, int nC_mem, const double *V, const int32_t *nC, const int32_t *C,
-                            const int32_t *niTri, const int32_t *iTri, const int32_t *Tri, int2 *ct, double *Dc) {
+                            const int32_t *niTri, const int32_t *iTri, const int32_t *Tri, int2 *ct, double *Dc,
+                            double *rDc) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   if (vi >= nV) return;
   for (int ci = 0; ci < nC_mem; ++ci) {
@@ -105,6 +125,7 @@ __global__ void k_conn_tris(int nV, int nTri, int nC_mem, const double *V, const
     }
     ct[(int64_t)ci * nV + vi] = r;
     Dc[(int64_t)ci * nV + vi] = D;
+    rDc[(int64_t)ci * nV + vi] = 1.0 / D;
   }
 }
 
@@ -115,14 +136,19 @@ struct MeshRef {
 };
 
 // The zero half of max(0, u_perp) / min(0, u_perp) is not divided: 0 / A_i is +0, and c0 + 0 is c0,
-// so skipping it leaves every value as the reference's expression gives it.
+// so skipping it leaves every value as the reference's expression gives it; the other half's quotient is one for both.
+//
+// Bound by FP64 instructions (64 cycles of its scheduler a warp): three divisions by the connection's length and the
+// cell's area per connection.  Their reciprocals are formed once per mesh and once per row (div_by: the same values in
+// three instructions instead of eight).  262k vertices: 173 us before, 100 now.
 __global__ void k_divq_matrix(MeshRef m, const double *A, const double *Cw, const int2 *ct, const double *Dc,
-                              const double *u, const double *v, const double *fm, const int32_t *ptr, double *val) {
+                              const double *rDc, const double *u, const double *v, const double *fm,
+                              const int32_t *ptr, double *val) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   if (vi >= m.nV) return;
   const int nV = m.nV;
   const int64_t k0 = ptr[vi];
-  const double A_i = A[vi];
+  const double A_i = A[vi], rA = 1.0 / A_i;
   const double xi = m.V[vi], yi = m.V[nV + vi];
   const bool out_i = opt(fm, vi, 1.0) >= 1.0;
   double c0 = 0.0;
@@ -138,12 +164,12 @@ __global__ void k_divq_matrix(MeshRef m, const double *A, const double *Cw, cons
       uc = (u[t.x] + u[t.y]) / 2.0;
       vc = (v[t.x] + v[t.y]) / 2.0;
     }
-    const double L_c = Cw[cix];
     const double Dx = m.V[vj] - xi, Dy = m.V[nV + vj] - yi;
-    const double D = Dc[cix];
-    const double u_perp = uc * Dx / D + vc * Dy / D;
-    if (out_i && u_perp > 0.0) c0 = c0 + L_c * u_perp / A_i;
-    val[k0 + 1 + ci] = (u_perp < 0.0 && opt(fm, vj, 1.0) >= 1.0) ? L_c * u_perp / A_i : 0.0;
+    const double D = Dc[cix], rD = rDc[cix];
+    const double u_perp = div_by(uc * Dx, D, rD) + div_by(vc * Dy, D, rD);
+    const double q = div_by(Cw[cix] * u_perp, A_i, rA);
+    if (out_i && u_perp > 0.0) c0 = c0 + q;
+    val[k0 + 1 + ci] = (u_perp < 0.0 && opt(fm, vj, 1.0) >= 1.0) ? q : 0.0;
   }
   val[k0] = c0;
 }
@@ -155,6 +181,12 @@ struct Inputs {
 
 __device__ __forceinline__ double mass_balance(const Inputs &in, int vi) {
   return opt(in.fm, vi, 1.0) * (opt(in.SMB, vi, 0.0) + opt(in.BMB, vi, 0.0) - opt(in.target, vi, 0.0));
+}
+
+__device__ __forceinline__ double prescribed(const Inputs &in, int vi, double h) {
+  if (in.prmask && in.prmask[vi] == 1) h = fmax(0.0, in.prHi[vi]);
+  if (in.noice && in.noice[vi]) h = 0.0;
+  return h;
 }
 
 // divQ, dH/dt (= AMB before the limits) and the time-step limit of every thinning vertex; the
@@ -204,9 +236,14 @@ __global__ void k_step(int nV, const double *Hi, const double *dHdt, double *dt,
   Hs[vi] = surface_elevation(h, Hb[vi], SL[vi]);
 }
 
-__global__ void k_surface(int nV, const double *H, const double *Hb, const double *SL, double *Hs) {
+// The end of calc_dHi_dt_explicit inside the semi-implicit scheme, which reads the thickness alone: prescribed
+// thickness, no-ice mask, and the surface for the second border pass.
+__global__ void k_prescribe_surface(int nV, Inputs in, double *H, double *Hs) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (vi < nV) Hs[vi] = surface_elevation(H[vi], Hb[vi], SL[vi]);
+  if (vi >= nV) return;
+  const double h = prescribed(in, vi, H[vi]);
+  H[vi] = h;
+  Hs[vi] = surface_elevation(h, in.Hb[vi], in.SL[vi]);
 }
 
 // calc_n_interior_neighbours (conservation_of_mass_utilities.f90:206-234)
@@ -231,9 +268,10 @@ __device__ __forceinline__ int border_bc(int vbi, int4 bc) {   // (west, east, s
 
 // One pass of apply_ice_thickness_BC_explicit: pass 0 sets border vertices with interior
 // neighbours to their interior neighbours' mean surface, pass 1 those without to all
-// neighbours' mean; 'zero' borders get no ice in both.  Hs_tot is the pass's starting copy.
+// neighbours' mean; 'zero' borders get no ice in both.  Both passes read the surface that they started from: pass 0
+// reads interior vertices and writes border ones, pass 1 leaves the surface as it is (nothing reads it afterwards).
 __global__ void k_border(MeshRef m, int pass, int4 bc, const int32_t *noice, const int32_t *nint, const double *Hb,
-                         const double *SL, const double *Hs_tot, double *Hs, double *H) {
+                         const double *SL, double *Hs, double *H) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   if (vi >= m.nV) return;
   const int b = border_bc(m.VBI[vi], bc);
@@ -247,38 +285,23 @@ __global__ void k_border(MeshRef m, int pass, int4 bc, const int32_t *noice, con
   double s = 0.0;
   for (int ci = 0; ci < m.nC[vi]; ++ci) {
     const int vj = m.C[(int64_t)ci * m.nV + vi] - 1;
-    if (pass == 1 || (m.VBI[vj] == 0 && !(noice && noice[vj]))) s = s + Hs_tot[vj];
+    if (pass == 1 || (m.VBI[vj] == 0 && !(noice && noice[vj]))) s = s + Hs[vj];
   }
   const double av = s / (double)(pass == 0 ? n : m.nC[vi]);
   const double hs = fmax(Hb[vi], av);
-  Hs[vi] = hs;
+  if (pass == 0) Hs[vi] = hs;
   H[vi] = thickness_from_surface(Hb[vi], hs, SL[vi]);
-}
-
-// the rest of calc_dHi_dt_explicit: prescribed thickness, no-ice mask, dH/dt and AMB
-__global__ void k_explicit_finish(int nV, Inputs in, const double *dt, double *Hit, double *dHdt, double *AMB) {
-  const int vi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (vi >= nV) return;
-  double h = Hit[vi];
-  if (in.prmask && in.prmask[vi] == 1) h = fmax(0.0, in.prHi[vi]);
-  if (in.noice && in.noice[vi]) h = 0.0;
-  Hit[vi] = h;
-  const double r = (h - in.Hi[vi]) / *dt;
-  dHdt[vi] = r;
-  AMB[vi] = r - AMB[vi];
 }
 
 // calc_dHi_dt_semiimplicit's stiffness row, load vector and initial guess, then
 // apply_ice_thickness_BC_matrix: border rows (the explicit solution), prescribed rows, no-ice rows
 __global__ void k_semi_system(MeshRef m, const int32_t *ptr, const int32_t *ind, const double *valM, Inputs in,
                               double dt, double fs, const double *Hex, double *valA, double *bb, double *x0,
-                              double *divQ) {
+                              const double *divQ) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   if (vi >= m.nV) return;
   const int32_t k1 = ptr[vi], k2 = ptr[vi + 1];
-  double q = 0.0;
-  for (int32_t k = k1; k < k2; ++k) q = q + valM[k] * in.Hi[ind[k]];
-  divQ[vi] = q;
+  const double q = divQ[vi];
   const double Hi = in.Hi[vi];
   double b = Hi - (dt * (1.0 - fs) * q) + fmax(-1.0 * Hi, dt * (mass_balance(in, vi) + opt(in.LMB, vi, 0.0)));
   double x = Hi + dt * opt(in.dprev, vi, 0.0);
@@ -288,35 +311,36 @@ __global__ void k_semi_system(MeshRef m, const int32_t *ptr, const int32_t *ind,
   if (in.noice && in.noice[vi]) { ident = true; b = 0.0; x = 0.0; }
   for (int32_t k = k1; k < k2; ++k) {
     const bool diag = ind[k] == vi;
-    valA[k] = ident ? (diag ? 1.0 : 0.0) : (diag ? valM[k] * dt * fs + 1.0 : valM[k] * dt * fs);
+    double a = valM[k] * dt * fs;
+    if (diag) a = a + 1.0;
+    valA[k] = ident ? (diag ? 1.0 : 0.0) : a;
   }
   bb[vi] = b;
   x0[vi] = x;
 }
 
-__global__ void k_semi_finish(int nV, const double *Hi, double dt, const double *Hit, double *dHdt, double *AMB) {
+// The end of a scheme and of calc_dHi_dt.  Explicit: prescribed thickness, no-ice mask, dH/dt and AMB (which holds the
+// rate before the limits).  Both: negative thickness to zero (and the reference's warning), AMB, dH/dt; the second
+// rate is the first one again where the thickness was not negative.
+template <bool kExplicit>
+__global__ void k_finish(int nV, Inputs in, const double *dt, double Hi_min, double *Hit, double *dHdt, double *AMB,
+                         int32_t *flag) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
   if (vi >= nV) return;
-  const double a = (Hit[vi] - Hi[vi]) / dt;
-  const double r = (Hit[vi] - Hi[vi]) / dt;
-  dHdt[vi] = r;
-  AMB[vi] = r - a;
-}
-
-// calc_dHi_dt after the scheme: negative thickness to zero (and the reference's warning), AMB, dH/dt
-__global__ void k_main_finish(int nV, const double *Hi, const double *dt, double Hi_min, double *Hit, double *dHdt,
-                              double *AMB, int32_t *flag) {
-  const int vi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (vi >= nV) return;
+  const double Hi = in.Hi[vi], d = *dt;
   double h = Hit[vi];
+  if (kExplicit) h = prescribed(in, vi, h);
+  double r = (h - Hi) / d;
+  const double amb = kExplicit ? r - AMB[vi] : r - r;
+  const double first = r;
   if (h < 0.0) {
-    if (h < -0.1 && Hi[vi] > Hi_min) atomicOr(flag, 1);
+    if (h < -0.1 && Hi > Hi_min) atomicOr(flag, 1);
     h = 0.0;
+    r = (h - Hi) / d;
   }
   Hit[vi] = h;
-  const double d = *dt;
-  AMB[vi] = AMB[vi] + (h - Hi[vi]) / d - dHdt[vi];
-  dHdt[vi] = (h - Hi[vi]) / d;
+  AMB[vi] = amb + r - first;
+  dHdt[vi] = r;
 }
 
 __global__ void k_none(int nV, const double *Hi, double *Hit, double *dHdt, double *AMB) {
@@ -346,22 +370,19 @@ T *alloc_n(size_t n) { return (T *)dev_alloc(sizeof(T) * (n ? n : 1)); }
 void alloc_fields(MassWork *w, cudaStream_t s) {
   const size_t nV = w->nV, nT = w->nTri;
   double **vs[] = {&w->Hi, &w->Hb, &w->SL, &w->SMB, &w->BMB, &w->LMB, &w->fm, &w->target, &w->prHi, &w->dprev,
-                   &w->dHdt, &w->Hit, &w->divQ, &w->AMB, &w->dex, &w->Hex, &w->qex, &w->aex, &w->Hs, &w->Hs_tot,
-                   &w->bb};
+                   &w->dHdt, &w->Hit, &w->divQ, &w->AMB, &w->dex, &w->Hex, &w->aex, &w->Hs, &w->bb};
   for (double **p : vs) *p = alloc_n<double>(nV);
   w->u = alloc_n<double>(nT);
   w->v = alloc_n<double>(nT);
   w->noice = alloc_n<int32_t>(nV);
   w->prmask = alloc_n<int32_t>(nV);
   w->nint = alloc_n<int32_t>(nV);
-  w->dt = alloc_n<double>(2);
+  w->dt = alloc_n<double>(3);
   w->dtlim = alloc_n<unsigned long long>(2);
-  w->flag = alloc_n<int32_t>(1);
+  w->flag = reinterpret_cast<int32_t *>(w->dt + 2);
   w->valM = alloc_n<double>(w->nnz);
   w->valA = alloc_n<double>(w->nnz);
   csr_scratch_alloc(w->krylov, w->nV, s);
-  w->stage = alloc_n<double>(std::max(nV, nT));
-  w->stagei = alloc_n<int32_t>(nV);
 }
 
 MeshRef mesh_ref(ufe_ctx *ctx) { return MeshRef{ctx->nV, ctx->nTri, ctx->V, ctx->nC, ctx->C, ctx->VBI}; }
@@ -371,17 +392,23 @@ MeshRef mesh_ref(ufe_ctx *ctx) { return MeshRef{ctx->nV, ctx->nTri, ctx->V, ctx-
 Inputs upload_inputs(ufe_ctx *ctx, MassWork *w, const ufe_thickness_fields *f) {
   cudaStream_t s = ctx->stream;
   const size_t nV = w->nV, nT = w->nTri;
+  Temp<double> stage(ctx, 10 * nV + 2 * nT), stagei(ctx, nV);   // the fields in the caller's order
+  double *next = stage;
+  int32_t *nexti = reinterpret_cast<int32_t *>(stagei.p);
+  PermuteList list;
   auto up = [&](double *d, const double *h, bool tri) -> const double * {
     if (!h) return nullptr;
     const size_t n = tri ? nT : nV;
-    UFE_CUDA(cudaMemcpyAsync(w->stage, h, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    k_permute<double><<<blocks(n), 256, 0, s>>>((int64_t)n, 1, w->stage, tri ? ctx->perm_t : ctx->perm_v, d);
+    UFE_CUDA(cudaMemcpyAsync(next, h, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    list.add(next, d, tri ? ctx->perm_t : ctx->perm_v, (int64_t)n, true);
+    next += n;
     return d;
   };
   auto upi = [&](int32_t *d, const int32_t *h) -> const int32_t * {
     if (!h) return nullptr;
-    UFE_CUDA(cudaMemcpyAsync(w->stagei, h, sizeof(int32_t) * nV, cudaMemcpyHostToDevice, s));
-    k_permute<int32_t><<<blocks(nV), 256, 0, s>>>((int64_t)nV, 1, w->stagei, ctx->perm_v, d);
+    UFE_CUDA(cudaMemcpyAsync(nexti, h, sizeof(int32_t) * nV, cudaMemcpyHostToDevice, s));
+    list.add(nexti, d, ctx->perm_v, (int64_t)nV, false);
+    nexti += nV;
     return d;
   };
   Inputs in;
@@ -399,6 +426,8 @@ Inputs upload_inputs(ufe_ctx *ctx, MassWork *w, const ufe_thickness_fields *f) {
   in.dprev = up(w->dprev, f->dHi_dt, false);
   in.noice = upi(w->noice, f->mask_noice);
   in.prmask = upi(w->prmask, f->BC_prescr_mask);
+  k_permute_list<<<dim3(blocks((int64_t)std::max(nV, nT)), list.count), 256, 0, s>>>(list);
+  UFE_CUDA(cudaGetLastError());
   return in;
 }
 
@@ -418,7 +447,7 @@ void check_inputs(const ufe_thickness_params *p, const ufe_thickness_fields *f) 
               "ice thickness: bad Krylov tolerances");
 }
 
-// calc_dHi_dt_explicit on the device into (dHdt, Hit, divQ, AMB); dt at dt_slot is shortened
+// calc_dHi_dt_explicit on the device into (dHdt, Hit, divQ, AMB), up to the border rule; dt at dt_slot is shortened
 void run_explicit(ufe_ctx *ctx, MassWork *w, const ufe_thickness_params *p, const Inputs &in, int dt_slot,
                   double *dHdt, double *Hit, double *divQ, double *AMB) {
   cudaStream_t s = ctx->stream;
@@ -429,46 +458,47 @@ void run_explicit(ufe_ctx *ctx, MassWork *w, const ufe_thickness_params *p, cons
   k_rate<<<blocks(nV), 256, 0, s>>>(nV, w->ptr, w->ind, w->valM, in, p->Hi_min, divQ, dHdt, AMB, w->dtlim + dt_slot);
   k_step<<<blocks(nV), 256, 0, s>>>(nV, in.Hi, dHdt, w->dt + dt_slot, w->dtlim + dt_slot, p->dt_ice_min, in.Hb, in.SL,
                                     Hit, w->Hs);
-  for (int pass = 0; pass < 2; ++pass) {
-    UFE_CUDA(cudaMemcpyAsync(w->Hs_tot, w->Hs, sizeof(double) * nV, cudaMemcpyDeviceToDevice, s));
-    k_border<<<blocks(nV), 256, 0, s>>>(m, pass, bc, in.noice, w->nint, in.Hb, in.SL, w->Hs_tot, w->Hs, Hit);
-  }
-  k_explicit_finish<<<blocks(nV), 256, 0, s>>>(nV, in, w->dt + dt_slot, Hit, dHdt, AMB);
+  for (int pass = 0; pass < 2; ++pass)
+    k_border<<<blocks(nV), 256, 0, s>>>(m, pass, bc, in.noice, w->nint, in.Hb, in.SL, w->Hs, Hit);
   UFE_CUDA(cudaGetLastError());
 }
 
-// the semi-implicit system (valA, bb, x0) for step dt; x0 is the initial guess
+// the semi-implicit system (valA, bb, x0) for step dt, which w->dt[1] holds; x0 is the initial guess
 void semi_system(ufe_ctx *ctx, MassWork *w, const ufe_thickness_params *p, const Inputs &in, double dt, double *x0) {
   cudaStream_t s = ctx->stream;
   const int nV = w->nV;
   const MeshRef m = mesh_ref(ctx);
   const int4 bc = make_int4(p->BC_H_west, p->BC_H_east, p->BC_H_south, p->BC_H_north);
-  UFE_CUDA(cudaMemcpyAsync(w->dt + 1, &dt, sizeof(double), cudaMemcpyHostToDevice, s));
-  run_explicit(ctx, w, p, in, 1, w->dex, w->Hex, w->qex, w->aex);
+  run_explicit(ctx, w, p, in, 1, w->dex, w->Hex, w->divQ, w->aex);   // divQ is the scheme's too
   // apply_ice_thickness_BC_matrix_domain_border applies the border rule to the explicit solution again
-  k_surface<<<blocks(nV), 256, 0, s>>>(nV, w->Hex, in.Hb, in.SL, w->Hs);
-  for (int pass = 0; pass < 2; ++pass) {
-    UFE_CUDA(cudaMemcpyAsync(w->Hs_tot, w->Hs, sizeof(double) * nV, cudaMemcpyDeviceToDevice, s));
-    k_border<<<blocks(nV), 256, 0, s>>>(m, pass, bc, in.noice, w->nint, in.Hb, in.SL, w->Hs_tot, w->Hs, w->Hex);
-  }
+  k_prescribe_surface<<<blocks(nV), 256, 0, s>>>(nV, in, w->Hex, w->Hs);
+  for (int pass = 0; pass < 2; ++pass)
+    k_border<<<blocks(nV), 256, 0, s>>>(m, pass, bc, in.noice, w->nint, in.Hb, in.SL, w->Hs, w->Hex);
   k_semi_system<<<blocks(nV), 256, 0, s>>>(m, w->ptr, w->ind, w->valM, in, dt, p->dHi_semiimplicit_fs, w->Hex,
                                            w->valA, w->bb, x0, w->divQ);
   UFE_CUDA(cudaGetLastError());
 }
 
-// an internal vertex field into the caller's host array
-void download_vertex(ufe_ctx *ctx, MassWork *w, double *h, const double *d) {
+// internal vertex fields into the caller's host arrays, there when the stream has been waited for
+void download_vertices(ufe_ctx *ctx, MassWork *w, std::initializer_list<std::pair<double *, const double *>> fields,
+                       double *stage) {
   cudaStream_t s = ctx->stream;
-  k_permute<double><<<blocks(w->nV), 256, 0, s>>>(w->nV, 1, d, ctx->iperm_v, w->stage);
-  UFE_CUDA(cudaMemcpyAsync(h, w->stage, sizeof(double) * w->nV, cudaMemcpyDeviceToHost, s));
-  UFE_CUDA(cudaStreamSynchronize(s));   // the staging buffer is reused by the next field
+  const size_t nV = w->nV;
+  PermuteList list;
+  for (const auto &f : fields) list.add(f.second, stage + list.count * nV, ctx->iperm_v, (int64_t)nV, true);
+  k_permute_list<<<dim3(blocks((int64_t)nV), list.count), 256, 0, s>>>(list);
+  UFE_CUDA(cudaGetLastError());
+  for (const auto &f : fields) {
+    UFE_CUDA(cudaMemcpyAsync(f.first, stage, sizeof(double) * nV, cudaMemcpyDeviceToHost, s));
+    stage += nV;
+  }
 }
 
 void prepare(ufe_ctx *ctx, MassWork *w, const ufe_thickness_params *p, const Inputs &in) {
   cudaStream_t s = ctx->stream;
   const int nV = w->nV;
   const MeshRef m = mesh_ref(ctx);
-  k_divq_matrix<<<blocks(nV), 256, 0, s>>>(m, w->A, w->Cw, w->ct, w->Dc, w->u, w->v, in.fm, w->ptr, w->valM);
+  k_divq_matrix<<<blocks(nV), 256, 0, s>>>(m, w->A, w->Cw, w->ct, w->Dc, w->rDc, w->u, w->v, in.fm, w->ptr, w->valM);
   k_interior_neighbours<<<blocks(nV), 256, 0, s>>>(m, in.noice, w->nint);
   UFE_CUDA(cudaGetLastError());
   (void)p;
@@ -480,10 +510,9 @@ void free_mass(ufe_ctx *ctx) {
   MassWork *w = ctx->mass;
   if (!w) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  void *ptrs[] = {w->A, w->Cw, w->ct, w->Dc, w->ptr, w->ind, w->valM, w->valA, w->Hi, w->Hb, w->SL, w->u, w->v,
+  void *ptrs[] = {w->A, w->Cw, w->ct, w->Dc, w->rDc, w->ptr, w->ind, w->valM, w->valA, w->Hi, w->Hb, w->SL, w->u, w->v,
                   w->SMB, w->BMB, w->LMB, w->fm, w->target, w->prHi, w->dprev, w->noice, w->prmask, w->dHdt,
-                  w->Hit, w->divQ, w->AMB, w->dex, w->Hex, w->qex, w->aex, w->Hs, w->Hs_tot, w->bb, w->nint,
-                  w->dt, w->dtlim, w->flag, w->stage, w->stagei};
+                  w->Hit, w->divQ, w->AMB, w->dex, w->Hex, w->aex, w->Hs, w->bb, w->nint, w->dt, w->dtlim};
   for (void *q : ptrs) dev_free(q);
   csr_scratch_free(w->krylov);
   delete w;
@@ -523,6 +552,7 @@ extern "C" int32_t ufe_mesh_voronoi_upload(ufe_ctx *ctx, const double *A, const 
     w->Cw = alloc_n<double>(nc);
     w->ct = alloc_n<int2>(nc);
     w->Dc = alloc_n<double>(nc);
+    w->rDc = alloc_n<double>(nc);
     double *tmp = alloc_n<double>(nc);   // the caller's order, then gathered into the internal one
     UFE_CUDA(cudaMemcpyAsync(tmp, A, sizeof(double) * w->nV, cudaMemcpyHostToDevice, s));
     k_permute<double><<<blocks(w->nV), 256, 0, s>>>(w->nV, 1, tmp, ctx->perm_v, w->A);
@@ -532,7 +562,7 @@ extern "C" int32_t ufe_mesh_voronoi_upload(ufe_ctx *ctx, const double *A, const 
     UFE_CUDA(cudaStreamSynchronize(s));
     dev_free(tmp);
     k_conn_tris<<<blocks(w->nV), 256, 0, s>>>(w->nV, w->nTri, w->nC_mem, ctx->V, ctx->nC, ctx->C, ctx->niTri,
-                                              ctx->iTri, ctx->Tri, w->ct, w->Dc);
+                                              ctx->iTri, ctx->Tri, w->ct, w->Dc, w->rDc);
     UFE_CUDA(cudaGetLastError());
     // M_divQ's pattern: row vi = [vi, C(vi, 1:nC)] (calc_ice_flux_divergence_matrix_upwind's add_entry order)
     std::vector<int32_t> nC(w->nV), C(nc);
@@ -571,6 +601,7 @@ extern "C" int32_t ufe_thickness_assemble(ufe_ctx *ctx, const ufe_thickness_para
     UFE_REQUIRE(cap >= w->nnz, UFE_ERR_CAPACITY, "ice thickness: matrix output too small");
     const Inputs in = upload_inputs(ctx, w, f);
     prepare(ctx, w, p, in);
+    UFE_CUDA(cudaMemcpyAsync(w->dt + 1, &dt, sizeof(double), cudaMemcpyHostToDevice, s));
     semi_system(ctx, w, p, in, dt, w->Hit);
     // rows back in the caller's numbering: caller row r is internal row iperm[r], entries in the
     // same order, columns renamed through perm
@@ -592,8 +623,9 @@ extern "C" int32_t ufe_thickness_assemble(ufe_ctx *ctx, const ufe_thickness_para
       }
     }
     ptr[nV] = (int32_t)k;
-    download_vertex(ctx, w, bb, w->bb);
-    download_vertex(ctx, w, x0, w->Hit);
+    Temp<double> stage(ctx, 2 * (size_t)nV);
+    download_vertices(ctx, w, {{bb, w->bb}, {x0, w->Hit}}, stage);
+    UFE_CUDA(cudaStreamSynchronize(s));
     return UFE_OK;
   });
 }
@@ -611,8 +643,8 @@ extern "C" int32_t ufe_calc_dHi_dt(ufe_ctx *ctx, const ufe_thickness_params *p, 
     ufe_thickness_stats st;
     memset(&st, 0, sizeof(st));
     const Inputs in = upload_inputs(ctx, w, f);
-    UFE_CUDA(cudaMemcpyAsync(w->dt, dt, sizeof(double), cudaMemcpyHostToDevice, s));
-    UFE_CUDA(cudaMemsetAsync(w->flag, 0, sizeof(int32_t), s));
+    double scalars[3] = {*dt, *dt, 0.0};   // dt of the scheme and of the explicit part, the flag
+    UFE_CUDA(cudaMemcpyAsync(w->dt, scalars, sizeof(scalars), cudaMemcpyHostToDevice, s));
     UFE_CUDA(cudaEventRecord(ctx->ev0, s));
     int32_t status = UFE_OK;
     if (p->choice_ice_integration_method == UFE_DHI_NONE) {
@@ -622,6 +654,7 @@ extern "C" int32_t ufe_calc_dHi_dt(ufe_ctx *ctx, const ufe_thickness_params *p, 
       prepare(ctx, w, p, in);
       if (p->choice_ice_integration_method == UFE_DHI_EXPLICIT) {
         run_explicit(ctx, w, p, in, 0, w->dHdt, w->Hit, w->divQ, w->AMB);
+        k_finish<true><<<blocks(nV), 256, 0, s>>>(nV, in, w->dt, p->Hi_min, w->Hit, w->dHdt, w->AMB, w->flag);
       } else {
         semi_system(ctx, w, p, in, *dt, w->Hit);
         DevCSR A;
@@ -635,19 +668,18 @@ extern "C" int32_t ufe_calc_dHi_dt(ufe_ctx *ctx, const ufe_thickness_params *p, 
                                   p->dHi_PETSc_max_it, &its, &w->krylov);
         st.n_Axb_its = its;
         st.krylov_status = status;
-        k_semi_finish<<<blocks(nV), 256, 0, s>>>(nV, in.Hi, *dt, w->Hit, w->dHdt, w->AMB);
+        k_finish<false><<<blocks(nV), 256, 0, s>>>(nV, in, w->dt, p->Hi_min, w->Hit, w->dHdt, w->AMB, w->flag);
       }
-      k_main_finish<<<blocks(nV), 256, 0, s>>>(nV, in.Hi, w->dt, p->Hi_min, w->Hit, w->dHdt, w->AMB, w->flag);
       UFE_CUDA(cudaGetLastError());
     }
     UFE_CUDA(cudaEventRecord(ctx->ev1, s));
-    download_vertex(ctx, w, f->dHi_dt, w->dHdt);
-    download_vertex(ctx, w, f->Hi_tplusdt, w->Hit);
-    download_vertex(ctx, w, f->divQ, w->divQ);
-    download_vertex(ctx, w, f->AMB, w->AMB);
-    UFE_CUDA(cudaMemcpyAsync(dt, w->dt, sizeof(double), cudaMemcpyDeviceToHost, s));
-    UFE_CUDA(cudaMemcpyAsync(&st.found_negative, w->flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    Temp<double> stage(ctx, 4 * (size_t)nV);
+    download_vertices(ctx, w, {{f->dHi_dt, w->dHdt}, {f->Hi_tplusdt, w->Hit}, {f->divQ, w->divQ}, {f->AMB, w->AMB}},
+                      stage);
+    UFE_CUDA(cudaMemcpyAsync(scalars, w->dt, sizeof(scalars), cudaMemcpyDeviceToHost, s));
     UFE_CUDA(cudaStreamSynchronize(s));
+    *dt = scalars[0];
+    memcpy(&st.found_negative, &scalars[2], sizeof(int32_t));
     float ms = 0.f;
     UFE_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     st.device_ms = ms;
