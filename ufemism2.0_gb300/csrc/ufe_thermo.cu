@@ -626,21 +626,20 @@ __global__ void __launch_bounds__(32) k_heat_retry(In in, ZOps z, Consts c, Vert
 // to sum, and one barrier for the new right-hand side.
 //
 // Unstable columns grow until they overflow, and what is left of such a column is decided by which of its sums become
-// infinite or undefined, so from kTeamLimit on (far enough below for the product's sums to stay finite) a substep is
-// the scans' of k_heat_retry, on the first warp; so is a level whose inverse holds an entry of 2^14 or more.
+// infinite or undefined.  So from the size on where the product's sums could overflow (32 products with the inverse's
+// largest entry) a substep is the scans' of k_heat_retry, on the first warp.
 //
 // That is three times the scans' FP64 instructions, so it is for lists that leave the schedulers idle otherwise: two
-// columns an SM.  All 1,022 substeps at 30 layers take 0.61 ms for up to 100 columns and 0.86 ms for 152 to 304; the
-// scans take 1.06 ms for up to 304 and 1.10 ms for 600, where the teams' second wave would end at 1.7 ms.
+// columns an SM.  All 1,022 substeps at 30 layers take 0.62 ms for up to 100 columns and 0.95 ms for 152 to 304; the
+// scans take 1.06 ms for up to 304 and 1.10 ms for 600, where the teams' second wave would end at 1.8 ms.
 constexpr int kTeamPad = 10;   // slots j at (j / 8) * 10 + j % 8: the four groups in different banks
-constexpr int kTeamLimit = (1023 + 1004) << 20;   // high words of 2^1004 and 2^14: 32 products stay below 2^1024
-constexpr int kTeamEntry = (1023 + 14) << 20;
 struct TeamShared {
   double M[kRetryLevels][kTeamRows * kTeamRows];
   double A[kTeamRows], C[kTeamRows], E1[kTeamRows], E2[kTeamRows];
   double W[kRetryLevels * kTeamRows], B[kRetryLevels * kTeamRows];
   double D[2][4 * kTeamPad];   // right-hand sides
   double d_gr[2];              // the basal one of the grounded flux condition
+  int m_exp;                   // largest exponent field in a level's inverse
   double x[kTeamRows], fwd[5][kTeamRows], bwd[5][kTeamRows], all[kTeamRows];   // the scans' substep
 };
 __device__ __forceinline__ int team_slot(int j) { return (j >> 3) * kTeamPad + (j & 7); }
@@ -736,7 +735,8 @@ __global__ void __launch_bounds__(128) k_heat_retry_team(In in, ZOps z, Consts c
   }
   const bool interior = group == 0 && row >= 1 && row < kb, above = group == 0 && row == kb - 1;
   double inv_dt = 0.0;
-  // the next substep's right-hand side; true when a value nears the overflow
+  int limit = 0;   // high word from which on a right-hand side is too large for the product
+  // the next substep's right-hand side; true when a value is
   auto publish = [&](int buf) -> bool {
     int hi = 0;
     if (interior) {
@@ -748,24 +748,32 @@ __global__ void __launch_bounds__(128) k_heat_retry_team(In in, ZOps z, Consts c
       const double d_gr = min_limit(x - flux_b, pmp_b);
       sh.D[buf][team_slot(kb)] = two_solves ? 0.0 : (grounded ? d_gr : pmp_b);
       sh.d_gr[buf] = d_gr;
+      hi = max(hi, __double2hiint(d_gr) & 0x7fffffff);
     }
-    return hi >= kTeamLimit;
+    return hi >= limit;
   };
+  __syncthreads();
   bool found = false;
   int buf = 0, slopes = -1;
   for (int l = 0; l < kRetryLevels && !found; ++l) {
     inv_dt = 1.0 / (c.dt * (1.0 / (double)(2 << l)));   // 0.5**(it_dt-1), exact
-    bool big = publish(buf);
-    __syncthreads();
     double m[8];
-    int m_hi = 0;
+    int m_exp = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       m[i] = row < nz && 8 * group + i < nz ? sh.M[l][row * kTeamRows + 8 * group + i] : 0.0;
-      m_hi = max(m_hi, __double2hiint(m[i]) & 0x7fffffff);
+      m_exp = max(m_exp, (__double2hiint(m[i]) & 0x7fffffff) >> 20);
     }
-    const bool scans = __syncthreads_or(m_hi >= kTeamEntry);   // of this level throughout
-    big = __syncthreads_or(scans || big);
+    m_exp = __reduce_max_sync(0xffffffffu, m_exp);
+    if (threadIdx.x == 0) sh.m_exp = 0;
+    __syncthreads();
+    if (lane == 0) atomicMax(&sh.m_exp, m_exp);
+    __syncthreads();
+    // 2^(d + 1) 2^(m + 1) 32 <= 2^1023 for the exponents d and m of a right-hand side and the largest entry, fields
+    // biased by 1023; no right-hand side is small enough for an inverse with infinities or NaN
+    m_exp = sh.m_exp;
+    limit = m_exp == 2047 ? 0 : min(3 * 1023 - 6 - m_exp, 2046) << 20;
+    bool big = __syncthreads_or(publish(buf));
     const double m_b = row < nz ? sh.M[l][row * kTeamRows + kb] : 0.0;
     const int nsub = 2 << l;
 #pragma unroll 1
@@ -802,7 +810,7 @@ __global__ void __launch_bounds__(128) k_heat_retry_team(In in, ZOps z, Consts c
       }
       x = two_solves ? fr * min_limit(x_sel, pmp) + (1.0 - fr) * min_limit(x_fl, pmp) : min_limit(x_sel, pmp);
       buf ^= 1;
-      big = __syncthreads_or(publish(buf) || scans);
+      big = __syncthreads_or(publish(buf));
     }
     found = !__syncthreads_or(row < nz && unstable_value(x));
   }
