@@ -447,8 +447,8 @@ def run_ours(args):
                     "path": head_name, "h2d_bytes_per_step": int(sum(v.nbytes for v in ice_h.values())),
                     "d2h_bytes_per_step": int(2 * 8 * mesh.nTri)}
     if rank == 0:
-        kname = {"fp64": "k_bicgstab_halo<double2,double4> (persistent FP64 BiCGStab)",
-                 "fp32_pair": "k_bicgstab_halo<dw2,dwblk> (persistent double-word BiCGStab)"}
+        kname = {"fp64": "k_bicgstab_resident<double2,double4> (persistent FP64 BiCGStab)",
+                 "fp32_pair": "k_bicgstab_resident<dw2,dwblk> (persistent double-word BiCGStab)"}
         kprec = {"fp32_pair_inexact": "fp32_pair"}.get(head_prec, head_prec)   # the persistent kernel it runs
         rk = kprec if kprec in us_it and us_it.get(kprec) else "fp64"
 
@@ -460,7 +460,7 @@ def run_ours(args):
             return {"bound": "hbm", "kernel": kname[name], "launch": "one BiCGStab iteration of the persistent kernel",
                     "achieved": round(ach, 1), "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                     "frac": round(ach / peaks.get("hbm_gbs"), 4), "peak_source": peak_kind,
-                    "traffic": traffic.get(f"k_bicgstab_halo_{name}_bytes_per_iteration"),
+                    "traffic": traffic.get(f"k_bicgstab_resident_{name}_bytes_per_iteration"),
                     "algorithmic_bytes_per_launch": int(bytes_it), "us_per_launch": round(us, 3)}
 
         roofline = roof(rk)

@@ -276,7 +276,7 @@ __global__ void k_icestream_yield(int nV, const double *Vy, double H, double tan
 // one FP64 division per layer instead of two (the reference's (tau zeta) / eta rounds differently
 // by an ulp or so).
 // A thread per triangle and layer: the division is a chain of its own (in k_finalize, a thread per triangle over all
-// layers, 15.6k triangles x 15 layers took 24 us; the two
+// layers, 15.6k triangles x 12 layers took 24 us; the two
 // kernels take 13 and 7).
 __global__ void k_diva_shear_b(int nTri, int nz, const double2 *tau_b, const double *eta_3D_b, const double *zeta,
                                double visc_eff_min, double2 *duz_b) {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(32 * kVertexSsaWarps) k_vertex_ssa(int nV, OpR
 // Dynamic shared memory: (kMaxNz + nz * blockDim.x) doubles.
 // Six warps per 32 vertices, the layers in turn: as in k_vertex_ssa, one warp's chain of FP64 instructions is what a
 // small mesh waits for, and a large one is evenly spread.  The sums over a row of the b->a operator are split over the
-// warps, the two integrals over the column and the friction go to one warp each.  7.8k vertices x 15 layers: 75 us with
+// warps, the two integrals over the column and the friction go to one warp each.  7.8k vertices x 12 layers: 75 us with
 // a thread per vertex, 34 like this (5, 8 and 16 warps: 36, 35, 36); 58k vertices, where the FP64 pipes are busy either
 // way: 176 and 176 us.
 constexpr int kVertexDivaWarps = 6;
