@@ -1237,7 +1237,8 @@ __device__ __forceinline__ void after_exchange(PhaseScalars<R> &ph, const double
           }
         }
       } else {
-        const double res2 = fmax(ss - w * (2.0 * st - w * den), 0.0);
+        // a negative difference of roundings is zero; an undefined one (an overflowed sum) stays undefined
+        const double raw = ss - w * (2.0 * st - w * den), res2 = raw > 0.0 || bits_nan(raw) ? raw : 0.0;
         if (lane == 0) {
           if (fail) {
             stop_failed(ph, zero ? UFE_ERR_DIVERGED : UFE_ERR_NAN);
