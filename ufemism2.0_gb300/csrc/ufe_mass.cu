@@ -139,8 +139,8 @@ struct MeshRef {
 // so skipping it leaves every value as the reference's expression gives it; the other half's quotient is one for both.
 //
 // Bound by FP64 instructions (64 cycles of its scheduler a warp): three divisions by the connection's length and the
-// cell's area per connection.  Their reciprocals are formed once per mesh and once per row (div_by: the same values in
-// three instructions instead of eight).  262k vertices: 173 us before, 100 now.
+// cell's area per connection.  Their reciprocals are formed once per mesh and once per row (div_by, in its range the
+// division's values, in three instructions instead of eight).  262k vertices: 173 us before, 100 now.
 __global__ void k_divq_matrix(MeshRef m, const double *A, const double *Cw, const int2 *ct, const double *Dc,
                               const double *rDc, const double *u, const double *v, const double *fm,
                               const int32_t *ptr, double *val) {

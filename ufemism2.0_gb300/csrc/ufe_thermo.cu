@@ -301,7 +301,7 @@ __device__ bool column_substep(const In &in, const ZOps &z, const Consts &c, int
 // ---- the three passes ------------------------------------------------------------------------
 // A thread per column, bound by FP64 instructions (85% of the pipes' cycles).  So the quotients that share a divisor
 // share its reciprocal, and minima and the stability check work on bit patterns: 101 FP64 instructions a row instead of
-// 115, all values the same to the bit.  Blocks of one warp: the columns' shared memory (3 x 8 bytes a layer) lets nine
+// 115, the values the same to the bit (the quotients in div_by's range).  Blocks of one warp: the columns' shared memory (3 x 8 bytes a layer) lets nine
 // of them on an SM at 30 layers, against two blocks of four, and the last wave is short.  200k columns x 30 layers:
 // 1.24 ms a step (blocks of 64 and 128: 1.27 and 1.32), 1.49 before.
 constexpr int kColumnThreads = 32;
