@@ -1,5 +1,7 @@
 // Context, mesh upload, operators and CSR-algebra entry points of the C ABI.
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <unordered_map>
 
 #include "ufe_internal.cuh"
@@ -14,6 +16,18 @@ void *dev_alloc(size_t bytes) {
 
 void dev_free(void *p) {
   if (p) cudaFree(p);
+}
+
+void raise_smem_limit(const void *kernel, size_t bytes) {
+  static std::mutex m;
+  static std::map<std::pair<int, const void *>, size_t> limits;
+  int device = 0;
+  UFE_CUDA(cudaGetDevice(&device));
+  std::lock_guard<std::mutex> lock(m);
+  size_t &limit = limits[{device, kernel}];
+  if (bytes <= limit) return;
+  UFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  limit = bytes;
 }
 
 void *temp_alloc(ufe_ctx *ctx, size_t bytes) {

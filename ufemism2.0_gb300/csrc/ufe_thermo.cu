@@ -1179,7 +1179,7 @@ template <class In, int R>
 void launch_retry_rows(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, const VertexFields &vf, int64_t nV,
                        double *Ti_next, const Lists &lists, Counters *cnt) {
   const size_t smem = (size_t)kRetryArrays * z.nz * sizeof(double);
-  UFE_CUDA(cudaFuncSetAttribute(k_heat_retry<In, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(k_heat_retry<In, R>, smem);
   k_heat_retry<In, R><<<kRetryBlocks, 32, smem, s>>>(in, z, c, vf, nV, Ti_next, lists, cnt);
   UFE_CUDA(cudaGetLastError());
 }
@@ -1187,8 +1187,7 @@ template <class In>
 void launch_retry(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, const VertexFields &vf, int64_t nV,
                   double *Ti_next, const Lists &lists, Counters *cnt) {
   if (z.nz <= kTeamRows) {   // one of the two finds work: the list's length is known on the device only
-    UFE_CUDA(cudaFuncSetAttribute(k_heat_retry_team<In>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(TeamShared)));
+    raise_smem_limit(k_heat_retry_team<In>, sizeof(TeamShared));
     k_heat_retry_team<In><<<kTeamColumns, 128, sizeof(TeamShared), s>>>(in, z, c, vf, nV, Ti_next, lists, cnt);
     UFE_CUDA(cudaGetLastError());
   }
@@ -1204,7 +1203,7 @@ void launch_step(ufe_ctx *ctx, ThermoWork *t, const In &in, const Consts &c, con
   const ZOps z = zops_of(t);
   const int T = kColumnThreads;
   const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
-  UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(k_heat_columns<In>, smem);
   cudaStream_t s = ctx->stream;
   const unsigned blocks = (unsigned)((nV + T - 1) / T);
   k_heat_columns<In><<<blocks, T, smem, s>>>(in, z, c, vf, nV, Ti_cur, Ti_next, t->lists, t->cnt);
@@ -1549,7 +1548,7 @@ extern "C" int32_t ufe_profile_heat_kernels(ufe_ctx *ctx, const ufe_thermo_param
     const ZOps z = zops_of(t);
     const int T = kColumnThreads;
     const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
-      UFE_CUDA(cudaFuncSetAttribute(k_heat_columns<HeatMesh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    raise_smem_limit(k_heat_columns<HeatMesh>, smem);
     const int64_t nV = t->nV;
     const unsigned blocks = (unsigned)((nV + T - 1) / T);
     reset_counters(ctx, t, nV);

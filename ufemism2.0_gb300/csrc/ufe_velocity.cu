@@ -1747,7 +1747,7 @@ struct Solver {
   // after another, and the grid never exceeds the co-resident count).
   template <class... KArgs, class... Args>
   void launch_coresident(void (*kern)(KArgs...), unsigned threads, size_t smem, Args... args) {
-    UFE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    raise_smem_limit(kern, smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(w->halo_G);
     cfg.blockDim = dim3(threads);
@@ -1964,7 +1964,7 @@ struct Solver {
   void enqueue_picard_pre(bool diva, CondArg inner) {
     if (diva) {
       const size_t smem = (size_t)(2 * kMaxNz + 2 * w->nz * 32) * sizeof(double);
-      UFE_CUDA(cudaFuncSetAttribute(k_vertex_diva, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      raise_smem_limit(k_vertex_diva, smem);
       k_vertex_diva<<<(w->nV + 31) / 32, 32 * kVertexDivaWarps, smem, s>>>(
           w->nV, w->nTri, w->nz, ba, w->uv, w->uv_base, w->duz_b, w->A_pow, w->Hi, ctx->zeta,
           sliding(), q, w->ps, w->eta_pred_a, w->eta_3D_a, w->N_a, w->F2a1, w->beta_a, w->beta_eff_a);
