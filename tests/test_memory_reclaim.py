@@ -1,0 +1,59 @@
+"""Unused buffers that the library keeps between calls are there for its other allocations: a limit on the device memory
+that a call can have (a library in front of the CUDA runtime refuses what goes past it) leaves room for the call only
+when the kept buffers are given back.  The contexts of a process keep 1 GiB of them together."""
+import pytest
+
+import cuda_shim
+
+KEEP = """
+def keep(s, mb):        # leaves about mb of unused buffers with the context: a product's operand and result
+    import scipy.sparse as sp
+    n, cols = 100_000, max(1, int(mb * 1e6 / 2 / 8 / 100_000))
+    A = pkg.CSR.from_scipy(sp.identity(n, format="csr"))
+    x = np.asfortranarray(np.random.default_rng(0).random((n, cols)))
+    y = pkg.VelocitySolver.multiply_CSR_matrix_with_vector_2D(s, A, x)
+    assert np.array_equal(x, y)
+
+def step(s):            # 12 fields of 20,000 x 30: 58 MB that the context keeps
+    zeta, cols = pkg.geometry.random_columns(20_000, 30, seed=1)
+    return s.thermo_step(pkg.abi.default_thermo_params(dt=1.0), zeta, cols)[0]
+
+MB = 1 << 20
+"""
+
+OWN_AND_OTHERS = KEEP + """
+with pkg.ColumnSolver() as alone:
+    want = step(alone)
+a, b, c = pkg.ColumnSolver(), pkg.ColumnSolver(), pkg.ColumnSolver()
+keep(a, 200)
+shim.shim_cap(shim.shim_held() + 20 * MB)
+assert np.array_equal(step(a), want)       # its own buffers
+shim.shim_cap((1 << 63))
+keep(a, 200)
+shim.shim_cap(shim.shim_held() + 20 * MB)
+assert np.array_equal(step(b), want)       # another context's
+shim.shim_cap((1 << 63))
+keep(a, 200)
+shim.shim_cap(shim.shim_held() + 20 * MB)
+keep(c, 150)                               # temporary buffers from another context's
+"""
+
+TOGETHER = KEEP + """
+some = [pkg.ColumnSolver() for _ in range(5)]
+base = shim.shim_held()
+for s in some:
+    keep(s, 400)
+assert shim.shim_held() - base <= 1025 * MB, (shim.shim_held() - base) / MB
+n = shim.shim_mallocs()
+keep(some[0], 400)                         # kept, not allocated again
+assert shim.shim_mallocs() == n
+for s in some:
+    s.close()
+assert shim.shim_held() < base
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER], ids=["own_and_others", "together"])
+def test_kept_buffers_are_given_back(gpu_lib, tmp_path, script):
+    cuda_shim.run(tmp_path, script)

@@ -1,4 +1,5 @@
 // Context, mesh upload, operators and CSR-algebra entry points of the C ABI.
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -7,12 +8,65 @@
 #include "ufe_internal.cuh"
 
 // ------------------------------------------------------------------------------------------
-void *dev_alloc(size_t bytes) {
+namespace {
+
+// All contexts' pools and their calls, under one lock (taken for a few tens of ns by a call's buffers).
+std::mutex g_pools;
+std::vector<ufe_ctx *> g_contexts;
+std::map<int, size_t> g_idle;            // bytes of unused blocks per device
+thread_local CallScope *t_call = nullptr;
+
+// Under the lock: frees unused blocks of a context, the largest first, while the device's pools keep more than `keep`.
+void trim(ufe_ctx *ctx, size_t keep) {
+  std::vector<TempPool::Block> &bl = ctx->temps.blocks;
+  size_t &idle = g_idle[ctx->device];
+  while (idle > keep) {
+    int big = -1;
+    for (int i = 0; i < (int)bl.size(); ++i)
+      if (!bl[i].used && (big < 0 || bl[i].bytes > bl[big].bytes)) big = i;
+    if (big < 0) return;
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);   // work that may still use it
+    dev_free(bl[big].p);
+    idle -= bl[big].bytes;
+    bl.erase(bl.begin() + big);
+  }
+}
+
+// cudaMalloc; where it fails, again after the unused blocks of the contexts on this device are given back: those whose
+// calls run in this thread, and those that no call is running on (another thread's stream may be capturing).
+void *malloc_or_reclaim(size_t bytes) {
   void *p = nullptr;
-  if (bytes == 0) bytes = 16;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  int device = 0;
+  UFE_CUDA(cudaGetDevice(&device));
+  {
+    std::lock_guard<std::mutex> lock(g_pools);
+    for (ufe_ctx *c : g_contexts) {
+      bool mine = false;
+      for (const CallScope *q = t_call; q; q = q->outer) mine |= q->ctx == c;
+      if (c->device == device && (mine || c->calls == 0)) trim(c, 0);
+    }
+  }
   UFE_CUDA(cudaMalloc(&p, bytes));
   return p;
 }
+
+}  // namespace
+
+CallScope::CallScope(ufe_ctx *c) : ctx(c), outer(t_call) {
+  std::lock_guard<std::mutex> lock(g_pools);
+  ++ctx->calls;
+  t_call = this;
+}
+
+CallScope::~CallScope() {
+  std::lock_guard<std::mutex> lock(g_pools);
+  --ctx->calls;
+  t_call = outer;
+}
+
+void *dev_alloc(size_t bytes) { return malloc_or_reclaim(bytes == 0 ? 16 : bytes); }
 
 void dev_free(void *p) {
   if (p) cudaFree(p);
@@ -32,53 +86,45 @@ void raise_smem_limit(const void *kernel, size_t bytes) {
 
 void *temp_alloc(ufe_ctx *ctx, size_t bytes) {
   std::vector<TempPool::Block> &bl = ctx->temps.blocks;
-  int best = -1;
-  for (int i = 0; i < (int)bl.size(); ++i)
-    if (!bl[i].used && bl[i].bytes >= bytes && bl[i].bytes / 4 <= bytes + (1 << 16) &&
-        (best < 0 || bl[i].bytes < bl[best].bytes))
-      best = i;
-  if (best < 0) {
-    const size_t size = (bytes + 65535) / 65536 * 65536 + (bytes == 0 ? 65536 : 0);
-    void *p = nullptr;
-    if (cudaMalloc(&p, size) != cudaSuccess) {
-      cudaGetLastError();
-      temp_trim(ctx, 0);
-      UFE_CUDA(cudaMalloc(&p, size));
+  {
+    std::lock_guard<std::mutex> lock(g_pools);
+    int best = -1;
+    for (int i = 0; i < (int)bl.size(); ++i)
+      if (!bl[i].used && bl[i].bytes >= bytes && bl[i].bytes / 4 <= bytes + (1 << 16) &&
+          (best < 0 || bl[i].bytes < bl[best].bytes))
+        best = i;
+    if (best >= 0) {
+      bl[best].used = true;
+      g_idle[ctx->device] -= bl[best].bytes;
+      return bl[best].p;
     }
-    bl.push_back({p, size, false});
-    best = (int)bl.size() - 1;
   }
-  bl[best].used = true;
-  return bl[best].p;
+  const size_t size = (bytes + 65535) / 65536 * 65536 + (bytes == 0 ? 65536 : 0);
+  void *p = malloc_or_reclaim(size);
+  std::lock_guard<std::mutex> lock(g_pools);
+  bl.push_back({p, size, true});
+  return p;
 }
 
 void temp_free(ufe_ctx *ctx, void *p) {
   if (!p) return;
+  std::lock_guard<std::mutex> lock(g_pools);
   for (auto &b : ctx->temps.blocks)
-    if (b.p == p) b.used = false;
-  temp_trim(ctx, kTempKeep);
+    if (b.p == p) {
+      b.used = false;
+      g_idle[ctx->device] += b.bytes;
+    }
+  trim(ctx, kTempKeep);
 }
 
-void temp_trim(ufe_ctx *ctx, size_t keep) {
-  std::vector<TempPool::Block> &bl = ctx->temps.blocks;
-  for (;;) {
-    size_t total = 0;
-    int big = -1;
-    for (int i = 0; i < (int)bl.size(); ++i)
-      if (!bl[i].used) {
-        total += bl[i].bytes;
-        if (big < 0 || bl[i].bytes > bl[big].bytes) big = i;
-      }
-    if (big < 0 || total <= keep) return;
-    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    dev_free(bl[big].p);
-    bl.erase(bl.begin() + big);
-  }
+void temp_clear(ufe_ctx *ctx) {
+  std::lock_guard<std::mutex> lock(g_pools);
+  trim(ctx, 0);
 }
 
 void temp_drop(ufe_ctx *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  temp_trim(ctx, 0);
+  temp_clear(ctx);
 }
 
 void free_operators(ufe_ctx *ctx) {
@@ -111,7 +157,7 @@ static void free_mesh(ufe_ctx *ctx) {
   ctx->V = ctx->TriGC = ctx->zeta = nullptr;
   ctx->nC = ctx->C = ctx->niTri = ctx->iTri = ctx->VBI = ctx->Tri = ctx->TriC = ctx->TriBI = nullptr;
   free_layout(ctx);
-  temp_trim(ctx, 0);
+  temp_clear(ctx);
   ctx->has_mesh = false;
 }
 
@@ -193,6 +239,10 @@ extern "C" int32_t ufe_ctx_create(int32_t device, ufe_ctx **out) {
     delete ctx;
     return rc;
   }
+  {
+    std::lock_guard<std::mutex> lock(g_pools);
+    g_contexts.push_back(ctx);
+  }
   *out = ctx;
   return UFE_OK;
 }
@@ -211,7 +261,11 @@ extern "C" void ufe_ctx_destroy(ufe_ctx *ctx) {
   dev_free(ctx->red.tickets);
   if (ctx->csr) csr_scratch_free(*ctx->csr);
   delete ctx->csr;
-  temp_trim(ctx, 0);
+  temp_clear(ctx);
+  {
+    std::lock_guard<std::mutex> lock(g_pools);
+    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+  }
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
