@@ -52,8 +52,32 @@ for s in some:
 assert shim.shim_held() < base
 """
 
+CSR_SOLVE = KEEP + """
+import scipy.sparse as sp
+def solve(s, m):        # 112 bytes of work vectors a row beside the system itself
+    rng = np.random.default_rng(m)
+    A = pkg.CSR.from_scipy(sp.diags([rng.uniform(-1, 0, m - 1), 3 + rng.random(m), rng.uniform(-1, 0, m - 1)],
+                                    [-1, 0, 1], format="csr"))
+    return pkg.VelocitySolver.solve_matrix_equation_CSR_PETSc(s, A, rng.random(m), np.zeros(m), 1e-10, 0.0)
+
+a = pkg.ColumnSolver()
+base = shim.shim_held()
+want = solve(a, 1_000_000)
+assert want[2] == 0
+n = shim.shim_mallocs()
+x, its, st = solve(a, 1_000_000)
+assert shim.shim_mallocs() == n and its == want[1] and np.array_equal(x, want[0])
+small = solve(a, 400_000)   # in the larger call's buffers
+with pkg.ColumnSolver() as fresh:
+    got = solve(fresh, 400_000)
+assert got[1] == small[1] and np.array_equal(got[0], small[0])
+shim.shim_cap(base + 80 * MB)
+step(a)
+assert shim.shim_held() <= base + 80 * MB
+"""
+
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER], ids=["own_and_others", "together"])
+@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER, CSR_SOLVE], ids=["own_and_others", "together", "csr_solve"])
 def test_kept_buffers_are_given_back(gpu_lib, tmp_path, script):
     cuda_shim.run(tmp_path, script)

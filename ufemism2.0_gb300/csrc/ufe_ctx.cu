@@ -259,8 +259,7 @@ extern "C" void ufe_ctx_destroy(ufe_ctx *ctx) {
   free_mesh(ctx);
   dev_free(ctx->red.partials);
   dev_free(ctx->red.tickets);
-  if (ctx->csr) csr_scratch_free(*ctx->csr);
-  delete ctx->csr;
+  if (ctx->csr_host) cudaFreeHost(ctx->csr_host);
   temp_clear(ctx);
   {
     std::lock_guard<std::mutex> lock(g_pools);

@@ -3150,21 +3150,27 @@ void csr_scratch_free(CsrSolveScratch &scr) {
   scr = CsrSolveScratch{};
 }
 
-// Work vectors that stay with the context after a solve (112 bytes a row): allocating them costs 0.5 ms, a tenth of
-// the smallest solves' time and nothing beside a solve of millions of rows.
-constexpr int64_t kCsrKeepRows = 1 << 22;
-
 int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double *x, double rtol, double abstol,
                          int32_t max_it, int32_t *its, CsrSolveScratch *scratch) {
   cudaStream_t s = ctx->stream;
   const int m = A.m;
-  if (!scratch) {   // the context's, grown to the largest system so far
-    if (!ctx->csr) ctx->csr = new CsrSolveScratch();
-    scratch = ctx->csr;
-    if (scratch->cap < m) {
-      csr_scratch_free(*scratch);
-      csr_scratch_alloc(*scratch, m, s);
-    }
+  if (!scratch) {   // this call's temporary buffers (112 bytes a row); the exchanges' stamps start anew in them
+    const size_t nslots = 2 * kCsrSet + 2 * (size_t)m;
+    Temp<double> vec(ctx, (size_t)m * 10);
+    Temp<ExSlot> slots(ctx, nslots);
+    struct Tail { GridSync gsync; KrylovScalars ks; };
+    Temp<Tail> tail(ctx, 1);
+    if (!ctx->csr_host) UFE_CUDA(cudaMallocHost(&ctx->csr_host, sizeof(KrylovScalars)));
+    UFE_CUDA(cudaMemsetAsync(slots, 0, sizeof(ExSlot) * nslots, s));
+    UFE_CUDA(cudaMemsetAsync(tail, 0, sizeof(Tail), s));
+    CsrSolveScratch scr;
+    scr.vec = vec;
+    scr.ks = &tail.p->ks;
+    scr.hks = ctx->csr_host;
+    scr.slots = slots;
+    scr.gsync = &tail.p->gsync;
+    scr.cap = m;
+    return solve_csr_device(ctx, A, b, x, rtol, abstol, max_it, its, &scr);
   }
   UFE_REQUIRE(scratch->cap >= m, UFE_ERR_INVALID, "CSR solve: work vectors too small");
   CsrSolveScratch &scr = *scratch;
@@ -3228,6 +3234,5 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
     cudaStreamSynchronize(s);
     throw;
   }
-  if (scratch == ctx->csr && scratch->cap > kCsrKeepRows) csr_scratch_free(*scratch);
   return status;
 }
