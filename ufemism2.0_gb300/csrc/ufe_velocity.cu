@@ -3119,7 +3119,8 @@ extern "C" int32_t ufe_profile_krylov_kernels(ufe_ctx *ctx, int32_t precision, i
 }
 
 // General CSR matrix-equation solve (solve_matrix_equation_CSR_PETSc): BiCGStab on scalar rows as one persistent
-// launch (k_csr_persist); with UFE_NO_PERSIST=1 five kernels per iteration, host-checked every eight.
+// launch (k_csr_persist); with UFE_NO_PERSIST=1, or where that launch is refused, five kernels per iteration,
+// host-checked every eight, with the same values.
 // inverse diagonal of a CSR matrix: the row's diagonal entries summed in storage order
 __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const double *val, double *dinv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3193,7 +3194,8 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
     k_krylov_init<CsrMat><<<krylov_grid(mat, kThreads, grid), kThreads, 0, s>>>(
         mat, v, ks, rtol, abstol, max_it, 0, ctx->red.partials, ctx->red.tickets, none);
     UFE_CUDA(cudaGetLastError());
-    if (persistent_krylov()) {
+    bool persist = persistent_krylov();
+    if (persist) {
       // the virtual blocks of the kernels' launch, up to four per block, one block per SM at most
       const int nvirt = std::min((int)krylov_grid(mat, 256, grid), kMaxVirt), sms = sm_count(ctx);
       const int q = std::max(1, std::min(4, (nvirt + sms - 1) / sms));
@@ -3207,11 +3209,18 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
       at[0].val.cooperative = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      UFE_CUDA(cudaLaunchKernelEx(&cfg, k_csr_persist<CsrMat>, mat, nvirt, v, ks, scr.slots + 2 * kCsrSet,
-                                  scr.slots + 2 * kCsrSet + m, scr.slots, scr.gsync));
-      UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
-      UFE_CUDA(cudaStreamSynchronize(s));
-    } else {
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, k_csr_persist<CsrMat>, mat, nvirt, v, ks, scr.slots + 2 * kCsrSet,
+                                               scr.slots + 2 * kCsrSet + m, scr.slots, scr.gsync);
+      if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+        cudaGetLastError();   // not all of these SMs are to be had: the kernels below need none at the same time
+        persist = false;
+      } else {
+        UFE_CUDA(e);
+        UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
+        UFE_CUDA(cudaStreamSynchronize(s));
+      }
+    }
+    if (!persist) {
       for (;;) {
         const unsigned gu = (unsigned)pick_blocks(m, kThreads, kMaxReduceBlocks);
         for (int c = 0; c < 8; ++c) {
