@@ -1,6 +1,6 @@
 """A library put in front of the CUDA runtime (LD_PRELOAD) in a child process.  It counts device memory, refuses
-allocations past a limit as a full device does, refuses cooperative launches as a device whose SMs are not all available
-does, and notes a kernel's shared-memory limit being lowered.  Nothing reaches the GPU that would not otherwise."""
+allocations past a limit as a full device does, counts cooperative launches or refuses them as a device whose SMs are not
+all available does, and notes a kernel's shared-memory limit being lowered.  Nothing reaches the GPU that would not otherwise."""
 import os
 import subprocess
 import sys
@@ -16,7 +16,7 @@ SOURCE = r"""
 
 static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;
 static struct { void *p; size_t bytes; } block[1 << 16];
-static int blocks, mallocs, lowered, refused, refuse_coop;
+static int blocks, mallocs, lowered, coop, refused, refuse_coop;
 static size_t held, cap = (size_t)-1;
 static struct { const void *f; int bytes; } limit[4096];
 static int limits;
@@ -30,6 +30,7 @@ static void *real(const char *name) {
 size_t shim_held(void) { return held; }
 int shim_mallocs(void) { return mallocs; }
 int shim_lowered(void) { return lowered; }
+int shim_coop(void) { return coop; }
 int shim_refused(void) { return refused; }
 void shim_cap(size_t bytes) { cap = bytes; }
 void shim_refuse_coop(int on) { refuse_coop = on; }
@@ -78,9 +79,12 @@ cudaError_t cudaFuncSetAttribute(const void *func, enum cudaFuncAttribute attr, 
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *cfg, const void *func, void **args) {
   cudaError_t (*f)(const cudaLaunchConfig_t *, const void *, void **) = real("cudaLaunchKernelExC");
   for (unsigned i = 0; i < cfg->numAttrs; ++i)
-    if (refuse_coop && cfg->attrs[i].id == cudaLaunchAttributeCooperative && cfg->attrs[i].val.cooperative) {
-      ++refused;
-      return cudaErrorCooperativeLaunchTooLarge;
+    if (cfg->attrs[i].id == cudaLaunchAttributeCooperative && cfg->attrs[i].val.cooperative) {
+      ++coop;
+      if (refuse_coop) {
+        ++refused;
+        return cudaErrorCooperativeLaunchTooLarge;
+      }
     }
   return f(cfg, func, args);
 }

@@ -1,5 +1,6 @@
-"""The scalar CSR solve where its persistent kernel cannot be launched: the kernels that need no co-residency take the
-solve, with the same iterates to the bit, in ufe_solve_csr and in the semi-implicit thickness step."""
+"""The scalar CSR solve where its persistent kernel is not launched: where the launch is refused (in ufe_solve_csr and in
+the semi-implicit thickness step) and above the rows up to which it is the faster form, the kernels that need no
+co-residency take the solve, with the same iterates to the bit."""
 import pytest
 
 import cuda_shim
@@ -34,6 +35,22 @@ assert h["stats"]["n_Axb_its"] == g["stats"]["n_Axb_its"] > 0
 for k in ("Hi_tplusdt", "dHi_dt", "divQ", "AMB"):
     assert np.array_equal(h[k], g[k])
 """
+
+ROWS = SOLVES + """
+with pkg.ColumnSolver() as s:
+    for m, coop in ((1 << 21, 1), ((1 << 21) + 1, 0)):
+        n = shim.shim_coop()
+        got = csr(s, m)
+        assert shim.shim_coop() - n == coop
+        shim.shim_refuse_coop(1)
+        assert same(csr(s, m), got) and got[2] == 0
+        shim.shim_refuse_coop(0)
+"""
+
+
+@pytest.mark.gpu
+def test_rows_up_to_which_the_solve_is_persistent(gpu_lib, tmp_path):
+    cuda_shim.run(tmp_path, ROWS)
 
 
 @pytest.mark.gpu

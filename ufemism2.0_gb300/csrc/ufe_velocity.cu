@@ -3119,7 +3119,7 @@ extern "C" int32_t ufe_profile_krylov_kernels(ufe_ctx *ctx, int32_t precision, i
 }
 
 // General CSR matrix-equation solve (solve_matrix_equation_CSR_PETSc): BiCGStab on scalar rows as one persistent
-// launch (k_csr_persist); with UFE_NO_PERSIST=1, or where that launch is refused, five kernels per iteration,
+// launch (k_csr_persist); for large systems, with UFE_NO_PERSIST=1 or where that launch is refused, five kernels per iteration,
 // host-checked every eight, with the same values.
 // inverse diagonal of a CSR matrix: the row's diagonal entries summed in storage order
 __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const double *val, double *dinv) {
@@ -3131,12 +3131,19 @@ __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const 
   dinv[i] = d != 0.0 ? 1.0 / d : 1.0;
 }
 
+// The persistent solve takes systems of up to 2^21 rows.  Its p and s travel as 16-byte words that are read past L1, twice
+// the bytes of the kernels' gathers, which counts once the vectors leave L2.  Five entries a row, microseconds an
+// iteration, persistent and kernels: 19 and 46 for 60k rows, 112 and 140 for 1M, 188 and 203 for 2M, 351 and 346 for 4M,
+// 656 and 612 for 8M, 1,257 and 1,143 for 16M.
+constexpr int64_t kCsrPersistRows = 1 << 21;
+static size_t csr_slots(int64_t m) { return m <= kCsrPersistRows ? 2 * kCsrSet + 2 * (size_t)m : 0; }
+
 void csr_scratch_alloc(CsrSolveScratch &scr, int64_t m, cudaStream_t s) {
   scr.vec = (double *)dev_alloc(sizeof(double) * (size_t)m * 10);
   scr.ks = (KrylovScalars *)dev_alloc(sizeof(KrylovScalars));
-  scr.slots = (ExSlot *)dev_alloc(sizeof(ExSlot) * (2 * kCsrSet + 2 * (size_t)m));
+  scr.slots = (ExSlot *)dev_alloc(sizeof(ExSlot) * csr_slots(m));
   scr.gsync = (GridSync *)dev_alloc(sizeof(GridSync));
-  UFE_CUDA(cudaMemsetAsync(scr.slots, 0, sizeof(ExSlot) * (2 * kCsrSet + 2 * (size_t)m), s));
+  UFE_CUDA(cudaMemsetAsync(scr.slots, 0, sizeof(ExSlot) * csr_slots(m), s));
   UFE_CUDA(cudaMemsetAsync(scr.gsync, 0, sizeof(GridSync), s));
   UFE_CUDA(cudaMallocHost(&scr.hks, sizeof(KrylovScalars)));
   scr.cap = m;
@@ -3156,7 +3163,7 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
   cudaStream_t s = ctx->stream;
   const int m = A.m;
   if (!scratch) {   // this call's temporary buffers (112 bytes a row); the exchanges' stamps start anew in them
-    const size_t nslots = 2 * kCsrSet + 2 * (size_t)m;
+    const size_t nslots = csr_slots(m);
     Temp<double> vec(ctx, (size_t)m * 10);
     Temp<ExSlot> slots(ctx, nslots);
     struct Tail { GridSync gsync; KrylovScalars ks; };
@@ -3194,7 +3201,7 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
     k_krylov_init<CsrMat><<<krylov_grid(mat, kThreads, grid), kThreads, 0, s>>>(
         mat, v, ks, rtol, abstol, max_it, 0, ctx->red.partials, ctx->red.tickets, none);
     UFE_CUDA(cudaGetLastError());
-    bool persist = persistent_krylov();
+    bool persist = persistent_krylov() && m <= kCsrPersistRows;
     if (persist) {
       // the virtual blocks of the kernels' launch, up to four per block, one block per SM at most
       const int nvirt = std::min((int)krylov_grid(mat, 256, grid), kMaxVirt), sms = sm_count(ctx);
