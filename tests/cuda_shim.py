@@ -16,7 +16,8 @@ SOURCE = r"""
 
 static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;
 static struct { void *p; size_t bytes; } block[1 << 16];
-static int blocks, mallocs, lowered, coop, refused, refuse_coop;
+static int blocks, mallocs, lowered, refused, refuse_coop;
+static __thread int coop;   // this thread's
 static size_t held, cap = (size_t)-1;
 static struct { const void *f; int bytes; } limit[4096];
 static int limits;

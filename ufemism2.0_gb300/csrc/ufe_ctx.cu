@@ -2,7 +2,6 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <unordered_map>
 
 #include "ufe_internal.cuh"
@@ -70,6 +69,11 @@ void *dev_alloc(size_t bytes) { return malloc_or_reclaim(bytes == 0 ? 16 : bytes
 
 void dev_free(void *p) {
   if (p) cudaFree(p);
+}
+
+std::shared_mutex &grid_lock(int device) {
+  static std::shared_mutex m[64];
+  return m[device % 64];
 }
 
 void raise_smem_limit(const void *kernel, size_t bytes) {

@@ -2317,6 +2317,7 @@ int32_t picard_collect(ufe_ctx *ctx, const ufe_solver_params &p, ufe_solve_stats
 
 // Run a resident Picard solve; fills stats; returns the status.
 int32_t run_picard(ufe_ctx *ctx, const ufe_solver_params &p, bool diva, ufe_solve_stats *stats) {
+  const std::shared_lock<std::shared_mutex> grids(grid_lock(ctx->device));
   picard_launch(ctx, p, diva);
   return picard_collect(ctx, p, stats);
 }
@@ -2955,6 +2956,7 @@ extern "C" int32_t ufe_solve_linearised(ufe_ctx *ctx, const ufe_solver_params *p
     Solver S(ctx, *p);
     CondArg none{0, 0};
     UFE_CUDA(cudaMemsetAsync(w->ks, 0, sizeof(KrylovScalars) * 3, S.s));
+    const std::shared_lock<std::shared_mutex> grids(grid_lock(ctx->device));
     S.enqueue_assemble(kFromTriangles, p->krylov_initial_guess == UFE_X0_CURRENT, none);
     for (;;) {
       if (p->precision == UFE_PREC_FP32_REFINE) {
@@ -3036,6 +3038,7 @@ extern "C" int32_t ufe_profile_krylov_persistent(ufe_ctx *ctx, int32_t precision
       UFE_CUDA(cudaGetLastError());
     }
     KrylovScalars *dks = w->ks + (fp32 ? 1 : 0);
+    const std::shared_lock<std::shared_mutex> grids(grid_lock(ctx->device));
     UFE_CUDA(cudaEventRecord(ctx->ev0, s));
     if (fp32) {
       k_reset_gsync<<<1, 1, 0, s>>>(w->gsync);
@@ -3119,8 +3122,8 @@ extern "C" int32_t ufe_profile_krylov_kernels(ufe_ctx *ctx, int32_t precision, i
 }
 
 // General CSR matrix-equation solve (solve_matrix_equation_CSR_PETSc): BiCGStab on scalar rows as one persistent
-// launch (k_csr_persist); for large systems, with UFE_NO_PERSIST=1 or where that launch is refused, five kernels per iteration,
-// host-checked every eight, with the same values.
+// launch (k_csr_persist); for large systems, beside other solves on the device, with UFE_NO_PERSIST=1 or where that
+// launch is refused, five kernels per iteration, host-checked every eight, with the same values.
 // inverse diagonal of a CSR matrix: the row's diagonal entries summed in storage order
 __global__ void k_csr_dinv(int m, const int32_t *ptr, const int32_t *ind, const double *val, double *dinv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3201,7 +3204,8 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
     k_krylov_init<CsrMat><<<krylov_grid(mat, kThreads, grid), kThreads, 0, s>>>(
         mat, v, ks, rtol, abstol, max_it, 0, ctx->red.partials, ctx->red.tickets, none);
     UFE_CUDA(cudaGetLastError());
-    bool persist = persistent_krylov() && m <= kCsrPersistRows;
+    std::unique_lock<std::shared_mutex> alone(grid_lock(ctx->device), std::defer_lock);
+    bool persist = persistent_krylov() && m <= kCsrPersistRows && alone.try_lock();
     if (persist) {
       // the virtual blocks of the kernels' launch, up to four per block, one block per SM at most
       const int nvirt = std::min((int)krylov_grid(mat, 256, grid), kMaxVirt), sms = sm_count(ctx);
@@ -3221,6 +3225,7 @@ int32_t solve_csr_device(ufe_ctx *ctx, const DevCSR &A, const double *b, double 
       if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
         cudaGetLastError();   // not all of these SMs are to be had: the kernels below need none at the same time
         persist = false;
+        alone.unlock();
       } else {
         UFE_CUDA(e);
         UFE_CUDA(cudaMemcpyAsync(hks, ks, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, s));
