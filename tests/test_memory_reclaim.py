@@ -1,6 +1,7 @@
 """Unused buffers that the library keeps between calls are there for its other allocations: a limit on the device memory
 that a call can have (a library in front of the CUDA runtime refuses what goes past it) leaves room for the call only
-when the kept buffers are given back.  The contexts of a process keep 1 GiB of them together."""
+when the kept buffers are given back.  The contexts of a process keep 1 GiB of them together.  A mesh's thickness steps
+find their buffers there."""
 import pytest
 
 import cuda_shim
@@ -76,8 +77,27 @@ step(a)
 assert shim.shim_held() <= base + 80 * MB
 """
 
+FIRST_STEP = KEEP + """
+mesh, f, p = pkg.geometry.thickness_case(res=8e3)
+for method in ("explicit", "semi-implicit"):
+    p.choice_ice_integration_method = pkg.abi.DHI[method]
+    with pkg.VelocitySolver(mesh) as s:
+        s.voronoi_upload()
+        n = shim.shim_mallocs()
+        first = s.calc_dHi_dt(p, f, 3.0)["Hi_tplusdt"]
+        assert shim.shim_mallocs() == n, method        # all buffers came with the mesh
+        try:
+            s.calc_dHi_dt(p, dict(f, Hi=None), 3.0)
+            assert False, "a missing field was accepted"
+        except pkg.UfeError:
+            pass
+        assert np.array_equal(s.calc_dHi_dt(p, f, 3.0)["Hi_tplusdt"], first)
+        assert shim.shim_mallocs() == n, method        # and outlive a refused call
+"""
+
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER, CSR_SOLVE], ids=["own_and_others", "together", "csr_solve"])
+@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER, CSR_SOLVE, FIRST_STEP],
+                         ids=["own_and_others", "together", "csr_solve", "first_step"])
 def test_kept_buffers_are_given_back(gpu_lib, tmp_path, script):
     cuda_shim.run(tmp_path, script)

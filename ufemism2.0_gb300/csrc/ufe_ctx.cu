@@ -126,9 +126,8 @@ void temp_clear(ufe_ctx *ctx) {
   trim(ctx, 0);
 }
 
-void temp_drop(ufe_ctx *ctx) {
+void wait_after_error(ufe_ctx *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  temp_clear(ctx);
 }
 
 void free_operators(ufe_ctx *ctx) {

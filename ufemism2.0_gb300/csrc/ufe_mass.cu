@@ -385,6 +385,12 @@ void alloc_fields(MassWork *w, cudaStream_t s) {
   csr_scratch_alloc(w->krylov, w->nV, s);
 }
 
+// a step's input fields in the caller's order (its outputs', of which there are four, fit the first buffer)
+struct Stage {
+  Temp<double> d, i;
+  Stage(ufe_ctx *ctx, const MassWork *w) : d(ctx, 10 * (size_t)w->nV + 2 * (size_t)w->nTri), i(ctx, w->nV) {}
+};
+
 MeshRef mesh_ref(ufe_ctx *ctx) { return MeshRef{ctx->nV, ctx->nTri, ctx->V, ctx->nC, ctx->C, ctx->VBI}; }
 
 // upload the fields the caller gave, in the internal numbering; returns the device-side view
@@ -392,9 +398,9 @@ MeshRef mesh_ref(ufe_ctx *ctx) { return MeshRef{ctx->nV, ctx->nTri, ctx->V, ctx-
 Inputs upload_inputs(ufe_ctx *ctx, MassWork *w, const ufe_thickness_fields *f) {
   cudaStream_t s = ctx->stream;
   const size_t nV = w->nV, nT = w->nTri;
-  Temp<double> stage(ctx, 10 * nV + 2 * nT), stagei(ctx, nV);   // the fields in the caller's order
-  double *next = stage;
-  int32_t *nexti = reinterpret_cast<int32_t *>(stagei.p);
+  Stage stage(ctx, w);
+  double *next = stage.d;
+  int32_t *nexti = reinterpret_cast<int32_t *>(stage.i.p);
   PermuteList list;
   auto up = [&](double *d, const double *h, bool tri) -> const double * {
     if (!h) return nullptr;
@@ -583,6 +589,7 @@ extern "C" int32_t ufe_mesh_voronoi_upload(ufe_ctx *ctx, const double *A, const 
     UFE_CUDA(cudaMemcpyAsync(w->ptr, ptr.data(), sizeof(int32_t) * (w->nV + 1), cudaMemcpyHostToDevice, s));
     UFE_CUDA(cudaMemcpyAsync(w->ind, ind.data(), sizeof(int32_t) * w->nnz, cudaMemcpyHostToDevice, s));
     alloc_fields(w, s);
+    Stage(ctx, w);   // with the mesh rather than in its first step
     UFE_CUDA(cudaStreamSynchronize(s));
     return UFE_OK;
   });
