@@ -1,7 +1,7 @@
 """Unused buffers that the library keeps between calls are there for its other allocations: a limit on the device memory
 that a call can have (a library in front of the CUDA runtime refuses what goes past it) leaves room for the call only
 when the kept buffers are given back.  The contexts of a process keep 1 GiB of them together.  A mesh's thickness steps
-find their buffers there."""
+find their buffers there, and a network that only predicts has no gradient buffers."""
 import pytest
 
 import cuda_shim
@@ -95,9 +95,29 @@ for method in ("explicit", "semi-implicit"):
         assert shim.shim_mallocs() == n, method        # and outlive a refused call
 """
 
+NETWORK = KEEP + """
+n = 60_000
+i = np.arange(n)
+nbr = np.stack([(i - 1) % n, (i + 1) % n, np.full(n, -1)], axis=1).astype(np.int32)
+rng = np.random.default_rng(0)
+x, y = rng.standard_normal((n, 16)).astype(np.float32), rng.standard_normal((n, 3)).astype(np.float32)
+w = np.full(n, 1 / n, np.float32)
+with pkg.ColumnSolver() as s:
+    base = shim.shim_held()
+    net = pkg.LearnedStart(s, seed=0)
+    assert shim.shim_held() - base < 10 * MB       # weights and the sums' scalars
+    net.forward(nbr[:100] % 100, x[:100])
+    small = net.loss_grad(nbr[:100] % 100, x[:100], y[:100], w[:100])
+    big = net.loss_grad(nbr, x, y, w)
+    again = net.loss_grad(nbr[:100] % 100, x[:100], y[:100], w[:100])
+    assert small[0] == again[0] and np.array_equal(small[1], again[1])
+    other = pkg.LearnedStart(s, seed=0).loss_grad(nbr, x, y, w)
+    assert big[0] == other[0] and np.array_equal(big[1], other[1])
+"""
+
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER, CSR_SOLVE, FIRST_STEP],
-                         ids=["own_and_others", "together", "csr_solve", "first_step"])
+@pytest.mark.parametrize("script", [OWN_AND_OTHERS, TOGETHER, CSR_SOLVE, FIRST_STEP, NETWORK],
+                         ids=["own_and_others", "together", "csr_solve", "first_step", "network"])
 def test_kept_buffers_are_given_back(gpu_lib, tmp_path, script):
     cuda_shim.run(tmp_path, script)

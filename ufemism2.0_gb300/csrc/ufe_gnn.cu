@@ -866,6 +866,7 @@ struct ufe_gnn {
   uint16_t *t[kLayers] = {};
   float *dacc[2] = {}, *dA[2] = {}, *ybuf = nullptr;   // dacc, dA: of the layer above and of this one, in turn
   float *part = nullptr, *dpart = nullptr;             // gradient partials per CTA
+  int part_ctas = 0;                                   // that part holds (0.3 MB each)
   double *loss_part = nullptr;
   double *loss_host = nullptr;       // pinned
   // scratch for explicit graphs and mesh features
@@ -958,6 +959,13 @@ void gnn_forward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x, co
 // backward after gnn_forward with targets: the full gradient in g->grad
 void gnn_backward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x) {
   const int G = (int)gnn_grid(gr.n, kBwdBlocks), D = (int)gnn_grid(gr.n, kFwdBlocks);
+  if (g->part_ctas < G) {   // networks that only predict have none
+    dev_free(g->part);
+    g->part = nullptr;
+    g->part_ctas = 0;
+    g->part = (float *)dev_alloc(sizeof(float) * (size_t)kPartSets * G * kPart);
+    g->part_ctas = G;
+  }
   auto set = [&](int q) { return g->part + (int64_t)q * G * kPart; };
   GradIn in{nullptr, nullptr, g->ybuf};
   for (int l = kLayers - 1, c = 0; l >= 0; --l, c ^= 1) {
@@ -1048,7 +1056,6 @@ extern "C" int32_t ufe_gnn_create(ufe_ctx *ctx, uint64_t seed, ufe_gnn **out) {
       g->v = (float *)dev_alloc(sizeof(float) * kParams);
       g->wbf = (uint16_t *)dev_alloc(sizeof(uint16_t) * kBfTotal);
       g->err = (int *)dev_alloc(sizeof(int));
-      g->part = (float *)dev_alloc(sizeof(float) * (size_t)kPartSets * kBwdBlocks * kPart);
       g->dpart = (float *)dev_alloc(sizeof(float) * kFwdBlocks * kDecParts);
       g->loss_part = (double *)dev_alloc(sizeof(double) * kFwdBlocks);
       UFE_CUDA(cudaMallocHost(&g->loss_host, sizeof(double) * kFwdBlocks));
