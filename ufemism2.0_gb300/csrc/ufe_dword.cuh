@@ -112,10 +112,6 @@ __device__ __forceinline__ dw dw_v(dw2 a) { return dw(a.q.y, a.q.w); }
 __device__ __forceinline__ dw2 make_dw2(dw u, dw v) { return dw2{make_float4(u.hi, v.hi, u.lo, v.lo)}; }
 __device__ __forceinline__ dw2 to_dw2(double2 a) { return make_dw2(dw(a.x), dw(a.y)); }
 __device__ __forceinline__ double2 to_double2(dw2 a) { return make_double2(dw_u(a).to_double(), dw_v(a).to_double()); }
-__device__ __forceinline__ dwblk to_dwblk(double4 a) {
-  const dw x(a.x), y(a.y), z(a.z), w(a.w);
-  return dwblk{make_float4(x.hi, y.hi, z.hi, w.hi), make_float4(x.lo, y.lo, z.lo, w.lo)};
-}
 
 // Vector operations of the BiCGStab recurrence (the double-word forms of the FP64 ones).
 // p_new = r - bw*v + beta*p

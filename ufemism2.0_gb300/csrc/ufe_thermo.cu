@@ -77,7 +77,6 @@ struct Counters {
 struct Lists {
   int32_t *retry;       // nV
   int32_t *unstable;    // nV
-  double *scratch;      // nV x nz (list-indexed current profiles of retried columns)
 };
 
 __device__ __forceinline__ double heat_capacity(const Consts &c, double T) {
@@ -1094,7 +1093,7 @@ struct ThermoWork {
   Counters *cnt = nullptr;
   Counters *cnt_host = nullptr; // pinned
   Lists lists{};
-  int64_t list_nv = 0, list_nl = 0;
+  int64_t list_nv = 0;
   // column-level inputs (uploaded per call)
   double *col_buf = nullptr;    // 12 x nV x nz + 6 x nV
   int32_t *col_mask = nullptr;
@@ -1113,7 +1112,7 @@ void free_thermo(ufe_ctx *ctx) {
   ThermoWork *t = ctx->thermo;
   if (!t) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  void *ptrs[] = {t->zops, t->cnt, t->lists.retry, t->lists.unstable, t->lists.scratch, t->col_buf, t->col_mask,
+  void *ptrs[] = {t->zops, t->cnt, t->lists.retry, t->lists.unstable, t->col_buf, t->col_mask,
                   t->Ti[0], t->Ti[1], t->u, t->v, t->w, t->phi, t->ub, t->vb, t->vert, t->mask, t->ti_up};
   for (void *p : ptrs) dev_free(p);
   if (t->cnt_host) cudaFreeHost(t->cnt_host);
@@ -1132,18 +1131,13 @@ ThermoWork *thermo_work(ufe_ctx *ctx) {
   return ctx->thermo;
 }
 
-void ensure_lists(ThermoWork *t, int64_t nV, int nz) {
+void ensure_lists(ThermoWork *t, int64_t nV) {
   if (t->list_nv < nV) {
     dev_free(t->lists.retry);
     dev_free(t->lists.unstable);
     t->lists.retry = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
     t->lists.unstable = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
     t->list_nv = nV;
-  }
-  if (t->list_nl < nV * nz) {
-    dev_free(t->lists.scratch);
-    t->lists.scratch = (double *)dev_alloc(sizeof(double) * nV * nz);
-    t->list_nl = nV * nz;
   }
 }
 
@@ -1282,7 +1276,7 @@ extern "C" int32_t ufe_thermo_step(ufe_ctx *ctx, const ufe_thermo_params *p, int
       t->col_mask = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
       t->col_mask_cap = nV;
     }
-    ensure_lists(t, nV, nz);
+    ensure_lists(t, nV);
     cudaStream_t s = ctx->stream;
     double *d = t->col_buf;
     for (int i = 0; i < 11; ++i)
@@ -1398,7 +1392,7 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     t->nV = nV;
     t->mesh_ready = false;
     set_zops(ctx, t, nz, ctx->zeta_host.data());
-    ensure_lists(t, nV, nz);
+    ensure_lists(t, nV);
     t->cur = 0;
     to_internal(ctx, t->Ti[0], f->Ti, false, nz);
     to_internal(ctx, t->u, f->u_3D, false, nz);

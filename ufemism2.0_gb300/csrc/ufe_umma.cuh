@@ -22,12 +22,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// byte offset of element (r, k) (k < 64) inside a 128B-swizzled K-major tile
-__device__ __forceinline__ uint32_t sw128_offset(int r, int k) {
-  const int chunk = k >> 3;
-  return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((chunk ^ (r & 7)) << 4) + ((k & 7) << 1));
-}
-// byte offset of 16-byte chunk c (0..7) of row r
+// byte offset of 16-byte chunk c (0..7) of row r inside a 128B-swizzled K-major tile
 __device__ __forceinline__ uint32_t sw128_chunk(int r, int c) {
   return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }

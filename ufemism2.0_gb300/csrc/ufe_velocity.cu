@@ -462,7 +462,7 @@ __device__ __forceinline__ bool pair_unsafe(double a, bool tiny_matters) {
          (tiny_matters && b != 0 && b < (unsigned long long)__double_as_longlong(1e-30));
 }
 
-// The double-word form of a block that is not pair_unsafe, as to_dwblk gives it.  The high word is the value rounded to
+// The double-word form of a block that is not pair_unsafe.  The high word is the value rounded to
 // 24 bits, to nearest and ties to even, which needs no FP64 conversion either way.
 __device__ __forceinline__ void pair_words(double x, float &hi, float &lo) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -1051,21 +1051,6 @@ __global__ void k_check_finite(const double *a, int64_t n, int *flag) {
   bool bad = false;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) bad |= !isfinite(a[i]);
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
-}
-
-__global__ void k_interleave(int n, const double *a, const double *b, double2 *out) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    out[i] = make_double2(a ? a[i] : 0.0, b ? b[i] : 0.0);
-}
-
-__global__ void k_deinterleave(int n, const double2 *in, double *a, double *b) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    double2 w = in[i];
-    a[i] = w.x;
-    b[i] = w.y;
-  }
 }
 
 // Export of the stiffness matrix in the reference's CSR layout (rows 2(ti-1)+uv, entries in the
