@@ -1086,10 +1086,14 @@ void validate_thermo_params(const ufe_thermo_params *p) {
 }  // namespace
 
 // ---- work area -------------------------------------------------------------------------------
+struct ZetaGrid {
+  int nz = 0;
+  double *ops = nullptr;        // 7 x nz
+};
 struct ThermoWork {
   int64_t nV = 0;
-  int nz = 0;
-  double *zops = nullptr;       // 7 x nz
+  // vertical grids of the column calls and of the mesh's resident state: each call keeps to its own
+  ZetaGrid col_zeta, mesh_zeta;
   Counters *cnt = nullptr;
   Counters *cnt_host = nullptr; // pinned
   Lists lists{};
@@ -1112,7 +1116,7 @@ void free_thermo(ufe_ctx *ctx) {
   ThermoWork *t = ctx->thermo;
   if (!t) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  void *ptrs[] = {t->zops, t->cnt, t->lists.retry, t->lists.unstable, t->col_buf, t->col_mask,
+  void *ptrs[] = {t->col_zeta.ops, t->mesh_zeta.ops, t->cnt, t->lists.retry, t->lists.unstable, t->col_buf, t->col_mask,
                   t->Ti[0], t->Ti[1], t->u, t->v, t->w, t->phi, t->ub, t->vb, t->vert, t->mask, t->ti_up};
   for (void *p : ptrs) dev_free(p);
   if (t->cnt_host) cudaFreeHost(t->cnt_host);
@@ -1141,23 +1145,23 @@ void ensure_lists(ThermoWork *t, int64_t nV) {
   }
 }
 
-void set_zops(ufe_ctx *ctx, ThermoWork *t, int nz, const double *zeta_host) {
+void set_zops(ufe_ctx *ctx, ZetaGrid &g, int nz, const double *zeta_host) {
   std::vector<double> h(7 * (size_t)nz);
   std::copy(zeta_host, zeta_host + nz, h.begin());
   UFE_REQUIRE(zeta_operators_host(nz, zeta_host, &h[nz], &h[2 * nz], &h[3 * nz], &h[4 * nz], &h[5 * nz],
                                   &h[6 * nz]),
               UFE_ERR_INVALID, "zeta operators: singular shape-function system (repeated zeta values?)");
-  if (t->nz != nz || !t->zops) {
-    dev_free(t->zops);
-    t->zops = (double *)dev_alloc(sizeof(double) * 7 * nz);
+  if (g.nz != nz || !g.ops) {
+    dev_free(g.ops);
+    g.ops = (double *)dev_alloc(sizeof(double) * 7 * nz);
   }
-  UFE_CUDA(cudaMemcpyAsync(t->zops, h.data(), sizeof(double) * 7 * nz, cudaMemcpyHostToDevice, ctx->stream));
-  t->nz = nz;
+  UFE_CUDA(cudaMemcpyAsync(g.ops, h.data(), sizeof(double) * 7 * nz, cudaMemcpyHostToDevice, ctx->stream));
+  g.nz = nz;
 }
 
-ZOps zops_of(const ThermoWork *t) {
-  const int nz = t->nz;
-  const double *b = t->zops;
+ZOps zops_of(const ZetaGrid &g) {
+  const int nz = g.nz;
+  const double *b = g.ops;
   return ZOps{b, b + nz, b + 2 * nz, b + 3 * nz, b + 4 * nz, b + 5 * nz, b + 6 * nz, nz};
 }
 
@@ -1192,9 +1196,8 @@ void launch_retry(cudaStream_t s, const In &in, const ZOps &z, const Consts &c, 
 }
 
 template <class In>
-void launch_step(ufe_ctx *ctx, ThermoWork *t, const In &in, const Consts &c, const VertexFields &vf, int64_t nV,
-                 const double *Ti_cur, double *Ti_next) {
-  const ZOps z = zops_of(t);
+void launch_step(ufe_ctx *ctx, ThermoWork *t, const ZOps &z, const In &in, const Consts &c, const VertexFields &vf,
+                 int64_t nV, const double *Ti_cur, double *Ti_next) {
   const int T = kColumnThreads;
   const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
   raise_smem_limit(k_heat_columns<In>, smem);
@@ -1263,7 +1266,7 @@ extern "C" int32_t ufe_thermo_step(ufe_ctx *ctx, const ufe_thermo_params *p, int
                 "thermo: UFE_GLBC_SUBGRID needs fraction_gr");
     UFE_CUDA(cudaSetDevice(ctx->device));
     ThermoWork *t = thermo_work(ctx);
-    set_zops(ctx, t, nz, zeta);
+    set_zops(ctx, t->col_zeta, nz, zeta);
     const int64_t nl = (int64_t)nV * nz;
     const int64_t need = 12 * nl + 6 * (int64_t)nV;
     if (t->col_cap < need) {
@@ -1297,7 +1300,7 @@ extern "C" int32_t ufe_thermo_step(ufe_ctx *ctx, const ufe_thermo_params *p, int
     VertexFields vf{vtx, vtx + nV, vtx + 2 * (int64_t)nV, vtx + 3 * (int64_t)nV, vtx + 4 * (int64_t)nV,
                     vtx + 5 * (int64_t)nV, t->col_mask};
     reset_counters(ctx, t, nV);
-    launch_step(ctx, t, in, make_consts(p), vf, nV, d, out);
+    launch_step(ctx, t, zops_of(t->col_zeta), in, make_consts(p), vf, nV, d, out);
     UFE_CUDA(cudaMemcpyAsync(Ti_next, out, sizeof(double) * nl, cudaMemcpyDeviceToHost, s));
     return finish_counters(ctx, t, n_unstable);
   });
@@ -1373,7 +1376,7 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     UFE_CUDA(cudaSetDevice(ctx->device));
     ThermoWork *t = thermo_work(ctx);
     cudaStream_t s = ctx->stream;
-    if (t->nV != nV || t->nz != nz || !t->Ti[0]) {
+    if (t->nV != nV || t->mesh_zeta.nz != nz || !t->Ti[0]) {
       void *old[] = {t->Ti[0], t->Ti[1], t->u, t->v, t->w, t->phi, t->ub, t->vb, t->vert, t->mask, t->ti_up};
       for (void *q : old) dev_free(q);
       const size_t nl = sizeof(double) * nV * nz;
@@ -1391,7 +1394,7 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     }
     t->nV = nV;
     t->mesh_ready = false;
-    set_zops(ctx, t, nz, ctx->zeta_host.data());
+    set_zops(ctx, t->mesh_zeta, nz, ctx->zeta_host.data());
     ensure_lists(t, nV);
     t->cur = 0;
     to_internal(ctx, t->Ti[0], f->Ti, false, nz);
@@ -1496,7 +1499,7 @@ extern "C" int32_t ufe_heat_step_resident(ufe_ctx *ctx, const ufe_thermo_params 
     for (int32_t st = 0; st < nsteps; ++st) {
       const int a = (cur0 + st) & 1;
       const HeatMesh in = heat_mesh_inputs(ctx, t, t->Ti[a]);
-      launch_step(ctx, t, in, c, vf, t->nV, t->Ti[a], t->Ti[a ^ 1]);
+      launch_step(ctx, t, zops_of(t->mesh_zeta), in, c, vf, t->nV, t->Ti[a], t->Ti[a ^ 1]);
     }
     UFE_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     int32_t rc;
@@ -1539,7 +1542,7 @@ extern "C" int32_t ufe_profile_heat_kernels(ufe_ctx *ctx, const ufe_thermo_param
     const VertexFields vf = heat_vertex_fields(t);
     const HeatMesh in = heat_mesh_inputs(ctx, t, t->Ti[t->cur]);
     double *out = t->Ti[t->cur ^ 1];
-    const ZOps z = zops_of(t);
+    const ZOps z = zops_of(t->mesh_zeta);
     const int T = kColumnThreads;
     const size_t smem = (size_t)3 * z.nz * T * sizeof(double);
     raise_smem_limit(k_heat_columns<HeatMesh>, smem);
@@ -1591,7 +1594,7 @@ extern "C" int32_t ufe_heat_download(ufe_ctx *ctx, double *Ti) {
     UFE_REQUIRE(t && t->mesh_ready, UFE_ERR_INVALID, "heat download: nothing uploaded");
     UFE_REQUIRE(Ti, UFE_ERR_INVALID, "heat download: NULL output");
     UFE_CUDA(cudaSetDevice(ctx->device));
-    to_external(ctx, Ti, t->Ti[t->cur], false, t->nz);
+    to_external(ctx, Ti, t->Ti[t->cur], false, t->mesh_zeta.nz);
     return UFE_OK;
   });
 }
