@@ -16,7 +16,7 @@ SOURCE = r"""
 
 static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;
 static struct { void *p; size_t bytes; } block[1 << 16];
-static int blocks, mallocs, lowered, refused, refuse_coop;
+static int blocks, mallocs, lowered, refused, refuse_coop, attempts, fail_from = 1 << 30;
 static __thread int coop;   // this thread's
 static size_t held, cap = (size_t)-1;
 static struct { const void *f; int bytes; } limit[4096];
@@ -34,13 +34,14 @@ int shim_lowered(void) { return lowered; }
 int shim_coop(void) { return coop; }
 int shim_refused(void) { return refused; }
 void shim_cap(size_t bytes) { cap = bytes; }
+void shim_fail_from(int n) { attempts = 0, fail_from = n; }   // the n-th allocation from now and all after it
 void shim_refuse_coop(int on) { refuse_coop = on; }
 
 cudaError_t cudaMalloc(void **p, size_t bytes) {
   cudaError_t (*f)(void **, size_t) = real("cudaMalloc");
   pthread_mutex_lock(&lock);
   cudaError_t e = cudaErrorMemoryAllocation;
-  if (held + bytes <= cap) e = f(p, bytes);
+  if (held + bytes <= cap && attempts++ < fail_from) e = f(p, bytes);
   if (e == cudaSuccess) {
     int i = 0;
     while (i < blocks && block[i].p) ++i;

@@ -911,13 +911,12 @@ void gnn_ensure(ufe_gnn *g, int64_t n) {
 
 void gnn_ensure_scratch(ufe_gnn *g, int64_t n) {
   if (g->gcap >= n) return;
-  void *ptrs[] = {g->gnbr, g->gx, g->gy, g->gw, g->gmask};
-  for (void *p : ptrs) dev_free(p);
-  g->gnbr = (int32_t *)dev_alloc(sizeof(int32_t) * 3 * n);
-  g->gx = (float *)dev_alloc(sizeof(float) * kFin * n);
-  g->gy = (float *)dev_alloc(sizeof(float) * kGnnOut * n);
-  g->gw = (float *)dev_alloc(sizeof(float) * n);
-  g->gmask = (float *)dev_alloc(sizeof(float) * n);
+  g->gcap = 0;
+  dev_replace(g->gnbr, 3 * (size_t)n);
+  dev_replace(g->gx, kFin * (size_t)n);
+  dev_replace(g->gy, kGnnOut * (size_t)n);
+  dev_replace(g->gw, n);
+  dev_replace(g->gmask, n);
   g->gcap = n;
 }
 
@@ -960,10 +959,8 @@ void gnn_forward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x, co
 void gnn_backward(ufe_gnn *g, cudaStream_t s, const Graph &gr, const float *x) {
   const int G = (int)gnn_grid(gr.n, kBwdBlocks), D = (int)gnn_grid(gr.n, kFwdBlocks);
   if (g->part_ctas < G) {   // networks that only predict have none
-    dev_free(g->part);
-    g->part = nullptr;
     g->part_ctas = 0;
-    g->part = (float *)dev_alloc(sizeof(float) * (size_t)kPartSets * G * kPart);
+    dev_replace(g->part, (size_t)kPartSets * G * kPart);
     g->part_ctas = G;
   }
   auto set = [&](int q) { return g->part + (int64_t)q * G * kPart; };

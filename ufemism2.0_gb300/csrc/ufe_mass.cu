@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "ufe_internal.cuh"
@@ -539,58 +540,68 @@ extern "C" void ufe_default_thickness_params(ufe_thickness_params *p) {
   p->Hi_min = 0.0;
 }
 
+static void fill_mass(ufe_ctx *ctx, MassWork *w, const double *A, const double *Cw) {
+  cudaStream_t s = ctx->stream;
+  w->nV = ctx->nV;
+  w->nTri = ctx->nTri;
+  w->nC_mem = ctx->nC_mem;
+  const size_t nc = (size_t)w->nV * w->nC_mem;
+  for (int64_t i = 0; i < w->nV; ++i)
+    UFE_REQUIRE(A[i] > 0.0 && std::isfinite(A[i]), UFE_ERR_INVALID, "Voronoi cell areas must be positive");
+  w->A = alloc_n<double>(w->nV);
+  w->Cw = alloc_n<double>(nc);
+  w->ct = alloc_n<int2>(nc);
+  w->Dc = alloc_n<double>(nc);
+  w->rDc = alloc_n<double>(nc);
+  {
+    // the caller's order, then gathered into the internal one
+    const std::unique_ptr<double, void (*)(void *)> tmp(alloc_n<double>(nc), dev_free);
+    UFE_CUDA(cudaMemcpyAsync(tmp.get(), A, sizeof(double) * w->nV, cudaMemcpyHostToDevice, s));
+    k_permute<double><<<blocks(w->nV), 256, 0, s>>>(w->nV, 1, tmp.get(), ctx->perm_v, w->A);
+    UFE_CUDA(cudaMemcpyAsync(tmp.get(), Cw, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
+    UFE_CUDA(cudaStreamSynchronize(s));
+    k_permute<double><<<blocks((int64_t)nc), 256, 0, s>>>(w->nV, w->nC_mem, tmp.get(), ctx->perm_v, w->Cw);
+    UFE_CUDA(cudaStreamSynchronize(s));
+  }
+  k_conn_tris<<<blocks(w->nV), 256, 0, s>>>(w->nV, w->nTri, w->nC_mem, ctx->V, ctx->nC, ctx->C, ctx->niTri,
+                                            ctx->iTri, ctx->Tri, w->ct, w->Dc, w->rDc);
+  UFE_CUDA(cudaGetLastError());
+  // M_divQ's pattern: row vi = [vi, C(vi, 1:nC)] (calc_ice_flux_divergence_matrix_upwind's add_entry order)
+  std::vector<int32_t> nC(w->nV), C(nc);
+  UFE_CUDA(cudaMemcpyAsync(nC.data(), ctx->nC, sizeof(int32_t) * w->nV, cudaMemcpyDeviceToHost, s));
+  UFE_CUDA(cudaMemcpyAsync(C.data(), ctx->C, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s));
+  UFE_CUDA(cudaStreamSynchronize(s));
+  std::vector<int32_t> ptr(w->nV + 1), ind;
+  ind.reserve((size_t)w->nV * 8);
+  for (int32_t vi = 0; vi < w->nV; ++vi) {
+    ptr[vi] = (int32_t)ind.size();
+    ind.push_back(vi);
+    for (int ci = 0; ci < nC[vi]; ++ci) ind.push_back(C[(size_t)ci * w->nV + vi] - 1);
+  }
+  ptr[w->nV] = (int32_t)ind.size();
+  w->nnz = (int64_t)ind.size();
+  w->ptr = alloc_n<int32_t>(w->nV + 1);
+  w->ind = alloc_n<int32_t>(w->nnz);
+  UFE_CUDA(cudaMemcpyAsync(w->ptr, ptr.data(), sizeof(int32_t) * (w->nV + 1), cudaMemcpyHostToDevice, s));
+  UFE_CUDA(cudaMemcpyAsync(w->ind, ind.data(), sizeof(int32_t) * w->nnz, cudaMemcpyHostToDevice, s));
+  alloc_fields(w, s);
+  Stage(ctx, w);   // with the mesh rather than in its first step
+  UFE_CUDA(cudaStreamSynchronize(s));
+}
+
 extern "C" int32_t ufe_mesh_voronoi_upload(ufe_ctx *ctx, const double *A, const double *Cw) {
   return guarded(ctx, [&]() -> int32_t {
     UFE_REQUIRE(ctx->has_mesh, UFE_ERR_INVALID, "upload a mesh first");
     UFE_REQUIRE(A && Cw, UFE_ERR_INVALID, "null Voronoi arrays");
     UFE_CUDA(cudaSetDevice(ctx->device));
     free_mass(ctx);
-    cudaStream_t s = ctx->stream;
-    MassWork *w = new MassWork;
-    ctx->mass = w;
-    w->nV = ctx->nV;
-    w->nTri = ctx->nTri;
-    w->nC_mem = ctx->nC_mem;
-    const size_t nc = (size_t)w->nV * w->nC_mem;
-    for (int64_t i = 0; i < w->nV; ++i)
-      UFE_REQUIRE(A[i] > 0.0 && std::isfinite(A[i]), UFE_ERR_INVALID, "Voronoi cell areas must be positive");
-    w->A = alloc_n<double>(w->nV);
-    w->Cw = alloc_n<double>(nc);
-    w->ct = alloc_n<int2>(nc);
-    w->Dc = alloc_n<double>(nc);
-    w->rDc = alloc_n<double>(nc);
-    double *tmp = alloc_n<double>(nc);   // the caller's order, then gathered into the internal one
-    UFE_CUDA(cudaMemcpyAsync(tmp, A, sizeof(double) * w->nV, cudaMemcpyHostToDevice, s));
-    k_permute<double><<<blocks(w->nV), 256, 0, s>>>(w->nV, 1, tmp, ctx->perm_v, w->A);
-    UFE_CUDA(cudaMemcpyAsync(tmp, Cw, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
-    UFE_CUDA(cudaStreamSynchronize(s));
-    k_permute<double><<<blocks((int64_t)nc), 256, 0, s>>>(w->nV, w->nC_mem, tmp, ctx->perm_v, w->Cw);
-    UFE_CUDA(cudaStreamSynchronize(s));
-    dev_free(tmp);
-    k_conn_tris<<<blocks(w->nV), 256, 0, s>>>(w->nV, w->nTri, w->nC_mem, ctx->V, ctx->nC, ctx->C, ctx->niTri,
-                                              ctx->iTri, ctx->Tri, w->ct, w->Dc, w->rDc);
-    UFE_CUDA(cudaGetLastError());
-    // M_divQ's pattern: row vi = [vi, C(vi, 1:nC)] (calc_ice_flux_divergence_matrix_upwind's add_entry order)
-    std::vector<int32_t> nC(w->nV), C(nc);
-    UFE_CUDA(cudaMemcpyAsync(nC.data(), ctx->nC, sizeof(int32_t) * w->nV, cudaMemcpyDeviceToHost, s));
-    UFE_CUDA(cudaMemcpyAsync(C.data(), ctx->C, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s));
-    UFE_CUDA(cudaStreamSynchronize(s));
-    std::vector<int32_t> ptr(w->nV + 1), ind;
-    ind.reserve((size_t)w->nV * 8);
-    for (int32_t vi = 0; vi < w->nV; ++vi) {
-      ptr[vi] = (int32_t)ind.size();
-      ind.push_back(vi);
-      for (int ci = 0; ci < nC[vi]; ++ci) ind.push_back(C[(size_t)ci * w->nV + vi] - 1);
+    ctx->mass = new MassWork;
+    try {
+      fill_mass(ctx, ctx->mass, A, Cw);
+    } catch (...) {
+      free_mass(ctx);
+      throw;
     }
-    ptr[w->nV] = (int32_t)ind.size();
-    w->nnz = (int64_t)ind.size();
-    w->ptr = alloc_n<int32_t>(w->nV + 1);
-    w->ind = alloc_n<int32_t>(w->nnz);
-    UFE_CUDA(cudaMemcpyAsync(w->ptr, ptr.data(), sizeof(int32_t) * (w->nV + 1), cudaMemcpyHostToDevice, s));
-    UFE_CUDA(cudaMemcpyAsync(w->ind, ind.data(), sizeof(int32_t) * w->nnz, cudaMemcpyHostToDevice, s));
-    alloc_fields(w, s);
-    Stage(ctx, w);   // with the mesh rather than in its first step
-    UFE_CUDA(cudaStreamSynchronize(s));
     return UFE_OK;
   });
 }

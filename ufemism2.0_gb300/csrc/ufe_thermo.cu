@@ -1129,18 +1129,22 @@ namespace {
 ThermoWork *thermo_work(ufe_ctx *ctx) {
   if (!ctx->thermo) {
     ctx->thermo = new ThermoWork();
-    ctx->thermo->cnt = (Counters *)dev_alloc(sizeof(Counters));
-    UFE_CUDA(cudaMallocHost(&ctx->thermo->cnt_host, sizeof(Counters)));
+    try {
+      dev_replace(ctx->thermo->cnt, 1);
+      UFE_CUDA(cudaMallocHost(&ctx->thermo->cnt_host, sizeof(Counters)));
+    } catch (...) {
+      free_thermo(ctx);
+      throw;
+    }
   }
   return ctx->thermo;
 }
 
 void ensure_lists(ThermoWork *t, int64_t nV) {
   if (t->list_nv < nV) {
-    dev_free(t->lists.retry);
-    dev_free(t->lists.unstable);
-    t->lists.retry = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
-    t->lists.unstable = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
+    t->list_nv = 0;
+    dev_replace(t->lists.retry, nV);
+    dev_replace(t->lists.unstable, nV);
     t->list_nv = nV;
   }
 }
@@ -1151,10 +1155,7 @@ void set_zops(ufe_ctx *ctx, ZetaGrid &g, int nz, const double *zeta_host) {
   UFE_REQUIRE(zeta_operators_host(nz, zeta_host, &h[nz], &h[2 * nz], &h[3 * nz], &h[4 * nz], &h[5 * nz],
                                   &h[6 * nz]),
               UFE_ERR_INVALID, "zeta operators: singular shape-function system (repeated zeta values?)");
-  if (g.nz != nz || !g.ops) {
-    dev_free(g.ops);
-    g.ops = (double *)dev_alloc(sizeof(double) * 7 * nz);
-  }
+  if (g.nz != nz || !g.ops) dev_replace(g.ops, 7 * (size_t)nz);
   UFE_CUDA(cudaMemcpyAsync(g.ops, h.data(), sizeof(double) * 7 * nz, cudaMemcpyHostToDevice, ctx->stream));
   g.nz = nz;
 }
@@ -1270,13 +1271,13 @@ extern "C" int32_t ufe_thermo_step(ufe_ctx *ctx, const ufe_thermo_params *p, int
     const int64_t nl = (int64_t)nV * nz;
     const int64_t need = 12 * nl + 6 * (int64_t)nV;
     if (t->col_cap < need) {
-      dev_free(t->col_buf);
-      t->col_buf = (double *)dev_alloc(sizeof(double) * need);
+      t->col_cap = 0;
+      dev_replace(t->col_buf, need);
       t->col_cap = need;
     }
     if (t->col_mask_cap < nV) {
-      dev_free(t->col_mask);
-      t->col_mask = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
+      t->col_mask_cap = 0;
+      dev_replace(t->col_mask, nV);
       t->col_mask_cap = nV;
     }
     ensure_lists(t, nV);
@@ -1376,24 +1377,17 @@ extern "C" int32_t ufe_heat_upload(ufe_ctx *ctx, const ufe_heat_fields *f) {
     UFE_CUDA(cudaSetDevice(ctx->device));
     ThermoWork *t = thermo_work(ctx);
     cudaStream_t s = ctx->stream;
-    if (t->nV != nV || t->mesh_zeta.nz != nz || !t->Ti[0]) {
-      void *old[] = {t->Ti[0], t->Ti[1], t->u, t->v, t->w, t->phi, t->ub, t->vb, t->vert, t->mask, t->ti_up};
-      for (void *q : old) dev_free(q);
-      const size_t nl = sizeof(double) * nV * nz;
-      t->Ti[0] = (double *)dev_alloc(nl);
-      t->Ti[1] = (double *)dev_alloc(nl);
-      t->u = (double *)dev_alloc(nl);
-      t->v = (double *)dev_alloc(nl);
-      t->w = (double *)dev_alloc(nl);
-      t->phi = (double *)dev_alloc(nl);
-      t->ub = (double *)dev_alloc(nl);
-      t->vb = (double *)dev_alloc(nl);
-      t->vert = (double *)dev_alloc(sizeof(double) * 13 * nV);
-      t->mask = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
-      t->ti_up = (int32_t *)dev_alloc(sizeof(int32_t) * nV);
-    }
-    t->nV = nV;
     t->mesh_ready = false;
+    if (t->nV != nV || t->mesh_zeta.nz != nz) {
+      t->nV = 0;
+      const size_t nl = (size_t)nV * nz;
+      double **fields[] = {&t->Ti[0], &t->Ti[1], &t->u, &t->v, &t->w, &t->phi, &t->ub, &t->vb};
+      for (double **q : fields) dev_replace(*q, nl);
+      dev_replace(t->vert, 13 * (size_t)nV);
+      dev_replace(t->mask, nV);
+      dev_replace(t->ti_up, nV);
+      t->nV = nV;
+    }
     set_zops(ctx, t->mesh_zeta, nz, ctx->zeta_host.data());
     ensure_lists(t, nV);
     t->cur = 0;

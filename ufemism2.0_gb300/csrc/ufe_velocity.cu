@@ -1316,11 +1316,7 @@ bool use_sell() {
   return v == 1;
 }
 
-Work *ensure_work(ufe_ctx *ctx) {
-  check_operators(ctx);
-  if (ctx->work) return ctx->work;
-  Work *w = new Work();
-  ctx->work = w;
+static void fill_work(ufe_ctx *ctx, Work *w) {
   const int nV = ctx->nV, nTri = ctx->nTri, nz = ctx->nz;
   w->nV = nV; w->nTri = nTri; w->nz = nz;
   w->nnzb = ctx->ops[UFE_OP_M2_DDX_B_B].nnz;
@@ -1388,12 +1384,9 @@ Work *ensure_work(ufe_ctx *ctx) {
   UFE_CUDA(cudaMemsetAsync(w->err, 0, sizeof(int), s));
   UFE_CUDA(cudaMemsetAsync(w->pred_flag, 0, sizeof(int32_t), s));
   UFE_CUDA(cudaStreamSynchronize(s));
-  return w;
 }
 
-void free_work(ufe_ctx *ctx) {
-  free_thermo(ctx);   // the resident heat state depends on the mesh and its operators
-  free_mass(ctx);     // so do the Voronoi geometry and the thickness matrix pattern
+static void free_solver(ufe_ctx *ctx) {
   Work *w = ctx->work;
   if (!w) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
@@ -1416,6 +1409,25 @@ void free_work(ufe_ctx *ctx) {
   if (w->ps_host) cudaFreeHost(w->ps_host);
   delete w;
   ctx->work = nullptr;
+}
+
+Work *ensure_work(ufe_ctx *ctx) {
+  check_operators(ctx);
+  if (ctx->work) return ctx->work;
+  ctx->work = new Work();
+  try {
+    fill_work(ctx, ctx->work);
+  } catch (...) {
+    free_solver(ctx);
+    throw;
+  }
+  return ctx->work;
+}
+
+void free_work(ufe_ctx *ctx) {
+  free_thermo(ctx);   // the resident heat state depends on the mesh and its operators
+  free_mass(ctx);     // so do the Voronoi geometry and the thickness matrix pattern
+  free_solver(ctx);
 }
 
 int32_t bsr_lanes(ufe_ctx *ctx) {
@@ -1497,9 +1509,9 @@ void build_icestream_copy(ufe_ctx *ctx, Work *w) {
     }
     ptr[t + 1] = (int32_t)idx.size();
   }
-  w->cp_ptr = alloc_n<int32_t>(nTri + 1);
-  w->cp_idx = alloc_n<int32_t>(idx.size());
-  w->cp_w = alloc_n<double>(wts.size());
+  dev_replace(w->cp_ptr, nTri + 1);
+  dev_replace(w->cp_idx, idx.size());
+  dev_replace(w->cp_w, wts.size());
   UFE_CUDA(cudaMemcpyAsync(w->cp_ptr, ptr.data(), sizeof(int32_t) * (nTri + 1), cudaMemcpyHostToDevice, s));
   if (!idx.empty()) {
     UFE_CUDA(cudaMemcpyAsync(w->cp_idx, idx.data(), sizeof(int32_t) * idx.size(), cudaMemcpyHostToDevice, s));
@@ -1571,7 +1583,7 @@ struct Solver {
     const DevCSR &mba = ctx->ops[UFE_OP_MAP_B_A];
     ba = OpRow{mba.ptr, mba.ind, mba.val, ctx->ops[UFE_OP_DDX_B_A].val, ctx->ops[UFE_OP_DDY_B_A].val};
     if (pair_ok()) ensure_pair();
-    if (icestream_bc(p) && !w->cp_ptr) build_icestream_copy(ctx, w);
+    if (icestream_bc(p) && !w->cp_w) build_icestream_copy(ctx, w);   // cp_w: the last of its arrays
   }
 
   int eblocks(int64_t n) const { return pick_blocks(n, kThreads, grid); }
@@ -1799,12 +1811,12 @@ struct Solver {
   // only when the double-word solve declined (k_pair_decide)
   bool pair_ok() const { return p.precision == UFE_PREC_FP32_PAIR && halo64_ok(); }
   void ensure_pair() {
-    if (w->sell_blkp) return;
+    if (w->pair_bad) return;   // the last of them
     const int n = w->nTri;
     dw2 **v[] = {&w->pX, &w->pR, &w->pRP, &w->pS, &w->pT, &w->pdinv, &w->pP[0], &w->pP[1], &w->pV[0], &w->pV[1]};
-    for (auto q : v) *q = static_cast<dw2 *>(dev_alloc(sizeof(dw2) * (size_t)(n ? n : 1)));
-    w->sell_blkp = static_cast<dwblk *>(dev_alloc(sizeof(dwblk) * (size_t)(w->nslots ? w->nslots : 1)));
-    w->pair_bad = static_cast<int *>(dev_alloc(sizeof(int)));
+    for (auto q : v) dev_replace(*q, n ? n : 1);
+    dev_replace(w->sell_blkp, w->nslots ? w->nslots : 1);
+    dev_replace(w->pair_bad, 1);
     UFE_CUDA(cudaMemsetAsync(w->sell_blkp, 0, sizeof(dwblk) * (size_t)(w->nslots ? w->nslots : 1), s));
     UFE_CUDA(cudaMemsetAsync(w->pair_bad, 0, sizeof(int), s));
   }
