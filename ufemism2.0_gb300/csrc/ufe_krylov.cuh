@@ -1013,7 +1013,7 @@ __device__ __forceinline__ void row_publish(ExRow *p, Vec x, unsigned int stamp)
   st_words(p->w, word(q.x, stamp), word(q.y, stamp));
   st_words(p->w + 2, word(q.z, stamp), word(q.w, stamp));
 }
-// FP64 butterfly sums of a (in lanes below 16) and b (in the others); not inlined, to be fetched once
+// FP64 butterfly sums of a (in lanes below 16) and b (in the others)
 __device__ __forceinline__ double warp_fold_sum(double a, double b) {
   const bool up = threadIdx.x & 16;
   double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
@@ -1023,7 +1023,7 @@ __device__ __forceinline__ double warp_fold_sum(double a, double b) {
 }
 __device__ __forceinline__ double fp64_div(double a, double b) { return a / b; }
 // Double-word sums.  Two butterflies' step in one addition: lanes with `bit` clear go on with a, the others
-// with b (fold(a, a, bit) is a butterfly step).  Not inlined: a double-word addition is 20 instructions.
+// with b (fold(a, a, bit) is a butterfly step).  A double-word addition is 20 instructions, so five sums are folded.
 __device__ __forceinline__ dw dw_fold(dw a, dw b, int bit) {
   const bool up = threadIdx.x & bit;
   const dw keep(up ? b.hi : a.hi, up ? b.lo : a.lo), send(up ? a.hi : b.hi, up ? a.lo : b.lo);

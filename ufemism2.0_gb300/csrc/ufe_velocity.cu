@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(32 * kVertexSsaWarps) k_vertex_ssa(int nV, OpR
 // reference's order, zeta increasing) and the F2 integral (from the base up).
 // In the first iteration of a solve the learned start armed, every layer takes the predicted
 // vertically averaged viscosity eta_pred instead (a depth-uniform first viscosity).
-// Dynamic shared memory: (kMaxNz + nz * blockDim.x) doubles.
+// Dynamic shared memory: (2 kMaxNz + 2 * 32 nz) doubles.
 // Six warps per 32 vertices, the layers in turn: as in k_vertex_ssa, one warp's chain of FP64 instructions is what a
 // small mesh waits for, and a large one is evenly spread.  The sums over a row of the b->a operator are split over the
 // warps, the two integrals over the column and the friction go to one warp each.  7.8k vertices x 12 layers: 75 us with
