@@ -1456,7 +1456,7 @@ struct ResidentLayout {
 // row of 13) and the scalar recurrence (~2,000 and ~3,300); the double-word form on 115k triangles is bound by
 // the L2 stream of the blocks that do not fit.  Per iteration, with the counter-barrier kernel it replaces
 // beside it: FP64 11.6 us (20.8) on 1,154 triangles, 14.0 (21.2) on 16,662, 35.0 (39.7) on 115,383; double-word
-// 19.3 us (25.4) on 115,383.  Fewer threads leave more registers and loads in flight to each, so the launch
+// 19.2 us (25.2) on 115,383.  Fewer threads leave more registers and loads in flight to each, so the launch
 // takes 512, 768 or 1024 by the rows per block.
 template <class Vec, class Blk, int NT>
 __global__ void __launch_bounds__(NT, 1) k_bicgstab_resident(HaloMat<Blk> m, KV<Vec> v, KrylovScalars *ks,
@@ -1651,9 +1651,9 @@ __global__ void __launch_bounds__(NT, 1) k_bicgstab_resident(HaloMat<Blk> m, KV<
 // in the same way.  A block of 256 q threads runs q virtual blocks at a time.
 //
 // What bounds it: latency (three exchanges of ~3,000 cycles, two gathers, the FP64 sums and scalars), and the
-// FP64 pipe for large systems.  A whole ufe_solve_csr of 60,000 rows of five entries: 3.1 ms, 5.8 ms with five
-// kernels an iteration (each ends in a last block's serial sums, 10 to 16 us however small the system) and a host
-// check every eight; the thickness step on 1.05M vertices: 2.58 ms, 2.83 ms with the kernels in a graph.
+// vectors' and matrix's way from L2 for large systems.  60,000 rows of five entries: 19 us an iteration, 46 with five
+// kernels (each ends in a last block's serial sums, 10 to 16 us however small the system) and a host check every
+// eight; larger systems at kCsrPersistRows.
 constexpr int kMaxVirt = 8 * 152;
 constexpr int kCsrSums = 3;
 constexpr size_t kCsrSet = (size_t)kReplicas * kCsrSums * kMaxVirt;   // slots of one exchange; two sets in turn
